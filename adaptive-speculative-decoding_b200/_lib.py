@@ -170,6 +170,7 @@ def lib() -> ctypes.CDLL:
         "asd_debug_gemm_trace": (i32, [vp, i32]),
         "asd_debug_attn_trace": (i32, [vp, i32]),
         "asd_engine_forward": (i32, [vp, vp, vp, vp, i32, vp, vp, i32, i32, i32, vp, i32, vp, c.c_longlong, vp]),
+        "asd_engine_forward_prompt": (i32, [vp, vp, vp, vp, i32, vp, vp, i32, i32, i32, vp, i32, vp, c.c_longlong, vp]),
         "asd_mezilix_create": (vp, [vp, vp]),
         "asd_mezilix_destroy": (None, [vp]),
         "asd_mezilix_set_globals": (i32, [vp, vp, vp, vp, vp]),

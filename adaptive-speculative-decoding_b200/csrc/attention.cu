@@ -81,10 +81,11 @@ struct AttnArgs {
     const int* page_table;
     int max_pages, nh, nkv, page_size, split_keys, nsplit_max, rg_count, kg_count;
     int page_shift;                // log2(page_size) when it is a power of two, else -1 (division fallback)
+    int nseq, q_tile;              // q_tile > 0: new positions per query tile (grid.x = tiles x sequences), else 0
     float scale_log2;
     float* o_part;                 // [M, nh, nsplit_max, hd]
     float* ml_part;                // [M, nh, nsplit_max, 2]
-    int* tickets;                  // [nseq_max * nkv], zero between launches
+    int* tickets;                  // [M * nkv], zero between launches
     __nv_bfloat16* out;            // [M, nh, hd]
     unsigned long long* trace;     // diagnostics: 16 globaltimer stamps per CTA (nullptr = off)
     // weights of the following GEMMs to pull into L2 while this kernel runs (see AttnLaunch::WeightPrefetch)
@@ -140,21 +141,29 @@ __global__ void __launch_bounds__(256) attn_mma_kernel(const AttnArgs a, const _
     uint8_t* sV = sK + NS * kKeyTile * ROWB;                  // [NS][64][HD]
     const uint32_t uQ = smem_u32(sQ), uK = smem_u32(sK), uV = smem_u32(sV);
 
-    const int seq = blockIdx.x, g = blockIdx.y, sp = blockIdx.z;
+    int seq = blockIdx.x, tq = 0;
+    const int g = blockIdx.y, sp = blockIdx.z;
+    if (a.q_tile > 0) {                      // the last tiles see the most keys: they start first
+        tq = (int)(gridDim.x / a.nseq) - 1 - (int)blockIdx.x / a.nseq;
+        seq = blockIdx.x % a.nseq;
+    }
     const int G = a.nh / a.nkv;
     attn_stamp(a, 0);
     // Everything up to the PDL wait reads only what earlier forwards (or the host) wrote: the batch
     // description, the page table and the K/V of keys older than this step's tokens.  The QKV GEMM that is
     // still running upstream only produces q and the K/V of the last qlen positions.
-    const int q0 = a.cu_q[seq], qlen = a.cu_q[seq + 1] - q0;
+    const int q0 = a.cu_q[seq] + tq * a.q_tile;
+    int qlen = a.cu_q[seq + 1] - q0;
     if (qlen <= 0) return;
+    if (a.q_tile > 0) qlen = min(qlen, a.q_tile);
     const int R = qlen * G;
     const int kv_len = a.positions[q0 + qlen - 1] + 1;
     const int kbeg = sp * a.split_keys;
     if (kbeg >= kv_len) return;
     const int kend = min(kv_len, kbeg + a.split_keys);
     const int nsplit_seq = (kv_len + a.split_keys - 1) / a.split_keys;
-    const int old_keys = kv_len - qlen;
+    const int old_keys = kv_len - qlen;                // keys before this tile's first position
+    const int ready_keys = old_keys - tq * a.q_tile;   // keys that this forward's QKV GEMM does not write
     // this CTA's slice of the sequence's page table, staged once (a lookup per key row would be a dependent
     // L2 round trip in front of every cp.async batch)
     int* s_pt = reinterpret_cast<int*>(sV + NS * kKeyTile * ROWB);
@@ -190,7 +199,7 @@ __global__ void __launch_bounds__(256) attn_mma_kernel(const AttnArgs a, const _
         }
     };
     const int ntiles = (kend - kbeg + kKeyTile - 1) / kKeyTile;
-    auto tile_is_old = [&](int t) { return kbeg + (t + 1) * kKeyTile <= old_keys; };
+    auto tile_is_old = [&](int t) { return kbeg + (t + 1) * kKeyTile <= ready_keys; };
 #pragma unroll
     for (int t = 0; t < NS - 1; ++t)     // prologue, part 1: the old tiles among the first NS-1
         if (t < ntiles && tile_is_old(t)) load_tile(t, t);
@@ -439,13 +448,13 @@ __global__ void __launch_bounds__(256) attn_mma_kernel(const AttnArgs a, const _
     }
     attn_stamp(a, 7);
     if (nsplit_seq == 1) return;
-    // the last CTA of this (sequence, kv head) to finish merges the splits (no separate combine launch)
+    // the last CTA of this (query tile, kv head) to finish merges the splits (no separate combine launch)
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int tk = atomicAdd(&a.tickets[seq * a.nkv + g], 1);
+        const int tk = atomicAdd(&a.tickets[q0 * a.nkv + g], 1);
         s_last = (tk == nsplit_seq - 1);
-        if (s_last) a.tickets[seq * a.nkv + g] = 0;
+        if (s_last) a.tickets[q0 * a.nkv + g] = 0;
     }
     __syncthreads();
     attn_stamp(a, 8);
@@ -518,7 +527,8 @@ int launch_attention(const AttnLaunch& L, cudaStream_t stream) {
         return 0;
     }
     const int G = L.nh / L.nkv;
-    const int rows = L.max_qlen * G;
+    const int rows = (L.q_tile > 0 ? L.q_tile : L.max_qlen) * G;
+    const int tiles = L.q_tile > 0 ? (L.max_qlen + L.q_tile - 1) / L.q_tile : 1;
     if (L.impl == 2 && L.kv_map != nullptr && L.hd == 128 && rows <= 128 && L.split_keys % 128 == 0)
         return launch_attention_tc(L, stream);
     const int rg = (rows + 15) / 16;
@@ -543,6 +553,8 @@ int launch_attention(const AttnLaunch& L, cudaStream_t stream) {
         if ((1 << b) == L.page_size) a.page_shift = b;
     a.split_keys = L.split_keys;
     a.nsplit_max = L.nsplit_max;
+    a.nseq = L.nseq;
+    a.q_tile = L.q_tile;
     a.rg_count = rg;
     a.kg_count = kg;
     a.scale_log2 = scale_log2;
@@ -553,7 +565,7 @@ int launch_attention(const AttnLaunch& L, cudaStream_t stream) {
     a.trace = nullptr;
     if (g_attn_trace && g_attn_trace_next < g_attn_trace_max)
         a.trace = g_attn_trace + (size_t)(g_attn_trace_next++) * 1024 * 16;
-    const dim3 grid(L.nseq, L.nkv, L.nsplit_max);
+    const dim3 grid(L.nseq * tiles, L.nkv, L.nsplit_max);
     if (grid.x * grid.y * grid.z > 1024) a.trace = nullptr;
     const int ns = (int)(grid.x * grid.y * grid.z) <= 148 ? 4 : 2;   // one CTA per SM: deeper K/V ring
     size_t smem = (size_t)rg * 16 * L.hd * 2 + 2 * (size_t)ns * kKeyTile * L.hd * 2;

@@ -4,6 +4,8 @@
 //
 // Work item = (sequence, kv head, kv split) as before: the query tile is all new positions x the GQA group
 // (rows = q_len * G <= 128, padded to the 128 TMEM lanes), so each K/V byte is read once per sequence.
+// A prompt has more rows than that: its positions are cut into tiles of floor(128 / G), each a work item of its own that
+// stops at its last position (K/V of a sequence is then re-read from L2 once per tile).
 // Per 128-key tile:
 //   S   = Q K^T     tcgen05.mma M=128 N=128 (8 k-steps over head_dim), both operands K-major SW128 in shared
 //                   memory; K pages arrive by TMA straight from the paged pool (one 2-D box of one page x 64
@@ -56,6 +58,7 @@ struct AttnTcArgs {
     const int* seq_slot;           // [nseq]
     const int* page_table;
     int max_pages, nh, nkv, split_keys, nsplit_max;
+    int nseq, q_tile;              // q_tile > 0: new positions per query tile (grid.x = tiles x sequences), else 0
     int page_shift;                // log2(positions per page): 4..7 (one TMA box = one page x 64 head-dim elements)
     int dbg;                       // diagnostics: 1 = skip the softmax arithmetic, 2 = also skip the fold
     long long k_row0, v_row0;      // first pool row (position-major rows of 128 dims) of this layer's K / V
@@ -177,10 +180,17 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     int* s_pt = reinterpret_cast<int*>(fin_s + 2 * 128);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int seq = blockIdx.x, g = blockIdx.y, sp = blockIdx.z;
+    int seq = blockIdx.x, tq = 0;
+    const int g = blockIdx.y, sp = blockIdx.z;
+    if (a.q_tile > 0) {                      // the last tiles see the most keys: they start first
+        tq = (int)(gridDim.x / a.nseq) - 1 - (int)blockIdx.x / a.nseq;
+        seq = blockIdx.x % a.nseq;
+    }
     const int G = a.nh / a.nkv;
-    const int q0 = a.cu_q[seq], qlen = a.cu_q[seq + 1] - q0;
+    const int q0 = a.cu_q[seq] + tq * a.q_tile;
+    int qlen = a.cu_q[seq + 1] - q0;
     if (qlen <= 0) return;
+    if (a.q_tile > 0) qlen = min(qlen, a.q_tile);
     const int R = qlen * G;
     const int nact = (R + 31) >> 5;          // softmax / fold warps that own at least one real row
     const int kv_len = a.positions[q0 + qlen - 1] + 1;
@@ -188,7 +198,8 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     if (kbeg >= kv_len) return;
     const int kend = min(kv_len, kbeg + a.split_keys);
     const int nsplit_seq = (kv_len + a.split_keys - 1) / a.split_keys;
-    const int old_keys = kv_len - qlen;
+    const int old_keys = kv_len - qlen;              // keys before this tile's first position
+    const int ready_keys = old_keys - tq * a.q_tile;   // keys that this forward's QKV GEMM does not write
     const int nt = (kend - kbeg + kAtTile - 1) / kAtTile;
     const int psh = a.page_shift;
     const int page0 = kbeg >> psh, npages = ((kend - 1) >> psh) - page0 + 1;
@@ -236,7 +247,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             for (int j = 0; j < nt; ++j) {
                 const int st = j & 1, use = j >> 1;
                 const int key0 = kbeg + j * kAtTile;
-                if (!waited && key0 + kAtTile > old_keys) {   // this tile holds keys the upstream QKV GEMM writes
+                if (!waited && key0 + kAtTile > ready_keys) {   // this tile holds keys the upstream QKV GEMM writes
                     grid_dep_wait();
                     waited = true;
                 }
@@ -475,13 +486,13 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     }
     if (threadIdx.x == 0) at_stamp(a, 10);
     if (nsplit_seq == 1) return;
-    // the last CTA of this (sequence, kv head) to finish merges the splits (no separate combine launch)
+    // the last CTA of this (query tile, kv head) to finish merges the splits (no separate combine launch)
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        const int tk = atomicAdd(&a.tickets[seq * a.nkv + g], 1);
+        const int tk = atomicAdd(&a.tickets[q0 * a.nkv + g], 1);
         *s_last = (tk == nsplit_seq - 1);
-        if (*s_last) a.tickets[seq * a.nkv + g] = 0;
+        if (*s_last) a.tickets[q0 * a.nkv + g] = 0;
     }
     __syncthreads();
     if (!*s_last) return;
@@ -534,6 +545,8 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     a.nkv = L.nkv;
     a.split_keys = L.split_keys;
     a.nsplit_max = L.nsplit_max;
+    a.nseq = L.nseq;
+    a.q_tile = L.q_tile;
     a.page_shift = 0;
     while ((1 << a.page_shift) < L.page_size) ++a.page_shift;
     a.dbg = tuning().attn_dbg;
@@ -545,13 +558,14 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     a.tickets = L.tickets;
     a.out = L.out;
     a.trace = nullptr;
-    if (g_attn_trace && g_attn_trace_next < g_attn_trace_max && L.nseq * L.nkv * L.nsplit_max <= 1024)
+    const int tiles = L.q_tile > 0 ? (L.max_qlen + L.q_tile - 1) / L.q_tile : 1;
+    if (g_attn_trace && g_attn_trace_next < g_attn_trace_max && (long long)tiles * L.nseq * L.nkv * L.nsplit_max <= 1024)
         a.trace = g_attn_trace + (size_t)(g_attn_trace_next++) * 1024 * 16;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(L.nseq, L.nkv, L.nsplit_max);
+    cfg.gridDim = dim3(L.nseq * tiles, L.nkv, L.nsplit_max);
     cfg.blockDim = dim3(kAtThreads);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;

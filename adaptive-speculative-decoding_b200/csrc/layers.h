@@ -40,8 +40,9 @@ struct AttnLaunch {
     __nv_bfloat16* out;     // [M, nh, hd]
     float* o_part;
     float* ml_part;
-    int* tickets;           // [nseq * nkv] zero-initialised, self-resetting
+    int* tickets;           // [M * nkv] zero-initialised, self-resetting (one per query tile and kv head: its first token's)
     int M, nseq, max_qlen, nh, nkv, hd, page_size, max_pages, split_keys, nsplit_max, impl;
+    int q_tile = 0;         // > 0: new positions per query tile, a sequence's positions spread over ceil(max_qlen / q_tile) CTAs
     // impl 2 (tcgen05 kernel, attention_tc.cu): 2-D TMA map over the whole paged pool viewed as rows of head_dim
     // elements (box = 64 elements x 16 positions) and the first row of this layer's K / V
     const CUtensorMap* kv_map = nullptr;
@@ -55,7 +56,7 @@ struct AttnLaunch {
     } pf[2];
 };
 // impl 0: one-warp cross-check kernel; 1: mma.sync kernel; 2: tcgen05 kernel when the shape allows (head_dim 128,
-// 16-position pages, q_len * group <= 128), else 1
+// 16-position pages, query tile * group <= 128), else 1
 int launch_attention(const AttnLaunch& L, cudaStream_t stream);
 int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream);
 

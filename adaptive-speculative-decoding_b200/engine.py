@@ -93,6 +93,13 @@ class _BatchOps:
         query rows on 128 lanes)"""
         return max(1, 128 // (self.cfg.num_attention_heads // self.cfg.num_key_value_heads))
 
+    def _prompt_chunk(self, nseq: int) -> int:
+        """new positions per sequence in one forward of a prompt (``_prompt_forward``)"""
+        return max(1, min(self.max_qlen(), self.max_tokens // nseq))
+
+    def _prompt_forward(self, *args):
+        return self.forward(*args)
+
     def forward_ragged(self, items, device=None, layer_out: bool = False):
         """One scheduler step over requests of unequal length: ``items`` = [(slot, start_pos, token ids, wanted
         indices)], every request's tokens continuing at ``start_pos`` from what the cache and state hold.  Runs as few
@@ -160,27 +167,31 @@ class _BatchOps:
     def forward_uniform(self, tokens2d: torch.Tensor, start_pos: torch.Tensor, slots: torch.Tensor, max_kv_len: int,
                         last_only: bool = False, want_logits: bool = True, logits_out=None, logits_ld: int = 0):
         """tokens2d int32 [nseq, q]; start_pos int32 [nseq] (position of column 0); slots int32 [nseq]."""
+        return self._uniform(self.forward, tokens2d, start_pos, slots, max_kv_len, last_only, want_logits, logits_out, logits_ld)
+
+    def _uniform(self, forward, tokens2d, start_pos, slots, max_kv_len, last_only, want_logits, logits_out=None, logits_ld=0):
         nseq, q = tokens2d.shape
         ix = self._uniform_index_on(nseq, q, tokens2d.device)
         positions = (start_pos[:, None] + ix["ar"]).reshape(-1)
         token_slot = slots[:, None].expand(nseq, q).reshape(-1) if q > 1 else slots
         rows = ix["last_rows"] if (last_only and want_logits and q > 1) else None
-        return self.forward(tokens2d.reshape(-1).contiguous(), positions.contiguous(), token_slot.contiguous(),
-                            ix["cu_q"], slots.contiguous(), q,
-                            max_kv_len, rows, logits_out, want_logits, logits_ld)
+        return forward(tokens2d.reshape(-1).contiguous(), positions.contiguous(), token_slot.contiguous(),
+                       ix["cu_q"], slots.contiguous(), q,
+                       max_kv_len, rows, logits_out, want_logits, logits_ld)
 
     def prefill(self, prompt_ids: torch.Tensor, slots: torch.Tensor, chunk: int = 0, want_logits: bool = True):
         """Chunked prefill of equal-length prompts [nseq, P]; returns the logits of the last position."""
         nseq, P = prompt_ids.shape
+        forward = self.forward
         if chunk <= 0:
-            chunk = max(1, min(self.max_qlen(), self.max_tokens // nseq))
+            forward = self._prompt_forward
+            chunk = self._prompt_chunk(nseq)
         logits = None
         zero = torch.zeros(nseq, dtype=torch.int32, device=prompt_ids.device)
         for s in range(0, P, chunk):
             e = min(P, s + chunk)
             last = e == P
-            logits = self.forward_uniform(prompt_ids[:, s:e].to(torch.int32), zero + s, slots, e, last_only=True,
-                                          want_logits=want_logits and last)
+            logits = self._uniform(forward, prompt_ids[:, s:e].to(torch.int32), zero + s, slots, e, True, want_logits and last)
         return logits
 
     def prefill_ragged(self, prompts, slots: torch.Tensor, chunk: int = 0, device=None):
@@ -192,8 +203,10 @@ class _BatchOps:
         nseq = len(prompts)
         lens = [len(p) for p in prompts]
         assert nseq == slots.numel() and min(lens) >= 1
+        forward = self.forward
         if chunk <= 0:
-            chunk = max(1, min(self.max_qlen(), self.max_tokens // nseq))
+            forward = self._prompt_forward
+            chunk = self._prompt_chunk(nseq)
         out = torch.empty(nseq, self.cfg.vocab_size, dtype=torch.float32, device=dev)
         slots_h = slots.cpu().tolist()
         for s0 in range(0, max(lens), chunk):
@@ -211,8 +224,8 @@ class _BatchOps:
                     rows.append(len(toks) - 1)
                     owners.append(b)
             mk = lambda x: torch.tensor(x, dtype=torch.int32).to(dev, non_blocking=True)
-            lg = self.forward(mk(toks), mk(pos), mk(tslot), mk(cu), mk(sslot), min(chunk, max(lens) - s0),
-                              min(max(lens), s0 + chunk), mk(rows) if rows else None, None, bool(rows))
+            lg = forward(mk(toks), mk(pos), mk(tslot), mk(cu), mk(sslot), min(chunk, max(lens) - s0),
+                         min(max(lens), s0 + chunk), mk(rows) if rows else None, None, bool(rows))
             if rows:
                 out[torch.tensor(owners, device=dev)] = lg
         return out
@@ -348,6 +361,21 @@ class QwenEngine(_BatchOps):
         draft stage placed on its own device, configs/qwen3_models.yaml:15,39,51) are copied over NVLink on a
         side stream of this engine's device and the logits are copied back; both streams are ordered by events,
         the host never waits."""
+        return self._forward("asd_engine_forward", tokens, positions, token_slot, cu_q, seq_slot, max_qlen, max_kv_len,
+                             logit_rows, logits_out, want_logits, logits_ld)
+
+    def _prompt_chunk(self, nseq: int) -> int:
+        # Attention tiles any number of new positions, so a forward is as large as max_tokens and the CTA-pair GEMM (4096
+        # tokens a call) allow.  A tensor-parallel rank keeps the short chunk: its exchanges grow with the tokens.
+        if self.tp_size > 1:
+            return super()._prompt_chunk(nseq)
+        return max(1, min(self.max_tokens, 4096) // nseq)
+
+    def _prompt_forward(self, *args):
+        return self._forward("asd_engine_forward_prompt", *args)
+
+    def _forward(self, entry: str, tokens, positions, token_slot, cu_q, seq_slot, max_qlen, max_kv_len, logit_rows=None,
+                 logits_out=None, want_logits=True, logits_ld=0):
         M, nseq = tokens.numel(), seq_slot.numel()
         for t in (tokens, positions, token_slot, cu_q, seq_slot):
             assert t.dtype == torch.int32 and t.is_contiguous() and t.is_cuda, "int32 contiguous CUDA tensors"
@@ -356,19 +384,19 @@ class QwenEngine(_BatchOps):
                            f"{self.max_pages * self.page_size} (page-table overrun refused)")
         n_rows = 0 if not want_logits else (M if logit_rows is None else logit_rows.numel())
         if tokens.device != self.device:
-            return _remote_forward(self, self.device, tokens, positions, token_slot, cu_q, seq_slot, max_qlen,
+            return _remote_forward(self, entry, self.device, tokens, positions, token_slot, cu_q, seq_slot, max_qlen,
                                    max_kv_len, logit_rows, logits_out, want_logits, logits_ld)
         if n_rows and logits_out is None:
             logits_out = torch.empty(n_rows, self.cfg.vocab_size, dtype=torch.float32, device=self.device)
         if n_rows and logits_out.device != self.device:
             raise AsdError("logits_out must live on the engine's device")
         with self._lock, torch.cuda.device(self.device):
-            rc = lib().asd_engine_forward(
+            rc = getattr(lib(), entry)(
                 self.h, tokens.data_ptr(), positions.data_ptr(), token_slot.data_ptr(), M, cu_q.data_ptr(),
                 seq_slot.data_ptr(), nseq, max_qlen, max_kv_len,
                 None if logit_rows is None else logit_rows.data_ptr(), n_rows,
                 None if not n_rows else logits_out.data_ptr(), logits_ld, _stream())
-        check(rc, "asd_engine_forward")
+        check(rc, entry)
         return logits_out if n_rows else None
 
     def _hop_stream(self):
@@ -386,9 +414,9 @@ class QwenEngine(_BatchOps):
         return buf[:n_rows]
 
 
-def _remote_forward(eng, dev, tokens, positions, token_slot, cu_q, seq_slot, max_qlen, max_kv_len, logit_rows,
+def _remote_forward(eng, entry, dev, tokens, positions, token_slot, cu_q, seq_slot, max_qlen, max_kv_len, logit_rows,
                     logits_out, want_logits, logits_ld):
-    """Run ``eng.forward`` on ``dev`` for a caller whose tensors (and current stream) are on another GPU."""
+    """Run ``eng._forward(entry, ...)`` on ``dev`` for a caller whose tensors (and current stream) are on another GPU."""
     src = tokens.device
     n_rows = 0 if not want_logits else (tokens.numel() if logit_rows is None else logit_rows.numel())
     V = eng.cfg.vocab_size
@@ -406,7 +434,7 @@ def _remote_forward(eng, dev, tokens, positions, token_slot, cu_q, seq_slot, max
             loc.append(t.to(dev, non_blocking=True))
             t.record_stream(side)
         local = eng._hop_logits(n_rows) if n_rows else None
-        eng.forward(loc[0], loc[1], loc[2], loc[3], loc[4], max_qlen, max_kv_len, loc[5], local, want_logits, 0)
+        eng._forward(entry, loc[0], loc[1], loc[2], loc[3], loc[4], max_qlen, max_kv_len, loc[5], local, want_logits, 0)
         if n_rows:
             if logits_out is None:
                 with torch.cuda.device(src):

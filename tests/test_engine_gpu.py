@@ -282,3 +282,38 @@ def test_engine_large_m_takes_the_tensor_bound_kernel(fuse_norm):
     check(outs[0], ref)
     check(outs[1], ref)
     assert (outs[0] - outs[1]).abs().max().item() <= 1e-2
+
+
+@pytest.mark.parametrize("hd,nh,nkv,page,attn_impl,min_keys,lens,max_tokens", [
+    (128, 7, 1, 16, 2, 1024, [18, 19, 36, 37, 1, 90], 600),      # tiles of 18 positions: exact, one over, one position
+    (128, 10, 2, 16, 2, 128, [301], 512),                        # one odd forward on the CTA-pair GEMM, split keys
+    (128, 10, 2, 64, 2, 1024, [257, 256, 130], 256),             # chunks of 85 over a cache that already holds positions
+    (128, 8, 2, 8, 2, 1024, [100, 33], 160),                     # pages too small for the TMA boxes: mma.sync kernel
+    (128, 8, 8, 16, 1, 64, [290], 300),                          # one head per group: tiles of 128 positions, split keys
+    (64, 14, 2, 16, 2, 1024, [19, 18, 75], 256),                 # head size 64
+])
+def test_prompt_query_tiles(hd, nh, nkv, page, attn_impl, min_keys, lens, max_tokens):
+    """prompts whose new positions x group exceed the 128 rows of a query tile, against the oracle: the last logits, and a
+    step on top of the caches that the prompts left"""
+    from asd_b200.engine import QwenEngine
+    cfg = Qwen2Config(512, 2, nh, nkv, 1024, 2048, head_dim=hd, name="tiles")
+    w = random_hf_weights(cfg, seed=17, logit_std=0.4)
+    g = torch.Generator().manual_seed(8)
+    ids = [torch.randint(0, cfg.vocab_size, (1, n + 3), generator=g) for n in lens]
+    refs = [qwen2_forward(w, cfg, t) for t in ids]
+    eng = QwenEngine(cfg, max_seqs=len(lens), max_seq_len=max(lens) + 16, max_tokens=max_tokens, page_size=page).load_hf_weights(w)
+    eng.set_option("attn_impl", attn_impl)
+    eng.set_option("attn_min_split_keys", min_keys)
+    slots = torch.arange(len(lens), dtype=torch.int32, device="cuda")
+    last = eng.prefill_ragged([t[0, :n].tolist() for t, n in zip(ids, lens)], slots)
+    new = torch.cat([t[:, n:] for t, n in zip(ids, lens)]).to(torch.int32).cuda()
+    ver = eng.forward_uniform(new, torch.tensor(lens, dtype=torch.int32, device="cuda"), slots, max(lens) + 3)
+    torch.cuda.synchronize()
+    check(last.cpu(), torch.stack([r[0, n - 1] for r, n in zip(refs, lens)]))
+    check(ver.view(len(lens), 3, -1).cpu(), torch.stack([r[0, n:] for r, n in zip(refs, lens)]))
+    # a step call still takes no more positions than one tile holds
+    if nh // nkv > 1:
+        q = eng.max_qlen() + 1
+        with pytest.raises(Exception):
+            eng.forward_uniform(new[:1, :1].expand(1, q).contiguous(), slots[:1] * 0, slots[:1], q)
+    eng.close()
