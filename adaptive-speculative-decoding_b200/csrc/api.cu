@@ -10,7 +10,7 @@ using namespace asd;
 extern "C" {
 
 size_t asd_reject_sample_workspace_bytes(int B, int k) { return reject_sample_workspace_bytes(B, k); }
-void asd_reject_sample_set_impl(int impl) { g_sampler_impl = impl; }
+void asd_reject_sample_set_impl(int impl) { (void)impl; }
 
 int asd_reject_sample(const float* target_logits, const float* draft_logits, const int32_t* draft_tokens,
                       const double* u_accept, const double* u_resid, int B, int k, int V, float temperature,

@@ -1,23 +1,23 @@
 // Fused logits -> softmax -> rejection sampling -> residual resample -> stop-rule features, as a STREAMING pass:
-// every logit of the verify step is read from HBM once, by an independent CTA, with no vocabulary-wide exchange
-// in front of the exponentials.
+// every logit of the verify step is read from HBM once, with no vocabulary-wide exchange in front of the exponentials.
 //
-//   sampler_stats_kernel   grid = rows x chunks (a chunk = 4096 consecutive logits of one row, the draft row's
-//     chunk next to the target's), 256 threads; the chunk pair lands in shared memory through two 1-D bulk (TMA)
-//     copies, so no register holds data in flight: 40 registers, 6 CTAs = 48 warps and 192 KB of loads per SM.
-//     Per chunk: maxima (warp shuffles + one shared-memory hop), exponentials
-//     relative to the CHUNK maximum (polynomial exp2 on the packed fp32x2 pipe), lane sums and the canonical
-//     warp scan; one 32-byte record per (row, chunk).  The last CTA of a row to finish (atomic ticket) merges the
-//     row's records (rescaling by 2^(m_c - M)), runs the min(1, p/q) accept test in binary64 and writes the
-//     features; the last row of a sequence finds the first-reject prefix and emits the accepted tokens.
-//   sampler_draw_kernel    grid = sequences x chunks, only for the ONE row per sequence that emits a new token (first
-//     rejected position or bonus row): residual max(0, p - q) chunk totals, then the last CTA of the sequence walks
-//     the chunk totals, re-reads the selected chunk (L2) and finishes the inverse-CDF draw inside it.  Launched
-//     programmatically behind the first kernel and gated per sequence by a flag, so it overlaps the first kernel's
-//     tail; not launched at all for greedy verification.
-// DRAM traffic = (1 + ~1/(k+1)) x the algorithmic bytes.  The previous design (a cluster of 8 CTAs holding a row
-// pair on chip through three dependent cluster-wide exchanges, round 1) read every byte exactly once but ran at
-// 0.15-0.19 of HBM speed: one row pair occupied 8 SMs for ~15 us of barrier latency.
+//   sampler_stats_kernel   item = (row, chunk): 4096 consecutive logits of one row, the draft row's chunk next to the
+//     target's; at most 3 CTAs of 256 threads per SM stay resident and walk the items.  Bound by HBM: a CTA keeps a ring
+//     of two chunk pairs (four chunks when greedy) filled by 1-D bulk (TMA) copies, so an SM has 96 to 192 KB of loads in
+//     flight all the time; a CTA per item, whose load, barriers, fence and ticket came one after the other, lived 7 us per
+//     32 KB and held the kernel at 0.57 of the copy bandwidth.  Per chunk: maximum (warp shuffles + one shared-memory
+//     hop; the runner-up only where it can be: between the threads' maxima, and inside the one thread that owns the
+//     maximum), exponentials relative to the CHUNK maximum (polynomial exp2 on the packed fp32x2 pipe), lane sums and
+//     the canonical warp scan; one 32-byte record per (row, chunk), and nothing that waits for another CTA.
+//   sampler_draw_kernel    grid = sequences x G (G CTAs share a sequence's chunks, enough to fill the SMs once), launched
+//     programmatically behind it.  Every CTA merges the records of its sequence's rows, a warp per row (rescaling by
+//     2^(m_c - M), lanes = chunks, sums chained in chunk order through shuffles), runs the min(1, p/q) accept test in
+//     binary64 and finds the first-reject prefix: repeating this in the G CTAs is cheaper than tickets between them.  The
+//     first of them writes the features and accepted tokens.  Then the ONE row that emits a new token: residual
+//     max(0, p - q) chunk totals; the last CTA of the sequence walks the totals, re-reads the selected chunk (L2) and
+//     finishes the inverse-CDF draw inside it.  Greedy verification needs the merge only (G = 1).
+// DRAM traffic = (1 + ~1/(k+1)) x the algorithmic bytes.
+// MEASURE_SAMPLER
 //
 // ARITHMETIC CONTRACT v2 (bit-exact with oracle/sampler_oracle.c - see that file's header): every contract
 // operation below is an explicit round-to-nearest intrinsic so that nvcc can neither contract nor reorder it.
@@ -31,6 +31,9 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <algorithm>
+#include <mutex>
+
 #include "asd_internal.h"
 #include "ptx.cuh"
 
@@ -41,6 +44,7 @@ constexpr int kST = 256;                 // threads per CTA = lanes per chunk
 constexpr int kSW = kST / 32;            // warps
 constexpr int kSlots = kChunk / 4 / kST; // float4 per thread and row (4)
 constexpr int kMaxChunks = 52;           // V <= 212992
+constexpr int kMaxRows = 65;             // k <= 64
 constexpr int kNFeat = ASD_NUM_FEATURES;
 
 struct SamplerParams {
@@ -49,7 +53,8 @@ struct SamplerParams {
     const int* draft_tokens;   // [B, k]
     const double* u_accept;    // [B, k]
     const double* u_resid;     // [B]
-    int B, k, V, NC, greedy, flags;   // flags: 4 = the draw kernel is gated per sequence (no grid-wide wait), 8 = acq_rel ticket
+    int B, k, V, NC, greedy;
+    int G;                     // CTAs of the draw kernel per sequence
     float c1;
     // outputs
     uint8_t* accept_mask;
@@ -57,20 +62,12 @@ struct SamplerParams {
     int* out_tokens;
     float* out_logprobs;
     float* features;
-    // workspace (tickets zero between launches)
-    int* row_ticket;    // [rows]
+    // workspace (ticket zero between launches)
     int* seq_ticket;    // [B]
-    int* seq_ticket2;   // [B]
-    int* need_row;      // [B] position that emits the new token
     float4* rec_p;      // [rows][NC] {m, m2, Z, S} of the target chunk
     float4* rec_q;      // [rows][NC] {mq, Zq, e at the chunk arg-max, arg-max index (bits)}
     float* row_px;      // [rows] chunk-relative e_p of the draft token
     float* row_qx;      // [rows] chunk-relative e_q of the draft token
-    float4* row_stat;   // [rows] {M, Zp, Mq, Zq}
-    int* row_accept;    // [rows]
-    float* row_lpx;     // [rows]
-    int* row_amax;      // [rows]
-    float* row_lpamax;  // [rows]
     float* seq_rc;      // [B][NC] residual chunk totals of the emitting row
 };
 
@@ -105,12 +102,6 @@ __device__ __forceinline__ float2 exp2p2(float2 t) {
                        __int_as_float(__float_as_int(q.y) + (__float_as_int(r.y) << 23)));
 }
 
-__device__ __forceinline__ int atom_add_release(int* p, int v) {
-    int old;
-    asm volatile("atom.add.acq_rel.gpu.global.s32 %0, [%1], %2;" : "=r"(old) : "l"(p), "r"(v) : "memory");
-    return old;
-}
-
 // Hillis-Steele inclusive scan inside the warp (the contract's order)
 __device__ __forceinline__ float warp_hs(float x, int lane) {
 #pragma unroll
@@ -130,264 +121,175 @@ __device__ __forceinline__ void exp4(float4& z, float2 c1v, float2 nmv, float2& 
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 1
-// The chunk (16 KB target + 16 KB draft) lands in shared memory through two 1-D bulk (TMA) copies, so no register
-// holds data in flight: 42 registers per thread, 6 CTAs = 48 warps per SM, up to 192 KB of loads in flight per SM.
-__global__ void __launch_bounds__(kST, 6) sampler_stats_kernel(const SamplerParams p) {
-    __shared__ __align__(128) float4 s_zt[kChunk / 4];
-    __shared__ __align__(128) float4 s_zq[kChunk / 4];
-    __shared__ __align__(16) float4 s_recp[kMaxChunks], s_recq[kMaxChunks];
-    __shared__ __align__(8) uint64_t s_bar;
-    __shared__ float s_red[kSW][4], s_red2[kSW][4];
+__device__ __forceinline__ float max4(const float4& z) { return fmaxf(fmaxf(z.x, z.y), fmaxf(z.z, z.w)); }
+
+template <bool GREEDY>
+__global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerParams p) {
+    constexpr int kStages = GREEDY ? 4 : 2, kPair = GREEDY ? kChunk / 4 : kChunk / 2;    // float4s per stage
+    extern __shared__ __align__(128) float4 s_ring[];     // [kStages][target chunk | draft chunk]
+    __shared__ __align__(8) uint64_t s_bar[kStages];
+    __shared__ float s_red[kSW][3], s_red2[kSW][3], s_own2;
     __shared__ unsigned long long s_key[kSW];
-    __shared__ int s_last;
     grid_dep_launch();      // the draw kernel may be scheduled; it waits for this grid before reading anything
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k1 = p.k + 1, V = p.V, NC = p.NC;
     const int total = p.B * k1 * NC;
     const float c1 = p.c1;
     const float2 c1v = make_float2(c1, c1);
-    // thread 0: bulk copies of one (row, chunk) item into the chunk buffers
-    auto issue = [&](int item) {
+    // thread 0: bulk copies of one (row, chunk) item into a stage of the ring
+    auto issue = [&](int item, int st) {
         const int row = item / NC, c = item - row * NC;
         const int b = row / k1, i = row - b * k1;
-        const bool hd = (i < p.k) && !p.greedy;
+        const bool hd = !GREEDY && i < p.k;
         const uint32_t bytes = (uint32_t)min(kChunk / 4, (V - c * kChunk) >> 2) * 16u;
-        mbar_expect_tx(&s_bar, hd ? 2 * bytes : bytes);
-        bulk_g2s(s_zt, p.target + (size_t)row * V + (size_t)c * kChunk, bytes, &s_bar);
-        if (hd) bulk_g2s(s_zq, p.draft + ((size_t)b * p.k + i) * V + (size_t)c * kChunk, bytes, &s_bar);
+        float4* dst = s_ring + st * kPair;
+        mbar_expect_tx(&s_bar[st], hd ? 2 * bytes : bytes);
+        bulk_g2s(dst, p.target + (size_t)row * V + (size_t)c * kChunk, bytes, &s_bar[st]);
+        if (hd) bulk_g2s(dst + kChunk / 4, p.draft + ((size_t)b * p.k + i) * V + (size_t)c * kChunk, bytes, &s_bar[st]);
     };
     if (tid == 0) {
-        mbar_init(&s_bar, 1);
+#pragma unroll
+        for (int st = 0; st < kStages; ++st) mbar_init(&s_bar[st], 1);
         fence_mbar_init();
-        issue(blockIdx.x);
+#pragma unroll
+        for (int st = 0; st < kStages; ++st)
+            if (blockIdx.x + (long long)st * gridDim.x < total) issue(blockIdx.x + st * gridDim.x, st);
     }
-    __syncthreads();            // the barrier is initialised
-    uint32_t phase = 0;
-    // Persistent CTAs, items dealt round-robin: the bulk copies of a CTA's NEXT item are issued as soon as every thread
-    // has consumed the current chunk, so they fly while thread 0 finishes the chunk (sums, record, fence, ticket).
-  for (int item = blockIdx.x; item < total; item += gridDim.x) {
-    const int row = item / NC, c = item - row * NC;
-    const int b = row / k1, i = row - b * k1;
-    const bool has_draft = (i < p.k) && !p.greedy;
-    const int n4 = min(kChunk / 4, (V - c * kChunk) >> 2);     // float4s of this chunk that exist
-    mbar_wait(&s_bar, phase);
-    phase ^= 1;
+    __syncthreads();            // the barriers are initialised
+    int it = 0;
+    for (int item = blockIdx.x; item < total; item += gridDim.x, ++it) {
+        const int st = it % kStages;
+        const int row = item / NC, c = item - row * NC;
+        const int b = row / k1, i = row - b * k1;
+        const bool has_draft = !GREEDY && i < p.k;
+        const int n4 = min(kChunk / 4, (V - c * kChunk) >> 2);     // float4s of this chunk that exist
+        const float4* zt = s_ring + st * kPair;
+        const float4* zq = zt + kChunk / 4;
+        mbar_wait(&s_bar[st], (it / kStages) & 1);
 
-    // ---- chunk maxima on the raw logits: rn multiplication by c1 > 0 is monotone, so the two largest a = z * c1 of
-    // the multiset are the products of the two largest z (exact, order independent)
-    float m1 = -INFINITY, m2 = -INFINITY, mq = -INFINITY;
+        // ---- chunk maxima on the raw logits: rn multiplication by c1 > 0 is monotone, so the two largest a = z * c1 of
+        // the multiset are the products of the two largest z (exact, order independent)
+        float m1 = -INFINITY, mq = -INFINITY;
 #pragma unroll
-    for (int s = 0; s < kSlots; ++s) {
-        if (s * kST + tid < n4) {
-            const float4 z = s_zt[s * kST + tid];
-            const float a[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                m2 = fmaxf(m2, fminf(m1, a[e]));
-                m1 = fmaxf(m1, a[e]);
+        for (int s = 0; s < kSlots; ++s)
+            if (s * kST + tid < n4) {
+                m1 = fmaxf(m1, max4(zt[s * kST + tid]));
+                if (has_draft) mq = fmaxf(mq, max4(zq[s * kST + tid]));
             }
-            if (has_draft) {
-                const float4 q = s_zq[s * kST + tid];
-                mq = fmaxf(mq, fmaxf(fmaxf(q.x, q.y), fmaxf(q.z, q.w)));
-            }
-        }
-    }
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const float o1 = __shfl_xor_sync(0xffffffffu, m1, d), o2 = __shfl_xor_sync(0xffffffffu, m2, d);
-        m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
-        m1 = fmaxf(m1, o1);
-        mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, d));
-    }
-    if (lane == 0) {
-        s_red[warp][0] = m1;
-        s_red[warp][1] = m2;
-        s_red[warp][2] = mq;
-    }
-    __syncthreads();
-    m1 = m2 = mq = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < kSW; ++w) {
-        const float o1 = s_red[w][0], o2 = s_red[w][1];
-        m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
-        m1 = fmaxf(m1, o1);
-        mq = fmaxf(mq, s_red[w][2]);
-    }
-    m1 = __fmul_rn(m1, c1);
-    m2 = __fmul_rn(m2, c1);
-    mq = __fmul_rn(mq, c1);
-
-    // ---- exponentials relative to the chunk maximum; a lane keeps two running sums (elements with even / odd local
-    // index, each left to right) on the packed fp32x2 pipe and adds them at the end
-    float2 zs2 = make_float2(0.f, 0.f), ss2 = zs2, qs2 = zs2;
-    unsigned long long key = ~0ull;                      // greedy: (lowest index attaining the maximum, its e)
-    const float2 nm1v = make_float2(-m1, -m1), nmqv = make_float2(-mq, -mq);
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s) {
-        if (s * kST + tid < n4) {
-            float4 z = s_zt[s * kST + tid];
-            const float4 zraw = z;
-            float2 t0, t1;
-            exp4(z, c1v, nm1v, t0, t1);
-            zs2 = __fadd2_rn(__fadd2_rn(zs2, make_float2(z.x, z.y)), make_float2(z.z, z.w));
-            ss2 = __fadd2_rn(__fadd2_rn(ss2, __fmul2_rn(make_float2(z.x, z.y), t0)), __fmul2_rn(make_float2(z.z, z.w), t1));
-            if (p.greedy) {
-                const float zz[4] = {zraw.x, zraw.y, zraw.z, zraw.w};
-                const float ee[4] = {z.x, z.y, z.z, z.w};
-#pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (__fmul_rn(zz[e], c1) == m1) {
-                        const unsigned long long kk =
-                            ((unsigned long long)(unsigned)(c * kChunk + (s * kST + tid) * 4 + e) << 32) | __float_as_uint(ee[e]);
-                        key = kk < key ? kk : key;
-                    }
-            }
-            if (has_draft) {
-                float4 q = s_zq[s * kST + tid];
-                float2 u0, u1;
-                exp4(q, c1v, nmqv, u0, u1);
-                qs2 = __fadd2_rn(__fadd2_rn(qs2, make_float2(q.x, q.y)), make_float2(q.z, q.w));
-            }
-        }
-    }
-    const float zs = __fadd_rn(zs2.x, zs2.y), ss = __fadd_rn(ss2.x, ss2.y), qs = __fadd_rn(qs2.x, qs2.y);
-    // ---- the draft token's exponentials (one thread recomputes them from the chunk in shared memory)
-    const int x = (i < p.k) ? p.draft_tokens[b * p.k + i] : -1;
-    const bool x_ok = (i < p.k) && x >= 0 && x < V;
-    if (tid == 32 && x_ok && x / kChunk == c) {
-        const int u = x - c * kChunk;
-        p.row_px[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(s_zt)[u], c1, -m1));
-        if (has_draft) p.row_qx[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(s_zq)[u], c1, -mq));
-    }
-    // ---- canonical chunk totals: Hillis-Steele inside the warp, sequential chain over the 8 warps
-    const float hz = warp_hs(zs, lane), hs_ = warp_hs(ss, lane), hq = warp_hs(qs, lane);
-    if (p.greedy) {
+        const float own = m1;
+        float m2 = -INFINITY;       // runner-up among the threads' maxima
 #pragma unroll
         for (int d = 16; d >= 1; d >>= 1) {
-            const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d);
-            key = o < key ? o : key;
+            const float o1 = __shfl_xor_sync(0xffffffffu, m1, d), o2 = __shfl_xor_sync(0xffffffffu, m2, d);
+            m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+            m1 = fmaxf(m1, o1);
+            mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, d));
         }
-    }
-    if (lane == 31) {
-        s_red2[warp][0] = hz;
-        s_red2[warp][1] = hs_;
-        s_red2[warp][2] = hq;
-    }
-    if (lane == 0) s_key[warp] = key;
-    __syncthreads();            // every thread is done with the chunk buffers
-    if (tid == 0) {
-        fence_proxy_async_smem();   // generic reads of the buffers ordered before the async-proxy writes of the next copy
-        if (item + (int)gridDim.x < total) issue(item + gridDim.x);
-        float Z = 0.0f, S = 0.0f, Zq = 0.0f;
-        unsigned long long kk = ~0ull;
+        if (lane == 0) {
+            s_red[warp][0] = m1;
+            s_red[warp][1] = m2;
+            s_red[warp][2] = mq;
+        }
+        __syncthreads();
+        m1 = m2 = mq = -INFINITY;
+#pragma unroll
         for (int w = 0; w < kSW; ++w) {
-            Z = __fadd_rn(Z, s_red2[w][0]);
-            S = __fadd_rn(S, s_red2[w][1]);
-            Zq = __fadd_rn(Zq, s_red2[w][2]);
-            kk = s_key[w] < kk ? s_key[w] : kk;
+            const float o1 = s_red[w][0], o2 = s_red[w][1];
+            m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
+            m1 = fmaxf(m1, o1);
+            mq = fmaxf(mq, s_red[w][2]);
         }
-        __stcg(&p.rec_p[(size_t)row * NC + c], make_float4(m1, m2, Z, S));
-        __stcg(&p.rec_q[(size_t)row * NC + c],
-               make_float4(mq, Zq, __uint_as_float((unsigned)(kk & 0xffffffffu)), __int_as_float((int)(kk >> 32))));
-        if (p.flags & 8) {
-            s_last = atom_add_release(&p.row_ticket[row], 1) == NC - 1;   // orders the record stores before the ticket
-        } else {
-            __threadfence();
-            s_last = atomicAdd(&p.row_ticket[row], 1) == NC - 1;
+        // the thread that owns the maximum adds its own runner-up; where several own it, m2 equals it already
+        if (own == m1) {
+            float a1 = -INFINITY, a2 = -INFINITY;
+            for (int s = 0; s < kSlots; ++s)
+                if (s * kST + tid < n4) {
+                    const float4 z = zt[s * kST + tid];
+                    const float a[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        a2 = fmaxf(a2, fminf(a1, a[e]));
+                        a1 = fmaxf(a1, a[e]);
+                    }
+                }
+            s_own2 = a2;
         }
-    }
-    __syncthreads();
-    if (!s_last) continue;
+        m1 = __fmul_rn(m1, c1);
+        mq = __fmul_rn(mq, c1);
 
-    // ================================================================ last CTA of the row: merge its chunk records
-    __threadfence();
-    if (tid < NC) {
-        s_recp[tid] = __ldcg(&p.rec_p[(size_t)row * NC + tid]);
-        s_recq[tid] = __ldcg(&p.rec_q[(size_t)row * NC + tid]);
-    }
-    __syncthreads();
-    if (tid != 0) continue;
-    float M = -INFINITY, M2 = -INFINITY, Mq = -INFINITY;
-    for (int c2 = 0; c2 < NC; ++c2) {
-        M2 = fmaxf(fminf(M, s_recp[c2].x), fmaxf(M2, s_recp[c2].y));
-        M = fmaxf(M, s_recp[c2].x);
-        Mq = fmaxf(Mq, s_recq[c2].x);
-    }
-    float Zp = 0.0f, St = 0.0f, Zq = 0.0f, s_x = 0.0f, sq_x = 0.0f, P_amax = 0.0f;
-    int amax = -1;
-    const int cx = x_ok ? x / kChunk : -1;
-    for (int c2 = 0; c2 < NC; ++c2) {
-        const float d = __fadd_rn(s_recp[c2].x, -M);
-        const float sc = exp2p(d);
-        Zp = __fadd_rn(Zp, __fmul_rn(s_recp[c2].z, sc));
-        St = __fadd_rn(St, __fmul_rn(__fmaf_rn(s_recp[c2].z, d, s_recp[c2].w), sc));
-        if (c2 == cx) s_x = sc;
-        if (p.greedy && amax < 0 && s_recp[c2].x == M) {
-            amax = __float_as_int(s_recq[c2].w);
-            P_amax = __fmul_rn(s_recq[c2].z, sc);
+        // ---- exponentials relative to the chunk maximum; a lane keeps two running sums (elements with even / odd local
+        // index, each left to right) on the packed fp32x2 pipe and adds them at the end
+        float2 zs2 = make_float2(0.f, 0.f), ss2 = zs2, qs2 = zs2;
+        const float2 nm1v = make_float2(-m1, -m1), nmqv = make_float2(-mq, -mq);
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s)
+            if (s * kST + tid < n4) {
+                float4 z = zt[s * kST + tid];
+                float2 t0, t1;
+                exp4(z, c1v, nm1v, t0, t1);
+                zs2 = __fadd2_rn(__fadd2_rn(zs2, make_float2(z.x, z.y)), make_float2(z.z, z.w));
+                ss2 = __fadd2_rn(__fadd2_rn(ss2, __fmul2_rn(make_float2(z.x, z.y), t0)), __fmul2_rn(make_float2(z.z, z.w), t1));
+                if (has_draft) {
+                    float4 q = zq[s * kST + tid];
+                    exp4(q, c1v, nmqv, t0, t1);
+                    qs2 = __fadd2_rn(__fadd2_rn(qs2, make_float2(q.x, q.y)), make_float2(q.z, q.w));
+                }
+            }
+        const float zs = __fadd_rn(zs2.x, zs2.y), ss = __fadd_rn(ss2.x, ss2.y), qs = __fadd_rn(qs2.x, qs2.y);
+        // ---- the draft token's exponentials (one thread recomputes them from the chunk in shared memory)
+        if (tid == 32 && i < p.k) {
+            const int x = p.draft_tokens[b * p.k + i];
+            if (x >= 0 && x < V && x / kChunk == c) {
+                const int u = x - c * kChunk;
+                p.row_px[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zt)[u], c1, -m1));
+                if (has_draft) p.row_qx[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zq)[u], c1, -mq));
+            }
         }
-        if (has_draft) {
-            const float sq = exp2p(__fadd_rn(s_recq[c2].x, -Mq));
-            Zq = __fadd_rn(Zq, __fmul_rn(s_recq[c2].y, sq));
-            if (c2 == cx) sq_x = sq;
+        // ---- canonical chunk totals: Hillis-Steele inside the warp, sequential chain over the 8 warps
+        const float hz = warp_hs(zs, lane), hs_ = warp_hs(ss, lane), hq = warp_hs(qs, lane);
+        if (GREEDY) {               // (lowest index attaining the maximum, its e): only threads whose maximum attains it look
+            unsigned long long key = ~0ull;
+            if (__fmul_rn(own, c1) == m1)
+                for (int s = kSlots - 1; s >= 0; --s)
+                    if (s * kST + tid < n4) {
+                        const float4 z = zt[s * kST + tid];
+                        const float zz[4] = {z.x, z.y, z.z, z.w};
+#pragma unroll
+                        for (int e = 3; e >= 0; --e)
+                            if (__fmul_rn(zz[e], c1) == m1)
+                                key = ((unsigned long long)(unsigned)(c * kChunk + (s * kST + tid) * 4 + e) << 32) |
+                                      __float_as_uint(exp2p(__fmaf_rn(zz[e], c1, -m1)));
+                    }
+#pragma unroll
+            for (int d = 16; d >= 1; d >>= 1) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d);
+                key = o < key ? o : key;
+            }
+            if (lane == 0) s_key[warp] = key;
+        }
+        if (lane == 31) {
+            s_red2[warp][0] = hz;
+            s_red2[warp][1] = hs_;
+            s_red2[warp][2] = hq;
+        }
+        __syncthreads();            // every thread is done with the stage
+        if (tid == 0) {
+            fence_proxy_async_smem();   // generic reads of the stage ordered before the async-proxy writes of the next copy
+            if (item + (long long)kStages * gridDim.x < total) issue(item + kStages * gridDim.x, st);
+            float Z = 0.0f, S = 0.0f, Zq = 0.0f;
+            unsigned long long kk = ~0ull;
+#pragma unroll
+            for (int w = 0; w < kSW; ++w) {
+                Z = __fadd_rn(Z, s_red2[w][0]);
+                S = __fadd_rn(S, s_red2[w][1]);
+                Zq = __fadd_rn(Zq, s_red2[w][2]);
+                if (GREEDY) kk = s_key[w] < kk ? s_key[w] : kk;
+            }
+            p.rec_p[(size_t)row * NC + c] = make_float4(m1, __fmul_rn(fmaxf(m2, s_own2), c1), Z, S);
+            p.rec_q[(size_t)row * NC + c] =
+                make_float4(mq, Zq, __uint_as_float((unsigned)(kk & 0xffffffffu)), __int_as_float((int)(kk >> 32)));
         }
     }
-    const float Px = x_ok ? __fmul_rn(__ldcg(&p.row_px[row]), s_x) : 0.0f;
-    int acc = 0;
-    if (p.greedy) {
-        acc = x_ok && x == amax;
-    } else if (has_draft && x_ok) {
-        const float Qx = __fmul_rn(__ldcg(&p.row_qx[row]), sq_x);
-        const double lhs = __dmul_rn(__dmul_rn(p.u_accept[b * p.k + i], (double)Qx), (double)Zp);
-        const double rhs = __dmul_rn((double)Px, (double)Zq);
-        acc = lhs <= rhs;
-    }
-    const float logZ = logf(Zp), log2Z = log2f(Zp);
-    float* f = p.features + (size_t)row * kNFeat;
-    f[0] = __fmul_rn(__fadd_rn(M, log2Z), 0x1.62e43p-1f);
-    f[1] = 1.0f / Zp;
-    f[2] = f[1] - exp2p(__fadd_rn(M2, -M)) / Zp;
-    f[3] = (log2Z - St / Zp) * 0x1.62e43p-1f;
-    f[4] = x_ok ? logf(Px) - logZ : -INFINITY;
-    __stcg(&p.row_stat[row], make_float4(M, Zp, Mq, Zq));
-    p.row_accept[row] = acc;
-    p.row_lpx[row] = f[4];
-    if (p.greedy) {
-        p.row_amax[row] = amax;
-        p.row_lpamax[row] = logf(P_amax) - logZ;
-    }
-    p.row_ticket[row] = 0;
-    __threadfence();
-    if (atomicAdd(&p.seq_ticket[b], 1) != p.k) continue;
-    // ================================================================ last row of the sequence: first-reject prefix
-    __threadfence();
-    int n = 0;
-    while (n < p.k && __ldcg(&p.row_accept[b * k1 + n])) ++n;
-    for (int t = 0; t < p.k; ++t) p.accept_mask[b * p.k + t] = t < n;
-    p.accepted_len[b] = n;
-    for (int t = 0; t < k1; ++t) {
-        if (t == n && !p.greedy) continue;          // written by the draw kernel
-        int tok = -1;
-        float lp = 0.0f;
-        if (t < n) {
-            tok = p.draft_tokens[b * p.k + t];
-            lp = __ldcg(&p.row_lpx[b * k1 + t]);
-        } else if (t == n) {
-            tok = __ldcg(&p.row_amax[b * k1 + t]);
-            lp = __ldcg(&p.row_lpamax[b * k1 + t]);
-        }
-        p.out_tokens[b * k1 + t] = tok;
-        p.out_logprobs[b * k1 + t] = lp;
-        p.features[(size_t)(b * k1 + t) * kNFeat + 5] = lp;
-    }
-    p.seq_ticket[b] = 0;
-    if (!p.greedy) {
-        // release: everything the draw kernel reads for this sequence (records, row statistics: written by other CTAs
-        // and observed here through the tickets) is ordered before the flag
-        __threadfence();
-        *reinterpret_cast<volatile int*>(&p.need_row[b]) = n + 1;
-    }
-  }
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 2
@@ -442,44 +344,166 @@ __device__ __forceinline__ float residual_chunk(const SamplerParams& p, int row,
     return rs;
 }
 
+// One row's statistics from its chunk records, by one warp (lanes = chunks lane and lane + 32; every sum is chained in
+// chunk order): {M, Zp, Mq, Zq}, whether the draft token is accepted, and - `write` - the row's features.
+struct RowMerge {
+    float4 stat;
+    int accept, amax;
+    float lpx, lp_amax;
+};
+__device__ __forceinline__ RowMerge merge_row(const SamplerParams& p, int b, int i, int lane, bool write) {
+    const unsigned all = 0xffffffffu;
+    const int NC = p.NC, row = b * (p.k + 1) + i;
+    const bool has_draft = i < p.k && !p.greedy;
+    const float4 none = make_float4(-INFINITY, -INFINITY, 0.f, 0.f);
+    float4 rp[2], rq[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const bool ok = lane + 32 * u < NC;
+        rp[u] = ok ? __ldcg(&p.rec_p[(size_t)row * NC + lane + 32 * u]) : none;
+        rq[u] = ok ? __ldcg(&p.rec_q[(size_t)row * NC + lane + 32 * u]) : none;
+    }
+    const int x = i < p.k ? p.draft_tokens[b * p.k + i] : -1;
+    const bool x_ok = i < p.k && x >= 0 && x < p.V;
+    const float px = x_ok ? __ldcg(&p.row_px[row]) : 0.0f, qx = x_ok && has_draft ? __ldcg(&p.row_qx[row]) : 0.0f;
+    const double u_acc = has_draft ? p.u_accept[b * p.k + i] : 0.0;
+    float M = fmaxf(rp[0].x, rp[1].x), M2 = fmaxf(fminf(rp[0].x, rp[1].x), fmaxf(rp[0].y, rp[1].y));
+    float Mq = fmaxf(rq[0].x, rq[1].x);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        const float o1 = __shfl_xor_sync(all, M, d), o2 = __shfl_xor_sync(all, M2, d);
+        M2 = fmaxf(fminf(M, o1), fmaxf(M2, o2));
+        M = fmaxf(M, o1);
+        Mq = fmaxf(Mq, __shfl_xor_sync(all, Mq, d));
+    }
+    float sc[2], tz[2], ts[2], sq[2], tq[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const float d = __fadd_rn(rp[u].x, -M);
+        sc[u] = exp2p(d);
+        tz[u] = __fmul_rn(rp[u].z, sc[u]);
+        ts[u] = __fmul_rn(__fmaf_rn(rp[u].z, d, rp[u].w), sc[u]);
+        sq[u] = exp2p(__fadd_rn(rq[u].x, -Mq));
+        tq[u] = __fmul_rn(rq[u].y, sq[u]);
+    }
+    float Zp = 0.0f, St = 0.0f, Zq = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll 8
+        for (int c = 0; c < min(32, NC - 32 * u); ++c) {
+            Zp = __fadd_rn(Zp, __shfl_sync(all, tz[u], c));
+            St = __fadd_rn(St, __shfl_sync(all, ts[u], c));
+            Zq = __fadd_rn(Zq, __shfl_sync(all, tq[u], c));
+        }
+    if (!has_draft) Zq = 0.0f;
+    const int cx = x_ok ? x / kChunk : 0;
+    const float s_x = __shfl_sync(all, cx < 32 ? sc[0] : sc[1], cx & 31);
+    const float sq_x = __shfl_sync(all, cx < 32 ? sq[0] : sq[1], cx & 31);
+    RowMerge r;
+    r.stat = make_float4(M, Zp, Mq, Zq);
+    const float Px = x_ok ? __fmul_rn(px, s_x) : 0.0f;
+    r.amax = -1;
+    float P_amax = 0.0f;
+    if (p.greedy) {             // the first chunk that attains the row maximum holds its lowest index
+        const unsigned h0 = __ballot_sync(all, rp[0].x == M && lane < NC), h1 = __ballot_sync(all, rp[1].x == M && lane + 32 < NC);
+        if (h0 | h1) {
+            const int src = h0 ? __ffs(h0) - 1 : __ffs(h1) - 1;
+            r.amax = __shfl_sync(all, __float_as_int(h0 ? rq[0].w : rq[1].w), src);
+            P_amax = __shfl_sync(all, h0 ? __fmul_rn(rq[0].z, sc[0]) : __fmul_rn(rq[1].z, sc[1]), src);
+        }
+    }
+    r.accept = 0;
+    if (p.greedy) {
+        r.accept = x_ok && x == r.amax;
+    } else if (has_draft && x_ok) {
+        const float Qx = __fmul_rn(qx, sq_x);
+        const double lhs = __dmul_rn(__dmul_rn(u_acc, (double)Qx), (double)Zp);
+        const double rhs = __dmul_rn((double)Px, (double)Zq);
+        r.accept = lhs <= rhs;
+    }
+    r.lpx = r.lp_amax = 0.0f;
+    if (write) {
+        const float logZ = logf(Zp), log2Z = log2f(Zp);
+        r.lpx = x_ok ? logf(Px) - logZ : -INFINITY;
+        if (p.greedy) r.lp_amax = logf(P_amax) - logZ;
+        if (lane == 0) {
+            float* f = p.features + (size_t)row * kNFeat;
+            f[0] = __fmul_rn(__fadd_rn(M, log2Z), 0x1.62e43p-1f);
+            f[1] = 1.0f / Zp;
+            f[2] = f[1] - exp2p(__fadd_rn(M2, -M)) / Zp;
+            f[3] = (log2Z - St / Zp) * 0x1.62e43p-1f;
+            f[4] = r.lpx;
+        }
+    }
+    return r;
+}
+
 __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParams p) {
-    __shared__ float s_red[kSW];
-    __shared__ float s_rc[kMaxChunks];
+    __shared__ float s_red[2][kSW];
+    __shared__ float s_rc[kMaxChunks], s_pre[kMaxChunks];
+    __shared__ float4 s_stat[kMaxRows];
+    __shared__ int s_acc[kMaxRows], s_amax[kMaxRows];
+    __shared__ float s_lpx[kMaxRows], s_lpamax[kMaxRows];
     __shared__ int s_flag, s_cstar, s_tstar[kSW];
-    __shared__ float s_tau, s_X;
-    // Launched programmatically: these CTAs become resident while the statistics kernel drains its last wave and wait
-    // for THEIR sequence only (flag = emitting position + 1, set by the sequence's finaliser with release semantics),
-    // so the draws of the early sequences overlap the statistics of the late ones.  No deadlock: this grid is only
-    // scheduled once every CTA of the statistics kernel has started, and those never wait for anything.
+    __shared__ float s_tau;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int k1 = p.k + 1, NC = p.NC;
-    const int b = blockIdx.x / NC, c = blockIdx.x - b * NC;
-    if (!(p.flags & 4)) grid_dep_wait();
-    if (tid == 0) {
-        int v;
-        do {
-            asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(v) : "l"(p.need_row + b) : "memory");
-        } while (v == 0);
-        s_cstar = v - 1;
+    const int k1 = p.k + 1, NC = p.NC, G = p.G;
+    const int b = blockIdx.x / G, g = blockIdx.x - b * G;
+    grid_dep_wait();
+    for (int i = warp; i < k1; i += kSW) {
+        const RowMerge r = merge_row(p, b, i, lane, g == 0);
+        if (lane == 0) {
+            s_stat[i] = r.stat;
+            s_acc[i] = r.accept;
+            s_amax[i] = r.amax;
+            s_lpx[i] = r.lpx;
+            s_lpamax[i] = r.lp_amax;
+        }
     }
     __syncthreads();
-    const int n = s_cstar;
-    __syncthreads();
+    int n = 0;                  // first-reject prefix
+    while (n < p.k && s_acc[n]) ++n;
+    if (g == 0) {
+        if (tid < p.k) p.accept_mask[b * p.k + tid] = tid < n;
+        if (tid == 0) p.accepted_len[b] = n;
+        if (tid < k1 && (tid != n || p.greedy)) {       // position n of a sampled sequence: the draw below
+            int tok = -1;
+            float lp = 0.0f;
+            if (tid < n) {
+                tok = p.draft_tokens[b * p.k + tid];
+                lp = s_lpx[tid];
+            } else if (tid == n) {
+                tok = s_amax[n];
+                lp = s_lpamax[n];
+            }
+            p.out_tokens[b * k1 + tid] = tok;
+            p.out_logprobs[b * k1 + tid] = lp;
+            p.features[(size_t)(b * k1 + tid) * kNFeat + 5] = lp;
+        }
+    }
+    if (p.greedy) return;
     const int row = b * k1 + n;
     const bool has_draft = n < p.k;
-    const float4 st = __ldcg(&p.row_stat[row]);
+    const float4 st = s_stat[n];
     float4 zt[kSlots], zq[kSlots];
     bool have[kSlots];
-    float rs = residual_chunk(p, row, b, n, c, has_draft, st, zt, zq, have);
-    float hs = warp_hs(rs, lane);
-    if (lane == 31) s_red[warp] = hs;
-    __syncthreads();
+    float rs = 0.0f, hs;
+    int c = -1;
+    for (int c2 = g, it = 0; c2 < NC; c2 += G, ++it) {
+        c = c2;
+        rs = residual_chunk(p, row, b, n, c, has_draft, st, zt, zq, have);
+        hs = warp_hs(rs, lane);
+        if (lane == 31) s_red[it & 1][warp] = hs;
+        __syncthreads();
+        if (tid == 0) {
+            float R = 0.0f;
+            for (int w = 0; w < kSW; ++w) R = __fadd_rn(R, s_red[it & 1][w]);
+            __stcg(&p.seq_rc[(size_t)b * NC + c], R);
+        }
+    }
     if (tid == 0) {
-        float R = 0.0f;
-        for (int w = 0; w < kSW; ++w) R = __fadd_rn(R, s_red[w]);
-        __stcg(&p.seq_rc[(size_t)b * NC + c], R);
         __threadfence();
-        s_flag = atomicAdd(&p.seq_ticket2[b], 1) == NC - 1;
+        s_flag = atomicAdd(&p.seq_ticket[b], 1) == G - 1;
     }
     __syncthreads();
     if (!s_flag) return;
@@ -488,37 +512,35 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
     __threadfence();
     if (tid < NC) s_rc[tid] = __ldcg(&p.seq_rc[(size_t)b * NC + tid]);
     __syncthreads();
-    if (tid == 0) {
+    if (warp == 0) {
         float R = 0.0f;
-        for (int c2 = 0; c2 < NC; ++c2) R = __fadd_rn(R, s_rc[c2]);
+        if (lane == 0) {
+            p.seq_ticket[b] = 0;
+#pragma unroll 8
+            for (int c2 = 0; c2 < NC; ++c2) s_pre[c2] = R = __fadd_rn(R, s_rc[c2]);
+        }
+        R = __shfl_sync(0xffffffffu, R, 0);
         int cstar = -1;
-        float X = 0.0f, tau = 0.0f;
+        float tau = 0.0f;
         if (R > 0.0f) {
             float ur = (float)p.u_resid[b];
             if (!(ur >= 0.0f)) ur = 0.0f;
             if (ur >= 1.0f) ur = 0x1.fffffep-1f;
             tau = __fmul_rn(ur, R);
             if (!(tau < R)) tau = 0.0f;
-            float pre = 0.0f;
-            for (int c2 = 0; c2 < NC; ++c2) {
-                const float nx = __fadd_rn(pre, s_rc[c2]);
-                if (nx > tau) {
-                    cstar = c2;
-                    X = pre;
-                    break;
-                }
-                pre = nx;
-            }
+            __syncwarp();
+            const unsigned h0 = __ballot_sync(0xffffffffu, lane < NC && s_pre[lane] > tau);
+            const unsigned h1 = __ballot_sync(0xffffffffu, lane + 32 < NC && s_pre[lane + 32] > tau);
+            cstar = h0 ? __ffs(h0) - 1 : (h1 ? 31 + __ffs(h1) : -1);
         }
-        s_cstar = cstar;
-        s_tau = tau;
-        s_X = X;
-        p.seq_ticket2[b] = 0;
-        p.need_row[b] = 0;          // every CTA of this sequence has read the flag (they ticket after reading it)
+        if (lane == 0) {
+            s_cstar = cstar;
+            s_tau = tau;
+        }
     }
     __syncthreads();
     const int cstar = s_cstar;
-    const float tau = s_tau, X = s_X;
+    const float tau = s_tau, X = cstar > 0 ? s_pre[cstar - 1] : 0.0f;
     const float logZ = logf(st.y);
     if (cstar < 0) {
         // residual mass is zero (p == q on this row): the draft token itself is a valid draw
@@ -538,11 +560,10 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
     }
     if (cstar != c) rs = residual_chunk(p, row, b, n, cstar, has_draft, st, zt, zq, have);
     hs = warp_hs(rs, lane);
-    __syncthreads();       // s_red is rewritten
-    if (lane == 31) s_red[warp] = hs;
+    if (lane == 31) s_red[0][warp] = hs;   // (thread 0 read both halves before its ticket)
     __syncthreads();
     float off = 0.0f;
-    for (int w = 0; w < warp; ++w) off = __fadd_rn(off, s_red[w]);
+    for (int w = 0; w < warp; ++w) off = __fadd_rn(off, s_red[0][w]);
     const float P = __fadd_rn(X, __fadd_rn(off, hs));
     const float Pprev = __shfl_up_sync(0xffffffffu, P, 1);
     const float Xl = lane == 0 ? __fadd_rn(X, off) : Pprev;
@@ -589,21 +610,14 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
     p.features[(size_t)row * kNFeat + 5] = lp;
 }
 
-// asd_reject_sample_set_impl bit flags: 2 = persistent statistics CTAs (experiment, slower), 4 = draw kernel gated per
-// sequence instead of the grid-wide wait (default: +4-7 % at B*k >= 512), 8 = single acq_rel ticket atomic (no gain)
-int g_sampler_impl = 5;
-
 static inline size_t align256(size_t x) { return (x + 255) / 256 * 256; }
 
 size_t reject_sample_workspace_bytes(int B, int k) {
     const size_t rows = (size_t)B * (k + 1);
     size_t n = 0;
-    n += align256(sizeof(int) * rows);                    // row_ticket
-    n += 3 * align256(sizeof(int) * (size_t)B);           // seq_ticket, seq_ticket2, need_row
+    n += align256(sizeof(int) * (size_t)B);               // seq_ticket
     n += 2 * align256(sizeof(float4) * rows * kMaxChunks);  // rec_p, rec_q
     n += 2 * align256(sizeof(float) * rows);              // row_px, row_qx
-    n += align256(sizeof(float4) * rows);                 // row_stat
-    n += 4 * align256(sizeof(float) * rows);              // row_accept, row_lpx, row_amax, row_lpamax
     n += align256(sizeof(float) * (size_t)B * kMaxChunks);  // seq_rc
     return n + 256;
 }
@@ -635,7 +649,8 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     p.V = V;
     p.NC = NC;
     p.greedy = greedy;
-    p.flags = g_sampler_impl;
+    // four draw CTAs fit an SM: one wave of them shares the chunks of all sequences
+    p.G = greedy ? 1 : std::max(1, std::min(NC, (4 * 148 + B - 1) / B));
     p.c1 = greedy ? 0x1.715476p+0f : (1.0f / temperature) * 0x1.715476p+0f;
     p.accept_mask = accept_mask;
     p.accepted_len = accepted_len;
@@ -649,46 +664,44 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
         off += align256(bytes);
         return q;
     };
-    p.row_ticket = reinterpret_cast<int*>(take(sizeof(int) * rows));
     p.seq_ticket = reinterpret_cast<int*>(take(sizeof(int) * (size_t)B));
-    p.seq_ticket2 = reinterpret_cast<int*>(take(sizeof(int) * (size_t)B));
-    p.need_row = reinterpret_cast<int*>(take(sizeof(int) * (size_t)B));
     p.rec_p = reinterpret_cast<float4*>(take(sizeof(float4) * rows * kMaxChunks));
     p.rec_q = reinterpret_cast<float4*>(take(sizeof(float4) * rows * kMaxChunks));
     p.row_px = reinterpret_cast<float*>(take(sizeof(float) * rows));
     p.row_qx = reinterpret_cast<float*>(take(sizeof(float) * rows));
-    p.row_stat = reinterpret_cast<float4*>(take(sizeof(float4) * rows));
-    p.row_accept = reinterpret_cast<int*>(take(sizeof(float) * rows));
-    p.row_lpx = reinterpret_cast<float*>(take(sizeof(float) * rows));
-    p.row_amax = reinterpret_cast<int*>(take(sizeof(float) * rows));
-    p.row_lpamax = reinterpret_cast<float*>(take(sizeof(float) * rows));
     p.seq_rc = reinterpret_cast<float*>(take(sizeof(float) * (size_t)B * kMaxChunks));
 
     static int sms[64];
+    static std::once_flag once[64];
+    constexpr int kRing = 2 * 2 * kChunk * 4;       // bytes: two chunk pairs, or four chunks
     int dev = 0;
     ASD_CUDA(cudaGetDevice(&dev));
-    if (sms[dev & 63] == 0) ASD_CUDA(cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev));
-    // One CTA per item by default.  impl 2 (asd_reject_sample_set_impl, experiments): persistent CTAs that prefetch
-    // their next item - measured 2.5x SLOWER on B200 (18 us per item and CTA), so the hardware block scheduler keeps
-    // the job of refilling SM slots.
-    const size_t items = rows * NC, resident = (size_t)6 * sms[dev & 63];
-    const size_t grid = (g_sampler_impl == 2 && items > resident) ? resident : items;
-    sampler_stats_kernel<<<dim3((unsigned)grid), kST, 0, stream>>>(p);
+    std::call_once(once[dev & 63], [&] {        // a second thread's first launch must not overtake the attributes
+        cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
+        cudaFuncSetAttribute(sampler_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
+        cudaFuncSetAttribute(sampler_stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
+        prefer_max_smem(sampler_stats_kernel<false>);
+        prefer_max_smem(sampler_stats_kernel<true>);
+    });
+    const size_t items = rows * NC, resident = (size_t)3 * sms[dev & 63];
+    const unsigned grid = (unsigned)std::max<size_t>(1, std::min(items, resident));
+    if (greedy)
+        sampler_stats_kernel<true><<<grid, kST, kRing, stream>>>(p);
+    else
+        sampler_stats_kernel<false><<<grid, kST, kRing, stream>>>(p);
     ASD_CUDA(cudaGetLastError());
     count_launch(1);
-    if (!greedy) {
-        cudaLaunchConfig_t cfg = {};
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[0].val.programmaticStreamSerializationAllowed = 1;
-        cfg.gridDim = dim3((unsigned)((size_t)B * NC));
-        cfg.blockDim = dim3(kST);
-        cfg.stream = stream;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        ASD_CUDA(cudaLaunchKernelEx(&cfg, sampler_draw_kernel, p));
-        count_launch(1);
-    }
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3((unsigned)((size_t)B * p.G));
+    cfg.blockDim = dim3(kST);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    ASD_CUDA(cudaLaunchKernelEx(&cfg, sampler_draw_kernel, p));
+    count_launch(1);
     return 0;
 }
 

@@ -56,8 +56,7 @@ ASD_API void asd_reset_launch_count(void);
  * token per row from softmax(target/T) (used for the draft model's own sampling).
  */
 ASD_API size_t asd_reject_sample_workspace_bytes(int B, int k);
-/* tuning switch of the streaming sampler (bit flags, default 5: 4 = the draw kernel is gated per sequence, 2 = persistent
- * statistics CTAs, 8 = single acq_rel ticket); every setting implements the same arithmetic contract bit for bit */
+/* kept for callers that set it: there is one form of the sampler, and every value selects it */
 ASD_API void asd_reject_sample_set_impl(int impl);
 ASD_API int asd_reject_sample(const float* target_logits, const float* draft_logits, const int32_t* draft_tokens,
                       const double* u_accept, const double* u_resid, int B, int k, int V, float temperature,

@@ -138,3 +138,31 @@ def test_full_batch_every_row_against_oracle(B):
     k, V, T = 8, 152064, 0.7
     tl, dl, dt, ua, ur = make_case(B, k, V, seed=500 + B, T=T)
     compare(run_gpu(tl, dl, dt, ua, ur, T), oracle.reject_sample(tl, dl, dt, ua, ur, T))
+
+
+@pytest.mark.parametrize("B,k,V,T", [
+    (70, 6, 12292, 0.8),        # 1960 items on 444 resident CTAs: every ring stage reused, rows without a draft among them
+    (300, 0, 16384, 1.0),       # two draw CTAs per sequence, two chunks each, no drafts
+    (600, 1, 8196, 0.6),        # one draw CTA per sequence walks all of its chunks, the last of 4 logits
+    (1, 64, 4096, 0.7),         # the longest draft: eight warps merge 65 rows
+    (33, 12, 40000, 0.0),       # greedy: four chunks in a ring, ring reused
+    (2, 3, 135172, 0.9),        # 34 chunks: two per lane in the merge, the last of 4 logits
+])
+def test_parity_rings_and_shares(B, k, V, T):
+    tl, dl, dt, ua, ur = make_case(B, k, V, seed=B + 7 * k, T=T, spread=1.5, noise=0.4)
+    tl = np.round(tl * 64) / 64         # equal logits: ties of the maximum inside a lane, a chunk and across chunks
+    compare(run_gpu(tl, dl if k else None, dt, ua, ur, T), oracle.reject_sample(tl, dl if k else None, dt, ua, ur, T))
+
+
+def test_parity_masked_logits():
+    """vocabularies with masked entries (-inf and the type's lowest value), whole chunks of them included"""
+    B, k, V, T = 3, 2, 12288, 0.7
+    tl, dl, dt, ua, ur = make_case(B, k, V, seed=5, T=T)
+    dt = dt % 4000
+    for m in (np.float32(-np.inf), np.finfo(np.float32).min):
+        a, d = tl.copy(), dl.copy()
+        a[:, :, 4096:8192] = d[:, :, 4096:8192] = m
+        a[:, :, 9000::7] = m
+        got, ref = run_gpu(a, d, dt, ua, ur, T), oracle.reject_sample(a, d, dt, ua, ur, T)
+        for key in ("accept_mask", "accepted_len", "out_tokens"):
+            assert np.array_equal(got[key], ref[key]), key
