@@ -5,7 +5,7 @@
 //     target's; at most 3 CTAs of 256 threads per SM stay resident and walk the items.  Bound by HBM: a CTA keeps a ring
 //     of two chunk pairs (four chunks when greedy) filled by 1-D bulk (TMA) copies, so an SM has 96 to 192 KB of loads in
 //     flight all the time; a CTA per item, whose load, barriers, fence and ticket came one after the other, lived 7 us per
-//     32 KB and held the kernel at 0.57 of the copy bandwidth.  Per chunk: maximum (warp shuffles + one shared-memory
+//     32 KB and held the kernel at 0.57 of the copy bandwidth.  Per chunk: maximum (warp reductions + one shared-memory
 //     hop; the runner-up only where it can be: between the threads' maxima, and inside the one thread that owns the
 //     maximum), exponentials relative to the CHUNK maximum (polynomial exp2 on the packed fp32x2 pipe), lane sums and
 //     the canonical warp scan; one 32-byte record per (row, chunk), and nothing that waits for another CTA.
@@ -17,7 +17,10 @@
 //     max(0, p - q) chunk totals; the last CTA of the sequence walks the totals, re-reads the selected chunk (L2) and
 //     finishes the inverse-CDF draw inside it.  Greedy verification needs the merge only (G = 1).
 // DRAM traffic = (1 + ~1/(k+1)) x the algorithmic bytes.
-// MEASURE_SAMPLER
+// Measured (V = 152064, all outputs the same bits), the CTA-per-item form -> this one: B = 64, k = 8: 195 -> 163 us (the
+// first kernel 176 -> 132 us, 5.0 TB/s; what is left is its 10 cycles per issued instruction at 24 warps, six of them a
+// scheduler's, and 31 us of the second kernel, of which 12 are the emitting rows' second read); B = 16, k = 5 greedy
+// 37 -> 29 us; V = 151936, B = 1, k = 4: 22 -> 14 us, launches and the chain record -> merge -> residual -> draw.
 //
 // ARITHMETIC CONTRACT v2 (bit-exact with oracle/sampler_oracle.c - see that file's header): every contract
 // operation below is an explicit round-to-nearest intrinsic so that nvcc can neither contract nor reorder it.
@@ -112,6 +115,26 @@ __device__ __forceinline__ float warp_hs(float x, int lane) {
     return x;
 }
 
+// warp_hs(x)'s last lane for three sums at once: the scan's last lane is the tree that pairs lanes 1, 2, 4, 8, 16 apart,
+// so a butterfly gives its bits, and after the first two steps one exchange serves all three (16 instructions instead of
+// 45).  Lanes with bit 1 set end up with q's total, the others with x's (bit 0 clear) or y's (bit 0 set).
+__device__ __forceinline__ float warp_tree3(float x, float y, float q, int lane) {
+    const unsigned all = 0xffffffffu;
+    const bool odd = lane & 1, high = lane & 2;
+    float a = __fadd_rn(odd ? y : x, __shfl_xor_sync(all, odd ? x : y, 1));
+    q = __fadd_rn(q, __shfl_xor_sync(all, q, 1));
+    a = __fadd_rn(high ? q : a, __shfl_xor_sync(all, high ? a : q, 2));
+#pragma unroll
+    for (int d = 4; d <= 16; d <<= 1) a = __fadd_rn(a, __shfl_xor_sync(all, a, d));
+    return a;
+}
+// maximum over the warp in one instruction (NaN loses against a number, as in fmaxf)
+__device__ __forceinline__ float warp_fmax(float x) {
+    float r;
+    asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 // e = exp2p(fma(z, c1, -m)) for the four logits of a float4, in place
 __device__ __forceinline__ void exp4(float4& z, float2 c1v, float2 nmv, float2& t0, float2& t1) {
     t0 = __ffma2_rn(make_float2(z.x, z.y), c1v, nmv);
@@ -128,22 +151,26 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
     constexpr int kStages = GREEDY ? 4 : 2, kPair = GREEDY ? kChunk / 4 : kChunk / 2;    // float4s per stage
     extern __shared__ __align__(128) float4 s_ring[];     // [kStages][target chunk | draft chunk]
     __shared__ __align__(8) uint64_t s_bar[kStages];
-    __shared__ float s_red[kSW][3], s_red2[kSW][3], s_own2;
+    __shared__ int4 s_item[kStages];                      // {row, chunk, float4s of the chunk | has_draft << 16, draft token in the chunk}
+    __shared__ __align__(16) float2 s_red[2][kSW];        // (the record of an item is written while the next one's maxima arrive)
+    __shared__ float s_own2[kSW], s_red2[kSW][3];
     __shared__ unsigned long long s_key[kSW];
     grid_dep_launch();      // the draw kernel may be scheduled; it waits for this grid before reading anything
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int k1 = p.k + 1, V = p.V, NC = p.NC;
-    const int total = p.B * k1 * NC;
+    const int total = p.B * (p.k + 1) * p.NC;
     const float c1 = p.c1;
     const float2 c1v = make_float2(c1, c1);
-    // thread 0: bulk copies of one (row, chunk) item into a stage of the ring
+    // thread 0: bulk copies of one (row, chunk) item into a stage of the ring, and what the others need to know about it
     auto issue = [&](int item, int st) {
-        const int row = item / NC, c = item - row * NC;
-        const int b = row / k1, i = row - b * k1;
+        const int V = p.V, row = item / p.NC, c = item - row * p.NC;
+        const int b = row / (p.k + 1), i = row - b * (p.k + 1);
         const bool hd = !GREEDY && i < p.k;
-        const uint32_t bytes = (uint32_t)min(kChunk / 4, (V - c * kChunk) >> 2) * 16u;
+        const int n4 = min(kChunk / 4, (V - c * kChunk) >> 2);
+        const uint32_t bytes = (uint32_t)n4 * 16u;
+        const int x = i < p.k ? p.draft_tokens[b * p.k + i] : -1;
+        s_item[st] = make_int4(row, c, n4 | (hd ? 1 << 16 : 0), x >= 0 && x < V && x / kChunk == c ? x - c * kChunk : -1);
         float4* dst = s_ring + st * kPair;
-        mbar_expect_tx(&s_bar[st], hd ? 2 * bytes : bytes);
+        mbar_expect_tx(&s_bar[st], hd ? 2 * bytes : bytes);     // (its release covers s_item)
         bulk_g2s(dst, p.target + (size_t)row * V + (size_t)c * kChunk, bytes, &s_bar[st]);
         if (hd) bulk_g2s(dst + kChunk / 4, p.draft + ((size_t)b * p.k + i) * V + (size_t)c * kChunk, bytes, &s_bar[st]);
     };
@@ -159,52 +186,52 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
     int it = 0;
     for (int item = blockIdx.x; item < total; item += gridDim.x, ++it) {
         const int st = it % kStages;
-        const int row = item / NC, c = item - row * NC;
-        const int b = row / k1, i = row - b * k1;
-        const bool has_draft = !GREEDY && i < p.k;
-        const int n4 = min(kChunk / 4, (V - c * kChunk) >> 2);     // float4s of this chunk that exist
         const float4* zt = s_ring + st * kPair;
         const float4* zq = zt + kChunk / 4;
         mbar_wait(&s_bar[st], (it / kStages) & 1);
+        const int4 what = s_item[st];
+        const int n4 = what.z & 0xffff;
+        const bool has_draft = !GREEDY && (what.z >> 16);
+        // pass over the float4s this thread owns; a whole chunk needs no bounds
+        auto each = [&](auto&& f) {
+            if (n4 == kChunk / 4) {
+#pragma unroll
+                for (int s = 0; s < kSlots; ++s) f(s * kST + tid);
+            } else {
+#pragma unroll 1
+                for (int v = tid; v < n4; v += kST) f(v);
+            }
+        };
 
         // ---- chunk maxima on the raw logits: rn multiplication by c1 > 0 is monotone, so the two largest a = z * c1 of
         // the multiset are the products of the two largest z (exact, order independent)
-        float m1 = -INFINITY, mq = -INFINITY;
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s)
-            if (s * kST + tid < n4) {
-                m1 = fmaxf(m1, max4(zt[s * kST + tid]));
-                if (has_draft) mq = fmaxf(mq, max4(zq[s * kST + tid]));
-            }
-        const float own = m1;
-        float m2 = -INFINITY;       // runner-up among the threads' maxima
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) {
-            const float o1 = __shfl_xor_sync(0xffffffffu, m1, d), o2 = __shfl_xor_sync(0xffffffffu, m2, d);
-            m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
-            m1 = fmaxf(m1, o1);
-            mq = fmaxf(mq, __shfl_xor_sync(0xffffffffu, mq, d));
-        }
-        if (lane == 0) {
-            s_red[warp][0] = m1;
-            s_red[warp][1] = m2;
-            s_red[warp][2] = mq;
-        }
+        float own = -INFINITY, mq = -INFINITY;
+        each([&](int v) {
+            own = fmaxf(own, max4(zt[v]));
+            if (has_draft) mq = fmaxf(mq, max4(zq[v]));
+        });
+        const float wm = warp_fmax(own);
+        mq = warp_fmax(mq);
+        if (lane == 0) s_red[it & 1][warp] = make_float2(wm, mq);
         __syncthreads();
-        m1 = m2 = mq = -INFINITY;
+        float m1 = -INFINITY;
+        mq = -INFINITY;
 #pragma unroll
-        for (int w = 0; w < kSW; ++w) {
-            const float o1 = s_red[w][0], o2 = s_red[w][1];
-            m2 = fmaxf(fminf(m1, o1), fmaxf(m2, o2));
-            m1 = fmaxf(m1, o1);
-            mq = fmaxf(mq, s_red[w][2]);
+        for (int w = 0; w < kSW; w += 2) {
+            const float4 o = *reinterpret_cast<const float4*>(&s_red[it & 1][w]);
+            m1 = fmaxf(m1, fmaxf(o.x, o.z));
+            mq = fmaxf(mq, fmaxf(o.y, o.w));
         }
-        // the thread that owns the maximum adds its own runner-up; where several own it, m2 equals it already
-        if (own == m1) {
+        // runner-up of a warp that owns the maximum: between its other lanes and inside the owner (of several owners the
+        // first leaves out its own maximum, and the others' stand in for the runner-up); of other warps: their maxima, below
+        float second = -INFINITY;
+        if (wm == m1) {
+            const unsigned owners = __ballot_sync(0xffffffffu, own == m1);
+            const bool first = lane == __ffs(owners) - 1;
             float a1 = -INFINITY, a2 = -INFINITY;
-            for (int s = 0; s < kSlots; ++s)
-                if (s * kST + tid < n4) {
-                    const float4 z = zt[s * kST + tid];
+            if (first)
+                for (int v = tid; v < n4; v += kST) {
+                    const float4 z = zt[v];
                     const float a[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
                     for (int e = 0; e < 4; ++e) {
@@ -212,8 +239,10 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
                         a1 = fmaxf(a1, a[e]);
                     }
                 }
-            s_own2 = a2;
+            __syncwarp();
+            second = warp_fmax(first ? a2 : own);
         }
+        const float raw1 = m1;
         m1 = __fmul_rn(m1, c1);
         mq = __fmul_rn(mq, c1);
 
@@ -221,45 +250,41 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
         // index, each left to right) on the packed fp32x2 pipe and adds them at the end
         float2 zs2 = make_float2(0.f, 0.f), ss2 = zs2, qs2 = zs2;
         const float2 nm1v = make_float2(-m1, -m1), nmqv = make_float2(-mq, -mq);
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s)
-            if (s * kST + tid < n4) {
-                float4 z = zt[s * kST + tid];
-                float2 t0, t1;
-                exp4(z, c1v, nm1v, t0, t1);
-                zs2 = __fadd2_rn(__fadd2_rn(zs2, make_float2(z.x, z.y)), make_float2(z.z, z.w));
-                ss2 = __fadd2_rn(__fadd2_rn(ss2, __fmul2_rn(make_float2(z.x, z.y), t0)), __fmul2_rn(make_float2(z.z, z.w), t1));
-                if (has_draft) {
-                    float4 q = zq[s * kST + tid];
-                    exp4(q, c1v, nmqv, t0, t1);
-                    qs2 = __fadd2_rn(__fadd2_rn(qs2, make_float2(q.x, q.y)), make_float2(q.z, q.w));
-                }
+        each([&](int v) {
+            float4 z = zt[v];
+            float2 t0, t1;
+            exp4(z, c1v, nm1v, t0, t1);
+            zs2 = __fadd2_rn(__fadd2_rn(zs2, make_float2(z.x, z.y)), make_float2(z.z, z.w));
+            ss2 = __fadd2_rn(__fadd2_rn(ss2, __fmul2_rn(make_float2(z.x, z.y), t0)), __fmul2_rn(make_float2(z.z, z.w), t1));
+            if (has_draft) {
+                float4 q = zq[v];
+                exp4(q, c1v, nmqv, t0, t1);
+                qs2 = __fadd2_rn(__fadd2_rn(qs2, make_float2(q.x, q.y)), make_float2(q.z, q.w));
             }
-        const float zs = __fadd_rn(zs2.x, zs2.y), ss = __fadd_rn(ss2.x, ss2.y), qs = __fadd_rn(qs2.x, qs2.y);
+        });
         // ---- the draft token's exponentials (one thread recomputes them from the chunk in shared memory)
-        if (tid == 32 && i < p.k) {
-            const int x = p.draft_tokens[b * p.k + i];
-            if (x >= 0 && x < V && x / kChunk == c) {
-                const int u = x - c * kChunk;
-                p.row_px[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zt)[u], c1, -m1));
-                if (has_draft) p.row_qx[row] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zq)[u], c1, -mq));
-            }
+        if (tid == 32 && what.w >= 0) {
+            p.row_px[what.x] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zt)[what.w], c1, -m1));
+            if (has_draft) p.row_qx[what.x] = exp2p(__fmaf_rn(reinterpret_cast<const float*>(zq)[what.w], c1, -mq));
         }
-        // ---- canonical chunk totals: Hillis-Steele inside the warp, sequential chain over the 8 warps
-        const float hz = warp_hs(zs, lane), hs_ = warp_hs(ss, lane), hq = warp_hs(qs, lane);
+        __syncwarp();
+        // ---- canonical chunk totals: the warp's scan tree, sequential chain over the 8 warps
+        const float sum = warp_tree3(__fadd_rn(zs2.x, zs2.y), __fadd_rn(ss2.x, ss2.y), __fadd_rn(qs2.x, qs2.y), lane);
+        if (lane < 3) s_red2[warp][lane] = sum;         // lanes 0, 1, 2: Z, S, Zq
+        if (lane == 3) s_own2[warp] = second;
         if (GREEDY) {               // (lowest index attaining the maximum, its e): only threads whose maximum attains it look
             unsigned long long key = ~0ull;
             if (__fmul_rn(own, c1) == m1)
-                for (int s = kSlots - 1; s >= 0; --s)
-                    if (s * kST + tid < n4) {
-                        const float4 z = zt[s * kST + tid];
-                        const float zz[4] = {z.x, z.y, z.z, z.w};
+                for (int v = tid; v < n4; v += kST) {
+                    const float4 z = zt[v];
+                    const float zz[4] = {z.x, z.y, z.z, z.w};
 #pragma unroll
-                        for (int e = 3; e >= 0; --e)
-                            if (__fmul_rn(zz[e], c1) == m1)
-                                key = ((unsigned long long)(unsigned)(c * kChunk + (s * kST + tid) * 4 + e) << 32) |
-                                      __float_as_uint(exp2p(__fmaf_rn(zz[e], c1, -m1)));
-                    }
+                    for (int e = 0; e < 4; ++e)
+                        if (key == ~0ull && __fmul_rn(zz[e], c1) == m1)
+                            key = ((unsigned long long)(unsigned)(what.y * kChunk + v * 4 + e) << 32) |
+                                  __float_as_uint(exp2p(__fmaf_rn(zz[e], c1, -m1)));
+                }
+            __syncwarp();
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1) {
                 const unsigned long long o = __shfl_xor_sync(0xffffffffu, key, d);
@@ -267,49 +292,45 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
             }
             if (lane == 0) s_key[warp] = key;
         }
-        if (lane == 31) {
-            s_red2[warp][0] = hz;
-            s_red2[warp][1] = hs_;
-            s_red2[warp][2] = hq;
-        }
         __syncthreads();            // every thread is done with the stage
         if (tid == 0) {
             fence_proxy_async_smem();   // generic reads of the stage ordered before the async-proxy writes of the next copy
             if (item + (long long)kStages * gridDim.x < total) issue(item + kStages * gridDim.x, st);
-            float Z = 0.0f, S = 0.0f, Zq = 0.0f;
+            float Z = 0.0f, S = 0.0f, Zq = 0.0f, m2 = -INFINITY;
             unsigned long long kk = ~0ull;
+            bool seen = false;          // the first warp that attains the maximum is the owner, the others are runners-up
 #pragma unroll
             for (int w = 0; w < kSW; ++w) {
                 Z = __fadd_rn(Z, s_red2[w][0]);
                 S = __fadd_rn(S, s_red2[w][1]);
                 Zq = __fadd_rn(Zq, s_red2[w][2]);
+                const float wmax = s_red[it & 1][w].x;
+                const bool owner = !seen && wmax == raw1;
+                seen |= owner;
+                m2 = fmaxf(m2, owner ? s_own2[w] : wmax);
                 if (GREEDY) kk = s_key[w] < kk ? s_key[w] : kk;
             }
-            p.rec_p[(size_t)row * NC + c] = make_float4(m1, __fmul_rn(fmaxf(m2, s_own2), c1), Z, S);
-            p.rec_q[(size_t)row * NC + c] =
-                make_float4(mq, Zq, __uint_as_float((unsigned)(kk & 0xffffffffu)), __int_as_float((int)(kk >> 32)));
+            const size_t at = (size_t)what.x * p.NC + what.y;
+            p.rec_p[at] = make_float4(m1, __fmul_rn(m2, c1), Z, S);
+            p.rec_q[at] = make_float4(mq, Zq, __uint_as_float((unsigned)(kk & 0xffffffffu)), __int_as_float((int)(kk >> 32)));
         }
     }
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 2
-// residual weights of this thread's elements of chunk c of the emitting row: r -> zq[], P -> zt[]; returns the lane sum
-__device__ __forceinline__ float residual_chunk(const SamplerParams& p, int row, int b, int n, int c, bool has_draft,
+// residual weights of this thread's elements of chunk c of the emitting row, whose logits lie at zt_s (draft: behind them):
+// r -> zq[], P -> zt[]; returns the lane sum
+__device__ __forceinline__ float residual_chunk(const SamplerParams& p, int row, int c, bool has_draft, const float4* zt_s,
                                                 const float4& st, float4 (&zt)[kSlots], float4 (&zq)[kSlots],
                                                 bool (&have)[kSlots]) {
-    const int tid = threadIdx.x, V = p.V;
-    const int n4 = min(kChunk / 4, (V - c * kChunk) >> 2);
-    const float4* zt_g = reinterpret_cast<const float4*>(p.target + (size_t)row * V + (size_t)c * kChunk);
-    const float4* zq_g =
-        has_draft ? reinterpret_cast<const float4*>(p.draft + ((size_t)b * p.k + n) * V + (size_t)c * kChunk) : nullptr;
+    const int tid = threadIdx.x;
+    const int n4 = min(kChunk / 4, (p.V - c * kChunk) >> 2);
 #pragma unroll
     for (int s = 0; s < kSlots; ++s) {
         have[s] = s * kST + tid < n4;
-        zt[s] = have[s] ? __ldcg(zt_g + s * kST + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
+        zt[s] = have[s] ? zt_s[s * kST + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+        zq[s] = (has_draft && have[s]) ? zt_s[kChunk / 4 + s * kST + tid] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-#pragma unroll
-    for (int s = 0; s < kSlots; ++s)
-        zq[s] = (has_draft && have[s]) ? __ldcg(zq_g + s * kST + tid) : make_float4(0.f, 0.f, 0.f, 0.f);
     const float4 rp = __ldcg(&p.rec_p[(size_t)row * p.NC + c]);
     const float4 rq = __ldcg(&p.rec_q[(size_t)row * p.NC + c]);
     const float M = st.x, Zp = st.y, Mq = st.z, Zq = st.w;
@@ -438,7 +459,9 @@ __device__ __forceinline__ RowMerge merge_row(const SamplerParams& p, int b, int
     return r;
 }
 
-__global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParams p) {
+__global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParams p) {
+    extern __shared__ __align__(128) float4 s_ring[];     // [2][target chunk | draft chunk]
+    __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ float s_red[2][kSW];
     __shared__ float s_rc[kMaxChunks], s_pre[kMaxChunks];
     __shared__ float4 s_stat[kMaxRows];
@@ -449,6 +472,11 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k1 = p.k + 1, NC = p.NC, G = p.G;
     const int b = blockIdx.x / G, g = blockIdx.x - b * G;
+    if (tid == 0) {
+        mbar_init(&s_bar[0], 1);
+        mbar_init(&s_bar[1], 1);
+        fence_mbar_init();
+    }
     grid_dep_wait();
     for (int i = warp; i < k1; i += kSW) {
         const RowMerge r = merge_row(p, b, i, lane, g == 0);
@@ -463,6 +491,20 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
     __syncthreads();
     int n = 0;                  // first-reject prefix
     while (n < p.k && s_acc[n]) ++n;
+    const int row = b * k1 + n;
+    const bool has_draft = n < p.k;
+    auto issue = [&](int c2, int stage) {       // thread 0
+        const uint32_t bytes = (uint32_t)min(kChunk / 4, (p.V - c2 * kChunk) >> 2) * 16u;
+        float4* dst = s_ring + stage * (kChunk / 2);
+        mbar_expect_tx(&s_bar[stage], has_draft ? 2 * bytes : bytes);
+        bulk_g2s(dst, p.target + (size_t)row * p.V + (size_t)c2 * kChunk, bytes, &s_bar[stage]);
+        if (has_draft)
+            bulk_g2s(dst + kChunk / 4, p.draft + ((size_t)b * p.k + n) * p.V + (size_t)c2 * kChunk, bytes, &s_bar[stage]);
+    };
+    if (tid == 0 && !p.greedy) {
+        issue(g, 0);
+        if (g + G < NC) issue(g + G, 1);
+    }
     if (g == 0) {
         if (tid < p.k) p.accept_mask[b * p.k + tid] = tid < n;
         if (tid == 0) p.accepted_len[b] = n;
@@ -482,24 +524,25 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
         }
     }
     if (p.greedy) return;
-    const int row = b * k1 + n;
-    const bool has_draft = n < p.k;
     const float4 st = s_stat[n];
     float4 zt[kSlots], zq[kSlots];
     bool have[kSlots];
     float rs = 0.0f, hs;
-    int c = -1;
-    for (int c2 = g, it = 0; c2 < NC; c2 += G, ++it) {
-        c = c2;
-        rs = residual_chunk(p, row, b, n, c, has_draft, st, zt, zq, have);
+    int c = g, it = 0;
+    for (;; c += G, ++it) {
+        mbar_wait(&s_bar[it & 1], (it >> 1) & 1);
+        rs = residual_chunk(p, row, c, has_draft, s_ring + (it & 1) * (kChunk / 2), st, zt, zq, have);
         hs = warp_hs(rs, lane);
         if (lane == 31) s_red[it & 1][warp] = hs;
         __syncthreads();
         if (tid == 0) {
+            fence_proxy_async_smem();
+            if (c + 2 * G < NC) issue(c + 2 * G, it & 1);
             float R = 0.0f;
             for (int w = 0; w < kSW; ++w) R = __fadd_rn(R, s_red[it & 1][w]);
             __stcg(&p.seq_rc[(size_t)b * NC + c], R);
         }
+        if (c + G >= NC) break;
     }
     if (tid == 0) {
         __threadfence();
@@ -558,7 +601,12 @@ __global__ void __launch_bounds__(kST, 4) sampler_draw_kernel(const SamplerParam
         }
         return;
     }
-    if (cstar != c) rs = residual_chunk(p, row, b, n, cstar, has_draft, st, zt, zq, have);
+    if (cstar != c) {           // the other stage is free: its chunk was consumed before this one
+        ++it;
+        if (tid == 0) issue(cstar, it & 1);
+        mbar_wait(&s_bar[it & 1], (it >> 1) & 1);
+        rs = residual_chunk(p, row, cstar, has_draft, s_ring + (it & 1) * (kChunk / 2), st, zt, zq, have);
+    }
     hs = warp_hs(rs, lane);
     if (lane == 31) s_red[0][warp] = hs;   // (thread 0 read both halves before its ticket)
     __syncthreads();
@@ -649,8 +697,8 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     p.V = V;
     p.NC = NC;
     p.greedy = greedy;
-    // four draw CTAs fit an SM: one wave of them shares the chunks of all sequences
-    p.G = greedy ? 1 : std::max(1, std::min(NC, (4 * 148 + B - 1) / B));
+    // three draw CTAs fit an SM: one wave of them shares the chunks of all sequences
+    p.G = greedy ? 1 : std::max(1, std::min(NC, 3 * 148 / B));
     p.c1 = greedy ? 0x1.715476p+0f : (1.0f / temperature) * 0x1.715476p+0f;
     p.accept_mask = accept_mask;
     p.accepted_len = accepted_len;
@@ -680,11 +728,13 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
         cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(sampler_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
         cudaFuncSetAttribute(sampler_stats_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
+        cudaFuncSetAttribute(sampler_draw_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
+        prefer_max_smem(sampler_draw_kernel);
         prefer_max_smem(sampler_stats_kernel<false>);
         prefer_max_smem(sampler_stats_kernel<true>);
     });
     const size_t items = rows * NC, resident = (size_t)3 * sms[dev & 63];
-    const unsigned grid = (unsigned)std::max<size_t>(1, std::min(items, resident));
+    const unsigned grid = (unsigned)std::min(items, resident);
     if (greedy)
         sampler_stats_kernel<true><<<grid, kST, kRing, stream>>>(p);
     else
@@ -697,6 +747,7 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.gridDim = dim3((unsigned)((size_t)B * p.G));
     cfg.blockDim = dim3(kST);
+    cfg.dynamicSmemBytes = greedy ? 0 : kRing;
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
