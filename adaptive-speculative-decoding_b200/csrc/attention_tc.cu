@@ -111,27 +111,6 @@ __device__ __forceinline__ void at_tma_box(void* dst, const void* tmap, int c0, 
         "l"(tmap), "r"(smem_u32(bar)), "r"(c0), "r"(c1)
         : "memory");
 }
-// D[tmem] (+)= A[tmem] * B[smem desc]: A = 128 lanes x (K = 16 bf16 = 8 packed 32-bit columns per instruction)
-__device__ __forceinline__ void at_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc,
-                                           uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(tmem_d),
-        "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-// 32 lanes x 16 consecutive 32-bit columns <- 16 registers per thread (thread = lane)
-__device__ __forceinline__ void at_tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
-        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
-        "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15])
-        : "memory");
-}
-__device__ __forceinline__ void at_tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // One 64-key half of the row maximum: element i of the half is visible iff i <= lim (lim >= 63: all of them).
 template <bool MASKED>
 __device__ __forceinline__ void at_max64(const uint32_t (&v0)[32], const uint32_t (&v1)[32], int lim, float (&m)[4]) {
@@ -301,7 +280,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 const uint32_t p = tmem_base + (uint32_t)(st * 128);     // bf16 P: 64 packed columns over S
 #pragma unroll
                 for (int k = 0; k < 8; ++k)
-                    at_umma_ts(d, p + (uint32_t)(k * 8), at_desc_mn(uV + st * kAtOp + k * 2048), idesc_pv, k != 0);
+                    umma_f16_ts(d, p + (uint32_t)(k * 8), at_desc_mn(uV + st * kAtOp + k * 2048), idesc_pv, k != 0);
                 umma_commit(&o_full[st]);
                 umma_commit(&v_empty[st]);
                 umma_commit(&s_empty[st]);
@@ -381,19 +360,19 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                     if (MASKED && wlim < h * 64) {
 #pragma unroll
                         for (int i = 0; i < 16; ++i) pk[i] = 0u;
-                        at_tmem_st16(tS + (uint32_t)(h * 32), pk);
-                        at_tmem_st16(tS + (uint32_t)(h * 32 + 16), pk);
+                        tmem_st_32x16(tS + (uint32_t)(h * 32), pk);
+                        tmem_st_32x16(tS + (uint32_t)(h * 32 + 16), pk);
                         continue;
                     }
                     tmem_ld_32x32(tS + (uint32_t)(h * 64), v0);
                     tmem_ld_32x32(tS + (uint32_t)(h * 64 + 32), v1);
                     tmem_ld_wait();
                     at_exp32<MASKED>(v0, lim - h * 64, scale, -ref, pk, ps);
-                    at_tmem_st16(tS + (uint32_t)(h * 32), pk);
+                    tmem_st_32x16(tS + (uint32_t)(h * 32), pk);
                     at_exp32<MASKED>(v1, lim - h * 64 - 32, scale, -ref, pk, ps);
-                    at_tmem_st16(tS + (uint32_t)(h * 32 + 16), pk);
+                    tmem_st_32x16(tS + (uint32_t)(h * 32 + 16), pk);
                 }
-                at_tmem_st_wait();
+                tmem_st_wait();
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {

@@ -4,6 +4,7 @@
 // none of them knows a model.  `f32` flags select the element type of a buffer: 0 = bf16, 1 = fp32.  Norms, scores,
 // softmax weights, router probabilities, the residual stream and the carried state are fp32 in both modes.
 #pragma once
+#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stddef.h>
 #include <stdint.h>
@@ -26,6 +27,8 @@ struct SimtLinear {
     const int* group_off = nullptr;
     const int* gather = nullptr;
     int epilogue = 0;         // 0 none, 1 relu(x)^2
+    // > 0 (linear_tc.cu, c_f32 = 0): C is three bf16 planes this many elements apart, the result = high + middle + low
+    long long c_terms = 0;
 };
 int launch_simt_linear(const SimtLinear& L, cudaStream_t stream);
 
@@ -105,17 +108,19 @@ struct PagedRows {
     int f32;
     const int* page_table;     // [slots][max_pages]
     int max_pages, page_size;
+    long long rows = 0;        // num_pages * page_size (0: not stated; kernels that read the pool by tensor maps are not taken)
 };
 // qd fp32 [M][heads * (dn + dr) + R + dr] = (queries head by head | latent | rotated key).  RMS-norms the latent (vector
 // weight), rotates the key part and appends both to the paged cache; rotates every head's query part into
 // q_lat[m][head][R .. R + dr) (fp32, row length R + dr).  inv_freq fp32 [rot_dims / 2].
 int launch_latent_post(const SeqIndex& ix, const float* qd, const LatentDims& d, const void* c_norm, int wf32, float eps,
-                       const float* inv_freq, const PagedRows& cache, float* q_lat, cudaStream_t stream);
+                       const float* inv_freq, const PagedRows& cache, float* q_lat, cudaStream_t stream,
+                       __nv_bfloat16* q_terms = nullptr);
 // The same with the queries and the (latent | rotated key) part in buffers of their own: q fp32 rows of ldq floats
 // (heads * (dn + dr) used), kv fp32 rows of ldkv floats (R + dr used).
 int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv,
                              const LatentDims& d, const void* c_norm, int wf32, float eps, const float* inv_freq,
-                             const PagedRows& cache, float* q_lat, cudaStream_t stream);
+                             const PagedRows& cache, float* q_lat, cudaStream_t stream, __nv_bfloat16* q_terms = nullptr);
 // Workspace of the register-tiled kernel when it cuts a long key range into shares (few query rows, long context):
 // o [o_elems] floats, ml [2 * rows] floats; (token, head) pairs x shares must fit `rows`.  tiled = 0 forces the
 // one-warp-per-pair kernel, which takes any latent size; 1 the register-tiled fp32 kernel where the sizes allow; 2 (default)
@@ -131,6 +136,16 @@ struct AttnSplit {
 int launch_latent_attention(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,
                             int max_kv_len, const float* q_lat, const LatentDims& d, const PagedRows& cache,
                             float* out_lat, const AttnSplit& ws, cudaStream_t stream);
+int launch_latent_combine(const float* ws_o, const float* ws_ml, int nsplit, int R, float* out_lat, long long rows,
+                          cudaStream_t stream);
+
+// ------------------------------------------------------------------------------------------- latent_attention_tc.cu
+// The same on tcgen05 for bf16 cache rows, where `takes` says so.  The query comes as three bf16 planes [3][M][heads][R + dr],
+// q = high + middle + low (SimtLinear::c_terms and the q_terms argument of launch_latent_post write them).
+bool latent_attention_tc_takes(const LatentDims& d, const PagedRows& cache, int max_qlen, int tiled);
+int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,
+                               int max_kv_len, const __nv_bfloat16* q_terms, const LatentDims& d, const PagedRows& cache,
+                               float* out_lat, const AttnSplit& ws, int* err, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------- moe.cu
 // Router: probs = softmax(logits) over all E experts (fp32); the `top` largest are kept with their probabilities as

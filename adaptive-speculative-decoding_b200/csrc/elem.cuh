@@ -52,6 +52,15 @@ __device__ __forceinline__ void stx4(void* p, long long i, int f32, const float 
     }
 }
 
+// x as three bf16 terms (24 bits) in planes `plane` elements apart
+__device__ __forceinline__ void store_terms(__nv_bfloat16* dst, long long plane, float x) {
+    const __nv_bfloat16 hi = __float2bfloat16(x);
+    const float r1 = x - __bfloat162float(hi);
+    const __nv_bfloat16 mid = __float2bfloat16(r1);
+    dst[0] = hi;
+    dst[plane] = mid;
+    dst[2 * plane] = __float2bfloat16(r1 - __bfloat162float(mid));
+}
 // two fp32 operations in one instruction (each rounded as its scalar form)
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     unsigned long long d;

@@ -656,6 +656,23 @@ int make_tmap_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t co
     return 0;
 }
 
+// [planes][rows][cols] bf16, contiguous; box = 64 columns x box_rows rows of all planes, 128-byte swizzle
+int make_tmap_bf16_planes(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint32_t planes, uint32_t box_rows) {
+    if (load_encode()) return -1;
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || cols * 2 % 16)
+        return set_error("tensor map: base and row stride must be 16-byte aligned");
+    if (box_rows == 0 || box_rows > 256) return set_error("tensor map: box rows must be in [1, 256]");
+    cuuint64_t gdim[3] = {cols, rows, planes};
+    cuuint64_t gstride[2] = {cols * 2, rows * cols * 2};
+    cuuint32_t box[3] = {(cuuint32_t)kBlockK, box_rows, planes};
+    cuuint32_t estr[3] = {1, 1, 1};
+    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r != CUDA_SUCCESS) return set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
+    return 0;
+}
+
 thread_local NextPrefetch g_gemm_next;   // set by the caller right before gemm_launch, consumed by it (per host thread)
 unsigned long long* g_gemm_trace = nullptr;   // diagnostics buffer [max launches][kTraceCtas][kTraceSlots]
 int g_gemm_trace_max = 0, g_gemm_trace_next = 0;

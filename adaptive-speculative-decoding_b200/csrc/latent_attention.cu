@@ -26,7 +26,7 @@ __device__ __forceinline__ long long cache_row(const PagedRows& c, int slot, int
 
 __global__ void latent_post_kernel(SeqIndex ix, const float* q, long long ldq, const float* kvp, long long ldkv,
                                    LatentDims d, const void* c_norm, int wf32, float eps, const float* inv_freq,
-                                   PagedRows cache, float* q_lat) {
+                                   PagedRows cache, float* q_lat, __nv_bfloat16* q_terms, long long plane) {
     __shared__ float red[33];
     const int m = blockIdx.x;
     const int pos = ix.positions[m], slot = ix.token_slot[m];
@@ -62,8 +62,13 @@ __global__ void latent_post_kernel(SeqIndex ix, const float* q, long long ldq, c
         }
         if (vec == 0)
             stx(cache.pool, crow + d.R + i, cache.f32, out);
-        else
-            q_lat[((long long)m * d.heads + (vec - 1)) * rw + d.R + i] = out;
+        else {
+            const long long at = ((long long)m * d.heads + (vec - 1)) * rw + d.R + i;
+            if (q_terms)
+                store_terms(q_terms + at, plane, out);
+            else
+                q_lat[at] = out;
+        }
     }
 }
 
@@ -385,7 +390,8 @@ __global__ void __launch_bounds__(256, 1) latent_attn_tiled(SeqIndex ix, const i
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Tensor-core form for bf16 cache rows (latent size a multiple of 8 and at most 512, row length a multiple of 16):
+// Tensor-core form for bf16 cache rows (latent size a multiple of 8 and at most 512, row length a multiple of 16) of the calls
+// that latent_attention_tc.cu does not take: few query rows, sizes that are no multiples of its 64 columns:
 // the two products of a tile run as mma.sync m16n8k16 with fp32 accumulation, and the fp32 operand of each (the query
 // in latent space, the softmax weights) enters as a sum of bf16 terms, x = hi + mid + lo with hi = bf16(x), mid =
 // bf16(x - hi), lo = bf16(x - hi - mid): three terms carry all 24 bits of the query, so a score is the same fp32 sum of
@@ -753,8 +759,7 @@ int launch_mma_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int n
     latent_attn_mma<MT><<<grid, 256, smem, stream>>>(ix, cu_q, seq_slot, TQ, HG, nsplit, q_lat, d, cache, out_lat, ws.o, ws.ml);
     count_launch(1);
     if (nsplit > 1) {
-        latent_combine_kernel<<<(unsigned)rows, 128, 0, stream>>>(ws.o, ws.ml, nsplit, d.R, out_lat);
-        count_launch(1);
+        if (launch_latent_combine(ws.o, ws.ml, nsplit, d.R, out_lat, rows, stream)) return -1;
     }
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -824,22 +829,33 @@ int launch_attn_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
 
 }  // namespace
 
+int launch_latent_combine(const float* ws_o, const float* ws_ml, int nsplit, int R, float* out_lat, long long rows,
+                          cudaStream_t stream) {
+    latent_combine_kernel<<<(unsigned)rows, 128, 0, stream>>>(ws_o, ws_ml, nsplit, R, out_lat);
+    count_launch(1);
+    ASD_CUDA(cudaGetLastError());
+    return 0;
+}
+
 int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv,
                              const LatentDims& d, const void* c_norm, int wf32, float eps, const float* inv_freq,
-                             const PagedRows& cache, float* q_lat, cudaStream_t stream) {
+                             const PagedRows& cache, float* q_lat, cudaStream_t stream, __nv_bfloat16* q_terms) {
     if (ix.M <= 0) return 0;
     if (d.rot_dims < 0 || d.rot_dims > d.dr || (d.rot_dims & 1))
         return set_error("latent attention: rot_dims %d must be even and <= %d", d.rot_dims, d.dr);
-    latent_post_kernel<<<ix.M, 128, 0, stream>>>(ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq, cache, q_lat);
+    latent_post_kernel<<<ix.M, 128, 0, stream>>>(ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq, cache, q_lat, q_terms,
+                                               (long long)ix.M * d.heads * (d.R + d.dr));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
 }
 
 int launch_latent_post(const SeqIndex& ix, const float* qd, const LatentDims& d, const void* c_norm, int wf32, float eps,
-                       const float* inv_freq, const PagedRows& cache, float* q_lat, cudaStream_t stream) {
+                       const float* inv_freq, const PagedRows& cache, float* q_lat, cudaStream_t stream,
+                       __nv_bfloat16* q_terms) {
     const int nq = d.heads * (d.dn + d.dr), ld = nq + d.R + d.dr;
-    return launch_latent_post_split(ix, qd, ld, qd + nq, ld, d, c_norm, wf32, eps, inv_freq, cache, q_lat, stream);
+    return launch_latent_post_split(ix, qd, ld, qd + nq, ld, d, c_norm, wf32, eps, inv_freq, cache, q_lat, stream,
+                                    q_terms);
 }
 
 int launch_latent_attention(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,

@@ -20,6 +20,7 @@
 
 #include "asd_internal.h"
 #include "blocks.h"
+#include "elem.cuh"
 #include "ptx.cuh"
 
 namespace asd {
@@ -171,10 +172,14 @@ __global__ void __launch_bounds__(kThreads) tc_linear_kernel(SimtLinear L, int M
                         v = v * v;
                     }
                     TC* dst = C + (long long)(row0 + m) * L.ldc + n;
-                    if constexpr (sizeof(TC) == 4)
+                    if constexpr (sizeof(TC) == 4) {
                         *dst = v;
-                    else
-                        *dst = __float2bfloat16(v);
+                    } else {
+                        if (L.c_terms > 0)
+                            store_terms(dst, L.c_terms, v);
+                        else
+                            *dst = __float2bfloat16(v);
+                    }
                 }
             }
         }

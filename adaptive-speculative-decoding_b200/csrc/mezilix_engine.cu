@@ -110,24 +110,36 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
             if (dense(e, e->hs, ly.wqd, e->qd, M, ly.nqd, D, ly.nqd, l * 8 + 0, s)) return -1;
         }
         const LatentDims dm{c.heads, c.dim, c.rot_dim, c.vdim, c.kv_rank, c.rot_dims, c.window, c.scale};
-        const PagedRows cache{e->pool + ly.cache_off * e->esz, f32, e->page_table, e->max_pages, e->c.page_size};
+        const PagedRows cache{e->pool + ly.cache_off * e->esz, f32,           e->page_table,
+                              e->max_pages,                     e->c.page_size, (long long)e->num_pages * e->c.page_size};
+        // q_lat[m][h][r] = sum_d q[m][h][d] * WukT[h][r][d], in fp32 or as the three bf16 planes the tcgen05 kernel reads
+        SimtLinear ql;
+        ql.a = e->qd, ql.a_f32 = 1, ql.lda = ly.nqd, ql.a_zs = c.dim + c.rot_dim;
+        ql.w = ly.wuk, ql.w_f32 = f32, ql.ldw = c.dim, ql.w_zs = (long long)c.dim * c.kv_rank;
+        ql.c = e->qlat, ql.c_f32 = 1, ql.ldc = (long long)c.heads * ly.rw, ql.c_zs = ly.rw;
+        ql.M = M, ql.N = c.kv_rank, ql.K = c.dim, ql.Z = c.heads;
+        __nv_bfloat16* q_terms = nullptr;
+        if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
+            latent_attention_tc_takes(dm, cache, max_qlen, e->attn_ws.tiled)) {
+            q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
+            ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
+        }
         {
             MZ_PROF(MZ_GLUE);
-            if (launch_latent_post(ix, e->qd, dm, ly.latent_gain, f32, e->c.eps, ly.inv_freq, cache, e->qlat, s)) return -1;
+            if (launch_latent_post(ix, e->qd, dm, ly.latent_gain, f32, e->c.eps, ly.inv_freq, cache, e->qlat, s,
+                                   q_terms))
+                return -1;
         }
-        {   // q_lat[m][h][r] = sum_d q[m][h][d] * WukT[h][r][d]
+        {
             MZ_PROF(MZ_HEADS);
-            SimtLinear L;
-            L.a = e->qd, L.a_f32 = 1, L.lda = ly.nqd, L.a_zs = c.dim + c.rot_dim;
-            L.w = ly.wuk, L.w_f32 = f32, L.ldw = c.dim, L.w_zs = (long long)c.dim * c.kv_rank;
-            L.c = e->qlat, L.c_f32 = 1, L.ldc = (long long)c.heads * ly.rw, L.c_zs = ly.rw;
-            L.M = M, L.N = c.kv_rank, L.K = c.dim, L.Z = c.heads;
-            if (linear(e, L, s)) return -1;
+            if (linear(e, ql, s)) return -1;
         }
         {
             MZ_PROF(MZ_ATTN);
-            if (launch_latent_attention(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qlat, dm, cache, e->olat,
-                                        e->attn_ws, s))
+            if (q_terms ? launch_latent_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache,
+                                                     e->olat, e->attn_ws, e->dev_error, s)
+                        : launch_latent_attention(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qlat, dm, cache,
+                                                  e->olat, e->attn_ws, s))
                 return -1;
         }
         {   // v[m][h][:] = Wuv[h] * out_lat[m][h][:]
@@ -253,7 +265,7 @@ asd_mezilix_engine_t* asd_mezilix_create(const asd_mezilix_config* cfg, const as
     rc |= dev_alloc(e, &e->xavg, MT * D);
     rc |= dev_alloc(e, &e->hn, MT * D);
     rc |= dev_alloc(e, &e->qd, MT * nqd);
-    rc |= dev_alloc(e, &e->qlat, MT * qlat);
+    rc |= dev_alloc(e, &e->qlat, (MT * qlat * 3 + 1) / 2);      // fp32, or three bf16 planes
     rc |= dev_alloc(e, &e->olat, MT * olat);
     rc |= dev_alloc(e, &e->mix, MT * D);
     rc |= dev_alloc(e, &e->rlog, MT * E);

@@ -130,26 +130,35 @@ static int mix_latent(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
     }
     LatentDims dm{c.heads, c.dim, c.rot_dim, c.vdim, c.kv_rank, c.rot_dims, c.window, c.scale};
     dm.interleaved = c.rot_interleaved;
-    const PagedRows cache{e->pool + run.cache_off * e->esz, f32, e->page_table, e->max_pages, e->c.page_size};
+    const PagedRows cache{e->pool + run.cache_off * e->esz, f32,           e->page_table,
+                          e->max_pages,                     e->c.page_size, (long long)e->num_pages * e->c.page_size};
+    // q_lat[m][h][r] = sum_d q[m][h][d] * WukT[h][r][d], in fp32 or as the three bf16 planes the tcgen05 kernel reads
+    SimtLinear ql;
+    ql.a = e->qbuf, ql.a_f32 = 1, ql.lda = nq, ql.a_zs = c.dim + c.rot_dim;
+    ql.w = ly.w("w_uk"), ql.w_f32 = f32, ql.ldw = c.dim, ql.w_zs = (long long)c.dim * c.kv_rank;
+    ql.c = e->qlat, ql.c_f32 = 1, ql.ldc = (long long)c.heads * rw, ql.c_zs = rw;
+    ql.M = M, ql.N = c.kv_rank, ql.K = c.dim, ql.Z = c.heads;
+    __nv_bfloat16* q_terms = nullptr;
+    if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) && latent_attention_tc_takes(dm, cache, b.max_qlen, e->attn_ws.tiled)) {
+        q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
+        ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
+    }
     {
         RV_PROF(RV_GLUE);
         if (launch_latent_post_split(b.ix, e->qbuf, nq, e->proj + c.q_rank, ly.n_in, dm, ly.f("kv_norm"), 1, e->c.eps,
-                                     ly.freq_k, cache, e->qlat, s))
+                                     ly.freq_k, cache, e->qlat, s, q_terms))
             return -1;
     }
-    {   // q_lat[m][h][r] = sum_d q[m][h][d] * WukT[h][r][d]
+    {
         RV_PROF(RV_HEADS);
-        SimtLinear L;
-        L.a = e->qbuf, L.a_f32 = 1, L.lda = nq, L.a_zs = c.dim + c.rot_dim;
-        L.w = ly.w("w_uk"), L.w_f32 = f32, L.ldw = c.dim, L.w_zs = (long long)c.dim * c.kv_rank;
-        L.c = e->qlat, L.c_f32 = 1, L.ldc = (long long)c.heads * rw, L.c_zs = rw;
-        L.M = M, L.N = c.kv_rank, L.K = c.dim, L.Z = c.heads;
-        if (linear(e, L, s)) return -1;
+        if (linear(e, ql, s)) return -1;
     }
     {
         RV_PROF(RV_LATENT_ATTN);
-        if (launch_latent_attention(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qlat, dm, cache, e->olat,
-                                    e->attn_ws, s))
+        if (q_terms ? launch_latent_attention_tc(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, q_terms, dm, cache,
+                                                 e->olat, e->attn_ws, e->dev_error, s)
+                    : launch_latent_attention(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qlat, dm, cache,
+                                              e->olat, e->attn_ws, s))
             return -1;
     }
     {   // v[m][h][:] = Wuv[h] * out_lat[m][h][:]
@@ -407,7 +416,7 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     rc |= dev_alloc(e, &e->y, MT * D);
     rc |= dev_alloc(e, &e->proj, MT * n_in);
     rc |= dev_alloc(e, &e->qbuf, MT * nq);
-    rc |= dev_alloc(e, &e->qlat, MT * qlat);
+    rc |= dev_alloc(e, &e->qlat, (MT * qlat * 3 + 1) / 2);      // fp32, or three bf16 planes
     rc |= dev_alloc(e, &e->olat, MT * olat);
     rc |= dev_alloc(e, &e->alpha, MT * nk);
     rc |= dev_alloc(e, &e->orec, MT * hv);

@@ -546,3 +546,56 @@ def test_trace_replay_command_on_a_checkpoint_directory(tmp_path, dtype):
     for step, ref in want.items():
         got = torch.from_numpy(np.fromfile(out / f"{step}.f32", dtype="<f4").reshape(ref.shape[0], -1).copy())
         assert rel_err(got, ref)[1] < tol, step
+
+
+@pytest.mark.parametrize("heads,kv_rank,rot_dim,window,page_size,scale,portions", [
+    (16, 512, 64, 1 << 20, 16, 0.3, [130, 1, 8, 9, 300, 1, 2, 250, 1]),      # two halves of the result, shares of the keys
+    (16, 512, 64, 200, 16, 2.0, [7, 400, 1, 129, 1, 64]),                    # a window inside the prompt, a sharp softmax
+    (3, 64, 64, 1000, 8, 0.5, [42, 43, 84, 1, 300]),                         # heads that do not divide the 128 rows
+    (130, 128, 128, 90, 32, 0.2, [100, 1, 30]),                              # more heads than rows: two head groups
+    (1, 384, 64, 500, 128, 1.0, [128, 129, 1, 200]),                         # one head, halves of 192 columns, one page a tile
+    (32, 256, 64, 1 << 20, 64, 0.1, [1, 1, 3, 257, 1, 1]),                   # single tokens of many heads
+])
+def test_latent_attention_on_tcgen05(heads, kv_rank, rot_dim, window, page_size, scale, portions):
+    """bf16 engine: the tcgen05 kernel against the fp32 CUDA-core kernel of the same engine, both held to the oracle; the pool
+    starts out as NaN, none of which may reach a result"""
+    cfg = config([layer(heads=heads, dim=16, rot_dim=rot_dim, vdim=16, kv_rank=kv_rank, window=window, scale=scale, experts=0)],
+                 width=64)
+    w = O.random_model(cfg, seed=51, scale=1.5)
+    n = sum(portions)
+    ids = tokens(n, 96, 52)
+    ref, _ = O.forward(cfg, w, ids)
+    outs = []
+    for mode in (2, 1):
+        eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512, max_seq_len=1024, page_size=page_size)
+        eng.set_option("attn_tiled", mode)
+        if mode == 2:
+            eng.cache_pool.fill_(255)
+        outs.append(feed(eng, eng.open_sequence(), ids, portions).cpu())
+        eng.check_device()
+        close(eng)
+    assert torch.isfinite(outs[0]).all()
+    e_tc, e_fp32 = rel_err(outs[0], ref)[0], rel_err(outs[1], ref)[0]
+    assert e_fp32 < 4e-2 and e_tc < 1.1 * e_fp32 + 1e-4, (e_tc, e_fp32)
+
+
+def test_latent_attention_on_tcgen05_unequal_prompts():
+    """three prompts of unequal length and single tokens of other sequences in one forward"""
+    cfg = config([layer(heads=16, dim=16, rot_dim=64, vdim=16, kv_rank=512, window=150, scale=0.5, experts=0)], width=64)
+    w = O.random_model(cfg, seed=53, scale=1.5)
+    lens = [300, 1, 77]
+    ids = [tokens(n + 1, 96, 54 + n) for n in lens]
+    refs = [O.forward(cfg, w, t)[0] for t in ids]
+    eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512, max_seq_len=512, max_seqs=4)
+    slots = [eng.open_sequence() for _ in lens]
+    for s, n in zip(slots, lens):
+        eng.reserve(s, n + 1)
+    got = eng.forward_ragged([(s, 0, t[:n], list(range(n))) for s, t, n in zip(slots, ids, lens)]).cpu()
+    step = eng.forward_ragged([(s, n, t[n:], [0]) for s, t, n in zip(slots, ids, lens)]).cpu()
+    eng.check_device()
+    at = 0
+    for i, n in enumerate(lens):
+        assert rel_err(got[at:at + n], refs[i][:n])[0] < 4e-2
+        assert rel_err(step[i:i + 1], refs[i][n:])[0] < 4e-2
+        at += n
+    close(eng)
