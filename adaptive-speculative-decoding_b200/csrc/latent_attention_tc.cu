@@ -19,8 +19,8 @@
 //     below 2^8 and the sums exact in fp32.
 //   * A thread needs ~200 clocks to wait for a barrier and issue one box or four products, so boxes are as large as the
 //     layout allows, a query slot feeds twelve products, three warps load, and the issuing warp walks its loops whole (a
-//     first form with 16 KB slots, one loader and one issuing thread took 666 us where this one takes 400).
-// Four prompts of 1024 tokens, 16 heads, latent 512 + 64: 1350 us on mma.sync, 400 here (185 GFLOP: 0.46 PFLOP/s).
+//     first form with 16 KB slots, one loader and one issuing thread took 666 us where this one takes 366).
+// Four prompts of 1024 tokens, 16 heads, latent 512 + 64: 1350 us on mma.sync, 366 here (185 GFLOP: 0.5 PFLOP/s).
 // Every wait is bounded: on expiry the kernel raises the caller's error flag, lets its copies land, frees its TMEM and ends.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -49,8 +49,8 @@ constexpr int kLtMaxV = 4;                 // chunks of 64 result columns per CT
 constexpr float kLtSlack = 8.0f;           // log2 growth of a row maximum that the weights tolerate before a rescale
 constexpr uint32_t kLtSpin = 1u << 20;
 // Query rows of a tile from which this kernel is the better one.  A tile costs what 128 rows cost, however many are real:
-// 64 single tokens of 32 heads at 1024 positions: 146 us on mma.sync, 117 us here; 16 of 16 heads at 1500: 58 us there, 72
-// here (4096 prompt tokens of 16 heads, 128 rows a tile: 1350 and 400).
+// 64 single tokens of 32 heads at 1024 positions: 146 us on mma.sync, 111 us here; 16 of 16 heads at 1500: 58 us there, 72
+// here (4096 prompt tokens of 16 heads, 128 rows a tile: 1350 and 366).
 constexpr int kLtMinRows = 32;
 
 struct LtArgs {
@@ -479,11 +479,15 @@ __global__ void __launch_bounds__(kLtThreads, 1)
             }
             __syncwarp();
             const unsigned live = __ballot_sync(0xffffffffu, real);
+            float* const to = direct ? a.out_lat : a.ws_o;
+            const long long at = (direct ? row : row * a.nsplit + split) * a.R + part * vcols;
+            const int q4 = vcols / 4;                          // at most 64
+#pragma unroll 8
             for (int r = 0; r < 32; ++r) {
-                const long long at = __shfl_sync(0xffffffffu, row, r);
-                if (!(live >> r & 1)) continue;
-                float* dst = (direct ? a.out_lat + at * a.R : a.ws_o + (at * a.nsplit + split) * a.R) + part * vcols;
-                for (int c = lane; c < vcols / 4; c += 32) reinterpret_cast<float4*>(dst)[c] = own[r * ld + c];
+                float4* dst = reinterpret_cast<float4*>(to + __shfl_sync(0xffffffffu, at, r));
+                const bool put = live >> r & 1;
+                if (put && lane < q4) dst[lane] = own[r * ld + lane];
+                if (put && lane + 32 < q4) dst[lane + 32] = own[r * ld + lane + 32];
             }
             if (real && !direct && part == 0) {
                 a.ws_ml[(row * a.nsplit + split) * 2] = ref * 0.69314718055994531f;    // natural units, as the merge expects
