@@ -19,6 +19,23 @@ void count_launch(int n);
             return ::asd::set_error("%s failed: %s (%s:%d)", #expr, cudaGetErrorString(_e), __FILE__, __LINE__); \
     } while (0)
 
+// Programmatic launch: the grid may become resident while its predecessor drains.  Only for kernels that begin with
+// pdl_enter() or otherwise wait (griddepcontrol.wait) before they touch memory.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Every kernel of a forward pass asks for the same (maximum) shared-memory carve-out: an SM only re-partitions
 // L1/shared memory when it is idle, so kernels with different carve-outs cannot be co-resident and a
 // programmatically launched GEMM could not start streaming weights next to the attention CTAs.

@@ -47,7 +47,7 @@ struct DenseRunner {
             }
             if (M >= tc_min_rows)
                 return gemm_tc_launch(it->second.big, it->second.tw, it->second.tx, y, ldc, N, 0, false, s, false, nullptr);
-            return gemm_launch(it->second.pl, it->second.tw, it->second.tx, y, ldc, N, false, s, false);
+            return gemm_launch(it->second.pl, it->second.tw, it->second.tx, y, ldc, N, true, s, false);
         }
         SimtLinear L;
         L.a = x, L.a_f32 = f32, L.lda = K;

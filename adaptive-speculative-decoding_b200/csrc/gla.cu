@@ -14,6 +14,7 @@
 #include "asd_internal.h"
 #include "blocks.h"
 #include "elem.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -35,6 +36,7 @@ constexpr int GD_TOK = 32, GD_CH = 256;   // tokens x channels per CTA of the de
 // reads as broadcasts.
 __global__ void __launch_bounds__(GD_CH) gla_decay_kernel(const float* a, long long lda, const float* w_decay,
                                                           const float* b_decay, GlaDims d, float* alpha, int M) {
+    pdl_enter();
     extern __shared__ float sm[];
     float* wT = sm;                      // [low][GD_CH]
     float* av = sm + d.low * GD_CH;      // [GD_TOK][low]
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) gla_recurrence_kern
                                                             const float* q, const float* k, const float* v, long long ld,
                                                             const float* alpha, GlaDims d, float* state, int ring,
                                                             float* out) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * 32;
     const int t0 = cu_q[seq], t1 = cu_q[seq + 1];
@@ -188,6 +191,7 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) gla_recurrence_kern
 
 __global__ void gla_out_kernel(const float* o, const float* gate, long long ldg, const float* w, float eps, void* y,
                                int of32, int heads, int dv) {
+    pdl_enter();
     // one warp per (token, head)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int h = blockIdx.y * (blockDim.x >> 5) + warp;
@@ -217,7 +221,7 @@ int launch_gla_decay(const float* a, long long lda, const float* w_decay, const 
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     dim3 grid((d.heads * d.dk + GD_CH - 1) / GD_CH, (M + GD_TOK - 1) / GD_TOK);
     if (grid.y > 65535) return set_error("gla: too many tokens");
-    gla_decay_kernel<<<grid, GD_CH, smem, stream>>>(a, lda, w_decay, b_decay, d, alpha, M);
+    ASD_CUDA(launch_pdl(gla_decay_kernel, grid, GD_CH, smem, stream, a, lda, w_decay, b_decay, d, alpha, M));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -243,7 +247,7 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
         auto fn = gla_recurrence_kernel<R, T, C>;                                                                        \
         static PerDeviceOnce once;                                                                                    \
         if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
-        fn<<<grid, RS * 32, smem, stream>>>(ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out);             \
+        ASD_CUDA(launch_pdl(fn, grid, RS * 32, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out));             \
     }
     if (RS > 8) ASD_GLA_CASE(32, 1024, GLA_CH / 4)
     else if (rows == 4) ASD_GLA_CASE(4, 256, GLA_CH)
@@ -261,7 +265,7 @@ int launch_gla_out(const float* o, const float* gate, long long ldg, const float
     if (M <= 0) return 0;
     const int wpb = heads < 8 ? heads : 8;
     dim3 grid(M, (heads + wpb - 1) / wpb);
-    gla_out_kernel<<<grid, wpb * 32, 0, stream>>>(o, gate, ldg, w, eps, y, of32, heads, dv);
+    ASD_CUDA(launch_pdl(gla_out_kernel, grid, wpb * 32, 0, stream, o, gate, ldg, w, eps, y, of32, heads, dv));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;

@@ -14,6 +14,7 @@
 #include "asd_internal.h"
 #include "blocks.h"
 #include "elem.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -27,6 +28,7 @@ __device__ __forceinline__ long long cache_row(const PagedRows& c, int slot, int
 __global__ void latent_post_kernel(SeqIndex ix, const float* q, long long ldq, const float* kvp, long long ldkv,
                                    LatentDims d, const void* c_norm, int wf32, float eps, const float* inv_freq,
                                    PagedRows cache, float* q_lat, __nv_bfloat16* q_terms, long long plane) {
+    pdl_enter();
     __shared__ float red[33];
     const int m = blockIdx.x;
     const int pos = ix.positions[m], slot = ix.token_slot[m];
@@ -76,6 +78,7 @@ template <typename T, int ACC>   // ACC = ceil(R / 32) accumulators per lane
 __global__ void __launch_bounds__(512) latent_attn_kernel(SeqIndex ix, const int* cu_q, const int* seq_slot, int TQ,
                                                           int HG, const float* q_lat, LatentDims d, PagedRows cache,
                                                           float* out_lat) {
+    pdl_enter();
     extern __shared__ float smem[];
     const int rw = d.R + d.dr, LD = rw | 1;          // odd row stride: lanes reading one column hit 32 banks
     float* ks = smem;                                 // [32][LD]
@@ -184,6 +187,7 @@ template <typename T, int RPT, int RC>
 __global__ void __launch_bounds__(256, 1) latent_attn_tiled(SeqIndex ix, const int* cu_q, const int* seq_slot, int TQ,
                                                             int HG, int nsplit, int vec, const float* q_lat, LatentDims d,
                                                             PagedRows cache, float* out_lat, float* ws_o, float* ws_ml) {
+    pdl_enter();
     constexpr int QT = 4 * RPT, KT = 32, RW = QT / 8;
     extern __shared__ float smem[];
     const int rw = d.R + d.dr, LD = rw + 4;
@@ -430,6 +434,7 @@ template <int MT>   // 16-row tiles per CTA: 1 (few rows: decode) or 2 (prompts:
 __global__ void __launch_bounds__(256, 1) latent_attn_mma(SeqIndex ix, const int* cu_q, const int* seq_slot, int TQ, int HG,
                                                           int nsplit, const float* q_lat, LatentDims d, PagedRows cache,
                                                           float* out_lat, float* ws_o, float* ws_ml) {
+    pdl_enter();
     constexpr int QT = 16 * MT, KT = 64, NTW = 8, RW = 2 * MT;                  // NTW: 8-wide latent tiles per warp (R <= 512)
     extern __shared__ __align__(16) uint8_t smem_b[];
     const int rw = d.R + d.dr, LDK = rw + 8;                  // bf16 elements per staged row (16-byte multiple)
@@ -664,6 +669,7 @@ __global__ void __launch_bounds__(256, 1) latent_attn_mma(SeqIndex ix, const int
 
 // out[row] = sum_s o_s exp(m_s - m) / sum_s l_s exp(m_s - m) over the shares of one (token, head)
 __global__ void latent_combine_kernel(const float* ws_o, const float* ws_ml, int nsplit, int R, float* out_lat) {
+    pdl_enter();
     const long long row = blockIdx.x;
     float m = -INFINITY;
     for (int s = 0; s < nsplit; ++s) m = fmaxf(m, ws_ml[(row * nsplit + s) * 2]);
@@ -716,10 +722,11 @@ int launch_tiled_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int
     ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid(q_tiles, nseq * nsplit, hgs);
     const int vec = sizeof(T) == 2 && (rw & 7) == 0 && (reinterpret_cast<uintptr_t>(cache.pool) & 15) == 0;
-    fn<<<grid, 256, smem, stream>>>(ix, cu_q, seq_slot, TQ, HG, nsplit, vec, q_lat, d, cache, out_lat, ws.o, ws.ml);
+    ASD_CUDA(launch_pdl(fn, grid, 256, smem, stream, ix, cu_q, seq_slot, TQ, HG, nsplit, vec, q_lat, d, cache, out_lat,
+                        ws.o, ws.ml));
     count_launch(1);
     if (nsplit > 1) {
-        latent_combine_kernel<<<(unsigned)rows, 128, 0, stream>>>(ws.o, ws.ml, nsplit, d.R, out_lat);
+        ASD_CUDA(launch_pdl(latent_combine_kernel, (unsigned)rows, 128, 0, stream, ws.o, ws.ml, nsplit, d.R, out_lat));
         count_launch(1);
     }
     ASD_CUDA(cudaGetLastError());
@@ -756,7 +763,8 @@ int launch_mma_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int n
     }
     ASD_CUDA(cudaFuncSetAttribute(latent_attn_mma<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid(q_tiles, nseq * nsplit, hgs);
-    latent_attn_mma<MT><<<grid, 256, smem, stream>>>(ix, cu_q, seq_slot, TQ, HG, nsplit, q_lat, d, cache, out_lat, ws.o, ws.ml);
+    ASD_CUDA(launch_pdl(latent_attn_mma<MT>, grid, 256, smem, stream, ix, cu_q, seq_slot, TQ, HG, nsplit, q_lat, d, cache,
+                        out_lat, ws.o, ws.ml));
     count_launch(1);
     if (nsplit > 1) {
         if (launch_latent_combine(ws.o, ws.ml, nsplit, d.R, out_lat, rows, stream)) return -1;
@@ -812,7 +820,7 @@ int launch_attn_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
     {                                                                                                                \
         auto fn = latent_attn_kernel<T, A>;                                                                          \
         if (smem > 48 * 1024) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
-        fn<<<grid, warps * 32, smem, stream>>>(ix, cu_q, seq_slot, TQ, HG, q_lat, d, cache, out_lat);                \
+        ASD_CUDA(launch_pdl(fn, grid, warps * 32, smem, stream, ix, cu_q, seq_slot, TQ, HG, q_lat, d, cache, out_lat));                \
     }
     if (smem > 220 * 1024) return set_error("latent attention: latent + rotated size %d does not fit shared memory", rw);
     if (acc <= 2) ASD_LAT_CASE(2)
@@ -831,7 +839,7 @@ int launch_attn_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
 
 int launch_latent_combine(const float* ws_o, const float* ws_ml, int nsplit, int R, float* out_lat, long long rows,
                           cudaStream_t stream) {
-    latent_combine_kernel<<<(unsigned)rows, 128, 0, stream>>>(ws_o, ws_ml, nsplit, R, out_lat);
+    ASD_CUDA(launch_pdl(latent_combine_kernel, (unsigned)rows, 128, 0, stream, ws_o, ws_ml, nsplit, R, out_lat));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -843,8 +851,9 @@ int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, 
     if (ix.M <= 0) return 0;
     if (d.rot_dims < 0 || d.rot_dims > d.dr || (d.rot_dims & 1))
         return set_error("latent attention: rot_dims %d must be even and <= %d", d.rot_dims, d.dr);
-    latent_post_kernel<<<ix.M, 128, 0, stream>>>(ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq, cache, q_lat, q_terms,
-                                               (long long)ix.M * d.heads * (d.R + d.dr));
+    ASD_CUDA(launch_pdl(latent_post_kernel, ix.M, 128, 0, stream, ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq,
+                        cache, q_lat, q_terms,
+                                               (long long)ix.M * d.heads * (d.R + d.dr)));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;

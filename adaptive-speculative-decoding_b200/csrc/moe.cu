@@ -9,6 +9,7 @@
 #include "asd_internal.h"
 #include "blocks.h"
 #include "elem.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -115,6 +116,7 @@ __device__ void choose_experts(const float* z, int E, const RouteChoice& c, floa
 __global__ void moe_route_kernel(const float* logits, const void* x, int xf32, const void* wr, int wf32, int D, float* z_out,
                                  int M, int E, int zld, RouteChoice c, int* expert_of, float* gate, int* counts,
                                  const float* bias) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int m = blockIdx.x * (blockDim.x >> 5) + warp;
@@ -153,6 +155,7 @@ __global__ void moe_route_kernel(const float* logits, const void* x, int xf32, c
 __global__ void __launch_bounds__(256) moe_route_small_kernel(const float* logits, int M, int E, int zld, RouteChoice c,
                                                               int* expert_of, float* gate, int* group_off, int* sorted_tok,
                                                               int* slot_of) {
+    pdl_enter();
     extern __shared__ float sm[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5, top = c.top;
     const int per = E + (c.groups > 1 ? c.groups : 0);
@@ -195,6 +198,7 @@ __global__ void __launch_bounds__(256) moe_route_small_kernel(const float* logit
 template <int NJ, int NTOK>
 __global__ void __launch_bounds__(128) moe_logits_kernel(const void* x, int xf32, const void* wr, int wf32, int D, int M, int E,
                                                          int rows, float* z_out, const float* bias, int vec) {
+    pdl_enter();
     __shared__ float red[4][NTOK][NJ];
     const int m0 = blockIdx.x * NTOK, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int e0 = 0; e0 < rows; e0 += NJ) {
@@ -246,6 +250,7 @@ __global__ void __launch_bounds__(128) moe_logits_kernel(const void* x, int xf32
 }
 
 __global__ void moe_offsets_kernel(int* counters, int* group_off, int E) {
+    pdl_enter();
     if (threadIdx.x == 0) {
         int o = 0;
         for (int e = 0; e < E; ++e) {
@@ -259,6 +264,7 @@ __global__ void moe_offsets_kernel(int* counters, int* group_off, int E) {
 
 __global__ void moe_scatter_kernel(const int* expert_of, int n, int top, int E, const int* group_off, int* counters,
                                    int* sorted_tok, int* slot_of, const float* gate, float* slot_gate) {
+    pdl_enter();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int e = expert_of[i];
@@ -272,8 +278,8 @@ template <int NJ, int NTOK>
 void launch_logits_as(const MoeRouterInput& in, int M, int E, int rows, cudaStream_t stream) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(in.x) | reinterpret_cast<uintptr_t>(in.w);
     const int vec = in.D % 4 == 0 && (at & 15) == 0;
-    moe_logits_kernel<NJ, NTOK><<<(M + NTOK - 1) / NTOK, 128, 0, stream>>>(in.x, in.x_f32, in.w, in.w_f32, in.D, M, E, rows,
-                                                                         in.logits_out, in.bias, vec);
+    launch_pdl(moe_logits_kernel<NJ, NTOK>, (M + NTOK - 1) / NTOK, 128, 0, stream, in.x, in.x_f32, in.w, in.w_f32, in.D, M, E,
+               rows, in.logits_out, in.bias, vec);
 }
 // the passes over a token's row are few and even
 void launch_logits(const MoeRouterInput& in, int M, int E, int rows, cudaStream_t stream) {
@@ -310,8 +316,9 @@ int launch_moe_route(const float* logits, const MoeRouterInput* in, int M, int E
     const size_t small_smem = (size_t)(8 * (E + (c.groups > 1 ? c.groups : 0)) + 2 * E + 1) * sizeof(float);
     if (in && in->logits_out && (long long)M * top <= 4096 && small_smem <= 48 * 1024) {
         launch_logits(*in, M, E, zld, stream);
-        moe_route_small_kernel<<<1, 256, small_smem, stream>>>(in->logits_out, M, E, zld, c, expert_of, gate, group_off,
-                                                               sorted_tok, slot_of);
+        ASD_CUDA(launch_pdl(moe_route_small_kernel, 1, 256, small_smem, stream, in->logits_out, M, E, zld, c, expert_of,
+                            gate, group_off,
+                                                               sorted_tok, slot_of));
         count_launch(2);
         ASD_CUDA(cudaGetLastError());
         return 0;
@@ -323,13 +330,14 @@ int launch_moe_route(const float* logits, const MoeRouterInput* in, int M, int E
         logits = in->logits_out;
         in = nullptr;
     }
-    moe_route_kernel<<<(M + 3) / 4, 128, (size_t)E * 8 * sizeof(float), stream>>>(
+    ASD_CUDA(launch_pdl(moe_route_kernel, (M + 3) / 4, 128, (size_t)E * 8 * sizeof(float), stream,
         logits, in ? in->x : nullptr, in ? in->x_f32 : 0, in ? in->w : nullptr, in ? in->w_f32 : 0, in ? in->D : 0,
-        nullptr, M, E, zld, c, expert_of, gate, counters, in ? in->bias : nullptr);
-    moe_offsets_kernel<<<1, 32, 0, stream>>>(counters, group_off, E);
+        nullptr, M, E, zld, c, expert_of, gate, counters, in ? in->bias : nullptr));
+    ASD_CUDA(launch_pdl(moe_offsets_kernel, 1, 32, 0, stream, counters, group_off, E));
     const int n = M * top;
-    moe_scatter_kernel<<<(n + 255) / 256, 256, 0, stream>>>(expert_of, n, top, E, group_off, counters, sorted_tok, slot_of,
-                                                            gate, c.slot_gate);
+    ASD_CUDA(launch_pdl(moe_scatter_kernel, (n + 255) / 256, 256, 0, stream, expert_of, n, top, E, group_off, counters,
+                        sorted_tok, slot_of,
+                                                            gate, c.slot_gate));
     count_launch(3);
     ASD_CUDA(cudaGetLastError());
     return 0;

@@ -9,6 +9,7 @@
 #include "asd_internal.h"
 #include "blocks.h"
 #include "elem.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -17,6 +18,7 @@ namespace {
 inline int row_threads(int D) { return D >= 2048 ? 512 : (D >= 1024 ? 256 : (D >= 256 ? 128 : 64)); }
 
 __global__ void embed_scaled_kernel(SeqIndex ix, const void* embed, int wf32, float scale, float* x0, float* x, int D) {
+    pdl_enter();
     const int m = blockIdx.x;
     const long long src = (long long)ix.tokens[m] * D, dst = (long long)m * D;
     for (int d = threadIdx.x; d < D; d += blockDim.x) {
@@ -30,6 +32,7 @@ __global__ void embed_scaled_kernel(SeqIndex ix, const void* embed, int wf32, fl
 // brought into one turn in fp64, so that a far position's angle is as exact as a near one's.
 __global__ void embed_sinusoid_kernel(SeqIndex ix, const void* embed, int wf32, float scale, const double* freq, float* x,
                                       int D) {
+    pdl_enter();
     const int m = blockIdx.x;
     const long long src = (long long)ix.tokens[m] * D, dst = (long long)m * D;
     const double pos = (double)ix.positions[m];
@@ -78,6 +81,7 @@ __device__ __forceinline__ void storevx(void* p, long long i, int f32, const flo
 // consecutive elements per thread and step: 4 where width, norm groups and addresses allow, else 1.
 template <int V>
 __global__ void row_close_kernel(RowClose c) {
+    pdl_enter();
     extern __shared__ __align__(16) float sm[];
     float* row = sm;
     float* red = sm + c.D;
@@ -188,6 +192,7 @@ __global__ void row_close_kernel(RowClose c) {
 // over the grid, V consecutive ones per thread.
 template <int V>
 __global__ void tanh_close_kernel(TanhClose c) {
+    pdl_enter();
     const int m = blockIdx.x, d = (blockIdx.y * blockDim.x + threadIdx.x) * V, D = c.D;
     if (d >= D) return;
     const long long base = (long long)m * D + d;
@@ -224,6 +229,7 @@ __global__ void tanh_close_kernel(TanhClose c) {
 // x[m] = group_norm(embed[token]) * w, fp32 (dynamic shared memory as row_close_kernel)
 __global__ void embed_normed_kernel(SeqIndex ix, const void* embed, int wf32, const float* w, int groups, float eps, float* x,
                                     int D) {
+    pdl_enter();
     extern __shared__ float sm[];
     float* row = sm;
     float* red = sm + D;
@@ -249,6 +255,7 @@ __device__ __forceinline__ float gelu_tanh_f(float z) {
 // out[r][f] = gelu_tanh(z[r][f]) (mode 0, z rows of F floats) or silu(z[r][f]) * z[r][F + f] (mode 1, rows of 2 F)
 // mode 2: relu(z[r][f])^2.  bias (optional) is added to z first: [F], or [2 F] in mode 1.
 __global__ void ff_act_kernel(const float* z, void* out, int of32, long long n, int F, int mode, const float* bias) {
+    pdl_enter();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     if (mode != 1) {
@@ -272,6 +279,7 @@ __global__ void ff_act_kernel(const float* z, void* out, int of32, long long n, 
 // gated activations: z rows of 2 F floats (gate half, then up half), V consecutive results per thread
 template <int V>
 __global__ void gated_act_kernel(const float* z, void* out, int of32, long long rows, int F, GatedAct p) {
+    pdl_enter();
     const int per = F / V;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= rows * per) return;
@@ -296,6 +304,7 @@ __global__ void gated_act_kernel(const float* z, void* out, int of32, long long 
 
 __global__ void rms_rows_kernel(const float* in, long long ld_in, const float* w, int plus_one, float eps, void* out,
                                 int of32, long long ld_out, int n) {
+    pdl_enter();
     __shared__ float red[33];
     const float* src = in + (long long)blockIdx.x * ld_in;
     float ss = 0.f;
@@ -307,6 +316,7 @@ __global__ void rms_rows_kernel(const float* in, long long ld_in, const float* w
 
 // dynamic shared memory: the row (F floats, if it fits: `staged`) + 33 for the block sums
 __global__ void polynorm_kernel(const float* z, const float* coeff, float eps, void* out, int of32, int F, int staged) {
+    pdl_enter();
     extern __shared__ float sm[];
     float* red = sm;
     float* row = sm + 33;
@@ -332,6 +342,7 @@ __global__ void polynorm_kernel(const float* z, const float* coeff, float eps, v
 }
 
 __global__ void softcap_kernel(float* logits, long long ld, int V, float cap) {
+    pdl_enter();
     float* row = logits + (long long)blockIdx.x * ld;
     const int i = blockIdx.y * blockDim.x + threadIdx.x;
     if (i < V) row[i] = cap * tanhf(row[i] / cap);
@@ -342,7 +353,7 @@ __global__ void softcap_kernel(float* logits, long long ld, int V, float cap) {
 int launch_embed_scaled(const SeqIndex& ix, const void* embed, int wf32, float scale, float* x0, float* x, int D,
                         cudaStream_t stream) {
     if (ix.M <= 0) return 0;
-    embed_scaled_kernel<<<ix.M, row_threads(D), 0, stream>>>(ix, embed, wf32, scale, x0, x, D);
+    ASD_CUDA(launch_pdl(embed_scaled_kernel, ix.M, row_threads(D), 0, stream, ix, embed, wf32, scale, x0, x, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -351,7 +362,7 @@ int launch_embed_scaled(const SeqIndex& ix, const void* embed, int wf32, float s
 int launch_embed_sinusoid(const SeqIndex& ix, const void* embed, int wf32, float scale, const double* freq, float* x, int D,
                           cudaStream_t stream) {
     if (ix.M <= 0) return 0;
-    embed_sinusoid_kernel<<<ix.M, row_threads(D), 0, stream>>>(ix, embed, wf32, scale, freq, x, D);
+    ASD_CUDA(launch_pdl(embed_sinusoid_kernel, ix.M, row_threads(D), 0, stream, ix, embed, wf32, scale, freq, x, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -378,9 +389,9 @@ int launch_row_close(const RowClose& c, cudaStream_t stream) {
                           (const void*)c.post_w2, (const void*)c.ff, (const void*)c.next_b, (const void*)c.hn_copy})
         at |= reinterpret_cast<uintptr_t>(p);
     if (c.D % 4 == 0 && (c.D / c.groups) % 4 == 0 && (at & 15) == 0)
-        row_close_kernel<4><<<c.M, row_threads(c.D), smem, stream>>>(c);
+        ASD_CUDA(launch_pdl(row_close_kernel<4>, c.M, row_threads(c.D), smem, stream, c));
     else
-        row_close_kernel<1><<<c.M, row_threads(c.D), smem, stream>>>(c);
+        ASD_CUDA(launch_pdl(row_close_kernel<1>, c.M, row_threads(c.D), smem, stream, c));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -395,7 +406,7 @@ int launch_embed_normed(const SeqIndex& ix, const void* embed, int wf32, const f
     if (smem > 200 * 1024) return set_error("embed_normed: width %d does not fit shared memory", D);
     static PerDeviceOnce once;
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(embed_normed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    embed_normed_kernel<<<ix.M, row_threads(D), smem, stream>>>(ix, embed, wf32, w, groups, eps, x, D);
+    ASD_CUDA(launch_pdl(embed_normed_kernel, ix.M, row_threads(D), smem, stream, ix, embed, wf32, w, groups, eps, x, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -407,7 +418,7 @@ int launch_ff_act(const float* z, void* out, int of32, long long rows, int F, in
     if (n <= 0) return 0;
     const long long blocks = (n + 255) / 256;
     if (blocks > 0x7fffffffLL) return set_error("ff_act: too many elements");
-    ff_act_kernel<<<(unsigned)blocks, 256, 0, stream>>>(z, out, of32, n, F, gated, bias);
+    ASD_CUDA(launch_pdl(ff_act_kernel, (unsigned)blocks, 256, 0, stream, z, out, of32, n, F, gated, bias));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -420,9 +431,9 @@ int launch_gated_act(const float* z, void* out, int of32, long long rows, int F,
     const long long blocks = (rows * (four ? F / 4 : F) + 255) / 256;
     if (blocks > 0x7fffffffLL) return set_error("gated_act: too many elements");
     if (four)
-        gated_act_kernel<4><<<(unsigned)blocks, 256, 0, stream>>>(z, out, of32, rows, F, p);
+        ASD_CUDA(launch_pdl(gated_act_kernel<4>, (unsigned)blocks, 256, 0, stream, z, out, of32, rows, F, p));
     else
-        gated_act_kernel<1><<<(unsigned)blocks, 256, 0, stream>>>(z, out, of32, rows, F, p);
+        ASD_CUDA(launch_pdl(gated_act_kernel<1>, (unsigned)blocks, 256, 0, stream, z, out, of32, rows, F, p));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -443,9 +454,9 @@ int launch_tanh_close(const TanhClose& c, cudaStream_t stream) {
     const int n = four ? c.D / 4 : c.D, threads = n >= 256 ? 256 : (n >= 128 ? 128 : 64);
     const dim3 grid(c.M, (n + threads - 1) / threads);
     if (four)
-        tanh_close_kernel<4><<<grid, threads, 0, stream>>>(c);
+        ASD_CUDA(launch_pdl(tanh_close_kernel<4>, grid, threads, 0, stream, c));
     else
-        tanh_close_kernel<1><<<grid, threads, 0, stream>>>(c);
+        ASD_CUDA(launch_pdl(tanh_close_kernel<1>, grid, threads, 0, stream, c));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -454,7 +465,7 @@ int launch_tanh_close(const TanhClose& c, cudaStream_t stream) {
 int launch_rms_rows(const float* in, long long ld_in, const float* w, int plus_one, float eps, void* out, int of32,
                     long long ld_out, int M, int n, cudaStream_t stream) {
     if (M <= 0 || n <= 0) return 0;
-    rms_rows_kernel<<<M, row_threads(n), 0, stream>>>(in, ld_in, w, plus_one, eps, out, of32, ld_out, n);
+    ASD_CUDA(launch_pdl(rms_rows_kernel, M, row_threads(n), 0, stream, in, ld_in, w, plus_one, eps, out, of32, ld_out, n));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -466,7 +477,7 @@ int launch_polynorm(const float* z, const float* coeff, float eps, void* out, in
     const size_t smem = (33 + (staged ? (size_t)F : 0)) * sizeof(float);
     static PerDeviceOnce once;
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(polynorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    polynorm_kernel<<<M, row_threads(F), smem, stream>>>(z, coeff, eps, out, of32, F, staged);
+    ASD_CUDA(launch_pdl(polynorm_kernel, M, row_threads(F), smem, stream, z, coeff, eps, out, of32, F, staged));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -475,7 +486,7 @@ int launch_polynorm(const float* z, const float* coeff, float eps, void* out, in
 int launch_softcap(float* logits, long long ld, int n, int V, float cap, cudaStream_t stream) {
     if (n <= 0 || V <= 0 || !(cap > 0.f)) return 0;
     dim3 grid(n, (V + 255) / 256);
-    softcap_kernel<<<grid, 256, 0, stream>>>(logits, ld, V, cap);
+    ASD_CUDA(launch_pdl(softcap_kernel, grid, 256, 0, stream, logits, ld, V, cap));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;

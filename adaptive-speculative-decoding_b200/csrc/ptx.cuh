@@ -218,4 +218,13 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// First statement of a kernel that is launched programmatically: nothing is read or written before the predecessor has
+// completed (and with it every kernel before that), and the successor may take up residence only from then on.  Letting it
+// in before the wait builds chains of grids that all hold their places while the first one runs; a prompt of the Rivetar
+// layers, CTA-pair GEMMs among them, did not end that way.
+__device__ __forceinline__ void pdl_enter() {
+    grid_dep_wait();
+    grid_dep_launch();
+}
+
 }  // namespace asd

@@ -6,6 +6,7 @@
 #include "asd_internal.h"
 #include "blocks.h"
 #include "elem.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -25,6 +26,7 @@ __device__ __forceinline__ bool owns_ring_entry(const SeqIndex& ix, int m, int r
 __global__ void embed_pair_kernel(SeqIndex ix, const void* embed, const void* table, int wf32, int buckets, int mul_prev,
                                   int mul_cur, const int* tok_ring, int ring, float* x0, const void* g, float eps,
                                   float* hn, int D) {
+    pdl_enter();
     __shared__ float red[33];
     const int m = blockIdx.x;
     const int tok = ix.tokens[m], pos = ix.positions[m], slot = ix.token_slot[m];
@@ -48,6 +50,7 @@ __global__ void embed_pair_kernel(SeqIndex ix, const void* embed, const void* ta
 }
 
 __global__ void commit_tokens_kernel(SeqIndex ix, int* tok_ring, int ring) {
+    pdl_enter();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= ix.M || !owns_ring_entry(ix, m, ring)) return;
     tok_ring[(long long)ix.token_slot[m] * ring + ix.positions[m] % ring] = ix.tokens[m];
@@ -55,6 +58,7 @@ __global__ void commit_tokens_kernel(SeqIndex ix, int* tok_ring, int ring) {
 
 __global__ void token_shift_kernel(SeqIndex ix, const float* hn, const float* state, int ring, const void* mu, int wf32,
                                    void* h, void* hs, int of32, int D) {
+    pdl_enter();
     const int m = blockIdx.x;
     const int pos = ix.positions[m];
     const float* prev = nullptr;
@@ -70,6 +74,7 @@ __global__ void token_shift_kernel(SeqIndex ix, const float* hn, const float* st
 }
 
 __global__ void commit_shift_kernel(SeqIndex ix, const float* hn, float* state, int ring, int D) {
+    pdl_enter();
     const int m = blockIdx.x;
     if (!owns_ring_entry(ix, m, ring)) return;
     float* dst = state + ((long long)ix.token_slot[m] * ring + ix.positions[m] % ring) * D;
@@ -77,6 +82,7 @@ __global__ void commit_shift_kernel(SeqIndex ix, const float* hn, float* state, 
 }
 
 __global__ void layer_close_kernel(LayerClose L, SeqIndex ix) {
+    pdl_enter();
     __shared__ float red[33];
     const int m = blockIdx.x, D = L.D;
     const long long base = (long long)m * D;
@@ -108,6 +114,7 @@ __global__ void layer_close_kernel(LayerClose L, SeqIndex ix) {
 }
 
 __global__ void select_rows_kernel(const float* src, const int* rows, void* dst, int of32, int D) {
+    pdl_enter();
     const int r = blockIdx.x;
     const long long s = (long long)(rows ? rows[r] : r) * D;
     for (int d = threadIdx.x; d < D; d += blockDim.x) stx(dst, (long long)r * D + d, of32, src[s + d]);
@@ -122,8 +129,9 @@ int launch_embed_pair(const SeqIndex& ix, const void* embed, const void* pair_ta
                       cudaStream_t stream) {
     if (ix.M <= 0) return 0;
     if (buckets <= 0 || ring <= 0) return set_error("embed_pair: buckets and ring must be positive");
-    embed_pair_kernel<<<ix.M, row_threads(D), 0, stream>>>(ix, embed, pair_table, wf32, buckets, mul_prev, mul_cur,
-                                                           tok_ring, ring, x0, g, eps, hn, D);
+    ASD_CUDA(launch_pdl(embed_pair_kernel, ix.M, row_threads(D), 0, stream, ix, embed, pair_table, wf32, buckets, mul_prev,
+                        mul_cur,
+                                                           tok_ring, ring, x0, g, eps, hn, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -131,7 +139,7 @@ int launch_embed_pair(const SeqIndex& ix, const void* embed, const void* pair_ta
 
 int launch_commit_tokens(const SeqIndex& ix, int* tok_ring, int ring, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
-    commit_tokens_kernel<<<(ix.M + 127) / 128, 128, 0, stream>>>(ix, tok_ring, ring);
+    ASD_CUDA(launch_pdl(commit_tokens_kernel, (ix.M + 127) / 128, 128, 0, stream, ix, tok_ring, ring));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -140,7 +148,8 @@ int launch_commit_tokens(const SeqIndex& ix, int* tok_ring, int ring, cudaStream
 int launch_token_shift(const SeqIndex& ix, const float* hn, const float* state_ring, int ring, const void* mu, int wf32,
                        void* h, void* hs, int of32, int D, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
-    token_shift_kernel<<<ix.M, row_threads(D), 0, stream>>>(ix, hn, state_ring, ring, mu, wf32, h, hs, of32, D);
+    ASD_CUDA(launch_pdl(token_shift_kernel, ix.M, row_threads(D), 0, stream, ix, hn, state_ring, ring, mu, wf32, h, hs,
+                        of32, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -149,7 +158,7 @@ int launch_token_shift(const SeqIndex& ix, const float* hn, const float* state_r
 int launch_commit_shift_state(const SeqIndex& ix, const float* hn, float* state_ring, int ring, int D,
                               cudaStream_t stream) {
     if (ix.M <= 0) return 0;
-    commit_shift_kernel<<<ix.M, row_threads(D), 0, stream>>>(ix, hn, state_ring, ring, D);
+    ASD_CUDA(launch_pdl(commit_shift_kernel, ix.M, row_threads(D), 0, stream, ix, hn, state_ring, ring, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -158,7 +167,8 @@ int launch_commit_shift_state(const SeqIndex& ix, const float* hn, float* state_
 int launch_layer_close(const LayerClose& L, cudaStream_t stream) {
     if (L.M <= 0) return 0;
     if (L.state_ring && (!L.ix || L.ring <= 0)) return set_error("layer_close: the carried state needs the batch index and a ring");
-    layer_close_kernel<<<L.M, row_threads(L.D), 0, stream>>>(L, L.ix ? *L.ix : SeqIndex{nullptr, nullptr, nullptr, 0});
+    ASD_CUDA(launch_pdl(layer_close_kernel, L.M, row_threads(L.D), 0, stream, L, L.ix ? *L.ix : SeqIndex{nullptr, nullptr,
+                        nullptr, 0}));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -166,7 +176,7 @@ int launch_layer_close(const LayerClose& L, cudaStream_t stream) {
 
 int launch_select_rows(const float* src, const int* rows, void* dst, int of32, int n, int D, cudaStream_t stream) {
     if (n <= 0) return 0;
-    select_rows_kernel<<<n, row_threads(D), 0, stream>>>(src, rows, dst, of32, D);
+    ASD_CUDA(launch_pdl(select_rows_kernel, n, row_threads(D), 0, stream, src, rows, dst, of32, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;

@@ -17,6 +17,7 @@
 #include "blocks.h"
 #include "elem.cuh"
 #include "mma_sync.cuh"
+#include "ptx.cuh"
 
 namespace asd {
 
@@ -52,6 +53,7 @@ __device__ __forceinline__ float turned(const float* src, int i, int n, int inte
 
 __global__ void window_post_kernel(SeqIndex ix, float* qkv, long long ld, WindowDims d, const float* freq_k,
                                    const float* freq_v, PagedRows cache) {
+    pdl_enter();
     extern __shared__ float row[];   // the token's q | k | v as projected
     const int m = blockIdx.x;
     const int pos = ix.positions[m], slot = ix.token_slot[m];
@@ -81,6 +83,7 @@ __global__ void __launch_bounds__(512) window_attn_kernel(SeqIndex ix, const int
                                                            int hpc, const float* q, long long ldq, WindowDims d,
                                                            const float* sink, const float* freq_v, PagedRows cache, void* out,
                                                            int of32) {
+    pdl_enter();
     extern __shared__ float smem[];
     const int group = d.heads / d.kv_heads;
     const int LDK = d.dk | 1;                          // odd row stride: lanes reading one column hit 32 banks
@@ -210,7 +213,7 @@ int launch_simple(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
         auto fn = window_attn_kernel<T, A>;                                                                          \
         static PerDeviceOnce once;                                                                                   \
         if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
-        fn<<<grid, warps * 32, smem, stream>>>(ix, cu_q, seq_slot, TQ, hpc, q, ldq, d, sink, freq_v, cache, out, of32); \
+        ASD_CUDA(launch_pdl(fn, grid, warps * 32, smem, stream, ix, cu_q, seq_slot, TQ, hpc, q, ldq, d, sink, freq_v, cache, out, of32)); \
     }
     if (acc <= 1) ASD_WIN_CASE(1)
     else if (acc <= 2) ASD_WIN_CASE(2)
@@ -244,6 +247,7 @@ __global__ void __launch_bounds__(128) window_attn_mma(SeqIndex ix, const int* c
                                                        const float* q, long long ldq, WindowDims d, const float* sink,
                                                        const float* freq_v, PagedRows cache, void* out, int of32,
                                                        int nsplit, float* ws_o, float* ws_ml, int q_alloc) {
+    pdl_enter();
     extern __shared__ __align__(16) unsigned char smraw[];
     const int dk = SQ ? 8 * NV : d.dk, dv = SQ ? 8 * NV : d.dv;
     const int LDQ = dk + 8, LDV = dv + 8;   // bf16 elements; 16 bytes of padding keep ldmatrix rows on distinct banks
@@ -583,6 +587,7 @@ __global__ void __launch_bounds__(128) window_attn_mma(SeqIndex ix, const int* c
 // normalisation and the turn back by the token's position
 __global__ void window_combine_kernel(SeqIndex ix, WindowDims d, const float* sink, const float* freq_v, int nsplit,
                                       const float* ws_o, const float* ws_ml, void* out, int of32) {
+    pdl_enter();
     extern __shared__ float row[];   // [dv]
     const long long pair = blockIdx.x;
     const int m = (int)(pair / d.heads), head = (int)(pair % d.heads);
@@ -648,8 +653,8 @@ int launch_mma(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nse
         auto fn = window_attn_mma<N, S, G, Q>;                                                                           \
         static PerDeviceOnce once;   /* the attribute is set once per device: a host call per launch costs microseconds */ \
         if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)); \
-        fn<<<grid, 128, smem, stream>>>(ix, cu_q, seq_slot, TQ, q, ldq, d, sink, freq_v, cache, out, of32, nsplit,   \
-                                        ws.o, ws.ml, q_alloc);                                                       \
+        ASD_CUDA(launch_pdl(fn, grid, 128, smem, stream, ix, cu_q, seq_slot, TQ, q, ldq, d, sink, freq_v, cache, out, of32, nsplit,   \
+                                        ws.o, ws.ml, q_alloc));                                                       \
     }
 #define ASD_WM_CASE(N, Q)         \
     {                             \
@@ -672,8 +677,8 @@ int launch_mma(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nse
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     if (nsplit > 1) {
-        window_combine_kernel<<<ix.M * d.heads, d.dv < 128 ? 64 : 128, d.dv * sizeof(float), stream>>>(
-            ix, d, sink, freq_v, nsplit, ws.o, ws.ml, out, of32);
+        ASD_CUDA(launch_pdl(window_combine_kernel, ix.M * d.heads, d.dv < 128 ? 64 : 128, d.dv * sizeof(float), stream,
+            ix, d, sink, freq_v, nsplit, ws.o, ws.ml, out, of32));
         count_launch(1);
         ASD_CUDA(cudaGetLastError());
     }
@@ -698,7 +703,7 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
     if (smem > 200 * 1024) return set_error("windowed attention: a token's q | k | v row does not fit shared memory");
     static PerDeviceOnce once;
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(window_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    window_post_kernel<<<ix.M, 256, smem, stream>>>(ix, qkv, ld, d, freq_k, freq_v, cache);
+    ASD_CUDA(launch_pdl(window_post_kernel, ix.M, 256, smem, stream, ix, qkv, ld, d, freq_k, freq_v, cache));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
