@@ -266,15 +266,19 @@ asd_mezilix_engine_t* asd_mezilix_create(const asd_mezilix_config* cfg, const as
     rc |= dev_alloc(e, &e->hn, MT * D);
     rc |= dev_alloc(e, &e->qd, MT * nqd);
     rc |= dev_alloc(e, &e->qlat, (MT * qlat * 3 + 1) / 2);      // fp32, or three bf16 planes
-    rc |= dev_alloc(e, &e->olat, MT * olat);
+    {   // the attention's result is read before the experts write: one region for it and for their buffers (the query's third
+        // plane is paid for by that)
+        const size_t eout = (MT * top * D + 63) & ~(size_t)63, act = (MT * top * ff * e->esz + 3) / 4;
+        rc |= dev_alloc(e, &e->olat, std::max(MT * olat, eout + act));
+        e->eout = e->olat;
+        e->act = reinterpret_cast<char*>(e->olat + eout);
+    }
     rc |= dev_alloc(e, &e->mix, MT * D);
     rc |= dev_alloc(e, &e->rlog, MT * E);
     rc |= dev_alloc(e, &e->gate, MT * top);
-    rc |= dev_alloc(e, &e->eout, MT * top * D);
     rc |= dev_alloc(e, (char**)&e->h, MT * D * e->esz);
     rc |= dev_alloc(e, (char**)&e->hs, MT * D * e->esz);
     rc |= dev_alloc(e, (char**)&e->vout, MT * hv * e->esz);
-    rc |= dev_alloc(e, (char**)&e->act, MT * top * ff * e->esz);
     rc |= dev_alloc(e, (char**)&e->xsel, MT * D * e->esz);
     rc |= dev_alloc(e, &e->expert_of, MT * top);
     rc |= dev_alloc(e, &e->counters, 2 * E + 1);

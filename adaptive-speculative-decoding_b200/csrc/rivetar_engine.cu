@@ -417,10 +417,11 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     rc |= dev_alloc(e, &e->proj, MT * n_in);
     rc |= dev_alloc(e, &e->qbuf, MT * nq);
     rc |= dev_alloc(e, &e->qlat, (MT * qlat * 3 + 1) / 2);      // fp32, or three bf16 planes
-    rc |= dev_alloc(e, &e->olat, MT * olat);
+    // the attention's result is read before the feed-forward writes: one region (the query's third plane is paid for by that)
+    rc |= dev_alloc(e, &e->olat, std::max(MT * olat, MT * ff));
+    e->up = e->olat;
     rc |= dev_alloc(e, &e->alpha, MT * nk);
     rc |= dev_alloc(e, &e->orec, MT * hv);
-    rc |= dev_alloc(e, &e->up, MT * ff);
     rc |= dev_alloc(e, (char**)&e->hn, MT * 2 * D * e->esz);
     rc |= dev_alloc(e, (char**)&e->cq, MT * qr * e->esz);
     rc |= dev_alloc(e, (char**)&e->mixed, MT * hv * e->esz);
