@@ -81,6 +81,8 @@ struct Engine {
     int attn_prefetch_mb = 0;
     // token counts above 256: QKV and O also run on the CTA-pair kernel (0 = weight-streaming kernel as for small steps)
     int tc_qkvo = 1;
+    // a step of one token of a small model runs its projections on the CUDA cores (gemv.cu); 0: weight-streaming kernel
+    int one_token = 1;
     PLayer* p_layers = nullptr;      // device array, rebuilt lazily after set_layer / set_kv
     bool p_layers_ok = false;
     unsigned* p_sync = nullptr;
@@ -256,13 +258,17 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         return persist_launch(PL, s);
     }
     int parts = 1;   // rows of e->sumsq that currently describe the residual (fused-norm mode)
+    // one token: every projection through gemv.cu (its norm statistics are one sum per block, side by side)
+    const bool one = e->one_token && fn && !tp && e->force_ksplit == 0 && e->force_stages == 0 && n_logit_rows <= 1 &&
+                     gemv_takes(M, std::max(std::max(h, e->qdim), c.ffn), (size_t)2 * e->ffp * h * 2);
+    const int ss_ld = one ? 1 : Mx, max_parts = Mx * ((h + 127) / 128);
     NormFusion cons;  // consumer-side descriptor, refreshed before each consumer GEMM
     auto consumer = [&](const float* ss) -> const NormFusion* {
         if (!fn) return nullptr;
         cons = NormFusion{};
         cons.sumsq_in = ss;
         cons.parts = parts;
-        cons.ld = Mx;
+        cons.ld = ss_ld;
         cons.hidden = h;
         cons.eps = c.rms_eps;
         return &cons;
@@ -330,6 +336,15 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         return launch_add_norm(e->resid, e->part, ns, stride, nullptr, nullptr, next_ln,
                                fn ? nullptr : (next_ln ? e->xnorm : nullptr), M, h, c.rms_eps, s,
                                fn ? e->resid_bf : nullptr, fn ? e->sumsq : nullptr);
+    };
+    auto project_residual_one = [&](const __nv_bfloat16* w, const __nv_bfloat16* x, int K, const __nv_bfloat16* next_ln) -> int {
+        NormFusion prod;
+        prod.sumsq_out = e->sumsq;
+        prod.ld = ss_ld;
+        prod.resid_bf = e->resid_bf;
+        prod.ln_w = next_ln;
+        PROF(PROF_GEMM);
+        return gemv_launch(GEMM_OUT_F32, x, w, K, h, e->resid, nullptr, &prod, max_parts, &parts, s);
     };
     auto project_residual = [&](const GemmPlan& pl, const CUtensorMap& tw, const CUtensorMap& tx,
                                 const __nv_bfloat16* next_ln) -> int {
@@ -426,10 +441,15 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
             q.nkv = nkv;
             q.hd = hd;
             q.page_size = c.page_size;
-            gemm_set_next(P->o, &L.t_o);
-            if (gemm_launch(P->qkv, L.t_qkv, P->x_norm, nullptr, e->nqkv, e->nqkv, e->pdl, s, false, &q,
-                            consumer(e->sumsq)))
-                return -1;
+            if (one) {
+                if (gemv_launch(GEMM_OUT_QKV, e->resid_bf, L.wqkv, h, e->nqkv, nullptr, &q, consumer(e->sumsq), 0, nullptr, s))
+                    return -1;
+            } else {
+                gemm_set_next(P->o, &L.t_o);
+                if (gemm_launch(P->qkv, L.t_qkv, P->x_norm, nullptr, e->nqkv, e->nqkv, e->pdl, s, false, &q,
+                                consumer(e->sumsq)))
+                    return -1;
+            }
         } else {
             {
                 PROF(PROF_GEMM);
@@ -493,6 +513,17 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
             PROF(PROF_ATTN);
             if (launch_attention(A, s)) return -1;
         }
+        if (one) {
+            if (project_residual_one(L.wo, e->attn, e->qdim, L.ln2)) return -1;
+            {
+                PROF(PROF_GEMM);
+                if (gemv_launch(GEMM_OUT_SWIGLU, e->resid_bf, L.wgu, h, c.ffn, e->act, nullptr, consumer(e->sumsq), 0, nullptr, s))
+                    return -1;
+            }
+            if (project_residual_one(L.wdown, e->act, c.ffn, l + 1 == c.n_layers ? e->final_norm : e->layers[l + 1].ln1))
+                return -1;
+            continue;
+        }
         gemm_set_next(P->gu, &L.t_gu);
         if (P->use_tc && e->tc_qkvo ? project_residual_tc(P->o_tc, L.t_o, P->x_attn_tc, L.ln2)
                                     : project_residual(P->o, L.t_o, P->x_attn, L.ln2))
@@ -524,7 +555,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     int key = M;
     if (logit_rows) {
         if (launch_gather_rows(src, logit_rows, e->xsel, n_logit_rows, h, s, fn ? e->sumsq : nullptr, e->sumsq_sel, parts,
-                               Mx))
+                               ss_ld))
             return -1;
         rows = n_logit_rows;
         src = e->xsel;
@@ -532,6 +563,10 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         key = -rows;
     } else if (n_logit_rows != M) {
         return set_error("engine: n_logit_rows must equal M when logit_rows is NULL");
+    }
+    if (one) {
+        PROF(PROF_LMHEAD);
+        return gemv_launch(GEMM_OUT_F32, src, e->lm_head, h, c.vocab, logits_out, nullptr, consumer(ss), 0, nullptr, s);
     }
     if (e->tune.gemm_big && rows > 256) {   // tensor-bound kernel; 152K vocabulary rows give plenty of units without a K split
         auto jt = e->lm_plans_tc.find(key);
@@ -579,7 +614,7 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
     {   // lazy module loading + spinning tensor-parallel kernels in one process = deadlock: load everything now
         static PerDeviceOnce loaded;
         if (loaded.need() && (preload_layers() || preload_attention() || preload_attention_tc() || preload_gemm() ||
-                              preload_gemm_tc()))
+                              preload_gemm_tc() || preload_gemv()))
             return nullptr;
     }
     Engine* e = new Engine();
@@ -833,6 +868,7 @@ int asd_engine_set_option(asd_engine_t* h, const char* name, int value) {
     else if (!strcmp(name, "attn_wide")) e->tune.attn_wide = value;
     else if (!strcmp(name, "attn_dbg")) e->tune.attn_dbg = value;
     else if (!strcmp(name, "tc_qkvo")) e->tc_qkvo = value;
+    else if (!strcmp(name, "one_token")) e->one_token = value;
     else if (!strcmp(name, "attn_prefetch_mb")) e->attn_prefetch_mb = value;
     else if (!strcmp(name, "gemm_big")) e->tune.gemm_big = value;
     else if (!strcmp(name, "persist")) e->persist = value;

@@ -89,4 +89,9 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
                    size_t slice_stride, bool pdl, cudaStream_t stream, bool accumulate, const NormFusion* norm);
 
+// ---- one token (gemv.cu): CUDA cores, weight rows straight into registers
+bool gemv_takes(int M, int max_k, size_t max_bytes);
+int gemv_launch(int mode, const __nv_bfloat16* x, const __nv_bfloat16* w, int K, int n_valid, void* out, const QkvEpilogue* qkv,
+                const NormFusion* norm, int max_parts, int* blocks_out, cudaStream_t stream);
+int preload_gemv();
 }  // namespace asd

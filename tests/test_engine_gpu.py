@@ -317,3 +317,40 @@ def test_prompt_query_tiles(hd, nh, nkv, page, attn_impl, min_keys, lens, max_to
         with pytest.raises(Exception):
             eng.forward_uniform(new[:1, :1].expand(1, q).contiguous(), slots[:1] * 0, slots[:1], q)
     eng.close()
+
+
+@pytest.mark.parametrize("cfg", [
+    Qwen2Config(896, 2, 14, 2, 1000, 1531, head_dim=64, name="one-odd"),          # odd vocabulary, ffn not a multiple of 64, K not of 256
+    Qwen2Config(512, 2, 10, 2, 4864, 40000, head_dim=128, name="one-split"),      # long rows: warps share a pair; many pairs: two at once
+    Qwen2Config(264, 1, 3, 1, 72, 96, head_dim=128, name="one-tiny"),             # fewer pairs than warps, rows shorter than a step
+])
+def test_engine_one_token(cfg):
+    """a step of one token runs its projections on the CUDA cores: all its logits, and selected ones, against the oracle and
+    against the tcgen05 kernels of the same engine; larger steps are the same with the option on and off"""
+    from asd_b200.engine import QwenEngine
+    w = random_hf_weights(cfg, seed=19, logit_std=0.4)
+    T = 40
+    ids = torch.randint(0, cfg.vocab_size, (2, T), generator=torch.Generator().manual_seed(9))
+    ref = qwen2_forward(w, cfg, ids)
+    eng = QwenEngine(cfg, max_seqs=2, max_seq_len=T + 8, max_tokens=64).load_hf_weights(w)
+    idc = ids.cuda().to(torch.int32)
+    for nseq, q in ((1, 1), (2, 1), (1, 2)):
+        slots = torch.arange(nseq, dtype=torch.int32, device="cuda")
+        eng.prefill(idc[:nseq, :T - q].contiguous(), slots, want_logits=False)
+        start = torch.full((nseq,), T - q, dtype=torch.int32, device="cuda")
+        got = {}
+        for on in (1, 0):
+            eng.set_option("one_token", on)
+            got[on] = eng.forward_uniform(idc[:nseq, T - q:].contiguous(), start, slots, T).view(nseq, q, -1).cpu()
+        check(got[1], ref[:nseq, T - q:])
+        if nseq * q == 1:
+            assert (got[1] - got[0]).abs().max().item() <= MAX_ABS
+        else:
+            assert torch.equal(got[1], got[0])
+    eng.set_option("one_token", 1)
+    one, slot = torch.tensor([0], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    pos, cu = slot + T - 1, torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    eng.prefill(idc[:1, :T - 1].contiguous(), slot, want_logits=False)
+    rows = eng.forward(idc[0, T - 1:].contiguous(), pos, slot, cu, slot, 1, T, logit_rows=one).cpu()
+    check(rows, ref[:1, T - 1])
+    eng.close()
