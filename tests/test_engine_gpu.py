@@ -354,3 +354,25 @@ def test_engine_one_token(cfg):
     rows = eng.forward(idc[0, T - 1:].contiguous(), pos, slot, cu, slot, 1, T, logit_rows=one).cpu()
     check(rows, ref[:1, T - 1])
     eng.close()
+
+
+@pytest.mark.parametrize("tokens", [160, 161, 211, 256])
+@pytest.mark.parametrize("cfg", [
+    Qwen2Config(1280, 1, 10, 2, 9600, 1024, head_dim=128, name="wave-wide"),      # 150 gate|up tiles: more than one per SM
+    Qwen2Config(512, 2, 8, 2, 1024, 1024, head_dim=64, name="wave-narrow"),       # 4 x 8 CTAs
+    Qwen2Config(1280, 1, 10, 2, 1024, 1024, head_dim=128, name="wave-between"),   # neither: weight-streaming up to 256 tokens
+])
+def test_engine_prompt_chunks_near_the_ridge(cfg, tokens):
+    """chunks of 161 to 256 tokens take the CTA-pair kernel where the weight-streaming one would need a second wave or leave
+    half of the SMs idle; both sides of each line against the oracle"""
+    from asd_b200.engine import QwenEngine
+    w = random_hf_weights(cfg, seed=23, logit_std=0.4)
+    ids = torch.randint(0, cfg.vocab_size, (1, tokens + 4), generator=torch.Generator().manual_seed(10))
+    ref = qwen2_forward(w, cfg, ids)
+    eng = QwenEngine(cfg, max_seqs=1, max_seq_len=tokens + 16, max_tokens=256).load_hf_weights(w)
+    slot, idc = torch.zeros(1, dtype=torch.int32, device="cuda"), ids.cuda().to(torch.int32)
+    last = eng.prefill(idc[:, :tokens].contiguous(), slot)
+    ver = eng.forward_uniform(idc[:, tokens:].contiguous(), slot + tokens, slot, tokens + 4)
+    check(last.cpu(), ref[:, tokens - 1])
+    check(ver.view(1, 4, -1).cpu(), ref[:, tokens:])
+    eng.close()
