@@ -46,7 +46,7 @@ struct DenseRunner {
                 it = cache.emplace(k, t).first;
             }
             if (M >= tc_min_rows)
-                return gemm_tc_launch(it->second.big, it->second.tw, it->second.tx, y, ldc, N, 0, false, s, false, nullptr);
+                return gemm_tc_launch(it->second.big, it->second.tw, it->second.tx, y, ldc, N, 0, s, false, nullptr);
             return gemm_launch(it->second.pl, it->second.tw, it->second.tx, y, ldc, N, true, s, false);
         }
         SimtLinear L;

@@ -35,7 +35,7 @@ struct Layer {
 struct Plans {
     GemmPlan qkv, o, gu, down;
     CUtensorMap x_norm, x_attn, x_act;
-    // token counts above the HBM/tensor ridge, or near it where that pays: the tensor-bound CTA-pair kernel (gemm_tc.cu)
+    // token counts above the HBM/tensor ridge: gate|up and down run on the tensor-bound CTA-pair kernel (gemm_tc.cu)
     bool use_tc = false;
     TcPlan gu_tc, down_tc, qkv_tc, o_tc;
     CUtensorMap x_norm_tc, x_act_tc, x_norm_qkv_tc, x_attn_tc;
@@ -79,7 +79,7 @@ struct Engine {
     int persist = 0, persist_ahead = 0;
     // MB of the O-projection / gate|up weights that the attention kernel pulls into L2 while it runs (0 = off)
     int attn_prefetch_mb = 0;
-    // steps on the CTA-pair kernel: QKV and O as well (0 = weight-streaming kernel as for small steps)
+    // token counts above 256: QKV and O also run on the CTA-pair kernel (0 = weight-streaming kernel as for small steps)
     int tc_qkvo = 1;
     // a step of one token of a small model runs its projections on the CUDA cores (gemv.cu); 0: weight-streaming kernel
     int one_token = 1;
@@ -150,14 +150,7 @@ static int ensure_plans(Engine* e, int M, Plans** out) {
     if (make_tmap_bf16(&p.x_norm, e->fuse_norm ? e->resid_bf : e->xnorm, M, h, h, p.qkv.MT)) return -1;
     if (make_tmap_bf16(&p.x_attn, e->attn, M, e->qdim, e->qdim, p.o.MT)) return -1;
     if (make_tmap_bf16(&p.x_act, e->act, M, e->c.ffn, e->c.ffn, p.down.MT)) return -1;
-    // From 257 tokens on the step is tensor bound.  From 161 on the weight-streaming kernel's ring for so many token columns
-    // leaves room for one CTA per SM: its gate|up then takes a second wave where it has more weight tiles than the chip has SMs,
-    // and a narrow model's row-parallel grids (8 K splits at most) leave half of the SMs idle while each thread walks its
-    // tokens.  Measured without the head, this kernel -> CTA pairs, 176 and 255 tokens: width 3584, 296 tiles, four layers
-    // 832 -> 688 and 991 -> 766 us (160 tokens: 618 -> 678); width 5120, two layers 684 -> 553 and 774 -> 636; width 896, 8 x 7
-    // CTAs, eight layers 586 -> 520 and 738 -> 564; width 1536, 140 tiles and 8 x 12 CTAs: 610 -> 688 and 731 -> 740, so it stays.
-    const bool second_wave = 2 * e->ffp / 128 > 148, half_idle = (h + 127) / 128 * 8 < 74;
-    p.use_tc = e->tune.gemm_big && (M > 256 || (M > 160 && e->c.tp_size == 1 && (second_wave || half_idle)));
+    p.use_tc = e->tune.gemm_big && M > 256;
     if (p.use_tc) {
         if (gemm_tc_plan(&p.gu_tc, M, 2 * e->ffp, h, GEMM_OUT_SWIGLU, 0, e->force_stages)) return -1;
         if (gemm_tc_plan(&p.down_tc, M, h, e->c.ffn, GEMM_OUT_F32, 0, e->force_stages)) return -1;
@@ -323,7 +316,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         float* dst = (p2p_ok && pl.ksplit == 1) ? e->tp_buf[e->tp_epoch & 1] : e->part;
         {
             PROF(PROF_GEMM);
-            if (gemm_tc_launch(pl, tw, tx, dst, h, h, stride, e->pdl, s, false, nullptr)) return -1;
+            if (gemm_tc_launch(pl, tw, tx, dst, h, h, stride, s, false, nullptr)) return -1;
         }
         if (p2p_ok) {
             if (pl.ksplit > 1) {
@@ -424,8 +417,8 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         if (P->use_tc && e->tune.gemm_big >= 1 && e->tc_qkvo) {   // tensor-bound step: CTA-pair GEMM + one glue kernel
             {
                 PROF(PROF_GEMM);
-                if (gemm_tc_launch(P->qkv_tc, L.t_qkv, P->x_norm_qkv_tc, e->part, e->nqkv, e->nqkv, (size_t)M * e->nqkv,
-                                   e->pdl, s, false, consumer(e->sumsq)))
+                if (gemm_tc_launch(P->qkv_tc, L.t_qkv, P->x_norm_qkv_tc, e->part, e->nqkv, e->nqkv, (size_t)M * e->nqkv, s,
+                                   false, consumer(e->sumsq)))
                     return -1;
             }
             PROF(PROF_GLUE);
@@ -537,7 +530,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
             return -1;
         if (P->use_tc) {
             PROF(PROF_GEMM);
-            if (gemm_tc_launch(P->gu_tc, L.t_gu, P->x_norm_tc, e->act, c.ffn, c.ffn, 0, e->pdl, s, false, consumer(e->sumsq)))
+            if (gemm_tc_launch(P->gu_tc, L.t_gu, P->x_norm_tc, e->act, c.ffn, c.ffn, 0, s, false, consumer(e->sumsq)))
                 return -1;
         } else {
             PROF(PROF_GEMM);
@@ -585,8 +578,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         }
         PROF(PROF_LMHEAD);
         const int ld = logits_ld > 0 ? (int)logits_ld : c.vocab;
-        return gemm_tc_launch(jt->second.first, e->t_lm, jt->second.second, logits_out, ld, c.vocab, 0, e->pdl, s, false,
-                              consumer(ss));
+        return gemm_tc_launch(jt->second.first, e->t_lm, jt->second.second, logits_out, ld, c.vocab, 0, s, false, consumer(ss));
     }
     auto it = e->lm_plans.find(key);
     if (it == e->lm_plans.end()) {

@@ -87,7 +87,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 // x tensor map: box rows = MT / 2 (each CTA of the pair loads half of the token tile); w tensor map: box rows = 128.
 // GEMM_OUT_F32: out fp32 [ksplit][slice_stride] slices of [M][ldo]; GEMM_OUT_SWIGLU: out bf16 [M][ldo].
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
-                   size_t slice_stride, bool pdl, cudaStream_t stream, bool accumulate, const NormFusion* norm);
+                   size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm);
 
 // ---- one token (gemv.cu): CUDA cores, weight rows straight into registers
 bool gemv_takes(int M, int max_k, size_t max_bytes);

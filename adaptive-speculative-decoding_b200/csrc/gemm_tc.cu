@@ -162,7 +162,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             const uint64_t pol_w = a.m_tiles > 1 ? policy_evict_normal() : policy_evict_first();
             const uint64_t pol_x = policy_evict_last();
             const uint32_t full_leader = mapa(smem_u32(full_bar), 0);
-            bool waited = false;
             int it = 0;
             for (int u = pair; u < units; u += npairs) {
                 const TcUnit t = tc_unit(a, u);
@@ -173,10 +172,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                     uint8_t* st = smem + (size_t)s * stage_bytes;
                     const uint32_t bar = full_leader + (uint32_t)s * 8u;
                     tma_load_2d_cg2(st, &tmap_w, (t.kb0 + kb) * kTcBlockK, t.w_tile * 256 + (int)rank * 128, bar, pol_w);
-                    if (!waited) {   // weights do not depend on the upstream kernel, activations do
-                        grid_dep_wait();
-                        waited = true;
-                    }
                     tma_load_2d_cg2(st + kTcABytes, &tmap_x, (t.kb0 + kb) * kTcBlockK,
                                     t.t_tile * a.MT + (int)rank * (a.MT / 2), bar, pol_x);
                 }
@@ -212,7 +207,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         // ------------------------------------------------------------------ epilogue (both CTAs)
         const int q = warp & 3, row = q * 32 + lane, et = threadIdx.x - 128;
         const bool scale = a.norm.sumsq_in != nullptr;
-        grid_dep_wait();
         if (scale) {
             for (int m = et; m < a.M; m += 128) {
                 float ssum = 0.0f;
@@ -383,7 +377,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 }
 
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
-                   size_t slice_stride, bool pdl, cudaStream_t stream, bool accumulate, const NormFusion* norm) {
+                   size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm) {
     if (g_tc_attr.need()) {
         ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
         prefer_max_smem(gemm_tc_kernel);
@@ -407,21 +401,8 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.out = out;
     a.slice_stride = slice_stride;
     a.norm = norm ? *norm : NormFusion{};
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute attr[1];
-    cfg.gridDim = dim3(2 * pl.pairs);
-    cfg.blockDim = dim3(kTcThreads);
-    cfg.dynamicSmemBytes = pl.smem_bytes;
-    cfg.stream = stream;
-    int na = 0;
-    if (pdl) {
-        attr[na].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[na].val.programmaticStreamSerializationAllowed = 1;
-        ++na;
-    }
-    cfg.attrs = attr;
-    cfg.numAttrs = na;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel, tmap_w, tmap_x, a));
+    gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, a);
+    ASD_CUDA(cudaGetLastError());
     count_launch(1);
     return 0;
 }
@@ -448,6 +429,5 @@ extern "C" int asd_linear_bf16_tc(const void* x, const void* w, void* out, int M
     if (make_tmap_bf16(&tx, x, M, K, K, pl.MT / 2)) return -1;
     if (ksplit_used) *ksplit_used = pl.ksplit;
     const int ldo = out_mode == 2 ? N / 2 : N;
-    return gemm_tc_launch(pl, tw, tx, out, ldo, ldo, (size_t)M * ldo, false, static_cast<cudaStream_t>(stream), false,
-                          nullptr);
+    return gemm_tc_launch(pl, tw, tx, out, ldo, ldo, (size_t)M * ldo, static_cast<cudaStream_t>(stream), false, nullptr);
 }

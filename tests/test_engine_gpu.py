@@ -360,11 +360,11 @@ def test_engine_one_token(cfg):
 @pytest.mark.parametrize("cfg", [
     Qwen2Config(1280, 1, 10, 2, 9600, 1024, head_dim=128, name="wave-wide"),      # 150 gate|up tiles: more than one per SM
     Qwen2Config(512, 2, 8, 2, 1024, 1024, head_dim=64, name="wave-narrow"),       # 4 x 8 CTAs
-    Qwen2Config(1280, 1, 10, 2, 1024, 1024, head_dim=128, name="wave-between"),   # neither: weight-streaming up to 256 tokens
+    Qwen2Config(1280, 1, 10, 2, 1024, 1024, head_dim=128, name="wave-between"),   # neither
 ])
 def test_engine_prompt_chunks_near_the_ridge(cfg, tokens):
-    """chunks of 161 to 256 tokens take the CTA-pair kernel where the weight-streaming one would need a second wave or leave
-    half of the SMs idle; both sides of each line against the oracle"""
+    """chunks up to 256 tokens (the weight-streaming kernel's largest token tile), of widths whose gate|up needs one wave of its
+    CTAs or two and whose row-parallel grids fill the chip or half of it, against the oracle"""
     from asd_b200.engine import QwenEngine
     w = random_hf_weights(cfg, seed=23, logit_std=0.4)
     ids = torch.randint(0, cfg.vocab_size, (1, tokens + 4), generator=torch.Generator().manual_seed(10))
@@ -376,3 +376,43 @@ def test_engine_prompt_chunks_near_the_ridge(cfg, tokens):
     check(last.cpu(), ref[:, tokens - 1])
     check(ver.view(1, 4, -1).cpu(), ref[:, tokens:])
     eng.close()
+
+
+def _rel(a, b):
+    return ((a - b).norm() / b.norm()).item()
+
+
+def test_prefill_of_the_benchmark_pair_ends():
+    """SpecDecoder.prefill of 16 x 512 tokens on the 32B / 7B pair at their real depths: 32 forwards of 256 tokens per model
+    back to back in one stream, thousands of launches without a host synchronisation"""
+    from asd_b200.engine import QwenEngine, SpecDecoder
+    from asd_b200.models.qwen2 import QWEN25
+    B, P = 16, 512
+    kw = dict(max_seqs=B, max_seq_len=P + 32, max_tokens=256)
+    t, d = QwenEngine(QWEN25["32b"], **kw).load_random(seed=1), QwenEngine(QWEN25["7b"], **kw).load_random(seed=0)
+    prompts = torch.randint(0, t.cfg.vocab_size, (B, P), generator=torch.Generator().manual_seed(1234))
+    first = [SpecDecoder(t, d, B, 5, 0.7, seed=4321).prefill(prompts).cpu() for _ in range(2)]
+    assert torch.equal(*first) and 0 <= int(first[0].min()) and int(first[0].max()) < t.cfg.vocab_size
+    t.close()
+    d.close()
+
+
+def test_prefill_at_depth_small_and_large_forwards():
+    """a 28-layer model's prompts by forwards of 256 tokens and of 2048 (CTA-pair GEMMs), many in a row: the same logits up to
+    the rounding of bf16 activations through the layers (each layer rounds its branches at 2^-9 relative; 28 layers x 2 branches
+    add to sqrt(56) 2^-9 = 1.5e-2 on either side, bound at twice their difference)"""
+    from asd_b200.engine import QwenEngine
+    from asd_b200.models.qwen2 import QWEN25
+    B, P = 16, 256
+    prompts = torch.randint(0, 150000, (B, P), generator=torch.Generator().manual_seed(5)).cuda().to(torch.int32)
+    slots = torch.arange(B, dtype=torch.int32, device="cuda")
+    logits = []
+    for max_tokens in (256, 2048):
+        eng = QwenEngine(QWEN25["7b"], max_seqs=B, max_seq_len=P + 16, max_tokens=max_tokens).load_random(seed=3)
+        outs = [eng.prefill(prompts, slots) for _ in range(20)]
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, outs[0]) for o in outs)
+        logits.append(outs[0].double().cpu())
+        eng.close()
+        del eng, outs
+    assert _rel(*logits) < 4.3e-2
