@@ -138,6 +138,8 @@ def lib() -> ctypes.CDLL:
         "asd_abi_version": (i32, []),
         "asd_last_error": (c.c_char_p, []),
         "asd_launch_count": (c.c_longlong, []),
+        "asd_wait_error": (i32, []),
+        "asd_debug_wait_expiry": (i32, [vp]),
         "asd_reset_launch_count": (None, []),
         "asd_reject_sample_workspace_bytes": (sz, [i32, i32]),
         "asd_reject_sample_set_impl": (None, [i32]),
@@ -166,6 +168,7 @@ def lib() -> ctypes.CDLL:
         "asd_engine_ipc_export": (i32, [vp, vp]),
         "asd_engine_ipc_import": (i32, [vp, vp]),
         "asd_engine_tp_error": (i32, [vp]),
+        "asd_engine_device_error": (i32, [vp]),
         "asd_engine_profile_read": (i32, [vp, vp, vp, i32]),
         "asd_debug_gemm_trace": (i32, [vp, i32]),
         "asd_debug_attn_trace": (i32, [vp, i32]),

@@ -68,6 +68,7 @@ int asd_reject_sample_host(const float* target_logits, const float* draft_logits
     if (rc == 0) {
         cudaError_t e = cudaStreamSynchronize(s);
         if (e != cudaSuccess) rc = set_error("asd_reject_sample_host: %s", cudaGetErrorString(e));
+        if (rc == 0) rc = asd_wait_error();
     }
     cudaFree(d);
     return rc;

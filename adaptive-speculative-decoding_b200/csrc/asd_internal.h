@@ -19,6 +19,23 @@ void count_launch(int n);
             return ::asd::set_error("%s failed: %s (%s:%d)", #expr, cudaGetErrorString(_e), __FILE__, __LINE__); \
     } while (0)
 
+// ---- Bounded device waits.  A kernel whose barrier does not complete gives up after some seconds (ptx.cuh, mbar_wait), writes
+// (kernel << 8 | place) into a word of mapped host memory and ends.  The host reads that word without touching the device: every
+// entry point of an engine does before it launches anything, and so does whoever hands results to the host.
+enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, WAIT_LINEAR, WAIT_LATENT, WAIT_PERSIST };
+int* wait_word_alloc();                                 // a zeroed word that every device and stream can write, or nullptr
+void wait_word_free(int* word);
+int wait_word_check(const int* word, const char* who);  // 0, or the error that names the kernel and the place
+int* device_wait_word();                                // of the current device: calls that belong to no engine
+int launch_wait_expiry(int* word, cudaStream_t stream); // a wait that runs out (two seconds), for the tests of what follows
+extern thread_local int* g_wait_word;
+inline int* wait_word() { return g_wait_word ? g_wait_word : device_wait_word(); }
+struct WaitScope {                                      // an engine's word, for the launches of one forward on this host thread
+    int* prev;
+    explicit WaitScope(int* w) : prev(g_wait_word) { g_wait_word = w; }
+    ~WaitScope() { g_wait_word = prev; }
+};
+
 // Programmatic launch: the grid may become resident while its predecessor drains.  Only for kernels that begin with
 // pdl_enter() or otherwise wait (griddepcontrol.wait) before they touch memory.
 template <typename... P, typename... A>

@@ -68,9 +68,11 @@ struct AttnTcArgs {
     int* tickets;
     __nv_bfloat16* out;            // [M, nh, 128]
     unsigned long long* trace;     // diagnostics: 16 globaltimer stamps per CTA (nullptr = off)
+    int* err;                      // where a wait that ran out is reported
 };
+template <bool TRACE>
 __device__ __forceinline__ void at_stamp(const AttnTcArgs& a, int slot) {
-    if (a.trace) {
+    if constexpr (TRACE) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
         const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -142,6 +144,7 @@ __device__ __forceinline__ void at_exp32(const uint32_t (&v)[32], int lim, float
     }
 }
 
+template <bool TRACE>      // with the stamps
 __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_constant__ CUtensorMap kv_map, const AttnTcArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -154,6 +157,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
              *c_full = bars + 18;   // c_full[4]
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
     int* s_last = reinterpret_cast<int*>(tmem_slot + 1);
+    const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 2), a.err, WAIT_ATTENTION << 8};
     float* corr_s = reinterpret_cast<float*>(tmem_slot + 4);   // [4][128] rescale factor of tile j (ring j & 3)
     float* fin_s = corr_s + 4 * 128;                           // [2][128] final row maximum / row sum
     int* s_pt = reinterpret_cast<int*>(fin_s + 2 * 128);
@@ -182,7 +186,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     const int nt = (kend - kbeg + kAtTile - 1) / kAtTile;
     const int psh = a.page_shift;
     const int page0 = kbeg >> psh, npages = ((kend - 1) >> psh) - page0 + 1;
-    if (threadIdx.x == 0) at_stamp(a, 0);
+    if (threadIdx.x == 0) at_stamp<TRACE>(a, 0);
 
     {   // this CTA's slice of the page table (static across forwards: safe before the PDL wait)
         const int* pt = a.page_table + (size_t)a.seq_slot[seq] * a.max_pages;
@@ -203,6 +207,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
         mbar_init(p_full, nact);
         mbar_init(q_full, 4);
         for (int i = 0; i < 4; ++i) mbar_init(&c_full[i], nact);
+        *guard.failed = 0;
         fence_mbar_init();
     }
     if (warp == 10) {
@@ -231,7 +236,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                     waited = true;
                 }
                 uint8_t* dst = ring + st * kAtOp;
-                if (use > 0) mbar_wait(&empty[st], (use - 1) & 1);
+                if (use > 0 && !mbar_wait(&empty[st], (use - 1) & 1, guard)) break;
                 mbar_expect_tx(&full[st], kAtOp);
 #pragma unroll 1
                 for (int p = 0; p < (kAtTile >> psh); ++p) {
@@ -241,7 +246,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                     at_tma_box(dst + ((p * 128) << psh), &kv_map, 0, row, &full[st]);
                     at_tma_box(dst + kAtHalf + ((p * 128) << psh), &kv_map, 64, row, &full[st]);
                 }
-                if (j == 0) at_stamp(a, 11 + kv);
+                if (j == 0) at_stamp<TRACE>(a, 11 + kv);
             }
             if (!waited) grid_dep_wait();
         }
@@ -252,10 +257,13 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             const uint32_t idesc_qk = umma_idesc_bf16(128, 128);
             const uint32_t idesc_pv = umma_idesc_bf16(128, 128) | (1u << 16);     // B (= V) is MN-major
             const uint32_t uQ = smem_u32(sQ), uK = smem_u32(sK), uV = smem_u32(sV);
+            bool ok = mbar_wait_far(q_full, 0, guard, 1);
             auto issue_qk = [&](int j) {
                 const int st = j & 1, use = j >> 1;
-                if (use > 0) mbar_wait(&s_empty[st], (use - 1) & 1);   // P V of tile j-2 has consumed P in this buffer
-                mbar_wait(&k_full[st], use & 1);
+                // P V of tile j-2 has consumed P in this buffer
+                if (use > 0) ok = ok && mbar_wait_far(&s_empty[st], (use - 1) & 1, guard, 2);
+                ok = ok && mbar_wait_far(&k_full[st], use & 1, guard, 3);
+                if (!ok) return;
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(st * 128);
 #pragma unroll
@@ -265,16 +273,15 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 }
                 umma_commit(&s_full[st]);
                 umma_commit(&k_empty[st]);
-                if (j == 0) at_stamp(a, 13);
+                if (j == 0) at_stamp<TRACE>(a, 13);
             };
-            mbar_wait(q_full, 0);
             issue_qk(0);
             for (int j = 0; j < nt; ++j) {
                 const int st = j & 1, use = j >> 1;
                 if (j + 1 < nt) issue_qk(j + 1);
-                mbar_wait(p_full, j & 1);
-                mbar_wait(&v_full[st], use & 1);
-                if (use > 0) mbar_wait(&o_empty[st], (use - 1) & 1);
+                ok = ok && mbar_wait_far(p_full, j & 1, guard, 4) && mbar_wait_far(&v_full[st], use & 1, guard, 5) &&
+                     (use == 0 || mbar_wait_far(&o_empty[st], (use - 1) & 1, guard, 6));
+                if (!ok) break;
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(256 + st * 128);
                 const uint32_t p = tmem_base + (uint32_t)(st * 128);     // bf16 P: 64 packed columns over S
@@ -284,8 +291,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 umma_commit(&o_full[st]);
                 umma_commit(&v_empty[st]);
                 umma_commit(&s_empty[st]);
-                if (j == 0) at_stamp(a, 14);
+                if (j == 0) at_stamp<TRACE>(a, 14);
             }
+            if (ok) mbar_wait_far(&o_full[(nt - 1) & 1], ((nt - 1) >> 1) & 1, guard, 7);      // the fold waits untimed
         }
         __syncwarp();
     } else if (warp < 4) {
@@ -306,7 +314,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) mbar_arrive(q_full);
-            if (r == 0) at_stamp(a, 1);
+            if (r == 0) at_stamp<TRACE>(a, 1);
         }
         if (warp < nact) {
             const int qpos = r < R ? kv_len - qlen + r / G : -1;
@@ -319,9 +327,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 const int st = j & 1, use = j >> 1;
                 const int lim = min(kend - 1, qpos) - (kbeg + j * kAtTile);   // element i of the tile visible iff i <= lim
                 const uint32_t tS = lane_base + (uint32_t)(st * 128);
-                mbar_wait(&s_full[st], use & 1);
+                mbar_wait(&s_full[st], use & 1, guard);
                 tc_fence_after();
-                if (r == 0 && (j < 2 || j == nt - 1)) at_stamp(a, j == 0 ? 2 : (j == 1 ? 4 : 7));
+                if (r == 0 && (j < 2 || j == nt - 1)) at_stamp<TRACE>(a, j == 0 ? 2 : (j == 1 ? 4 : 7));
                 if (a.dbg >= 1) {
                     corr_s[(j & 3) * 128 + r] = 1.0f;
                     tc_fence_before();
@@ -350,7 +358,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 const float ref = mn == -INFINITY ? 0.0f : mn;
                 const float corr = at_ex2(mx - ref);      // mx = -inf -> 0
                 corr_s[(j & 3) * 128 + r] = corr;
-                if (r == 0 && j == 1) at_stamp(a, 15);
+                if (r == 0 && j == 1) at_stamp<TRACE>(a, 15);
                 float ps[4] = {0.0f, 0.0f, 0.0f, 0.0f};
                 // second pass: the packed probabilities of columns [32c, 32c + 32) overwrite columns [16c, 16c + 16) of
                 // the same buffer, which this thread has already read (its own lane only)
@@ -379,7 +387,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                     mbar_arrive(p_full);
                     mbar_arrive(&c_full[j & 3]);
                 }
-                if (r == 0 && j < 2) at_stamp(a, j == 0 ? 3 : 5);
+                if (r == 0 && j < 2) at_stamp<TRACE>(a, j == 0 ? 3 : 5);
                 l = l * corr + ((ps[0] + ps[1]) + (ps[2] + ps[3]));
                 mx = mn;
             };
@@ -397,7 +405,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             fin_s[128 + r] = l;
             __syncwarp();
             if (lane == 0) mbar_arrive(&c_full[nt & 3]);
-            if (r == 0) at_stamp(a, 8);
+            if (r == 0) at_stamp<TRACE>(a, 8);
         }
     } else {
         // ------------------------------------------------------------------ fold: o = o * corr + O_tile (thread = row)
@@ -410,9 +418,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             for (int i = 0; i < 128; ++i) o[i] = 0.0f;
             for (int j = 0; j < nt; ++j) {
                 const int st = j & 1, use = j >> 1;
-                mbar_wait(&c_full[j & 3], (j >> 2) & 1);
+                mbar_wait(&c_full[j & 3], (j >> 2) & 1, guard);
                 const float corr = corr_s[(j & 3) * 128 + r];
-                mbar_wait(&o_full[st], use & 1);
+                mbar_wait(&o_full[st], use & 1, guard);
                 tc_fence_after();
                 if (a.dbg < 2) {
 #pragma unroll
@@ -427,11 +435,11 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&o_empty[st]);
-                if (r == 0 && j == 0) at_stamp(a, 6);
+                if (r == 0 && j == 0) at_stamp<TRACE>(a, 6);
             }
-            mbar_wait(&c_full[nt & 3], (nt >> 2) & 1);
+            mbar_wait(&c_full[nt & 3], (nt >> 2) & 1, guard);
             const float mx = fin_s[r], l = fin_s[128 + r];
-            if (r == 0) at_stamp(a, 9);
+            if (r == 0) at_stamp<TRACE>(a, 9);
             // ---- results: final output when the sequence has a single split, else partials + last-CTA combine
             if (r < R) {
                 const int t = r / G, gq = r - t * G;
@@ -457,13 +465,14 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             }
         }
     }
+    wait_settle(guard);
     tc_fence_before();
     __syncthreads();
     if (warp == 10) {
         tc_fence_after();
         tmem_dealloc(tmem_base, 512);
     }
-    if (threadIdx.x == 0) at_stamp(a, 10);
+    if (threadIdx.x == 0) at_stamp<TRACE>(a, 10);
     if (nsplit_seq == 1) return;
     // the last CTA of this (query tile, kv head) to finish merges the splits (no separate combine launch)
     __threadfence();
@@ -509,8 +518,10 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     const size_t smem = 1024 + 5 * (size_t)kAtOp + 22 * 8 + 16 + 6 * 128 * 4 +
                         ((size_t)L.split_keys / L.page_size + 2) * 4 + 64;
     if (once.need()) {
-        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        prefer_max_smem(attn_tc_kernel);
+        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        prefer_max_smem(attn_tc_kernel<false>);
+        prefer_max_smem(attn_tc_kernel<true>);
     }
     if (smem > 227 * 1024) return set_error("attention_tc: split of %d keys does not fit the page-table slice", L.split_keys);
     AttnTcArgs a;
@@ -536,6 +547,7 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     a.ml_part = L.ml_part;
     a.tickets = L.tickets;
     a.out = L.out;
+    a.err = wait_word();
     a.trace = nullptr;
     const int tiles = L.q_tile > 0 ? (L.max_qlen + L.q_tile - 1) / L.q_tile : 1;
     if (g_attn_trace && g_attn_trace_next < g_attn_trace_max && (long long)tiles * L.nseq * L.nkv * L.nsplit_max <= 1024)
@@ -550,7 +562,7 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = tuning().glue_pdl ? 1 : 0;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, attn_tc_kernel, *L.kv_map, a));
+    ASD_CUDA(cudaLaunchKernelEx(&cfg, a.trace ? attn_tc_kernel<true> : attn_tc_kernel<false>, *L.kv_map, a));
     count_launch(1);
     return 0;
 }
@@ -559,7 +571,7 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_attention_tc() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, attn_tc_kernel));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, attn_tc_kernel<false>));
     return 0;
 }
 

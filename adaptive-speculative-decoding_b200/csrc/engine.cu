@@ -95,6 +95,7 @@ struct Engine {
     float* tp_buf[2] = {nullptr, nullptr};
     uint32_t* tp_flags = nullptr;
     int* tp_error = nullptr;
+    int* wait_err = nullptr;         // a bounded wait of one of this engine's kernels ran out (mapped host memory)
     const float* peer_buf[2][8] = {};
     uint32_t* peer_flags[8] = {};
     bool p2p = false;
@@ -253,7 +254,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         PL.logit_rows = logit_rows, PL.n_logit_rows = n_logit_rows, PL.logits = logits_out;
         PL.logits_ld = logits_ld > 0 ? logits_ld : c.vocab;
         PL.prefetch_ahead = e->persist_ahead;
-        PL.sync = e->p_sync, PL.part_ws = e->p_ws, PL.error = e->tp_error, PL.trace = e->p_trace;
+        PL.sync = e->p_sync, PL.part_ws = e->p_ws, PL.error = e->wait_err, PL.trace = e->p_trace;
         PROF(PROF_GEMM);
         return persist_launch(PL, s);
     }
@@ -662,8 +663,6 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
         }
     }
     if (c.tp_size == 1) {
-        alloc((void**)&e->tp_error, 256);       // device-side wait bound exceeded (persistent kernel)
-        if (ok) cudaMemset(e->tp_error, 0, 256);
         alloc((void**)&e->p_layers, sizeof(PLayer) * c.n_layers);
         alloc((void**)&e->p_sync, sizeof(unsigned) * kPersistSyncWords);
         alloc((void**)&e->p_ws, persist_part_ws_bytes());
@@ -673,6 +672,7 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
     alloc((void**)&e->q, Mx * e->qdim * 2);
     alloc((void**)&e->attn, Mx * e->qdim * 2);
     alloc((void**)&e->act, Mx * (size_t)c.ffn * 2);
+    if (ok && !(e->wait_err = wait_word_alloc())) ok = false;
     if (!ok) {
         asd_engine_destroy(reinterpret_cast<asd_engine_t*>(e));
         return nullptr;
@@ -688,6 +688,7 @@ void asd_engine_destroy(asd_engine_t* h) {
                     e->p_layers, e->p_sync, e->p_ws};
     for (void* b : bufs)
         if (b) cudaFree(b);
+    wait_word_free(e->wait_err);
     delete e;
 }
 
@@ -841,9 +842,18 @@ int asd_engine_peer_connect(asd_engine_t** hs, int n) {
     return 0;
 }
 
+int asd_engine_device_error(asd_engine_t* h) {
+    Engine* e = reinterpret_cast<Engine*>(h);
+    if (!e) return set_error("asd_engine_device_error: NULL handle");
+    ASD_CUDA(cudaStreamSynchronize(nullptr));
+    return wait_word_check(e->wait_err, "asd_engine_device_error");
+}
+
 int asd_engine_tp_error(asd_engine_t* h) {
     Engine* e = reinterpret_cast<Engine*>(h);
-    if (!e || !e->tp_error) return 0;
+    if (!e) return 0;
+    if (*static_cast<const volatile int*>(e->wait_err)) return 1;
+    if (!e->tp_error) return 0;
     int v = 0, prev = 0;
     cudaGetDevice(&prev);
     if (prev != e->device) cudaSetDevice(e->device);
@@ -855,6 +865,7 @@ int asd_engine_tp_error(asd_engine_t* h) {
 int asd_engine_set_option(asd_engine_t* h, const char* name, int value) {
     Engine* e = reinterpret_cast<Engine*>(h);
     if (!e || !name) return set_error("asd_engine_set_option: NULL argument");
+    if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->wait_err, nullptr);
     if (!strcmp(name, "attn_impl")) e->attn_impl = value;
     else if (!strcmp(name, "pdl")) e->pdl = value;
     else if (!strcmp(name, "ksplit")) e->force_ksplit = value;
@@ -933,6 +944,8 @@ static int engine_forward(asd_engine_t* h, const int32_t* tokens, const int32_t*
     if ((long long)max_kv_len > (long long)e->max_pages * e->c.page_size)
         return set_error("asd_engine_forward: max_kv_len = %d exceeds the page table (%d pages of %d positions)",
                          max_kv_len, e->max_pages, e->c.page_size);
+    if (wait_word_check(e->wait_err, "asd_engine_forward")) return -1;
+    WaitScope wait_scope(e->wait_err);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (e->c.tp_size > 1 && e->p2p) {
         // the peer-memory all-reduce numbers its exchanges with a host-side epoch baked into the kernel arguments:

@@ -87,7 +87,7 @@ __device__ __forceinline__ void wait_counter(const unsigned* p, unsigned target,
     while (ld_acquire_u32(p) < target) {
         __nanosleep(20);
         if (clock64() - t0 > kPSpinLimit) {
-            *err = 1;
+            *const_cast<volatile int*>(err) = WAIT_PERSIST << 8 | 4;
             break;
         }
     }
@@ -98,7 +98,7 @@ __device__ __forceinline__ void wait_flag_eq(const unsigned* p, unsigned value, 
     while (ld_acquire_u32(p) != value) {
         __nanosleep(20);
         if (clock64() - t0 > kPSpinLimit) {
-            *err = 1;
+            *const_cast<volatile int*>(err) = WAIT_PERSIST << 8 | 4;
             break;
         }
     }
@@ -476,6 +476,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
     uint64_t* acc_empty = acc_full + 2;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
     int* s_last = reinterpret_cast<int*>(tmem_slot + 1);
+    const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 2), a.L.error, WAIT_PERSIST << 8};
     float* scratch = reinterpret_cast<float*>(tmem_slot + 4);          // [8]
     float* rstd_s = scratch + 8;                                       // [128]
     int* kvrow_s = reinterpret_cast<int*>(rstd_s + 128);               // [128]
@@ -495,6 +496,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], 4);     // lane 0 of each epilogue warp
         }
+        *guard.failed = 0;
         fence_mbar_init();
     }
     if (warp == 2) {
@@ -578,7 +580,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
                 }
                 const int tile = (int)(b_l / kb_l), k = (int)(b_l - (long long)tile * kb_l);
                 const int s = it % a.stages, round = it / a.stages;
-                if (round > 0) mbar_wait(&empty_bar[s], (round - 1) & 1);
+                if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, guard)) break;
                 mbar_expect_tx(&full_bar[s], kPWBytes);
                 tma_load_2d_hint(ring + (size_t)s * a.stage_bytes, wmap(gi_l), k * kPBlockK, tile * kPTile, &full_bar[s],
                                  pol_w);
@@ -591,12 +593,13 @@ __global__ void __launch_bounds__(kPThreads, 1)
         if (lane == 0) {
             const uint64_t pol_x = policy_evict_last();
             int it = 0;
-            for (int gi = 0; gi < n_gemms; ++gi) {
+            bool ok = true;
+            for (int gi = 0; gi < n_gemms && ok; ++gi) {
                 const GemmPhase ph = gemm_phase(gi);
                 SegIter si(ph.tiles, ph.kblocks, c, P);
                 int tile, ka, kb;
                 bool waited = false;
-                while (si.next(tile, ka, kb)) {
+                while (ok && si.next(tile, ka, kb)) {
                     if (!waited) {
                         wait_counter(a.counters + ph.phase - 1, (unsigned)P, L.error);
                         fence_proxy_async_all();     // peers' generic-proxy stores -> my async-proxy (TMA) loads
@@ -604,7 +607,8 @@ __global__ void __launch_bounds__(kPThreads, 1)
                     }
                     for (int k = ka; k < kb; ++k, ++it) {
                         const int s = it % a.stages, round = it / a.stages;
-                        if (round > 0) mbar_wait(&empty_bar[s], (round - 1) & 1);
+                        if (round > 0) ok = mbar_wait(&empty_bar[s], (round - 1) & 1, guard);
+                        if (!ok) break;
                         mbar_expect_tx(&full_bar[s], (uint32_t)ph.mt * 128u);
                         tma_load_2d_hint(ring + (size_t)s * a.stage_bytes + kPWBytes, ph.tx, k * kPBlockK, 0, &full_bar[s],
                                          pol_x);
@@ -616,19 +620,21 @@ __global__ void __launch_bounds__(kPThreads, 1)
         // ------------------------------------------------------------------ MMA issuer
         if (lane == 0) {
             int it = 0, nseg = 0;
-            for (int gi = 0; gi < n_gemms; ++gi) {
+            bool ok = true;
+            for (int gi = 0; gi < n_gemms && ok; ++gi) {
                 const GemmPhase ph = gemm_phase(gi);
                 const uint32_t idesc = umma_idesc_bf16(kPTile, ph.mt);
                 SegIter si(ph.tiles, ph.kblocks, c, P);
                 int tile, ka, kb;
-                while (si.next(tile, ka, kb)) {
+                while (ok && si.next(tile, ka, kb)) {
                     const int acc = nseg & 1, use = nseg >> 1;
-                    if (use > 0) mbar_wait(&acc_empty[acc], (use - 1) & 1);
+                    if (use > 0) ok = mbar_wait_far(&acc_empty[acc], (use - 1) & 1, guard, 1);
                     tc_fence_after();
                     const uint32_t d = tmem_base + (uint32_t)(acc * 128);
-                    for (int k = ka; k < kb; ++k, ++it) {
+                    for (int k = ka; k < kb && ok; ++k, ++it) {
                         const int s = it % a.stages, round = it / a.stages;
-                        mbar_wait(&full_bar[s], round & 1);
+                        ok = mbar_wait_far(&full_bar[s], round & 1, guard, 2);
+                        if (!ok) break;
                         tc_fence_after();
                         const uint32_t sa = smem_u32(ring + (size_t)s * a.stage_bytes);
                         const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kPWBytes);
@@ -637,7 +643,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
                             umma_f16(d, da + 2 * kk, db + 2 * kk, idesc, (uint32_t)((k > ka) | kk));
                         umma_commit(&empty_bar[s]);
                     }
-                    umma_commit(&acc_full[acc]);
+                    if (ok) umma_commit(&acc_full[acc]);
                     ++nseg;
                 }
             }
@@ -924,7 +930,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
                     }
                     const int acc = nseg & 1, use = nseg >> 1;
                     ++nseg;
-                    mbar_wait(&acc_full[acc], use & 1);
+                    mbar_wait_far(&acc_full[acc], use & 1, guard, 3);
                     tc_fence_after();
                     if (piece == 0) tstamp(1, ph.phase);
                     tstamp(2, ph.phase);
@@ -1029,6 +1035,7 @@ __global__ void __launch_bounds__(kPThreads, 1)
             if (ph.mode == PM_RESID) parts = t_h;
         }
     }
+    wait_settle(guard);
     tc_fence_before();
     __syncthreads();
     if (warp == 2) {

@@ -65,11 +65,13 @@ struct GemmArgs {
     int next_ntiles, next_ksplit, next_kblocks, next_kp;   // next_kp = k-blocks per next-kernel CTA to prefetch (0 = off)
     TpFusion tp;        // world > 1: all-reduce over peer memory inside the owner epilogue
     unsigned long long* trace;  // diagnostics: kTraceSlots globaltimer stamps per CTA (nullptr = off)
+    int* err;           // where a wait that ran out is reported
 };
 
 constexpr int kTraceSlots = 16;
+template <bool TRACE>
 __device__ __forceinline__ void trace_stamp(const GemmArgs& a, int slot) {
-    if (a.trace) {
+    if constexpr (TRACE) {
         unsigned long long t;
         asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
         const int cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -96,6 +98,8 @@ __device__ __forceinline__ void prefetch_next_weights(const GemmArgs& a, const C
     }
 }
 
+// TRACE: with the stamps.  A launch without them does not fetch their code, which pays for the bounded waits'.
+template <bool TRACE>
 __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_constant__ CUtensorMap tmap_w,
                                                                 const __grid_constant__ CUtensorMap tmap_x,
                                                                 const __grid_constant__ CUtensorMap tmap_next,
@@ -109,14 +113,15 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
     uint64_t* tmem_full = empty_bar + a.stages;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tmem_full + 1);
     uint64_t* rstd_bar = reinterpret_cast<uint64_t*>(tmem_slot + 4);
+    const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 1), a.err, WAIT_GEMM << 8};
     float* rstd_s = reinterpret_cast<float*>(rstd_bar + 1);   // [MT] per-token rstd (fused RMSNorm consumer)
     float* xbuf = rstd_s + a.MT;  // SwiGLU exchange [2][64][33] floats / sum-of-squares exchange [256 + ks*MT]
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tile_n = blockIdx.x, split = blockIdx.y, tile_m = blockIdx.z;
     if (threadIdx.x == 0) {
-        trace_stamp(a, 0);
-        if (a.trace) {
+        trace_stamp<TRACE>(a, 0);
+        if constexpr (TRACE) {
             unsigned sm;
             asm volatile("mov.u32 %0, %smid;" : "=r"(sm));
             a.trace[(size_t)(blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z)) * kTraceSlots + 9] = sm;
@@ -135,6 +140,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
         }
         mbar_init(tmem_full, 1);
         mbar_init(rstd_bar, 1);
+        *guard.failed = 0;
         fence_mbar_init();
     }
     if (warp == 1) {
@@ -145,7 +151,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
-    if (threadIdx.x == 0) trace_stamp(a, 1);
+    if (threadIdx.x == 0) trace_stamp<TRACE>(a, 1);
     // early trigger: the dependent grid becomes schedulable once every CTA of this grid is resident, so its
     // weight stream fills the SMs that this grid's tail leaves idle (it still waits before reading our output)
     if (a.early_trigger) grid_dep_launch();
@@ -166,7 +172,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
             for (int kb = 0; kb < nkb; ++kb) {
                 const int s = kb % a.stages, round = kb / a.stages;
                 if (s % nprod != pidx) continue;
-                if (round > 0) mbar_wait(&empty_bar[s], (round & 1) ^ 1);
+                if (round > 0 && !mbar_wait(&empty_bar[s], (round & 1) ^ 1, guard)) break;
                 mbar_expect_tx(&full_bar[s], stage_bytes);
                 uint8_t* st = smem + (size_t)s * stage_bytes;
                 // weights do not depend on the upstream kernel: issue them before the PDL wait
@@ -174,7 +180,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                 if (!waited) {
                     grid_dep_wait();
                     waited = true;
-                    if (pidx == 0) trace_stamp(a, 2);
+                    if (pidx == 0) trace_stamp<TRACE>(a, 2);
                 }
                 tma_load_2d_hint(st + kABytes, &tmap_x, (kb0 + kb) * kBlockK, tile_m * a.MT, &full_bar[s], pol_x);
             }
@@ -201,10 +207,10 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
         int s = 0;
         uint32_t ph = 0;
         for (int kb = 0; kb < nkb; ++kb) {
-            mbar_wait(&full_bar[s], ph);
+            const bool ready = mbar_wait(&full_bar[s], ph, guard);
             tc_fence_after();
-            if (lane == 0) {
-                if (kb == 0) trace_stamp(a, 3);
+            if (lane == 0 && ready) {
+                if (kb == 0) trace_stamp<TRACE>(a, 3);
                 const uint32_t sa = smem_u32(smem + (size_t)s * stage_bytes);
                 const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kABytes);
 #pragma unroll
@@ -221,7 +227,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
         }
         if (nkb == 0 && lane == 0) mbar_arrive(tmem_full);
         if (!a.reduce && a.next_kp > 0 && lane < 4) {   // no cluster phase: prefetch once this CTA's MMAs are done
-            mbar_wait(tmem_full, 0);
+            mbar_wait(tmem_full, 0, guard);
             prefetch_next_weights(a, &tmap_next, lane, 4);
         }
     } else {
@@ -229,13 +235,13 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
         const int q = warp & 3;                    // TMEM lane quarter this warp may read
         const int row = q * 32 + lane;             // accumulator row = weight row inside the tile
         const int m0 = tile_m * a.MT;
-        mbar_wait(tmem_full, 0);
+        mbar_wait_timed(tmem_full, 0, guard, 1);
         tc_fence_after();
-        if (threadIdx.x == 64) trace_stamp(a, 4);
+        if (threadIdx.x == 64) trace_stamp<TRACE>(a, 4);
         grid_dep_wait();     // (already satisfied) makes the upstream grid's writes to `out` visible here
         grid_dep_launch();
         const bool scale = a.norm.sumsq_in != nullptr;
-        if (scale) mbar_wait(rstd_bar, 0);
+        if (scale) mbar_wait(rstd_bar, 0, guard);
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16);
         if (a.reduce) {
             // handled below by the whole cluster
@@ -261,7 +267,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                 for (int i = 0; i < 32; ++i)
                     if (c0 + i < a.MT) T[(c0 + i) * kTileN + row] = __uint_as_float(r[i]);
             }
-            if (threadIdx.x == 64) trace_stamp(a, 5);
+            if (threadIdx.x == 64) trace_stamp<TRACE>(a, 5);
             asm volatile("bar.sync 1, 128;" ::: "memory");
             const bool wide = (a.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 #pragma unroll 1
@@ -289,7 +295,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                         if (j0 + i < a.n_valid) o[i] = __float2bfloat16(v[i]);
                 }
             }
-            if (threadIdx.x == 64) trace_stamp(a, 10);
+            if (threadIdx.x == 64) trace_stamp<TRACE>(a, 10);
         } else {
             const int n = tile_n * kTileN + row;
             for (int c0 = 0; c0 < a.MT; c0 += 32) {
@@ -397,7 +403,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                 }
             }
         }
-        if (warp < 2) mbar_wait(tmem_full, 0);  // own MMAs done => nothing reads or fills the ring any more
+        if (warp < 2) mbar_wait(tmem_full, 0, guard);  // own MMAs done => nothing reads or fills the ring any more
         tc_fence_after();
         uint8_t* recv_base = smem;               // the receive buffer overlays the (idle) tile ring ...
         if (a.recv_dedicated) {                  // ... or, for small token tiles, has its own shared memory
@@ -407,7 +413,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
             fence_proxy_async_smem();
             cluster_sync();                      // every CTA of the cluster is done with its ring
         }
-        if (threadIdx.x == 64) trace_stamp(a, 5);
+        if (threadIdx.x == 64) trace_stamp<TRACE>(a, 5);
         // receive layout in the owner: recv[src][owned column][128 rows] - the 32 lanes of a warp (32 consecutive
         // accumulator rows) write one contiguous 128-byte run per column
         if (warp >= 2) {
@@ -432,9 +438,9 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
             }
             tc_fence_before();
         }
-        if (threadIdx.x == 64) trace_stamp(a, 6);
+        if (threadIdx.x == 64) trace_stamp<TRACE>(a, 6);
         cluster_sync();
-        if (threadIdx.x == 64) trace_stamp(a, 7);
+        if (threadIdx.x == 64) trace_stamp<TRACE>(a, 7);
         // every CTA of the cluster has streamed its weights: HBM idles from here to the next kernel's first tile
         if (warp == 1 && lane < 4 && a.next_kp > 0) prefetch_next_weights(a, &tmap_next, lane, 4);
         const float* recv = reinterpret_cast<const float*>(recv_base);
@@ -473,7 +479,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                                      : "memory");
                     }
                 }
-                if (threadIdx.x == 64) trace_stamp(a, 13);
+                if (threadIdx.x == 64) trace_stamp<TRACE>(a, 13);
             }
             const float* mine = tpf ? a.tp.recv[a.tp.rank] : nullptr;
 #pragma unroll 1
@@ -555,7 +561,7 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                 }
             }
         }
-        if (threadIdx.x == 64) trace_stamp(a, 10);
+        if (threadIdx.x == 64) trace_stamp<TRACE>(a, 10);
         if ((emit || tpf) && !qkv && !vec) __trap();   // the host only asks for these on vectorisable shapes
         if (qkv && warp >= 2) {
             // bias + RoPE + q store / paged K,V append: 4 rotary pairs (dims i..i+3 and i+half..) per thread and step
@@ -611,11 +617,12 @@ __global__ void __launch_bounds__(kGemmThreads, 3) gemm_ws_kernel(const __grid_c
                 *reinterpret_cast<uint2*>(dstp + qi) = lo;
                 *reinterpret_cast<uint2*>(dstp + qi + half) = hi;
             }
-            if (threadIdx.x == 64) trace_stamp(a, 11);
+            if (threadIdx.x == 64) trace_stamp<TRACE>(a, 11);
         }
     }
+    wait_settle(guard);
     __syncthreads();
-    if (threadIdx.x == 0) trace_stamp(a, 8);
+    if (threadIdx.x == 0) trace_stamp<TRACE>(a, 8);
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, a.tmem_cols);
@@ -799,8 +806,10 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
                 const NormFusion* norm, const TpFusion* tp) {
     if (g_gemm_attr.need()) {
         if (device_props()) return -1;
-        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
-        prefer_max_smem(gemm_ws_kernel);
+        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
+        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
+        prefer_max_smem(gemm_ws_kernel<false>);
+        prefer_max_smem(gemm_ws_kernel<true>);
     }
     GemmArgs a;
     a.M = pl.M;
@@ -837,6 +846,7 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
         if ((size_t)pl.M * ldo > tp->slot_stride) return set_error("gemm: receive slot smaller than the output");
         a.tp = *tp;
     }
+    a.err = wait_word();
     a.trace = nullptr;
     if (g_gemm_trace && g_gemm_trace_next < g_gemm_trace_max) {
         a.trace = g_gemm_trace + (size_t)g_gemm_trace_next * kTraceCtas * kTraceSlots;
@@ -879,7 +889,7 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
     }
     cfg.attrs = attr;
     cfg.numAttrs = na;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, gemm_ws_kernel, tmap_w, tmap_x, *tnext, a));
+    ASD_CUDA(cudaLaunchKernelEx(&cfg, a.trace ? gemm_ws_kernel<true> : gemm_ws_kernel<false>, tmap_w, tmap_x, *tnext, a));
     count_launch(1);
     return 0;
 }
@@ -888,7 +898,7 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_gemm() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_ws_kernel));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_ws_kernel<false>));
     return 0;
 }
 

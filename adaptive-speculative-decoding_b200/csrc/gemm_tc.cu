@@ -46,6 +46,7 @@ struct TcArgs {
     void* out;
     size_t slice_stride;   // elements between the K-split slices of the fp32 output
     NormFusion norm;       // consumer side only (sumsq_in / parts / ld / hidden / eps)
+    int* err;              // where a wait that ran out is reported
 };
 
 // ---- cta_group::2 flavours of the PTX wrappers
@@ -124,6 +125,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     uint64_t* tfull_bar = empty_bar + a.stages;   // [2] accumulator ready (per CTA)
     uint64_t* tempty_bar = tfull_bar + 2;         // [2] accumulator drained (leader's copy is the one waited on)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
+    const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 1), a.err, WAIT_GEMM_PAIR << 8};
     float* rstd_s = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));   // [M]
     float* stage_t = rstd_s + ((a.norm.sumsq_in != nullptr ? a.M : 0) + 3) / 4 * 4;   // SwiGLU exchange [2][32][128]
 
@@ -144,6 +146,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             mbar_init(&tfull_bar[i], 1);
             mbar_init(&tempty_bar[i], 8);    // 4 epilogue warps x 2 CTAs
         }
+        *guard.failed = 0;
         fence_mbar_init();
     }
     if (warp == 2) {
@@ -157,7 +160,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer (both CTAs)
-        if (lane == 0) {
+        auto load = [&]() {
             // weights are shared by the m_tiles pairs that stream the same tile: keep them in L2 for those
             const uint64_t pol_w = a.m_tiles > 1 ? policy_evict_normal() : policy_evict_first();
             const uint64_t pol_x = policy_evict_last();
@@ -167,7 +170,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                 const TcUnit t = tc_unit(a, u);
                 for (int kb = 0; kb < t.nkb; ++kb, ++it) {
                     const int s = it % a.stages, round = it / a.stages;
-                    if (round > 0) mbar_wait(&empty_bar[s], (round - 1) & 1);
+                    if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, guard)) return;
                     if (leader) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
                     uint8_t* st = smem + (size_t)s * stage_bytes;
                     const uint32_t bar = full_leader + (uint32_t)s * 8u;
@@ -176,22 +179,23 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                                     t.t_tile * a.MT + (int)rank * (a.MT / 2), bar, pol_x);
                 }
             }
-        }
+        };
+        if (lane == 0) load();
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------------------------------------------ MMA issuer (leader CTA only)
-        if (leader && lane == 0) {
+        auto multiply = [&]() {
             const uint32_t idesc = umma_idesc_bf16(256, a.MT);
             int it = 0, tile = 0;
             for (int u = pair; u < units; u += npairs, ++tile) {
                 const TcUnit t = tc_unit(a, u);
                 const int acc = tile & 1, use = tile >> 1;
-                if (use > 0) mbar_wait(&tempty_bar[acc], (use - 1) & 1);
+                if (use > 0 && !mbar_wait(&tempty_bar[acc], (use - 1) & 1, guard)) return;
                 tc_fence_after();
                 const uint32_t d = tmem_base + (uint32_t)(acc * kTcAccCols);
                 for (int kb = 0; kb < t.nkb; ++kb, ++it) {
                     const int s = it % a.stages, round = it / a.stages;
-                    mbar_wait(&full_bar[s], round & 1);
+                    if (!mbar_wait(&full_bar[s], round & 1, guard)) return;
                     tc_fence_after();
                     const uint32_t sa = smem_u32(smem + (size_t)s * stage_bytes);
                     const uint64_t da = umma_desc_sw128(sa), db = umma_desc_sw128(sa + kTcABytes);
@@ -201,7 +205,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                 }
                 umma_commit_cg2(&tfull_bar[acc]);
             }
-        }
+        };
+        if (leader && lane == 0) multiply();
         __syncwarp();
     } else if (warp >= 4) {
         // ------------------------------------------------------------------ epilogue (both CTAs)
@@ -220,7 +225,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         for (int u = pair; u < units; u += npairs, ++tile) {
             const TcUnit t = tc_unit(a, u);
             const int acc = tile & 1, use = tile >> 1;
-            mbar_wait(&tfull_bar[acc], use & 1);
+            mbar_wait_timed(&tfull_bar[acc], use & 1, guard, 1);
             tc_fence_after();
             if (tile == 0) grid_dep_launch();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTcAccCols);
@@ -290,6 +295,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             if (lane == 0) mbar_arrive_cluster(tempty_leader + (uint32_t)acc * 8u);
         }
     }
+    wait_settle(guard);
     tc_fence_before();
     cluster_sync();      // the leader's MMAs read the peer's shared memory and both CTAs' TMEM until here
     if (warp == 2) {
@@ -401,6 +407,7 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.out = out;
     a.slice_stride = slice_stride;
     a.norm = norm ? *norm : NormFusion{};
+    a.err = wait_word();
     gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, a);
     ASD_CUDA(cudaGetLastError());
     count_launch(1);

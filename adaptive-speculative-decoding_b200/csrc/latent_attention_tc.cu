@@ -73,13 +73,19 @@ struct LtBars {
     int failed;
 };
 
+__device__ __forceinline__ void lt_report(LtBars* B, int* err) {
+    *reinterpret_cast<volatile int*>(&B->failed) = 1;
+    if (err) {
+        *const_cast<volatile int*>(err) = WAIT_LATENT << 8 | 1;
+        __threadfence_system();
+    }
+}
 __device__ __forceinline__ bool lt_wait(uint64_t* bar, uint32_t parity, LtBars* B, int* err) {
     for (uint32_t i = 0; i < kLtSpin; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*reinterpret_cast<volatile int*>(&B->failed)) return false;
     }
-    *reinterpret_cast<volatile int*>(&B->failed) = 1;
-    if (err) atomicExch(err, 1);
+    lt_report(B, err);
     return false;
 }
 // the same by a whole warp, one answer for all lanes: what follows stays uniform
@@ -88,8 +94,7 @@ __device__ __forceinline__ bool lt_wait_warp(uint64_t* bar, uint32_t parity, LtB
         if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
         if (__any_sync(0xffffffffu, *reinterpret_cast<volatile int*>(&B->failed))) return false;
     }
-    *reinterpret_cast<volatile int*>(&B->failed) = 1;
-    if (err) atomicExch(err, 1);
+    lt_report(B, err);
     return false;
 }
 // a place in a ring of barriers and the parity of its current round

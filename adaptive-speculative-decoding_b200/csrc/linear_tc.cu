@@ -49,7 +49,10 @@ __device__ __forceinline__ bool wait_bounded(uint64_t* bar, uint32_t parity, vol
     for (uint32_t i = 0; i < kSpinLimit; ++i)
         if (mbar_try_wait(bar, parity)) return true;
     *failed = 1;
-    if (err) atomicExch(err, 1);
+    if (err) {
+        *const_cast<volatile int*>(err) = WAIT_LINEAR << 8 | 1;
+        __threadfence_system();
+    }
     return false;
 }
 

@@ -293,8 +293,7 @@ asd_lukopel_engine_t* asd_lukopel_create(const asd_lukopel_config* cfg, const as
     rc |= dev_alloc(e, &e->attn_ws.part, (size_t)e->attn_ws.part_elems);
     e->attn_ws.score_elems = 8ll << 20;      // scores of steps of few tokens: tokens x heads x keys
     rc |= dev_alloc(e, &e->attn_ws.scores, (size_t)e->attn_ws.score_elems);
-    rc |= dev_alloc(e, &e->dev_error, 1);
-    if (!rc && cudaMemset(e->dev_error, 0, sizeof(int)) != cudaSuccess) rc = -1;
+    if (!rc && !(e->dev_error = wait_word_alloc())) rc = -1;
     if (rc) {
         asd_lukopel_destroy(e);
         return nullptr;
@@ -306,6 +305,7 @@ void asd_lukopel_destroy(asd_lukopel_engine_t* h) {
     LkEngine* e = static_cast<LkEngine*>(h);
     if (!e) return;
     for (void* p : e->owned) cudaFree(p);
+    wait_word_free(e->dev_error);
     delete e;
 }
 
@@ -354,6 +354,7 @@ int asd_lukopel_set_cache(asd_lukopel_engine_t* h, void* pool, int num_pages, co
 int asd_lukopel_set_option(asd_lukopel_engine_t* h, const char* name, int value) {
     LkEngine* e = static_cast<LkEngine*>(h);
     if (!e || !name) return set_error("asd_lukopel_set_option: NULL argument");
+    if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
     if (!strcmp(name, "tc_linear")) {
         e->dn.tc_linear = value;
         return 0;
@@ -404,6 +405,8 @@ int asd_lukopel_forward(asd_lukopel_engine_t* h, const int32_t* tokens, const in
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != e->device) return set_error("asd_lukopel_forward: called on device %d, engine lives on %d", dev, e->device);
+    if (wait_word_check(e->dev_error, "asd_lukopel_forward")) return -1;
+    WaitScope wait_scope(e->dev_error);
     const LkBatch b{SeqIndex{tokens, positions, token_slot, M}, cu_q, seq_slot, nseq, max_qlen, max_kv_len};
     return forward(e, b, logit_rows, logit_rows ? n_logit_rows : (n_logit_rows > 0 ? M : 0), logits_out, logits_ld,
                    layer_out, static_cast<cudaStream_t>(stream));
@@ -419,10 +422,8 @@ int asd_lukopel_profile_read(asd_lukopel_engine_t* h, float* ms_by_class, int* l
 int asd_lukopel_device_error(asd_lukopel_engine_t* h) {
     LkEngine* e = static_cast<LkEngine*>(h);
     if (!e) return set_error("asd_lukopel_device_error: NULL engine");
-    int v = 0;
-    ASD_CUDA(cudaMemcpy(&v, e->dev_error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v) return set_error("a Lukopel kernel gave up a bounded wait (tcgen05 linear)");
-    return 0;
+    ASD_CUDA(cudaStreamSynchronize(nullptr));
+    return wait_word_check(e->dev_error, "asd_lukopel_device_error");
 }
 
 }  // extern "C"

@@ -505,8 +505,7 @@ asd_mavipel_engine_t* asd_mavipel_create(const asd_mavipel_config* cfg, const as
         e->attn_ws.rows = (long long)MT;
         if (!rc && cudaMemset(e->attn_ws.ml, 0, MT * sizeof(float)) != cudaSuccess) rc = -1;
     }
-    rc |= dev_alloc(e, &e->dev_error, 1);
-    if (!rc && cudaMemset(e->dev_error, 0, sizeof(int)) != cudaSuccess) rc = -1;
+    if (!rc && !(e->dev_error = wait_word_alloc())) rc = -1;
     if (rc) {
         asd_mavipel_destroy(e);
         return nullptr;
@@ -518,6 +517,7 @@ void asd_mavipel_destroy(asd_mavipel_engine_t* h) {
     MvEngine* e = static_cast<MvEngine*>(h);
     if (!e) return;
     for (void* p : e->owned) cudaFree(p);
+    wait_word_free(e->dev_error);
     delete e;
 }
 
@@ -581,6 +581,7 @@ int asd_mavipel_set_cache(asd_mavipel_engine_t* h, void* pool, int num_pages, co
 int asd_mavipel_set_option(asd_mavipel_engine_t* h, const char* name, int value) {
     MvEngine* e = static_cast<MvEngine*>(h);
     if (!e || !name) return set_error("asd_mavipel_set_option: NULL argument");
+    if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
     if (!strcmp(name, "tc_linear")) {
         e->dn.tc_linear = value;
         return 0;
@@ -625,6 +626,8 @@ int asd_mavipel_forward(asd_mavipel_engine_t* h, const int32_t* tokens, const in
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != e->device) return set_error("asd_mavipel_forward: called on device %d, engine lives on %d", dev, e->device);
+    if (wait_word_check(e->dev_error, "asd_mavipel_forward")) return -1;
+    WaitScope wait_scope(e->dev_error);
     const Batch b{SeqIndex{tokens, positions, token_slot, M}, cu_q, seq_slot, nseq, max_qlen, max_kv_len};
     return forward(e, b, logit_rows, logit_rows ? n_logit_rows : (n_logit_rows > 0 ? M : 0), logits_out, logits_ld,
                    layer_out, static_cast<cudaStream_t>(stream));
@@ -640,10 +643,8 @@ int asd_mavipel_profile_read(asd_mavipel_engine_t* h, float* ms_by_class, int* l
 int asd_mavipel_device_error(asd_mavipel_engine_t* h) {
     MvEngine* e = static_cast<MvEngine*>(h);
     if (!e) return set_error("asd_mavipel_device_error: NULL engine");
-    int v = 0;
-    ASD_CUDA(cudaMemcpy(&v, e->dev_error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v) return set_error("a Mavipel kernel gave up a bounded wait (tcgen05 linear)");
-    return 0;
+    ASD_CUDA(cudaStreamSynchronize(nullptr));
+    return wait_word_check(e->dev_error, "asd_mavipel_device_error");
 }
 
 }  // extern "C"

@@ -35,9 +35,77 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
-__device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
-    while (!mbar_try_wait(bar, parity)) {
+// Waits that end.  In every kernel the role that all the others end up waiting for has a clock: it gives up after `ticks` steps
+// of 2^32 cycles of the SM (at least 8.7 s at 1.965 GHz), far above any legitimate wait (a programmatically launched kernel waits
+// here for all of its predecessor, an exchange with another GPU of two seconds included), and reports it.  All waits of that CTA
+// then end: loaders and MMA issuers stop issuing, the others walk through (what they write is invalid and reported as such), and
+// the CTA calls wait_settle() before its shared memory and TMEM go to the next one.
+// The form matters, since a launch fetches every instruction on its way: a counter or the flag in a loop of plain tries cost the
+// GEMMs 1 to 3 % (16 and 96 tokens of four and three layers, prompts of the Rivetar layers), a call from their loops 2 to 4 %.
+// Tries with a time hint stay asleep in one instruction, so the loops below are hardly entered.
+struct WaitGuard {
+    volatile int* failed;      // in shared memory, zero before the first wait
+    int* err;                  // mapped host memory (may be null)
+    int kernel;                // WaitKernel << 8
+    uint32_t ticks = 4;
+};
+__device__ __forceinline__ bool mbar_try_long(uint64_t* bar, uint32_t parity) {        // up to 10 ms, as the hardware allows
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(10000000u)
+        : "memory");
+    return ok != 0;
+}
+__device__ __forceinline__ uint32_t clock_steps() {
+    uint32_t t;
+    asm volatile("mov.u32 %0, %%clock_hi;" : "=r"(t));
+    return t;
+}
+__device__ __forceinline__ void wait_report(volatile int* failed, int* err, int code) {
+    *failed = 1;
+    if (err) {
+        *const_cast<volatile int*>(err) = code;
+        __threadfence_system();
     }
+}
+// without a clock: ends when the barrier completes or another wait of the CTA has given up
+__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, const WaitGuard& g) {
+    if (mbar_try_long(bar, parity)) return true;
+    do {
+        if (*g.failed) return false;
+    } while (!mbar_try_long(bar, parity));
+    return true;
+}
+__device__ __forceinline__ bool mbar_wait_timed(uint64_t* bar, uint32_t parity, const WaitGuard& g, int place) {
+    if (mbar_try_long(bar, parity)) return true;
+    const uint32_t t0 = clock_steps();
+    do {
+        if (*g.failed) return false;
+        if (clock_steps() - t0 > g.ticks) {
+            wait_report(g.failed, g.err, g.kernel | place);
+            return false;
+        }
+    } while (!mbar_try_long(bar, parity));
+    return true;
+}
+// the same out of line, for kernels with many such waits off their critical path
+static __device__ __noinline__ bool mbar_wait_clock(uint64_t* bar, uint32_t parity, volatile int* failed, int* err, int code,
+                                                    uint32_t ticks) {
+    const WaitGuard g{failed, err, code, ticks};
+    return mbar_wait_timed(bar, parity, g, 0);
+}
+__device__ __forceinline__ bool mbar_wait_far(uint64_t* bar, uint32_t parity, const WaitGuard& g, int place) {
+    return mbar_try_wait(bar, parity) || mbar_wait_clock(bar, parity, g.failed, g.err, g.kernel | place, g.ticks);
+}
+static __device__ __noinline__ void wait_settle_some() {      // copies and products land within microseconds
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+}
+__device__ __forceinline__ void wait_settle(const WaitGuard& g) {
+    if (*g.failed) wait_settle_some();
 }
 
 // ---------------------------------------------------------------- async-proxy copies

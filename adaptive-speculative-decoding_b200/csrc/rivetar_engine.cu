@@ -431,8 +431,7 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     e->attn_ws.o_elems = e->attn_ws.rows * 512;
     rc |= dev_alloc(e, &e->attn_ws.o, (size_t)e->attn_ws.o_elems);
     rc |= dev_alloc(e, &e->attn_ws.ml, (size_t)e->attn_ws.rows * 2);
-    rc |= dev_alloc(e, &e->dev_error, 1);
-    if (!rc && cudaMemset(e->dev_error, 0, sizeof(int)) != cudaSuccess) rc = -1;
+    if (!rc && !(e->dev_error = wait_word_alloc())) rc = -1;
     if (rc) {
         asd_rivetar_destroy(e);
         return nullptr;
@@ -444,6 +443,7 @@ void asd_rivetar_destroy(asd_rivetar_engine_t* h) {
     RvEngine* e = static_cast<RvEngine*>(h);
     if (!e) return;
     for (void* p : e->owned) cudaFree(p);
+    wait_word_free(e->dev_error);
     delete e;
 }
 
@@ -501,6 +501,7 @@ int asd_rivetar_set_cache(asd_rivetar_engine_t* h, void* pool, int num_pages, co
 int asd_rivetar_set_option(asd_rivetar_engine_t* h, const char* name, int value) {
     RvEngine* e = static_cast<RvEngine*>(h);
     if (!e || !name) return set_error("asd_rivetar_set_option: NULL argument");
+    if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
     if (!strcmp(name, "tc_linear")) {
         e->dn.tc_linear = value;
         return 0;
@@ -550,6 +551,8 @@ int asd_rivetar_forward(asd_rivetar_engine_t* h, const int32_t* tokens, const in
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev != e->device) return set_error("asd_rivetar_forward: called on device %d, engine lives on %d", dev, e->device);
+    if (wait_word_check(e->dev_error, "asd_rivetar_forward")) return -1;
+    WaitScope wait_scope(e->dev_error);
     const Batch b{SeqIndex{tokens, positions, token_slot, M}, cu_q, seq_slot, nseq, max_qlen, max_kv_len};
     return forward(e, b, logit_rows, logit_rows ? n_logit_rows : (n_logit_rows > 0 ? M : 0), logits_out, logits_ld,
                    layer_out, static_cast<cudaStream_t>(stream));
@@ -565,10 +568,8 @@ int asd_rivetar_profile_read(asd_rivetar_engine_t* h, float* ms_by_class, int* l
 int asd_rivetar_device_error(asd_rivetar_engine_t* h) {
     RvEngine* e = static_cast<RvEngine*>(h);
     if (!e) return set_error("asd_rivetar_device_error: NULL engine");
-    int v = 0;
-    ASD_CUDA(cudaMemcpy(&v, e->dev_error, sizeof(int), cudaMemcpyDeviceToHost));
-    if (v) return set_error("a Rivetar kernel gave up a bounded wait (tcgen05 linear)");
-    return 0;
+    ASD_CUDA(cudaStreamSynchronize(nullptr));
+    return wait_word_check(e->dev_error, "asd_rivetar_device_error");
 }
 
 }  // extern "C"

@@ -72,6 +72,7 @@ struct SamplerParams {
     float* row_px;      // [rows] chunk-relative e_p of the draft token
     float* row_qx;      // [rows] chunk-relative e_q of the draft token
     float* seq_rc;      // [B][NC] residual chunk totals of the emitting row
+    int* err;           // where a wait that ran out is reported
 };
 
 __device__ __forceinline__ float exp2p(float t) {
@@ -155,6 +156,8 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
     __shared__ __align__(16) float2 s_red[2][kSW];        // (the record of an item is written while the next one's maxima arrive)
     __shared__ float s_own2[kSW], s_red2[kSW][3];
     __shared__ unsigned long long s_key[kSW];
+    __shared__ int s_failed;
+    const WaitGuard guard{&s_failed, p.err, WAIT_SAMPLER << 8};
     grid_dep_launch();      // the draw kernel may be scheduled; it waits for this grid before reading anything
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int total = p.B * (p.k + 1) * p.NC;
@@ -177,6 +180,7 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
     if (tid == 0) {
 #pragma unroll
         for (int st = 0; st < kStages; ++st) mbar_init(&s_bar[st], 1);
+        s_failed = 0;
         fence_mbar_init();
 #pragma unroll
         for (int st = 0; st < kStages; ++st)
@@ -188,7 +192,7 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
         const int st = it % kStages;
         const float4* zt = s_ring + st * kPair;
         const float4* zq = zt + kChunk / 4;
-        mbar_wait(&s_bar[st], (it / kStages) & 1);
+        mbar_wait_far(&s_bar[st], (it / kStages) & 1, guard, 1);
         const int4 what = s_item[st];
         const int n4 = what.z & 0xffff;
         const bool has_draft = !GREEDY && (what.z >> 16);
@@ -295,7 +299,7 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
         __syncthreads();            // every thread is done with the stage
         if (tid == 0) {
             fence_proxy_async_smem();   // generic reads of the stage ordered before the async-proxy writes of the next copy
-            if (item + (long long)kStages * gridDim.x < total) issue(item + kStages * gridDim.x, st);
+            if (item + (long long)kStages * gridDim.x < total && !*guard.failed) issue(item + kStages * gridDim.x, st);
             float Z = 0.0f, S = 0.0f, Zq = 0.0f, m2 = -INFINITY;
             unsigned long long kk = ~0ull;
             bool seen = false;          // the first warp that attains the maximum is the owner, the others are runners-up
@@ -315,6 +319,7 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
             p.rec_q[at] = make_float4(mq, Zq, __uint_as_float((unsigned)(kk & 0xffffffffu)), __int_as_float((int)(kk >> 32)));
         }
     }
+    wait_settle(guard);
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 2
@@ -467,14 +472,16 @@ __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParam
     __shared__ float4 s_stat[kMaxRows];
     __shared__ int s_acc[kMaxRows], s_amax[kMaxRows];
     __shared__ float s_lpx[kMaxRows], s_lpamax[kMaxRows];
-    __shared__ int s_flag, s_cstar, s_tstar[kSW];
+    __shared__ int s_flag, s_cstar, s_tstar[kSW], s_failed;
     __shared__ float s_tau;
+    const WaitGuard guard{&s_failed, p.err, WAIT_SAMPLER << 8};
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int k1 = p.k + 1, NC = p.NC, G = p.G;
     const int b = blockIdx.x / G, g = blockIdx.x - b * G;
     if (tid == 0) {
         mbar_init(&s_bar[0], 1);
         mbar_init(&s_bar[1], 1);
+        s_failed = 0;
         fence_mbar_init();
     }
     grid_dep_wait();
@@ -530,20 +537,21 @@ __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParam
     float rs = 0.0f, hs;
     int c = g, it = 0;
     for (;; c += G, ++it) {
-        mbar_wait(&s_bar[it & 1], (it >> 1) & 1);
+        mbar_wait_far(&s_bar[it & 1], (it >> 1) & 1, guard, 2);
         rs = residual_chunk(p, row, c, has_draft, s_ring + (it & 1) * (kChunk / 2), st, zt, zq, have);
         hs = warp_hs(rs, lane);
         if (lane == 31) s_red[it & 1][warp] = hs;
         __syncthreads();
         if (tid == 0) {
             fence_proxy_async_smem();
-            if (c + 2 * G < NC) issue(c + 2 * G, it & 1);
+            if (c + 2 * G < NC && !*guard.failed) issue(c + 2 * G, it & 1);
             float R = 0.0f;
             for (int w = 0; w < kSW; ++w) R = __fadd_rn(R, s_red[it & 1][w]);
             __stcg(&p.seq_rc[(size_t)b * NC + c], R);
         }
         if (c + G >= NC) break;
     }
+    wait_settle(guard);
     if (tid == 0) {
         __threadfence();
         s_flag = atomicAdd(&p.seq_ticket[b], 1) == G - 1;
@@ -603,8 +611,8 @@ __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParam
     }
     if (cstar != c) {           // the other stage is free: its chunk was consumed before this one
         ++it;
-        if (tid == 0) issue(cstar, it & 1);
-        mbar_wait(&s_bar[it & 1], (it >> 1) & 1);
+        if (tid == 0 && !*guard.failed) issue(cstar, it & 1);
+        mbar_wait_far(&s_bar[it & 1], (it >> 1) & 1, guard, 3);
         rs = residual_chunk(p, row, cstar, has_draft, s_ring + (it & 1) * (kChunk / 2), st, zt, zq, have);
     }
     hs = warp_hs(rs, lane);
@@ -705,6 +713,11 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     p.out_tokens = out_tokens;
     p.out_logprobs = out_logprobs;
     p.features = features;
+    p.err = device_wait_word();
+    if (wait_word_check(p.err, "asd_reject_sample")) {      // reported once
+        *static_cast<volatile int*>(p.err) = 0;
+        return -1;
+    }
     uint8_t* ws = static_cast<uint8_t*>(workspace);
     size_t off = 0;
     auto take = [&](size_t bytes) {

@@ -349,6 +349,10 @@ class QwenEngine(_BatchOps):
     def tp_error(self) -> int:
         return int(lib().asd_engine_tp_error(self.h))
 
+    def check_device(self) -> None:
+        """raises if a kernel of this engine gave up a bounded wait (synchronises)"""
+        check(lib().asd_engine_device_error(self.h), "asd_engine_device_error")
+
     def set_allreduce(self, comm_ptr: int, fn_ptr: int):
         check(lib().asd_engine_set_allreduce(self.h, ctypes.c_void_p(comm_ptr), ctypes.c_void_p(fn_ptr)),
               "asd_engine_set_allreduce")
@@ -939,6 +943,11 @@ class TPQwenEngine(_BatchOps):
     def tp_error(self) -> int:
         return max(e.tp_error() for e in self.ranks)
 
+    def check_device(self) -> None:
+        for e in self.ranks:
+            with torch.cuda.device(e.device):
+                e.check_device()
+
     def profile_read(self):
         return self.ranks[0].profile_read()
 
@@ -1161,9 +1170,7 @@ class SpecDecoder:
             host_accepted.copy_(out["accepted_len"], non_blocking=True)
             host_state.copy_(torch.stack([self.last_tok, self.prev_tok, self.pos]), non_blocking=True)
             torch.cuda.current_stream().synchronize()
-        for e in (self.t, self.d):
-            if e is not None and getattr(e, "tp_size", 1) > 1 and e.tp_error():
-                raise AsdError("tensor-parallel peer did not answer within the spin bound (asd_engine_tp_error)")
+        self._check_device()
         return host_tokens, host_accepted
 
     def generate(self, prompts, max_new_tokens: int):
@@ -1210,10 +1217,19 @@ class SpecDecoder:
             feats_dev = feats[:, :n].contiguous()      # stays on the device for asd_cascade_decide (scorer -> stop rule)
             res = (toks[:, :n].cpu(), lps[:, :n].cpu(), feats_dev.cpu(),
                    {"accepted": int(accepted.item()), "steps": steps, "features_device": feats_dev})
-        for e in (self.t, self.d):
-            if e is not None and getattr(e, "tp_size", 1) > 1 and e.tp_error():
-                raise AsdError("tensor-parallel peer did not answer within the spin bound (asd_engine_tp_error)")
+        self._check_device()
         return res
+
+    def _check_device(self):
+        """before results go to the host: raises if a kernel that made them gave up a wait"""
+        with torch.cuda.device(self.device):
+            check(lib().asd_wait_error(), "asd_reject_sample")
+        for e in (self.t, self.d):
+            if e is None:
+                continue
+            if getattr(e, "tp_size", 1) > 1 and e.tp_error():
+                raise AsdError("tensor-parallel peer did not answer within the spin bound (asd_engine_tp_error)")
+            e.check_device()
 
     def _sample_rows_strided(self, i: int) -> torch.Tensor:
         # the fused sampler wants contiguous rows: draft step i wrote rows with stride k*V

@@ -99,6 +99,7 @@ def run(model_dir: str, dtype: str, out_dir: str, max_tokens: int, stdin=None, s
         logits = sess.step(req.get("entries", []), req.get("end", []))
         if logits is not None:
             data = logits.detach().to("cpu", torch.float32).contiguous().numpy().astype("<f4", copy=False)
+            sess.engine.check_device()
             tmp = os.path.join(out_dir, f".{req['step']}.part")
             with open(tmp, "wb") as f:
                 f.write(data.tobytes())

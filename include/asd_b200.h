@@ -37,6 +37,13 @@ ASD_API const char* asd_last_error(void);
 /* number of kernels this library has launched since load / since the last reset (bench "gpu_launches") */
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
+/* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:
+ * engines then refuse every later forward (asd_*_device_error names the kernel), a sampler call is refused once.
+ * asd_wait_error reports and clears what calls without an engine (sampler, asd_linear_*) left on the current device; it does
+ * not synchronise. */
+ASD_API int asd_wait_error(void);
+/* diagnostics: a kernel whose wait runs out after two seconds and is reported like any other (engines: option "debug_wait") */
+ASD_API int asd_debug_wait_expiry(void* stream);
 
 /* ---------------------------------------------------------------------------------------------
  * Fused logits -> softmax -> rejection sampling -> residual resample -> stop-rule features.
@@ -175,10 +182,12 @@ ASD_API int asd_engine_set_allreduce(asd_engine_t* e, void* comm, void* nccl_all
  * receive buffers; option "tp_fused", default at 2 ranks / small exchanges) or are followed by ONE kernel that
  * all-reduces through P2P loads (one-shot, or two-shot with a home rank per row: option "tp_two_shot"), adds the
  * residual and emits the norm statistics.  All paths give bit-identical residuals on every rank.
- * asd_engine_tp_error returns 1 if a peer ever failed to show up within the spin bound. */
+ * asd_engine_tp_error returns 1 if a peer ever failed to show up within the spin bound, or a kernel gave up a wait. */
 ASD_API int asd_engine_ipc_export(asd_engine_t* e, void* handles_out);
 ASD_API int asd_engine_ipc_import(asd_engine_t* e, const void* all_handles);
 ASD_API int asd_engine_tp_error(asd_engine_t* e);
+/* non-zero (and an error message) if a kernel of this engine gave up a bounded wait since creation; synchronises */
+ASD_API int asd_engine_device_error(asd_engine_t* e);
 /* In-process tensor parallelism (what Stage(tensor_parallel_size = t, gpu_ids = [...]) builds, mirroring
  * configs/qwen3_models.yaml:10-51 and src/serving/real_model_pipeline.py:98-108): the t rank engines were created in
  * ONE process, rank r on its own device.  Enables peer access between the devices and wires every rank's receive
