@@ -92,17 +92,28 @@ __device__ __forceinline__ bool mbar_wait_timed(uint64_t* bar, uint32_t parity, 
     } while (!mbar_try_long(bar, parity));
     return true;
 }
-// the same out of line, for kernels with many such waits off their critical path
+// the same out of line and by plain tries, for kernels of few waits
 static __device__ __noinline__ bool mbar_wait_clock(uint64_t* bar, uint32_t parity, volatile int* failed, int* err, int code,
                                                     uint32_t ticks) {
-    const WaitGuard g{failed, err, code, ticks};
-    return mbar_wait_timed(bar, parity, g, 0);
+    const uint32_t t0 = clock_steps();
+    while (!mbar_try_wait(bar, parity)) {
+        if (*failed) return false;
+        if (clock_steps() - t0 > ticks) {
+            wait_report(failed, err, code);
+            return false;
+        }
+    }
+    return true;
 }
 __device__ __forceinline__ bool mbar_wait_far(uint64_t* bar, uint32_t parity, const WaitGuard& g, int place) {
     return mbar_try_wait(bar, parity) || mbar_wait_clock(bar, parity, g.failed, g.err, g.kernel | place, g.ticks);
 }
-static __device__ __noinline__ void wait_settle_some() {      // copies and products land within microseconds
-    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+// Copies and products land within microseconds: a millisecond.  (By the clock: with a nanosleep in their code the sampler's kernels
+// took 20 us a call instead of 15 where the host is the slower side.)
+static __device__ __noinline__ void wait_settle_some() {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {
+    }
 }
 __device__ __forceinline__ void wait_settle(const WaitGuard& g) {
     if (*g.failed) wait_settle_some();
