@@ -26,7 +26,7 @@ enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, W
 int* wait_word_alloc();                                 // a zeroed word that every device and stream can write, or nullptr
 void wait_word_free(int* word);
 int wait_word_check(const int* word, const char* who);  // 0, or the error that names the kernel and the place
-int* device_wait_word();                                // of the current device: calls that belong to no engine
+int* device_wait_word(int dev = -1);                    // of a device (-1: the current one): calls that belong to no engine
 int launch_wait_expiry(int* word, cudaStream_t stream); // a wait that runs out (two seconds), for the tests of what follows
 extern thread_local int* g_wait_word;
 inline int* wait_word() { return g_wait_word ? g_wait_word : device_wait_word(); }

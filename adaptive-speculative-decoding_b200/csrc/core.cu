@@ -85,14 +85,16 @@ int launch_wait_expiry(int* word, cudaStream_t stream) {
     ASD_CUDA(cudaGetLastError());
     return 0;
 }
-int* device_wait_word() {
-    static int* words[64] = {};
+int* device_wait_word(int dev) {
+    static std::atomic<int*> words[64] = {};
+    if (dev < 0 && cudaGetDevice(&dev) != cudaSuccess) return nullptr;
+    if (dev < 0 || dev >= 64) return nullptr;
+    int* w = words[dev].load(std::memory_order_acquire);
+    if (w) return w;
     static std::mutex m;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(m);
-    if (!words[dev]) words[dev] = wait_word_alloc();
-    return words[dev];
+    if (!words[dev].load(std::memory_order_relaxed)) words[dev].store(wait_word_alloc(), std::memory_order_release);
+    return words[dev].load(std::memory_order_relaxed);
 }
 
 }  // namespace asd

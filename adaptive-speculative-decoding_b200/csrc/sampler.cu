@@ -15,7 +15,8 @@
 //     binary64 and finds the first-reject prefix: repeating this in the G CTAs is cheaper than tickets between them.  The
 //     first of them writes the features and accepted tokens.  Then the ONE row that emits a new token: residual
 //     max(0, p - q) chunk totals; the last CTA of the sequence walks the totals, re-reads the selected chunk (L2) and
-//     finishes the inverse-CDF draw inside it.  Greedy verification needs the merge only (G = 1).
+//     finishes the inverse-CDF draw inside it.  Greedy verification needs the merge only (G = 1), and where
+//     its items all fit the chip at once the first kernel's last CTA of a sequence does it: one launch.
 // DRAM traffic = (1 + ~1/(k+1)) x the algorithmic bytes.
 // Measured (V = 152064, all outputs the same bits), the CTA-per-item form -> this one: B = 64, k = 8: 195 -> 163 us (the
 // first kernel 176 -> 132 us, 5.0 TB/s; what is left is its 10 cycles per issued instruction at 24 warps, six of them a
@@ -58,6 +59,7 @@ struct SamplerParams {
     const double* u_resid;     // [B]
     int B, k, V, NC, greedy;
     int G;                     // CTAs of the draw kernel per sequence
+    int fused;                 // greedy, an item per CTA: the sequence's last CTA merges in the first kernel
     float c1;
     // outputs
     uint8_t* accept_mask;
@@ -144,6 +146,143 @@ __device__ __forceinline__ void exp4(float4& z, float2 c1v, float2 nmv, float2& 
     z = make_float4(e0.x, e0.y, e1.x, e1.y);
 }
 
+// One row's statistics from its chunk records, by one warp (lanes = chunks lane and lane + 32; every sum is chained in
+// chunk order): {M, Zp, Mq, Zq}, whether the draft token is accepted, and - `write` - the row's features.
+struct RowMerge {
+    float4 stat;
+    int accept, amax;
+    float lpx, lp_amax;
+};
+__device__ __forceinline__ RowMerge merge_row(const SamplerParams& p, int b, int i, int lane, bool write) {
+    const unsigned all = 0xffffffffu;
+    const int NC = p.NC, row = b * (p.k + 1) + i;
+    const bool has_draft = i < p.k && !p.greedy;
+    const float4 none = make_float4(-INFINITY, -INFINITY, 0.f, 0.f);
+    float4 rp[2], rq[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const bool ok = lane + 32 * u < NC;
+        rp[u] = ok ? __ldcg(&p.rec_p[(size_t)row * NC + lane + 32 * u]) : none;
+        rq[u] = ok ? __ldcg(&p.rec_q[(size_t)row * NC + lane + 32 * u]) : none;
+    }
+    const int x = i < p.k ? p.draft_tokens[b * p.k + i] : -1;
+    const bool x_ok = i < p.k && x >= 0 && x < p.V;
+    const float px = x_ok ? __ldcg(&p.row_px[row]) : 0.0f, qx = x_ok && has_draft ? __ldcg(&p.row_qx[row]) : 0.0f;
+    const double u_acc = has_draft ? p.u_accept[b * p.k + i] : 0.0;
+    float M = fmaxf(rp[0].x, rp[1].x), M2 = fmaxf(fminf(rp[0].x, rp[1].x), fmaxf(rp[0].y, rp[1].y));
+    float Mq = fmaxf(rq[0].x, rq[1].x);
+#pragma unroll
+    for (int d = 16; d >= 1; d >>= 1) {
+        const float o1 = __shfl_xor_sync(all, M, d), o2 = __shfl_xor_sync(all, M2, d);
+        M2 = fmaxf(fminf(M, o1), fmaxf(M2, o2));
+        M = fmaxf(M, o1);
+        Mq = fmaxf(Mq, __shfl_xor_sync(all, Mq, d));
+    }
+    float sc[2], tz[2], ts[2], sq[2], tq[2];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const float d = __fadd_rn(rp[u].x, -M);
+        sc[u] = exp2p(d);
+        tz[u] = __fmul_rn(rp[u].z, sc[u]);
+        ts[u] = __fmul_rn(__fmaf_rn(rp[u].z, d, rp[u].w), sc[u]);
+        sq[u] = exp2p(__fadd_rn(rq[u].x, -Mq));
+        tq[u] = __fmul_rn(rq[u].y, sq[u]);
+    }
+    float Zp = 0.0f, St = 0.0f, Zq = 0.0f;
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+#pragma unroll 8
+        for (int c = 0; c < min(32, NC - 32 * u); ++c) {
+            Zp = __fadd_rn(Zp, __shfl_sync(all, tz[u], c));
+            St = __fadd_rn(St, __shfl_sync(all, ts[u], c));
+            Zq = __fadd_rn(Zq, __shfl_sync(all, tq[u], c));
+        }
+    if (!has_draft) Zq = 0.0f;
+    const int cx = x_ok ? x / kChunk : 0;
+    const float s_x = __shfl_sync(all, cx < 32 ? sc[0] : sc[1], cx & 31);
+    const float sq_x = __shfl_sync(all, cx < 32 ? sq[0] : sq[1], cx & 31);
+    RowMerge r;
+    r.stat = make_float4(M, Zp, Mq, Zq);
+    const float Px = x_ok ? __fmul_rn(px, s_x) : 0.0f;
+    r.amax = -1;
+    float P_amax = 0.0f;
+    if (p.greedy) {             // the first chunk that attains the row maximum holds its lowest index
+        const unsigned h0 = __ballot_sync(all, rp[0].x == M && lane < NC), h1 = __ballot_sync(all, rp[1].x == M && lane + 32 < NC);
+        if (h0 | h1) {
+            const int src = h0 ? __ffs(h0) - 1 : __ffs(h1) - 1;
+            r.amax = __shfl_sync(all, __float_as_int(h0 ? rq[0].w : rq[1].w), src);
+            P_amax = __shfl_sync(all, h0 ? __fmul_rn(rq[0].z, sc[0]) : __fmul_rn(rq[1].z, sc[1]), src);
+        }
+    }
+    r.accept = 0;
+    if (p.greedy) {
+        r.accept = x_ok && x == r.amax;
+    } else if (has_draft && x_ok) {
+        const float Qx = __fmul_rn(qx, sq_x);
+        const double lhs = __dmul_rn(__dmul_rn(u_acc, (double)Qx), (double)Zp);
+        const double rhs = __dmul_rn((double)Px, (double)Zq);
+        r.accept = lhs <= rhs;
+    }
+    r.lpx = r.lp_amax = 0.0f;
+    if (write) {
+        const float logZ = logf(Zp), log2Z = log2f(Zp);
+        r.lpx = x_ok ? logf(Px) - logZ : -INFINITY;
+        if (p.greedy) r.lp_amax = logf(P_amax) - logZ;
+        if (lane == 0) {
+            float* f = p.features + (size_t)row * kNFeat;
+            f[0] = __fmul_rn(__fadd_rn(M, log2Z), 0x1.62e43p-1f);
+            f[1] = 1.0f / Zp;
+            f[2] = f[1] - exp2p(__fadd_rn(M2, -M)) / Zp;
+            f[3] = (log2Z - St / Zp) * 0x1.62e43p-1f;
+            f[4] = r.lpx;
+        }
+    }
+    return r;
+}
+
+// All rows of a sequence, a warp per row; returns the first-reject prefix.
+struct SeqMerge {
+    float4 stat[kMaxRows];
+    int acc[kMaxRows], amax[kMaxRows];
+    float lpx[kMaxRows], lpamax[kMaxRows];
+};
+__device__ __forceinline__ int merge_rows(const SamplerParams& p, int b, SeqMerge& s, bool write) {
+    const int lane = threadIdx.x & 31, k1 = p.k + 1;
+    for (int i = threadIdx.x >> 5; i < k1; i += kSW) {
+        const RowMerge r = merge_row(p, b, i, lane, write);
+        if (lane == 0) {
+            s.stat[i] = r.stat;
+            s.acc[i] = r.accept;
+            s.amax[i] = r.amax;
+            s.lpx[i] = r.lpx;
+            s.lpamax[i] = r.lp_amax;
+        }
+    }
+    __syncthreads();
+    int n = 0;
+    while (n < p.k && s.acc[n]) ++n;
+    return n;
+}
+__device__ __forceinline__ void write_prefix(const SamplerParams& p, int b, int n, const SeqMerge& s) {
+    const int tid = threadIdx.x, k1 = p.k + 1;
+    if (tid < p.k) p.accept_mask[b * p.k + tid] = tid < n;
+    if (tid == 0) p.accepted_len[b] = n;
+    if (tid < k1 && (tid != n || p.greedy)) {       // position n of a sampled sequence: the draw
+        int tok = -1;
+        float lp = 0.0f;
+        if (tid < n) {
+            tok = p.draft_tokens[b * p.k + tid];
+            lp = s.lpx[tid];
+        } else if (tid == n) {
+            tok = s.amax[n];
+            lp = s.lpamax[n];
+        }
+        p.out_tokens[b * k1 + tid] = tok;
+        p.out_logprobs[b * k1 + tid] = lp;
+        p.features[(size_t)(b * k1 + tid) * kNFeat + 5] = lp;
+    }
+}
+
 // ------------------------------------------------------------------------------------------------ kernel 1
 __device__ __forceinline__ float max4(const float4& z) { return fmaxf(fmaxf(z.x, z.y), fmaxf(z.z, z.w)); }
 
@@ -156,7 +295,8 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
     __shared__ __align__(16) float2 s_red[2][kSW];        // (the record of an item is written while the next one's maxima arrive)
     __shared__ float s_own2[kSW], s_red2[kSW][3];
     __shared__ unsigned long long s_key[kSW];
-    __shared__ int s_failed;
+    __shared__ int s_failed, s_last;
+    __shared__ SeqMerge s_seq;
     const WaitGuard guard{&s_failed, p.err, WAIT_SAMPLER << 8};
     grid_dep_launch();      // the draw kernel may be scheduled; it waits for this grid before reading anything
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -320,6 +460,19 @@ __global__ void __launch_bounds__(kST, 3) sampler_stats_kernel(const SamplerPara
         }
     }
     wait_settle(guard);
+    if (GREEDY && p.fused) {        // this CTA had one item
+        const int b = blockIdx.x / (p.NC * (p.k + 1));
+        if (tid == 0) {
+            __threadfence();        // the record, and the draft token's term before the last barrier
+            s_last = atomicAdd(&p.seq_ticket[b], 1) == p.NC * (p.k + 1) - 1;
+        }
+        __syncthreads();
+        if (!s_last) return;
+        __threadfence();
+        if (tid == 0) p.seq_ticket[b] = 0;
+        const int n = merge_rows(p, b, s_seq, true);
+        write_prefix(p, b, n, s_seq);
+    }
 }
 
 // ------------------------------------------------------------------------------------------------ kernel 2
@@ -370,108 +523,12 @@ __device__ __forceinline__ float residual_chunk(const SamplerParams& p, int row,
     return rs;
 }
 
-// One row's statistics from its chunk records, by one warp (lanes = chunks lane and lane + 32; every sum is chained in
-// chunk order): {M, Zp, Mq, Zq}, whether the draft token is accepted, and - `write` - the row's features.
-struct RowMerge {
-    float4 stat;
-    int accept, amax;
-    float lpx, lp_amax;
-};
-__device__ __forceinline__ RowMerge merge_row(const SamplerParams& p, int b, int i, int lane, bool write) {
-    const unsigned all = 0xffffffffu;
-    const int NC = p.NC, row = b * (p.k + 1) + i;
-    const bool has_draft = i < p.k && !p.greedy;
-    const float4 none = make_float4(-INFINITY, -INFINITY, 0.f, 0.f);
-    float4 rp[2], rq[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const bool ok = lane + 32 * u < NC;
-        rp[u] = ok ? __ldcg(&p.rec_p[(size_t)row * NC + lane + 32 * u]) : none;
-        rq[u] = ok ? __ldcg(&p.rec_q[(size_t)row * NC + lane + 32 * u]) : none;
-    }
-    const int x = i < p.k ? p.draft_tokens[b * p.k + i] : -1;
-    const bool x_ok = i < p.k && x >= 0 && x < p.V;
-    const float px = x_ok ? __ldcg(&p.row_px[row]) : 0.0f, qx = x_ok && has_draft ? __ldcg(&p.row_qx[row]) : 0.0f;
-    const double u_acc = has_draft ? p.u_accept[b * p.k + i] : 0.0;
-    float M = fmaxf(rp[0].x, rp[1].x), M2 = fmaxf(fminf(rp[0].x, rp[1].x), fmaxf(rp[0].y, rp[1].y));
-    float Mq = fmaxf(rq[0].x, rq[1].x);
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) {
-        const float o1 = __shfl_xor_sync(all, M, d), o2 = __shfl_xor_sync(all, M2, d);
-        M2 = fmaxf(fminf(M, o1), fmaxf(M2, o2));
-        M = fmaxf(M, o1);
-        Mq = fmaxf(Mq, __shfl_xor_sync(all, Mq, d));
-    }
-    float sc[2], tz[2], ts[2], sq[2], tq[2];
-#pragma unroll
-    for (int u = 0; u < 2; ++u) {
-        const float d = __fadd_rn(rp[u].x, -M);
-        sc[u] = exp2p(d);
-        tz[u] = __fmul_rn(rp[u].z, sc[u]);
-        ts[u] = __fmul_rn(__fmaf_rn(rp[u].z, d, rp[u].w), sc[u]);
-        sq[u] = exp2p(__fadd_rn(rq[u].x, -Mq));
-        tq[u] = __fmul_rn(rq[u].y, sq[u]);
-    }
-    float Zp = 0.0f, St = 0.0f, Zq = 0.0f;
-#pragma unroll
-    for (int u = 0; u < 2; ++u)
-#pragma unroll 8
-        for (int c = 0; c < min(32, NC - 32 * u); ++c) {
-            Zp = __fadd_rn(Zp, __shfl_sync(all, tz[u], c));
-            St = __fadd_rn(St, __shfl_sync(all, ts[u], c));
-            Zq = __fadd_rn(Zq, __shfl_sync(all, tq[u], c));
-        }
-    if (!has_draft) Zq = 0.0f;
-    const int cx = x_ok ? x / kChunk : 0;
-    const float s_x = __shfl_sync(all, cx < 32 ? sc[0] : sc[1], cx & 31);
-    const float sq_x = __shfl_sync(all, cx < 32 ? sq[0] : sq[1], cx & 31);
-    RowMerge r;
-    r.stat = make_float4(M, Zp, Mq, Zq);
-    const float Px = x_ok ? __fmul_rn(px, s_x) : 0.0f;
-    r.amax = -1;
-    float P_amax = 0.0f;
-    if (p.greedy) {             // the first chunk that attains the row maximum holds its lowest index
-        const unsigned h0 = __ballot_sync(all, rp[0].x == M && lane < NC), h1 = __ballot_sync(all, rp[1].x == M && lane + 32 < NC);
-        if (h0 | h1) {
-            const int src = h0 ? __ffs(h0) - 1 : __ffs(h1) - 1;
-            r.amax = __shfl_sync(all, __float_as_int(h0 ? rq[0].w : rq[1].w), src);
-            P_amax = __shfl_sync(all, h0 ? __fmul_rn(rq[0].z, sc[0]) : __fmul_rn(rq[1].z, sc[1]), src);
-        }
-    }
-    r.accept = 0;
-    if (p.greedy) {
-        r.accept = x_ok && x == r.amax;
-    } else if (has_draft && x_ok) {
-        const float Qx = __fmul_rn(qx, sq_x);
-        const double lhs = __dmul_rn(__dmul_rn(u_acc, (double)Qx), (double)Zp);
-        const double rhs = __dmul_rn((double)Px, (double)Zq);
-        r.accept = lhs <= rhs;
-    }
-    r.lpx = r.lp_amax = 0.0f;
-    if (write) {
-        const float logZ = logf(Zp), log2Z = log2f(Zp);
-        r.lpx = x_ok ? logf(Px) - logZ : -INFINITY;
-        if (p.greedy) r.lp_amax = logf(P_amax) - logZ;
-        if (lane == 0) {
-            float* f = p.features + (size_t)row * kNFeat;
-            f[0] = __fmul_rn(__fadd_rn(M, log2Z), 0x1.62e43p-1f);
-            f[1] = 1.0f / Zp;
-            f[2] = f[1] - exp2p(__fadd_rn(M2, -M)) / Zp;
-            f[3] = (log2Z - St / Zp) * 0x1.62e43p-1f;
-            f[4] = r.lpx;
-        }
-    }
-    return r;
-}
-
 __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParams p) {
     extern __shared__ __align__(128) float4 s_ring[];     // [2][target chunk | draft chunk]
     __shared__ __align__(8) uint64_t s_bar[2];
     __shared__ float s_red[2][kSW];
     __shared__ float s_rc[kMaxChunks], s_pre[kMaxChunks];
-    __shared__ float4 s_stat[kMaxRows];
-    __shared__ int s_acc[kMaxRows], s_amax[kMaxRows];
-    __shared__ float s_lpx[kMaxRows], s_lpamax[kMaxRows];
+    __shared__ SeqMerge s_seq;
     __shared__ int s_flag, s_cstar, s_tstar[kSW], s_failed;
     __shared__ float s_tau;
     const WaitGuard guard{&s_failed, p.err, WAIT_SAMPLER << 8};
@@ -485,19 +542,7 @@ __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParam
         fence_mbar_init();
     }
     grid_dep_wait();
-    for (int i = warp; i < k1; i += kSW) {
-        const RowMerge r = merge_row(p, b, i, lane, g == 0);
-        if (lane == 0) {
-            s_stat[i] = r.stat;
-            s_acc[i] = r.accept;
-            s_amax[i] = r.amax;
-            s_lpx[i] = r.lpx;
-            s_lpamax[i] = r.lp_amax;
-        }
-    }
-    __syncthreads();
-    int n = 0;                  // first-reject prefix
-    while (n < p.k && s_acc[n]) ++n;
+    const int n = merge_rows(p, b, s_seq, g == 0);
     const int row = b * k1 + n;
     const bool has_draft = n < p.k;
     auto issue = [&](int c2, int stage) {       // thread 0
@@ -512,26 +557,9 @@ __global__ void __launch_bounds__(kST, 3) sampler_draw_kernel(const SamplerParam
         issue(g, 0);
         if (g + G < NC) issue(g + G, 1);
     }
-    if (g == 0) {
-        if (tid < p.k) p.accept_mask[b * p.k + tid] = tid < n;
-        if (tid == 0) p.accepted_len[b] = n;
-        if (tid < k1 && (tid != n || p.greedy)) {       // position n of a sampled sequence: the draw below
-            int tok = -1;
-            float lp = 0.0f;
-            if (tid < n) {
-                tok = p.draft_tokens[b * p.k + tid];
-                lp = s_lpx[tid];
-            } else if (tid == n) {
-                tok = s_amax[n];
-                lp = s_lpamax[n];
-            }
-            p.out_tokens[b * k1 + tid] = tok;
-            p.out_logprobs[b * k1 + tid] = lp;
-            p.features[(size_t)(b * k1 + tid) * kNFeat + 5] = lp;
-        }
-    }
+    if (g == 0) write_prefix(p, b, n, s_seq);
     if (p.greedy) return;
-    const float4 st = s_stat[n];
+    const float4 st = s_seq.stat[n];
     float4 zt[kSlots], zq[kSlots];
     bool have[kSlots];
     float rs = 0.0f, hs;
@@ -713,7 +741,9 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     p.out_tokens = out_tokens;
     p.out_logprobs = out_logprobs;
     p.features = features;
-    p.err = device_wait_word();
+    int dev = 0;
+    ASD_CUDA(cudaGetDevice(&dev));
+    p.err = device_wait_word(dev);
     if (wait_word_check(p.err, "asd_reject_sample")) {      // reported once
         *static_cast<volatile int*>(p.err) = 0;
         return -1;
@@ -735,8 +765,6 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     static int sms[64];
     static std::once_flag once[64];
     constexpr int kRing = 2 * 2 * kChunk * 4;       // bytes: two chunk pairs, or four chunks
-    int dev = 0;
-    ASD_CUDA(cudaGetDevice(&dev));
     std::call_once(once[dev & 63], [&] {        // a second thread's first launch must not overtake the attributes
         cudaDeviceGetAttribute(&sms[dev & 63], cudaDevAttrMultiProcessorCount, dev);
         cudaFuncSetAttribute(sampler_stats_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing);
@@ -748,12 +776,18 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     });
     const size_t items = rows * NC, resident = (size_t)3 * sms[dev & 63];
     const unsigned grid = (unsigned)std::min(items, resident);
+    // Greedy calls whose items all fit the chip at once: a ticket per sequence and the merge by its last CTA, one launch.  Such
+    // calls are bound by the host: V = 151936, B = 4, k = 1: 13.9 us with two launches, 12.7 so; V = 32000, B = 1, k = 4: 14.0 and
+    // 12.7, host time alone 13.3 and 11.7.  More items than that: the ring would wait for a ticket per item, and the second
+    // launch is cheaper (B = 4, k = 5: 13.9 us, 18.7 with tickets).
+    p.fused = greedy && items <= resident;
     if (greedy)
         sampler_stats_kernel<true><<<grid, kST, kRing, stream>>>(p);
     else
         sampler_stats_kernel<false><<<grid, kST, kRing, stream>>>(p);
     ASD_CUDA(cudaGetLastError());
     count_launch(1);
+    if (p.fused) return 0;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

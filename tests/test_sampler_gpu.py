@@ -154,6 +154,19 @@ def test_parity_rings_and_shares(B, k, V, T):
     compare(run_gpu(tl, dl if k else None, dt, ua, ur, T), oracle.reject_sample(tl, dl if k else None, dt, ua, ur, T))
 
 
+@pytest.mark.parametrize("B,k,V", [
+    (4, 2, 151552),      # 12 rows x 37 chunks = 444 items: every resident CTA has one, the sequence's last one merges
+    (89, 4, 4096),       # 445: one more, merged by a second launch
+    (1, 0, 4), (1, 64, 4096), (148, 2, 4092), (7, 6, 32000)])
+def test_parity_greedy_one_and_two_launches(B, k, V):
+    """greedy calls around the number of CTAs that fit a 148-SM chip at once, against the oracle, called twice"""
+    tl, _, dt, ua, ur = make_case(B, k, V, seed=B + k, T=1.0)
+    dt = tl.argmax(-1).astype(np.int32)[:, :k].copy()
+    dt[1::3] = (dt[1::3] + 1) % V
+    tl[:, 0, V // 2] = tl[:, 0, V // 4] = tl[:, 0].max() + 1.0          # a tie, over chunks where there are several
+    compare(run_gpu(tl, None, dt, ua, ur, 0.0), oracle.reject_sample(tl, None, dt, ua, ur, 0.0))
+
+
 def test_parity_masked_logits():
     """vocabularies with masked entries (-inf and the type's lowest value), whole chunks of them included"""
     B, k, V, T = 3, 2, 12288, 0.7
