@@ -944,6 +944,10 @@ static int engine_forward(asd_engine_t* h, const int32_t* tokens, const int32_t*
     if ((long long)max_kv_len > (long long)e->max_pages * e->c.page_size)
         return set_error("asd_engine_forward: max_kv_len = %d exceeds the page table (%d pages of %d positions)",
                          max_kv_len, e->max_pages, e->c.page_size);
+    if (prompt && e->tune.gemm_big && M > kTcMaxTokens)
+        return set_error("asd_engine_forward_prompt: %d tokens; at most %d a call", M, kTcMaxTokens);
+    if (prompt && e->c.n_heads / e->c.n_kv_heads > 128)
+        return set_error("asd_engine_forward_prompt: more than 128 heads per key/value head");
     if (wait_word_check(e->wait_err, "asd_engine_forward")) return -1;
     WaitScope wait_scope(e->wait_err);
     cudaStream_t s = static_cast<cudaStream_t>(stream);

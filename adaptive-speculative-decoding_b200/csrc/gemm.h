@@ -83,6 +83,7 @@ struct TcPlan {
     int M, N, K, mode;
     int MT, m_tiles, w_tiles, kblocks, ksplit, stages, smem_bytes, pairs;
 };
+constexpr int kTcMaxTokens = 4096;       // of one call
 int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages);
 // x tensor map: box rows = MT / 2 (each CTA of the pair loads half of the token tile); w tensor map: box rows = 128.
 // GEMM_OUT_F32: out fp32 [ksplit][slice_stride] slices of [M][ldo]; GEMM_OUT_SWIGLU: out bf16 [M][ldo].

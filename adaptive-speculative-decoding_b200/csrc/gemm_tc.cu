@@ -37,7 +37,7 @@ constexpr int kTcThreads = 256;          // warp 0 TMA, warp 1 MMA (leader), war
 constexpr int kTcBlockK = 64;
 constexpr int kTcABytes = 128 * kTcBlockK * 2;
 constexpr int kTcAccCols = 256;          // TMEM column stride between the two accumulators
-constexpr int kTcMaxM = 4096;            // per-token rstd table in shared memory
+constexpr int kTcMaxM = kTcMaxTokens;    // per-token rstd table in shared memory
 
 struct TcArgs {
     int M, N, K;

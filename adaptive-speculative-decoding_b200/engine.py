@@ -145,12 +145,17 @@ class _BatchOps:
                 out[torch.tensor(dest, device=dev)] = lg
         return (out, streams) if layer_out else out
 
+    MAX_PROMPT_SHAPES = 64
+
     def _uniform_index(self, nseq: int, q: int):
-        """static index tensors of a uniform (nseq x q) call, built once per shape"""
+        """static index tensors of a uniform (nseq x q) call, built once per shape.  Steps have few shapes; prompts have one per
+        length, so only the first ``MAX_PROMPT_SHAPES`` of them stay (none is dropped: a captured step may hold the tensors)"""
         key = (nseq, q)
         c = self._index_cache.get(key)
         if c is None:
-            c = self._index_cache[key] = {}
+            c = {}
+            if q <= self.max_qlen() or sum(k[1] > self.max_qlen() for k in self._index_cache) < self.MAX_PROMPT_SHAPES:
+                self._index_cache[key] = c
         return c
 
     def _uniform_index_on(self, nseq: int, q: int, dev):

@@ -247,8 +247,9 @@ ASD_API int asd_engine_forward(asd_engine_t* e, const int32_t* tokens, const int
                        const int32_t* token_slot, int M, const int32_t* cu_q, const int32_t* seq_slot, int nseq,
                        int max_qlen, int max_kv_len, const int32_t* logit_rows, int n_logit_rows, float* logits_out,
                        long long logits_ld, void* stream);
-/* The same for prompts: a sequence may bring any number of new positions (M <= max_tokens); beyond 128 / (heads per
- * key/value head) of them attention runs in query tiles of that many positions. */
+/* The same for prompts: a sequence may bring any number of new positions (M <= max_tokens, and 4096 a call); beyond
+ * 128 / (heads per key/value head) of them attention runs in query tiles of that many positions.  At most 128 heads per
+ * key/value head. */
 ASD_API int asd_engine_forward_prompt(asd_engine_t* e, const int32_t* tokens, const int32_t* positions,
                        const int32_t* token_slot, int M, const int32_t* cu_q, const int32_t* seq_slot, int nseq,
                        int max_qlen, int max_kv_len, const int32_t* logit_rows, int n_logit_rows, float* logits_out,

@@ -374,3 +374,22 @@ def test_generations_sharing_a_gpu_take_the_same_device_lock_in_index_order():
     a[0].release()
     t.join(2)
     assert got == [1]
+
+
+def test_index_tensors_of_prompts_are_bounded():
+    """a server sees one prompt shape per length: the step shapes stay cached, of the prompt shapes only so many"""
+    from types import SimpleNamespace
+    import torch
+    from asd_b200.engine import _BatchOps
+    ops = _BatchOps()
+    ops.cfg, ops._index_cache = SimpleNamespace(num_attention_heads=28, num_key_value_heads=4), {}
+    assert ops.max_qlen() == 18
+    for q in range(1, 500):
+        for _ in range(2):
+            ix = ops._uniform_index_on(2, q, torch.device("cpu"))
+            assert ix["cu_q"].tolist() == [0, q, 2 * q] and ix["last_rows"].tolist() == [q - 1, 2 * q - 1]
+            assert ix["ar"].tolist() == [list(range(q))]
+    assert len(ops._index_cache) == 18 + ops.MAX_PROMPT_SHAPES
+    kept = ops._index_cache[(2, 7)]
+    ops._uniform_index_on(2, 7, torch.device("cpu"))
+    assert ops._index_cache[(2, 7)] is kept

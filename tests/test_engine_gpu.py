@@ -416,3 +416,21 @@ def test_prefill_at_depth_small_and_large_forwards():
         eng.close()
         del eng, outs
     assert _rel(*logits) < 4.3e-2
+
+
+def test_forward_prompt_limits():
+    """what a prompt call cannot take is refused before anything is launched, by name"""
+    from asd_b200._lib import AsdError, lib
+    from asd_b200.engine import QwenEngine
+    cfg = tiny_config(num_hidden_layers=1)
+    eng = QwenEngine(cfg, max_seqs=1, max_seq_len=4200, max_tokens=4160).load_random(seed=2)
+    slot = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ids = torch.zeros(4097, dtype=torch.int32, device="cuda")
+    pos = torch.arange(4097, dtype=torch.int32, device="cuda")
+    cu = torch.tensor([0, 4097], dtype=torch.int32, device="cuda")
+    before = lib().asd_launch_count()
+    with pytest.raises(AsdError, match="at most 4096 a call"):
+        eng._prompt_forward(ids, pos, torch.zeros_like(pos), cu, slot, 4097, 4097, None, None, False, 0)
+    assert lib().asd_launch_count() == before
+    assert torch.isfinite(eng.prefill(ids[None], slot)).all()          # prefill cuts it itself
+    eng.close()
