@@ -138,6 +138,7 @@ def lib() -> ctypes.CDLL:
         "asd_abi_version": (i32, []),
         "asd_last_error": (c.c_char_p, []),
         "asd_launch_count": (c.c_longlong, []),
+        "asd_kernel_launches": (c.c_longlong, [c.c_char_p]),
         "asd_wait_error": (i32, []),
         "asd_debug_wait_expiry": (i32, [vp]),
         "asd_reset_launch_count": (None, []),

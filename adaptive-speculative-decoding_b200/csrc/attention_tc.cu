@@ -563,7 +563,7 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     cfg.attrs = attr;
     cfg.numAttrs = tuning().glue_pdl ? 1 : 0;
     ASD_CUDA(cudaLaunchKernelEx(&cfg, a.trace ? attn_tc_kernel<true> : attn_tc_kernel<false>, *L.kv_map, a));
-    count_launch(1);
+    count_kernel(KERNEL_ATTENTION_TC);
     return 0;
 }
 

@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdarg.h>
 #include <stdio.h>
+#include <string.h>
 
 #include <atomic>
 #include <mutex>
@@ -27,6 +28,11 @@ int set_error(const char* fmt, ...) {
     return -1;
 }
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
+static std::atomic<long long> g_kernels[KERNEL_COUNTED];
+void count_kernel(CountedKernel k) {
+    g_kernels[k].fetch_add(1, std::memory_order_relaxed);
+    count_launch(1);
+}
 
 // ---- bounded device waits
 thread_local int* g_wait_word = nullptr;
@@ -107,6 +113,12 @@ int asd_abi_version(void) { return ASD_B200_ABI_VERSION; }
 const char* asd_last_error(void) { return g_err; }
 long long asd_launch_count(void) { return g_launches.load(); }
 void asd_reset_launch_count(void) { g_launches.store(0); }
+long long asd_kernel_launches(const char* name) {
+    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemv", "attention_tc", "latent_tc", "sampler_draw"};
+    for (int i = 0; name && i < KERNEL_COUNTED; ++i)
+        if (!strcmp(name, names[i])) return g_kernels[i].load();
+    return set_error("asd_kernel_launches: unknown kernel %s", name ? name : "(null)");
+}
 int asd_debug_wait_expiry(void* stream) { return launch_wait_expiry(device_wait_word(), static_cast<cudaStream_t>(stream)); }
 int asd_wait_error(void) {
     int* w = device_wait_word();

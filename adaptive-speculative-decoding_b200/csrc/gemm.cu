@@ -890,7 +890,7 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
     cfg.attrs = attr;
     cfg.numAttrs = na;
     ASD_CUDA(cudaLaunchKernelEx(&cfg, a.trace ? gemm_ws_kernel<true> : gemm_ws_kernel<false>, tmap_w, tmap_x, *tnext, a));
-    count_launch(1);
+    count_kernel(KERNEL_GEMM);
     return 0;
 }
 

@@ -410,7 +410,7 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.err = wait_word();
     gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, a);
     ASD_CUDA(cudaGetLastError());
-    count_launch(1);
+    count_kernel(KERNEL_GEMM_PAIR);
     return 0;
 }
 

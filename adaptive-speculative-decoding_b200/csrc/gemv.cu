@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kGvThreads, 2) gemv_kernel(const GvArgs a) {
 template <int UN>
 int gv_launch(const GvArgs& a, int blocks, size_t smem, cudaStream_t stream) {
     ASD_CUDA(launch_pdl(gemv_kernel<UN>, blocks, kGvThreads, smem, stream, a));
-    count_launch(1);
+    count_kernel(KERNEL_GEMV);
     return 0;
 }
 

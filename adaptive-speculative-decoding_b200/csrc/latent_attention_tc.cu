@@ -568,7 +568,7 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     ASD_CUDA(cudaFuncSetAttribute(latent_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const dim3 grid(p.q_tiles * p.hgs * p.parts, nseq * a.nsplit);
     latent_attn_tc<<<grid, kLtThreads, smem, stream>>>(mq, mk, a);
-    count_launch(1);
+    count_kernel(KERNEL_LATENT_TC);
     ASD_CUDA(cudaGetLastError());
     if (a.nsplit > 1) return launch_latent_combine(ws.o, ws.ml, a.nsplit, d.R, out_lat, rows, stream);
     return 0;

@@ -799,7 +799,7 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     ASD_CUDA(cudaLaunchKernelEx(&cfg, sampler_draw_kernel, p));
-    count_launch(1);
+    count_kernel(KERNEL_SAMPLER_DRAW);
     return 0;
 }
 

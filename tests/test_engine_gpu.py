@@ -341,7 +341,11 @@ def test_engine_one_token(cfg):
         got = {}
         for on in (1, 0):
             eng.set_option("one_token", on)
-            got[on] = eng.forward_uniform(idc[:nseq, T - q:].contiguous(), start, slots, T).view(nseq, q, -1).cpu()
+
+            def step():
+                got[on] = eng.forward_uniform(idc[:nseq, T - q:].contiguous(), start, slots, T).view(nseq, q, -1).cpu()
+
+            assert _launched("gemv", step) == (4 * cfg.num_hidden_layers + 1 if on and nseq * q == 1 else 0)
         check(got[1], ref[:nseq, T - q:])
         if nseq * q == 1:
             assert (got[1] - got[0]).abs().max().item() <= MAX_ABS
@@ -371,11 +375,22 @@ def test_engine_prompt_chunks_near_the_ridge(cfg, tokens):
     ref = qwen2_forward(w, cfg, ids)
     eng = QwenEngine(cfg, max_seqs=1, max_seq_len=tokens + 16, max_tokens=256).load_hf_weights(w)
     slot, idc = torch.zeros(1, dtype=torch.int32, device="cuda"), ids.cuda().to(torch.int32)
-    last = eng.prefill(idc[:, :tokens].contiguous(), slot)
+    last = []
+    assert _launched("gemm_pair", lambda: last.append(eng.prefill(idc[:, :tokens].contiguous(), slot))) == 0
+    last = last[0]
     ver = eng.forward_uniform(idc[:, tokens:].contiguous(), slot + tokens, slot, tokens + 4)
     check(last.cpu(), ref[:, tokens - 1])
     check(ver.view(1, 4, -1).cpu(), ref[:, tokens:])
     eng.close()
+
+
+def _launched(name, call):
+    """how often a kernel was launched by call()"""
+    from asd_b200._lib import lib
+    before = lib().asd_kernel_launches(name.encode())
+    assert before >= 0
+    call()
+    return lib().asd_kernel_launches(name.encode()) - before
 
 
 def _rel(a, b):
@@ -409,7 +424,9 @@ def test_prefill_at_depth_small_and_large_forwards():
     logits = []
     for max_tokens in (256, 2048):
         eng = QwenEngine(QWEN25["7b"], max_seqs=B, max_seq_len=P + 16, max_tokens=max_tokens).load_random(seed=3)
-        outs = [eng.prefill(prompts, slots) for _ in range(20)]
+        outs = []
+        pairs = _launched("gemm_pair", lambda: outs.extend(eng.prefill(prompts, slots) for _ in range(20)))
+        assert pairs == (0 if max_tokens == 256 else 20 * 2 * 28 * 4)
         torch.cuda.synchronize()
         assert all(torch.equal(o, outs[0]) for o in outs)
         logits.append(outs[0].double().cpu())

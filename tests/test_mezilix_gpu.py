@@ -571,7 +571,12 @@ def test_latent_attention_on_tcgen05(heads, kv_rank, rot_dim, window, page_size,
         eng.set_option("attn_tiled", mode)
         if mode == 2:
             eng.cache_pool.fill_(255)
+        before = lib().asd_kernel_launches(b"latent_tc")
         outs.append(feed(eng, eng.open_sequence(), ids, portions).cpu())
+        ran = lib().asd_kernel_launches(b"latent_tc") - before
+        # of 128 // heads positions a tile, those portions that fill 32 rows of it
+        want = sum(min(128 // min(heads, 128), p) * min(heads, 128) >= 32 for p in portions) if mode == 2 else 0
+        assert before >= 0 and ran == want
         eng.check_device()
         close(eng)
     assert torch.isfinite(outs[0]).all()

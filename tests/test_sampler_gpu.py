@@ -164,7 +164,12 @@ def test_parity_greedy_one_and_two_launches(B, k, V):
     dt = tl.argmax(-1).astype(np.int32)[:, :k].copy()
     dt[1::3] = (dt[1::3] + 1) % V
     tl[:, 0, V // 2] = tl[:, 0, V // 4] = tl[:, 0].max() + 1.0          # a tie, over chunks where there are several
+    import torch
+    from asd_b200._lib import lib
+    before = lib().asd_kernel_launches(b"sampler_draw")
     compare(run_gpu(tl, None, dt, ua, ur, 0.0), oracle.reject_sample(tl, None, dt, ua, ur, 0.0))
+    one = B * (k + 1) * ((V + 4095) // 4096) <= 3 * torch.cuda.get_device_properties(0).multi_processor_count
+    assert lib().asd_kernel_launches(b"sampler_draw") - before == (0 if one else 2)
 
 
 def test_parity_masked_logits():
@@ -179,3 +184,9 @@ def test_parity_masked_logits():
         got, ref = run_gpu(a, d, dt, ua, ur, T), oracle.reject_sample(a, d, dt, ua, ur, T)
         for key in ("accept_mask", "accepted_len", "out_tokens"):
             assert np.array_equal(got[key], ref[key]), key
+        # log-probabilities and features as in compare(), where the oracle has a number; elsewhere the same kind of value
+        for key in ("out_logprobs", "features"):
+            g, r = got[key], ref[key]
+            fin = np.isfinite(r)
+            assert np.array_equal(np.isnan(g), np.isnan(r)) and np.array_equal(g[np.isinf(r)], r[np.isinf(r)]), key
+            np.testing.assert_allclose(g[fin], r[fin], rtol=FEAT_RTOL, atol=2e-5)
