@@ -559,6 +559,7 @@ def test_trace_replay_command_on_a_checkpoint_directory(tmp_path, dtype):
 def test_latent_attention_on_tcgen05(heads, kv_rank, rot_dim, window, page_size, scale, portions):
     """bf16 engine: the tcgen05 kernel against the fp32 CUDA-core kernel of the same engine, both held to the oracle; the pool
     starts out as NaN, none of which may reach a result"""
+    from asd_b200._lib import lib
     cfg = config([layer(heads=heads, dim=16, rot_dim=rot_dim, vdim=16, kv_rank=kv_rank, window=window, scale=scale, experts=0)],
                  width=64)
     w = O.random_model(cfg, seed=51, scale=1.5)
