@@ -94,6 +94,8 @@ struct TuningScope {
     ~TuningScope() { g_tuning = prev; }
 };
 
+int sm_count();      // multiprocessors of the current device
+
 // cudaFuncSetAttribute is per device: remember which devices a kernel's attributes were set on
 struct PerDeviceOnce {
     unsigned long long mask = 0;

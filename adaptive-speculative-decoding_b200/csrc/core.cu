@@ -34,6 +34,18 @@ void count_kernel(CountedKernel k) {
     count_launch(1);
 }
 
+int sm_count() {
+    static std::atomic<int> counts[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0) dev = 0;
+    int n = counts[dev & 63].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) return 1;
+        counts[dev & 63].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 // ---- bounded device waits
 thread_local int* g_wait_word = nullptr;
 

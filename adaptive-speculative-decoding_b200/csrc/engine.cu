@@ -95,6 +95,7 @@ struct Engine {
     float* tp_buf[2] = {nullptr, nullptr};
     uint32_t* tp_flags = nullptr;
     int* tp_error = nullptr;
+    size_t sumsq_floats = 0;         // of sumsq and of sumsq_sel
     int* wait_err = nullptr;         // a bounded wait of one of this engine's kernels ran out (mapped host memory)
     const float* peer_buf[2][8] = {};
     uint32_t* peer_flags[8] = {};
@@ -262,7 +263,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     // one token: every projection through gemv.cu (its norm statistics are one sum per block, side by side)
     const bool one = e->one_token && fn && !tp && e->force_ksplit == 0 && e->force_stages == 0 && n_logit_rows <= 1 &&
                      gemv_takes(M, std::max(std::max(h, e->qdim), c.ffn), (size_t)2 * e->ffp * h * 2);
-    const int ss_ld = one ? 1 : Mx, max_parts = Mx * ((h + 127) / 128);
+    const int ss_ld = one ? 1 : Mx, max_parts = (int)std::min<size_t>(e->sumsq_floats, 1 << 30);
     NormFusion cons;  // consumer-side descriptor, refreshed before each consumer GEMM
     auto consumer = [&](const float* ss) -> const NormFusion* {
         if (!fn) return nullptr;
@@ -640,8 +641,10 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
     alloc((void**)&e->ml_part, Mx * c.n_heads * (size_t)e->max_attn_splits * 2 * 4);
     alloc((void**)&e->rope_cs, Mx * (c.head_dim / 2) * sizeof(float2));
     alloc((void**)&e->resid_bf, Mx * c.hidden * 2);
-    alloc((void**)&e->sumsq, Mx * (size_t)((c.hidden + 127) / 128) * 4);
-    alloc((void**)&e->sumsq_sel, Mx * (size_t)((c.hidden + 127) / 128) * 4);
+    // norm statistics: one sum per token and 128 columns, or per block of a one-token projection
+    e->sumsq_floats = std::max(Mx * ((c.hidden + 127) / 128), (size_t)gemv_max_blocks());
+    alloc((void**)&e->sumsq, e->sumsq_floats * 4);
+    alloc((void**)&e->sumsq_sel, e->sumsq_floats * 4);
     alloc((void**)&e->tickets, Mx * c.n_kv_heads * 4);
     if (ok && cudaMemset(e->tickets, 0, Mx * c.n_kv_heads * 4) != cudaSuccess) ok = false;
     if (c.tp_size > 1) {

@@ -94,5 +94,6 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
 bool gemv_takes(int M, int max_k, size_t max_bytes);
 int gemv_launch(int mode, const __nv_bfloat16* x, const __nv_bfloat16* w, int K, int n_valid, void* out, const QkvEpilogue* qkv,
                 const NormFusion* norm, int max_parts, int* blocks_out, cudaStream_t stream);
+int gemv_max_blocks();
 int preload_gemv();
 }  // namespace asd

@@ -254,7 +254,7 @@ int gv_launch(const GvArgs& a, int blocks, size_t smem, cudaStream_t stream) {
 bool gemv_takes(int M, int max_k, size_t max_bytes) { return M == 1 && max_k <= 16384 && max_bytes <= (size_t)128 << 20; }
 
 // x bf16 [K], w bf16 [N][K] row major; max_parts bounds the blocks of a launch that writes sums of squares (one per block, norm.ld
-// apart), *blocks_out their number.
+// apart; gemv_max_blocks() never bounds it), *blocks_out their number.
 int gemv_launch(int mode, const __nv_bfloat16* x, const __nv_bfloat16* w, int K, int n_valid, void* out, const QkvEpilogue* qkv,
                 const NormFusion* norm, int max_parts, int* blocks_out, cudaStream_t stream) {
     if (K <= 0 || K > 16384 || (K & 7) || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15))
@@ -266,19 +266,21 @@ int gemv_launch(int mode, const __nv_bfloat16* x, const __nv_bfloat16* w, int K,
     a.units = mode == GEMM_OUT_QKV ? n_valid / 2 : (mode == GEMM_OUT_SWIGLU ? n_valid : (n_valid + 1) / 2);
     // Two blocks of eight warps per SM.  Enough pairs: each warp takes two at once (an activation read serves four rows);
     // too few for the chip: warps share a pair's k range, 512 elements or more each.
-    const int want = 2 * 148 * kGvWarps;
+    const int at_a_time = 2 * sm_count(), want = at_a_time * kGvWarps;
     const int un = a.units >= 2 * want ? 2 : 1;
     const int steps = (K + kGvStep - 1) / kGvStep;
     a.ksplit = 1;
     while (un == 1 && a.ksplit < kGvWarps && 4 * a.units * a.ksplit < 3 * want && steps / (2 * a.ksplit) >= 2) a.ksplit *= 2;
     a.steps = (steps + a.ksplit - 1) / a.ksplit;
     const int groups = (a.units + un - 1) / un, at_once = kGvWarps / a.ksplit;
-    int blocks = std::min((groups + at_once - 1) / at_once, 2 * 148);
+    int blocks = std::min((groups + at_once - 1) / at_once, at_a_time);
     if (a.norm.sumsq_out) blocks = std::max(1, std::min(blocks, max_parts));
     if (blocks_out) *blocks_out = blocks;
     const size_t smem = (size_t)steps * kGvStep * 2;
     return un == 2 ? gv_launch<2>(a, blocks, smem, stream) : gv_launch<1>(a, blocks, smem, stream);
 }
+
+int gemv_max_blocks() { return 2 * sm_count(); }
 
 int preload_gemv() {
     cudaFuncAttributes fa;

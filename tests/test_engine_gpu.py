@@ -360,6 +360,23 @@ def test_engine_one_token(cfg):
     eng.close()
 
 
+def test_engine_one_token_of_an_engine_for_one():
+    """an engine that takes one token at a time has room for the statistics of as many blocks as any other"""
+    from asd_b200.engine import QwenEngine
+    cfg = Qwen2Config(896, 2, 14, 2, 4864, 1024, head_dim=64, name="one-only")
+    w = random_hf_weights(cfg, seed=29, logit_std=0.4)
+    ids = torch.randint(0, cfg.vocab_size, (1, 6), generator=torch.Generator().manual_seed(4))
+    ref = qwen2_forward(w, cfg, ids)
+    idc, slot = ids.cuda().to(torch.int32), torch.zeros(1, dtype=torch.int32, device="cuda")
+    outs = []
+    for max_tokens in (1, 64):
+        eng = QwenEngine(cfg, max_seqs=1, max_seq_len=16, max_tokens=max_tokens).load_hf_weights(w)
+        outs.append(torch.cat([eng.forward_uniform(idc[:, i:i + 1].contiguous(), slot + i, slot, i + 1) for i in range(6)]).cpu())
+        eng.close()
+    check(outs[0], ref[0])
+    assert torch.equal(outs[0], outs[1])        # the same grids
+
+
 @pytest.mark.parametrize("tokens", [160, 161, 211, 256])
 @pytest.mark.parametrize("cfg", [
     Qwen2Config(1280, 1, 10, 2, 9600, 1024, head_dim=128, name="wave-wide"),      # 150 gate|up tiles: more than one per SM
