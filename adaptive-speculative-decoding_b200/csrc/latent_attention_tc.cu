@@ -29,6 +29,7 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <mutex>
 
 #include "asd_internal.h"
 #include "blocks.h"
@@ -554,9 +555,10 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     // few query tiles: the keys are cut into shares until every SM has a CTA, of at least two tiles each
     a.nsplit = 1;
     const long long ctas = (long long)p.q_tiles * p.hgs * p.parts * nseq;
-    if (ws.o && ws.ml && ctas < 148) {
+    const int sms = sm_count();
+    if (ws.o && ws.ml && ctas < sms) {
         const long long keys = std::min<long long>(d.window, max_kv_len) + p.TQ + kLtKeys;
-        long long n = std::min<long long>(148 / ctas, keys / (2 * kLtKeys));
+        long long n = std::min<long long>(sms / ctas, keys / (2 * kLtKeys));
         n = std::min(n, std::min(ws.rows / rows, ws.o_elems / (rows * d.R)));
         a.nsplit = (int)std::max<long long>(1, std::min<long long>(n, 64));
     }
@@ -565,7 +567,12 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     if (make_tmap_bf16_planes(&mq, q_terms, rows, rw, 3, a.box_rows)) return -1;
     if (make_tmap_bf16(&mk, cache.pool, cache.rows, rw, rw, cache.page_size)) return -1;
     const int smem = 1024 + (kLtVSlots + kLtKSlots + 3 * kLtQSlots) * kLtSlot + (int)sizeof(LtBars);
-    ASD_CUDA(cudaFuncSetAttribute(latent_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static std::once_flag once[64];     // (a second thread's first launch must not overtake the attribute)
+    int dev = 0;
+    ASD_CUDA(cudaGetDevice(&dev));
+    cudaError_t rc = cudaSuccess;
+    std::call_once(once[dev & 63], [&] { rc = cudaFuncSetAttribute(latent_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
+    ASD_CUDA(rc);
     const dim3 grid(p.q_tiles * p.hgs * p.parts, nseq * a.nsplit);
     latent_attn_tc<<<grid, kLtThreads, smem, stream>>>(mq, mk, a);
     count_kernel(KERNEL_LATENT_TC);

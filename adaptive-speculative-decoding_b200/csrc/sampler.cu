@@ -733,8 +733,6 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
     p.V = V;
     p.NC = NC;
     p.greedy = greedy;
-    // three draw CTAs fit an SM: one wave of them shares the chunks of all sequences
-    p.G = greedy ? 1 : std::max(1, std::min(NC, 3 * 148 / B));
     p.c1 = greedy ? 0x1.715476p+0f : (1.0f / temperature) * 0x1.715476p+0f;
     p.accept_mask = accept_mask;
     p.accepted_len = accepted_len;
@@ -775,6 +773,8 @@ int launch_reject_sample(const float* target, const float* draft, const int* dra
         prefer_max_smem(sampler_stats_kernel<true>);
     });
     const size_t items = rows * NC, resident = (size_t)3 * sms[dev & 63];
+    // three draw CTAs fit an SM: one wave of them shares the chunks of all sequences
+    p.G = greedy ? 1 : std::max(1, std::min(NC, (int)resident / B));
     const unsigned grid = (unsigned)std::min(items, resident);
     // Greedy calls whose items all fit the chip at once: a ticket per sequence and the merge by its last CTA, one launch.  Such
     // calls are bound by the host: V = 151936, B = 4, k = 1: 13.9 us with two launches, 12.7 so; V = 32000, B = 1, k = 4: 14.0 and
