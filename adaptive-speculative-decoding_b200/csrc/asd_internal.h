@@ -40,7 +40,7 @@ struct WaitScope {                                      // an engine's word, for
 };
 
 // Programmatic launch: the grid may become resident while its predecessor drains.  Only for kernels that begin with
-// pdl_enter() or otherwise wait (griddepcontrol.wait) before they touch memory.
+// pdl_enter() or otherwise wait (griddepcontrol.wait) before they touch memory, and that keep ptx.cuh's rules on TMEM.
 template <typename... P, typename... A>
 inline cudaError_t launch_pdl(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args) {
     cudaLaunchConfig_t cfg = {};

@@ -2,7 +2,7 @@
 //
 // Why: with one launch per GEMM (gemm.cu) the weight stream stops at every kernel boundary - cluster barrier, DSMEM
 // scatter, owner epilogue, exit, the next grid's entry and first activation tile: 8-12 us of idle HBM per boundary,
-// five boundaries per layer (DESIGN.md section 8; 25-45 % of a layer at 16-96 tokens).  Here 148 CTAs (one per SM) stay
+// five boundaries per layer (25-45 % of a layer at 16-96 tokens).  Here 148 CTAs (one per SM) stay
 // resident for the whole forward and the weight stream never stops for a boundary:
 //   * warp 0 (one thread) is the WEIGHT producer: it walks the static schedule of every GEMM of the forward
 //     (QKV, O, gate|up, down of each layer, lm_head) and keeps TMA loads of 128 x 64 weight blocks in flight into a

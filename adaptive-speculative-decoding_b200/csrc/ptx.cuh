@@ -297,10 +297,17 @@ __device__ __forceinline__ bool elect_one() {
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Programmatic launch and TMEM.  A grid may become resident once every CTA of its predecessor has triggered (or ended), so
+//   * no CTA triggers (griddepcontrol.launch_dependents) before its own tcgen05.alloc has returned: otherwise the successor's CTA
+//     may take the columns and then wait for a grid that waits for those columns.  gemm.cu, gemm_tc.cu and attention_tc.cu
+//     allocate, synchronise the CTA (the pair), and trigger later; latent_attention_tc.cu and linear_tc.cu never trigger;
+//   * a kernel that allocates for a CTA pair (gemm_tc.cu) is launched plainly: its columns then never depend on another grid's;
+//   * nobody triggers before it waits, unless it was launched plainly itself (qkv_rope_kernel, sampler_stats_kernel): otherwise
+//     chains of grids hold their places while the first one runs.
+// Kernels of different streams are outside of these rules: generations that share a device are serialised by the caller.
+//
 // First statement of a kernel that is launched programmatically: nothing is read or written before the predecessor has
-// completed (and with it every kernel before that), and the successor may take up residence only from then on.  Letting it
-// in before the wait builds chains of grids that all hold their places while the first one runs; a prompt of the Rivetar
-// layers, CTA-pair GEMMs among them, did not end that way.
+// completed (and with it every kernel before that), and the successor may take up residence only from then on.
 __device__ __forceinline__ void pdl_enter() {
     grid_dep_wait();
     grid_dep_launch();

@@ -123,7 +123,7 @@ def validate_gpu_assignment(stages) -> None:
 _ORDER = threading.Lock()
 _NEXT_ORDER = [0]
 # one lock per GPU: generations that touch the same device run one after the other.  Kernels of different streams on
-# one SM are not covered by the forward's TMEM hand-over invariant: a 512-column tcgen05.alloc
+# one SM are not covered by the forward's TMEM hand-over invariant (csrc/ptx.cuh): a 512-column tcgen05.alloc
 # of one stream can hold the allocation permit while a clustered GEMM of the other waits for a sibling that needs it.
 _DEVICE_LOCKS = {}
 

@@ -142,7 +142,7 @@ def config_dict(wl, n_gpus, extra=None):
 def run_reference(args):
     """CPU arm.  The line's ``value`` is the same metric on the same config as our arm; a full
     7B -> 32B step on CPU takes minutes, so it is a bounded sample multiplied out (``"extrapolated": true``).
-    Next to it ``cpu_baselines`` holds three MEASURED, un-extrapolated baselines (BASELINE.md section 4): the stop
+    Next to it ``cpu_baselines`` holds three MEASURED, un-extrapolated baselines: the stop
     rule over 10^5 triples in CPython, the C sampler oracle on two config-2 grid points, and configs[0] end to end
     (HF Qwen2ForCausalLM fp32, 0.5B -> 1.5B, k = 4, greedy) - our arm reports the same three on the GPU."""
     rank = int(os.environ.get("RANK", "0"))

@@ -207,10 +207,10 @@ ASD_API int asd_engine_peer_connect(asd_engine_t** engines, int n);
  * per-token sum of squares, the consuming QKV / gate|up / lm_head epilogues apply rstd),
  * "attn_target_ctas", "attn_min_split_keys" (keys per flash-decoding split, default 1024), "glue_pdl",
  * "ksplit", "stages" (0 = automatic), "headroom" (shared memory left for the next kernel's CTAs on <= 32-token
- * tiles), "recv_dedicated", "early_trigger", "next_prefetch_mb" (tuning knobs, see DESIGN.md section 8),
+ * tiles), "recv_dedicated", "early_trigger", "next_prefetch_mb" (tuning knobs),
  * "tp_fused" (0 never, 1 where it pays, 2 always), "tp_two_shot" (-1 never, 0 where it pays, 1 always), "p2p",
  * "persist" (1: single-rank forwards of <= 128 tokens run as ONE cooperative launch of the persistent forward
- * kernel, forward_persist.cu; 0, default: one launch per GEMM / attention - measured faster, DESIGN.md section 8),
+ * kernel, forward_persist.cu; 0, default: one launch per GEMM / attention - measured faster),
  * "persist_ahead" (L2 prefetch distance of the persistent kernel's weight producer, 0 = off), "profile" (0/1) */
 ASD_API int asd_engine_set_option(asd_engine_t* e, const char* name, int value);
 /* With option "profile" = 1 every launch is bracketed by CUDA events on the launching stream;

@@ -352,7 +352,7 @@ def test_safetensors_round_trip(tmp_path):
 
 def test_generations_sharing_a_gpu_take_the_same_device_lock_in_index_order():
     """Stage.generate serialises generations that touch the same GPU (kernels of different streams are outside the
-    forward's TMEM hand-over invariant): one re-entrant lock per device, handed out sorted by
+    forward's TMEM hand-over invariant, csrc/ptx.cuh): one re-entrant lock per device, handed out sorted by
     device index so that two cascades with overlapping GPU sets can never wait for each other in a cycle."""
     import threading
     from asd_b200.models import stage

@@ -1,5 +1,5 @@
 """Raw NVLink peer bandwidth of the box (torch copies between two GPUs): the yardstick for the tensor-parallel
-exchange numbers in DESIGN.md section 4 (measured: 734 GB/s for cudaMemcpyPeer 1 -> 0 on 2 x B200)."""
+exchange (measured: 734 GB/s for cudaMemcpyPeer 1 -> 0 on 2 x B200)."""
 import torch, time
 n = torch.cuda.device_count()
 print("gpus", n)

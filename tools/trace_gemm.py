@@ -5,11 +5,13 @@ MMA committed), bar1 / scatter / bar2 (cluster split-K reduction; for the SwiGLU
 
 Prints, for each distinct GEMM of the verify forward (by position inside a layer), the median over the
 middle layers of: launch-to-launch period, kernel span, and the phase stamps relative to the first CTA's
-entry.  The raw stamps go to gpurun_out/gemm_trace.npy for offline reading."""
+entry.  The raw stamps go to gemm_trace.npy and attn_trace.npy in the folder $TRACE_OUT (default: the current one)."""
 import os
 import sys
 
 sys.path.insert(0, os.path.dirname(os.path.dirname(os.path.abspath(__file__))))
+OUT = os.environ.get("TRACE_OUT", ".")
+os.makedirs(OUT, exist_ok=True)
 import numpy as np
 import torch
 from asd_b200 import _lib
@@ -42,10 +44,9 @@ torch.cuda.synchronize()
 L.asd_debug_gemm_trace(None, 0)
 L.asd_debug_attn_trace(None, 0)
 atr = abuf.cpu().numpy().reshape(MAXL, 1024, 16)
-np.save("gpurun_out/attn_trace.npy", atr[:, :512].copy())
+np.save(os.path.join(OUT, "attn_trace.npy"), atr[:, :512].copy())
 tr = buf.cpu().numpy().reshape(MAXL, stride // 16, 16)
-os.makedirs("gpurun_out", exist_ok=True)
-np.save("gpurun_out/gemm_trace.npy", tr[:, :512].copy())
+np.save(os.path.join(OUT, "gemm_trace.npy"), tr[:, :512].copy())
 
 used = [i for i in range(MAXL) if tr[i, 0, 0] != 0]
 print("launches traced:", len(used))
