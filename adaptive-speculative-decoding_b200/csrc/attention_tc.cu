@@ -519,9 +519,7 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
                         ((size_t)L.split_keys / L.page_size + 2) * 4 + 64;
     if (once.need()) {
         ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         prefer_max_smem(attn_tc_kernel<false>);
-        prefer_max_smem(attn_tc_kernel<true>);
     }
     if (smem > 227 * 1024) return set_error("attention_tc: split of %d keys does not fit the page-table slice", L.split_keys);
     AttnTcArgs a;
@@ -552,6 +550,10 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     const int tiles = L.q_tile > 0 ? (L.max_qlen + L.q_tile - 1) / L.q_tile : 1;
     if (g_attn_trace && g_attn_trace_next < g_attn_trace_max && (long long)tiles * L.nseq * L.nkv * L.nsplit_max <= 1024)
         a.trace = g_attn_trace + (size_t)(g_attn_trace_next++) * 1024 * 16;
+    if (a.trace) {      // (not before it is asked for: setting an attribute loads the kernel)
+        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        prefer_max_smem(attn_tc_kernel<true>);
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

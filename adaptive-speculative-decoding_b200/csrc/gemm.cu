@@ -807,9 +807,7 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
     if (g_gemm_attr.need()) {
         if (device_props()) return -1;
         ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
-        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
         prefer_max_smem(gemm_ws_kernel<false>);
-        prefer_max_smem(gemm_ws_kernel<true>);
     }
     GemmArgs a;
     a.M = pl.M;
@@ -852,6 +850,10 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
         a.trace = g_gemm_trace + (size_t)g_gemm_trace_next * kTraceCtas * kTraceSlots;
         if (pl.n_tiles * pl.ksplit * pl.m_tiles > kTraceCtas) a.trace = nullptr;
         ++g_gemm_trace_next;
+    }
+    if (a.trace) {      // (not before it is asked for: setting an attribute loads the kernel)
+        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
+        prefer_max_smem(gemm_ws_kernel<true>);
     }
     if (a.norm.sumsq_out != nullptr) {
         if (!pl.reduce || pl.mode != GEMM_OUT_F32)
