@@ -408,8 +408,8 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.slice_stride = slice_stride;
     a.norm = norm ? *norm : NormFusion{};
     a.err = wait_word();
-    // plainly (ptx.cuh); its successor may start early.  Programmatically launched, two prompts of 2048 tokens through 32B layers
-    // took the same time: 13.4 to 13.7 ms, and 13.5
+    // plainly (ptx.cuh); its successor may start early.  Eight prompts of 500 to 1000 tokens through two 32B layers, forwards of
+    // 2048 tokens: 13.4 to 13.7 ms launched programmatically, 13.5 to 14.4 so (power cap; boxes differ by as much)
     gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_PAIR);
