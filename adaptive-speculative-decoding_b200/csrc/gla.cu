@@ -1,15 +1,18 @@
 // Gated linear attention: a recurrence with a [dk][dv] state per head and a decay per key channel,
 //   S_t = diag(alpha_t) S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t,   alpha_t = sigmoid(z_t)^(1 / tau).
-// gla_decay_kernel:  alpha from the inner decay projection (one thread per channel and 32 tokens, fp32).
+// gla_decay_kernel:  alpha from the inner decay projection (a thread has 1 or 4 channels of 8 tokens, fp32).
 // gla_recurrence_kernel: one CTA per (sequence, head, 32 value columns).  Columns of S never mix, so a CTA owns its
-//   columns for the whole run of new positions: lane = column, warp = a slice of 4 to 32 consecutive key rows' worth of
-//   state held in registers (up to eight warps).  The new positions are staged CH at a time in shared memory (q, k,
-//   decay rows and the CTA's 32 value columns) by cp.async, one chunk ahead; per position every thread
-//   updates its rows and forms its slice's part of o, and after the chunk the slices are added in index order.  The arithmetic per position is the same whatever the
-//   chunking or the batch, so a sequence's outputs do not depend on how its tokens were cut into forwards.
+//   columns for the whole run of new positions: a thread keeps 8 key rows x 4 columns of the state in registers.  The
+//   new positions are staged CH at a time in shared memory (q, k, decay rows and the CTA's 32 value columns) by
+//   cp.async, one chunk ahead; per position every thread updates its part and forms its rows' share of o, and after the
+//   chunk the shares are added in index order.  The arithmetic per position is the same whatever the chunking or the
+//   batch, so a sequence's outputs do not depend on how its tokens were cut into forwards.
 //   The state lives in fp32 [slot][ring][head][dk][dv]; entry p % ring is the state after position p.
 // gla_out_kernel: RMS norm of every head's o over dv (plain weight), times silu(gate).
 #include <cuda_bf16.h>
+
+#include <algorithm>
+#include <type_traits>
 
 #include "asd_internal.h"
 #include "blocks.h"
@@ -20,8 +23,10 @@ namespace asd {
 
 namespace {
 
-constexpr int GLA_CH = 16;   // positions staged per chunk
-constexpr int GLA_NR = 32;   // state rows per thread at most
+constexpr int GLA_R = 8;     // key rows of the state per thread
+constexpr int GLA_C = 4;     // and columns
+constexpr int GLA_COLS = 32; // value columns per CTA
+constexpr int GLA_CG = GLA_COLS / GLA_C;
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
     const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
@@ -29,113 +34,200 @@ __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool val
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(addr), "l"(src), "r"(sz) : "memory");
 }
 
-constexpr int GD_TOK = 32, GD_CH = 256;   // tokens x channels per CTA of the decay kernel
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+    const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
+    const int sz = valid ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(addr), "l"(src), "r"(sz) : "memory");
+}
 
-// One CTA = 256 channels x 32 tokens: the channels' projection rows are staged transposed ([low][256], so that the
-// threads of a warp read consecutive words) and reused for all the tile's tokens, whose inner vectors every thread
-// reads as broadcasts.
-__global__ void __launch_bounds__(GD_CH) gla_decay_kernel(const float* a, long long lda, const float* w_decay,
+constexpr int GD_TOK = 32, GD_LANES = 64, GD_THREADS = 256;   // per CTA of the decay kernel: tokens, channel lanes, threads
+
+// One CTA = 64 * CPT channels x 32 tokens: the channels' projection rows are staged transposed, [low][channels] with an odd
+// row length (the stores of a warp, which go down a column, then meet 32 banks; with 256 floats a row they met one and the
+// staging alone took a third of the kernel); a thread has CPT channels 64 apart and 8 tokens, so that a staged value feeds CPT
+// or 8 products.  2151 tokens x 2048 channels, 32 inner: 53 -> 36 us (what is left is log1p, exp and expm1 of
+// every element); 16 tokens: 18 -> 7 us (CPT 1: more CTAs).
+template <int CPT>
+__global__ void __launch_bounds__(GD_THREADS) gla_decay_kernel(const float* a, long long lda, const float* w_decay,
                                                           const float* b_decay, GlaDims d, float* alpha, int M) {
     pdl_enter();
     extern __shared__ float sm[];
-    float* wT = sm;                      // [low][GD_CH]
-    float* av = sm + d.low * GD_CH;      // [GD_TOK][low]
+    constexpr int CH = GD_LANES * CPT, ST = CH + 1, TT = GD_TOK / (GD_THREADS / GD_LANES);
+    float* wT = sm;                      // [low][ST]
+    float* av = sm + d.low * ST;         // [GD_TOK][low]
     const int n = d.heads * d.dk;
-    const int c0 = blockIdx.x * GD_CH, m0 = blockIdx.y * GD_TOK;
+    const int c0 = blockIdx.x * CH, m0 = blockIdx.y * GD_TOK;
     const int nt = min(GD_TOK, M - m0);
-    for (int i = threadIdx.x; i < GD_CH * d.low; i += GD_CH) {
-        const int c = i / d.low, r = i - c * d.low;
-        wT[r * GD_CH + c] = c0 + c < n ? w_decay[(long long)(c0 + c) * d.low + r] : 0.f;
-    }
-    for (int i = threadIdx.x; i < GD_TOK * d.low; i += GD_CH) {
-        const int t = i / d.low, r = i - t * d.low;
-        av[i] = t < nt ? a[(long long)(m0 + t) * lda + r] : 0.f;
-    }
+    // eight loads on their way at a time; (outer, inner) of consecutive places GD_THREADS apart without a division each
+    auto stage = [&](int total, auto load, auto store) {
+        const int d_out = GD_THREADS / d.low, d_in = GD_THREADS - d_out * d.low;
+        int out = threadIdx.x / d.low, in = threadIdx.x - out * d.low;
+        for (int i = threadIdx.x; i < total; i += 8 * GD_THREADS) {
+            float x[8];
+            int o = out, r = in;
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                x[j] = i + j * GD_THREADS < total ? load(o, r) : 0.f;
+                o += d_out, r += d_in;
+                if (r >= d.low) r -= d.low, ++o;
+            }
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                if (i + j * GD_THREADS < total) store(out, in, x[j]);
+                out += d_out, in += d_in;
+                if (in >= d.low) in -= d.low, ++out;
+            }
+        }
+    };
+    stage(CH * d.low, [&](int c, int r) { return c0 + c < n ? w_decay[(long long)(c0 + c) * d.low + r] : 0.f; },
+          [&](int c, int r, float x) { wT[r * ST + c] = x; });
+    stage(GD_TOK * d.low, [&](int t, int r) { return t < nt ? a[(long long)(m0 + t) * lda + r] : 0.f; },
+          [&](int t, int r, float x) { av[t * d.low + r] = x; });
     __syncthreads();
-    const int c = c0 + threadIdx.x;
-    if (c >= n) return;
-    float z[GD_TOK];
+    const int lane = threadIdx.x & (GD_LANES - 1), first = threadIdx.x / GD_LANES * TT;
+    float z[CPT][TT];
 #pragma unroll
-    for (int t = 0; t < GD_TOK; ++t) z[t] = 0.f;
+    for (int i = 0; i < CPT; ++i)
+#pragma unroll
+        for (int t = 0; t < TT; ++t) z[i][t] = 0.f;
     for (int r = 0; r < d.low; ++r) {
-        const float w = wT[r * GD_CH + threadIdx.x];
+        float w[CPT];
 #pragma unroll
-        for (int t = 0; t < GD_TOK; ++t) z[t] = fmaf(w, av[t * d.low + r], z[t]);
+        for (int i = 0; i < CPT; ++i) w[i] = wT[r * ST + i * GD_LANES + lane];
+#pragma unroll
+        for (int t = 0; t < TT; ++t) {
+            const float x = av[(first + t) * d.low + r];
+#pragma unroll
+            for (int i = 0; i < CPT; ++i) z[i][t] = fmaf(w[i], x, z[i][t]);
+        }
     }
-    const float bias = b_decay[c], inv_tau = 1.f / d.tau;
+    const float inv_tau = 1.f / d.tau;
 #pragma unroll
-    for (int t = 0; t < GD_TOK; ++t) {
-        if (t < nt) {
-            const float zz = z[t] + bias;
-            // log sigmoid(z) = min(z, 0) - log1p(exp(-|z|)).  A slow decay lies just below 1, where expf's two units in
-            // the last place are a relative error of 1e-7 that hundreds of steps multiply; 1 + expm1 is rounded once
-            const float ls = fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)));
-            alpha[(long long)(m0 + t) * n + c] = 1.f + expm1f(ls * inv_tau);
+    for (int i = 0; i < CPT; ++i) {
+        const int c = c0 + i * GD_LANES + lane;
+        const float bias = c < n ? b_decay[c] : 0.f;
+#pragma unroll
+        for (int t = 0; t < TT; ++t) {
+            if (c < n && first + t < nt) {
+                const float zz = z[i][t] + bias;
+                // log sigmoid(z) = min(z, 0) - log1p(exp(-|z|)).  A slow decay lies just below 1, where expf's two units in
+                // the last place are a relative error of 1e-7 that hundreds of steps multiply; 1 + expm1 is rounded once
+                const float ls = fminf(zz, 0.f) - log1pf(expf(-fabsf(zz)));
+                alpha[(long long)(m0 + first + t) * n + c] = 1.f + expm1f(ls * inv_tau);
+            }
         }
     }
 }
 
-// ROWS state rows per thread (a multiple of 4: the staged q, k and decay rows are read as float4); the staged rows are
-// padded with zeros up to warps x ROWS, so rows beyond dk keep a zero state and add nothing.
-// CH positions are staged per chunk; MAXT bounds the CTA's threads (32 per slice of ROWS key rows).
-template <int ROWS, int MAXT, int CH>
-__global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) gla_recurrence_kernel(SeqIndex ix, const int* cu_q, const int* seq_slot,
-                                                            const float* q, const float* k, const float* v, long long ld,
-                                                            const float* alpha, GlaDims d, float* state, int ring,
-                                                            float* out) {
+struct Staged {                         // one position's values for a thread: its key rows in pairs, its columns
+    float2 a[GLA_R / 2], k[GLA_R / 2], q[GLA_R / 2];
+    float v[GLA_C];
+};
+
+// What bounds it: three fp32 operations per state element and position, and the staged values' way from shared memory into
+// registers (128 bytes a clock and SM, broadcast or not).  With one column and 16 rows per thread (the form before) a position
+// brought 12 bytes per element into registers, 780 clocks on an SM with two CTAs; with 8 rows x 4 columns it is 3.5, below the
+// arithmetic, which runs on packed pairs of rows.  3 prompts of up to 777 positions, 16 heads of 128 x 128: 321 -> 174 us
+// (436 clocks a position where an SM has two of the 192 CTAs, 245 where it has one; fp32 pipe 0.54 busy on the former).
+// Rows beyond dk are staged as zeros and take no k v^T (an infinite v times zero would be NaN): they add nothing.  `vec`: sizes and addresses allow 16-byte
+// copies.  MAXT: threads at most (8 per 8 key rows); PIPE: loads a position ahead.
+template <int MAXT, int MINB, bool PIPE>
+__global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix, const int* cu_q, const int* seq_slot, const float* q,
+                                                              const float* k, const float* v, long long ld, const float* alpha,
+                                                              GlaDims d, float* state, int ring, float* out, int CH, int vec) {
     pdl_enter();
     extern __shared__ __align__(16) float sm[];
-    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * 32;
+    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * GLA_COLS;
     const int t0 = cu_q[seq], t1 = cu_q[seq + 1];
     if (t0 >= t1) return;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, RS = blockDim.x >> 5, nthr = blockDim.x;
-    const int dkp = RS * ROWS;                          // padded key size
-    const int r0 = warp * ROWS;
-    const int col = col0 + lane;
-    const bool col_ok = col < d.dv;
+    const int tid = threadIdx.x, nthr = blockDim.x, RG = nthr / GLA_CG;
+    const int dkp = RG * GLA_R;                         // padded key size
+    const int rg = tid / GLA_CG, r0 = rg * GLA_R, ca = tid % GLA_CG * GLA_C;   // the thread's rows and columns
     const int slot = seq_slot[seq];
     const int p0 = ix.positions[t0];
-    // shared: two buffers of { q, k, decay [CH][dkp] each, v [CH][32] }, then the partial o [RS][CH][32]
-    const int buf_elems = 3 * CH * dkp + CH * 32;
+    // shared: two buffers of { q, k, decay [CH][dkp] each, v [CH][32] }, then the shares of o [RG][CH][32]
+    const int buf_elems = 3 * CH * dkp + CH * GLA_COLS, share = CH * GLA_COLS;
     float* part = sm + 2 * buf_elems;
-    const long long st_head = ((long long)head * d.dk) * d.dv;
     const long long st_entry = (long long)d.heads * d.dk * d.dv;
-    float* st_slot = state + (long long)slot * ring * st_entry;
-    float S[ROWS];
+    float* st_cta = state + (long long)slot * ring * st_entry + (long long)head * d.dk * d.dv + col0;
+    float2 S[GLA_R / 2][GLA_C];                         // [pair of rows][column]
+    auto copy_state = [&](float* entry, bool store) {
 #pragma unroll
-    for (int r = 0; r < ROWS; ++r) S[r] = 0.f;
-    if (p0 > 0 && col_ok) {
-        const float* src = st_slot + (long long)((p0 - 1) % ring) * st_entry + st_head;
+        for (int p = 0; p < GLA_R / 2; ++p)
 #pragma unroll
-        for (int r = 0; r < ROWS; ++r)
-            if (r0 + r < d.dk) S[r] = src[(long long)(r0 + r) * d.dv + col];
-    }
+            for (int h = 0; h < 2; ++h) {
+                const int r = r0 + 2 * p + h;
+                if (r >= d.dk) continue;
+                float* at = entry + (long long)r * d.dv + ca;
+                float x[GLA_C];
+#pragma unroll
+                for (int e = 0; e < GLA_C; ++e) x[e] = h ? S[p][e].y : S[p][e].x;
+                if (vec) {
+                    if (col0 + ca < d.dv) {
+                        if (store)
+                            *reinterpret_cast<float4*>(at) = make_float4(x[0], x[1], x[2], x[3]);
+                        else
+                            *reinterpret_cast<float4*>(x) = *reinterpret_cast<const float4*>(at);
+                    }
+                } else {
+#pragma unroll
+                    for (int e = 0; e < GLA_C; ++e)
+                        if (col0 + ca + e < d.dv) {
+                            if (store)
+                                at[e] = x[e];
+                            else
+                                x[e] = at[e];
+                        }
+                }
+                if (!store) {
+#pragma unroll
+                    for (int e = 0; e < GLA_C; ++e) {
+                        if (h)
+                            S[p][e].y = x[e];
+                        else
+                            S[p][e].x = x[e];
+                    }
+                }
+            }
+    };
+#pragma unroll
+    for (int p = 0; p < GLA_R / 2; ++p)
+#pragma unroll
+        for (int c = 0; c < GLA_C; ++c) S[p][c] = make_float2(0.f, 0.f);
     const int hq = head * d.dk, hv = head * d.dv;
     const int n_alpha = d.heads * d.dk;
-    // a chunk's rows arrive by 4-byte cp.async (any alignment), one chunk ahead of the arithmetic; rows beyond the
-    // chunk's positions and key channels beyond dk are filled with zeros
-    auto fetch = [&](int buf, int c0) {
-        const int nt = min(CH, t1 - c0);
-        float* qd = sm + buf * buf_elems;
-        float* kd = qd + CH * dkp;
-        float* ad = kd + CH * dkp;
-        float* vd = ad + CH * dkp;
-        for (int i = threadIdx.x; i < nt * dkp; i += nthr) {        // rows beyond the chunk's positions are never read
-            const int t = i / dkp, c = i - t * dkp;
-            const bool ok = c < d.dk;
-            const long long row = ok ? (long long)(c0 + t) * ld + hq + c : 0;
-            cp_async4(qd + i, q + row, ok);
-            cp_async4(kd + i, k + row, ok);
-            cp_async4(ad + i, alpha + (ok ? (long long)(c0 + t) * n_alpha + hq + c : 0), ok);
-        }
-        for (int i = threadIdx.x; i < nt * 32; i += nthr) {
-            const int t = i >> 5, c = i & 31;
-            const bool ok = col0 + c < d.dv;
-            cp_async4(vd + i, v + (ok ? (long long)(c0 + t) * ld + hv + col0 + c : 0), ok);
+    // W floats per copy, one chunk ahead of the arithmetic; a thread has the same places of every position
+    auto fetch_w = [&](int buf, int c0, auto width) {
+        constexpr int W = decltype(width)::value;
+        const int nt = min(CH, t1 - c0), per = dkp / W;
+        for (int i = tid; i < 3 * per + GLA_COLS / W; i += nthr) {
+            const int arr = i >= 2 * per ? (i >= 3 * per ? 3 : 2) : (i >= per ? 1 : 0);
+            const int c = (i - arr * per) * W;
+            const bool ok = arr == 3 ? col0 + c < d.dv : c < d.dk;
+            const long long step = arr == 2 ? n_alpha : ld;
+            const float* src = arr == 0 ? q : (arr == 1 ? k : (arr == 2 ? alpha : v));
+            if (ok) src += c0 * step + (arr == 3 ? hv + col0 + c : hq + c);
+            const int width_s = arr == 3 ? GLA_COLS : dkp;
+            float* dst = sm + buf * buf_elems + arr * CH * dkp + c;
+            for (int t = 0; t < nt; ++t) {              // places beyond the chunk's positions are never read
+                if constexpr (W == 4)
+                    cp_async16(dst, src, ok);
+                else
+                    cp_async4(dst, src, ok);
+                dst += width_s;
+                if (ok) src += step;
+            }
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    auto fetch = [&](int buf, int c0) {
+        if (vec)
+            fetch_w(buf, c0, std::integral_constant<int, 4>{});
+        else
+            fetch_w(buf, c0, std::integral_constant<int, 1>{});
+    };
     fetch(0, t0);
+    if (p0 > 0) copy_state(st_cta + (long long)((p0 - 1) % ring) * st_entry, false);
     int it = 0;
     for (int c0 = t0; c0 < t1; c0 += CH, ++it) {
         const int nt = min(CH, t1 - c0);
@@ -145,67 +237,137 @@ __global__ void __launch_bounds__(MAXT, MAXT <= 256 ? 2 : 1) gla_recurrence_kern
         } else {
             asm volatile("cp.async.wait_group 0;" ::: "memory");
         }
-        __syncthreads();   // this chunk's rows have landed for every thread; the previous partial sums have been read
-        const float* qs = sm + (it & 1) * buf_elems;
-        const float* ks = qs + CH * dkp;
-        const float* as = ks + CH * dkp;
-        const float* vs = as + CH * dkp;
-        for (int t = 0; t < nt; ++t) {
-            const float vt = vs[t * 32 + lane];
-            const float4* qt = reinterpret_cast<const float4*>(qs + t * dkp + r0);
-            const float4* kt = reinterpret_cast<const float4*>(ks + t * dkp + r0);
-            const float4* at = reinterpret_cast<const float4*>(as + t * dkp + r0);
-            float o0 = 0.f, o1 = 0.f, o2 = 0.f, o3 = 0.f;
+        __syncthreads();   // this chunk's rows have landed for every thread; the previous shares have been read
+        const float* qs = sm + (it & 1) * buf_elems + r0;
+        const float* vs = sm + (it & 1) * buf_elems + 3 * CH * dkp;
+        float* ps = part + rg * share;
+        auto load = [&](int t, Staged& x) {
 #pragma unroll
-            for (int r = 0; r < ROWS; r += 4) {
-                const float4 a4 = at[r >> 2], k4 = kt[r >> 2], q4 = qt[r >> 2];
-                S[r] = fmaf(a4.x, S[r], k4.x * vt);
-                S[r + 1] = fmaf(a4.y, S[r + 1], k4.y * vt);
-                S[r + 2] = fmaf(a4.z, S[r + 2], k4.z * vt);
-                S[r + 3] = fmaf(a4.w, S[r + 3], k4.w * vt);
-                o0 = fmaf(S[r], q4.x, o0);
-                o1 = fmaf(S[r + 1], q4.y, o1);
-                o2 = fmaf(S[r + 2], q4.z, o2);
-                o3 = fmaf(S[r + 3], q4.w, o3);
+            for (int i = 0; i < 2; ++i) {
+                *reinterpret_cast<float4*>(&x.a[2 * i]) = *reinterpret_cast<const float4*>(qs + 2 * CH * dkp + t * dkp + 4 * i);
+                *reinterpret_cast<float4*>(&x.k[2 * i]) = *reinterpret_cast<const float4*>(qs + CH * dkp + t * dkp + 4 * i);
+                *reinterpret_cast<float4*>(&x.q[2 * i]) = *reinterpret_cast<const float4*>(qs + t * dkp + 4 * i);
             }
-            part[(warp * CH + t) * 32 + lane] = (o0 + o1) + (o2 + o3);
-            // the last `ring` new positions leave their state behind
-            const int m = c0 + t;
-            if (t1 - m <= ring && col_ok) {
-                float* dst = st_slot + (long long)((p0 + (m - t0)) % ring) * st_entry + st_head;
+            *reinterpret_cast<float4*>(x.v) = *reinterpret_cast<const float4*>(vs + t * GLA_COLS + ca);
+        };
+        auto position = [&](int t, const Staged& x, auto beyond) {
+            float o[GLA_C];
 #pragma unroll
-                for (int r = 0; r < ROWS; ++r)
-                    if (r0 + r < d.dk) dst[(long long)(r0 + r) * d.dv + col] = S[r];
+            for (int c = 0; c < GLA_C; ++c) {
+                const float2 vc = make_float2(x.v[c], x.v[c]);
+                float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int p = 0; p < GLA_R / 2; ++p) {
+                    float2 kv = mul2(x.k[p], vc);
+                    if constexpr (decltype(beyond)::value) {
+                        if (r0 + 2 * p >= d.dk) kv.x = 0.f;
+                        if (r0 + 2 * p + 1 >= d.dk) kv.y = 0.f;
+                    }
+                    S[p][c] = fma2(x.a[p], S[p][c], kv);
+                    s = p ? fma2(S[p][c], x.q[p], s) : mul2(S[p][c], x.q[p]);
+                }
+                o[c] = s.x + s.y;
+            }
+            *reinterpret_cast<float4*>(ps + t * GLA_COLS + ca) = make_float4(o[0], o[1], o[2], o[3]);
+        };
+        // the last `ring` new positions leave their state behind
+        const int quiet = min(nt, max(0, t1 - ring - c0));
+        int t = 0;
+        if (PIPE && r0 + GLA_R <= d.dk && quiet > 0) {
+            // the next position's values are on their way while this one's are used (one past the last reads what is there, in
+            // bounds, for nothing); a share's store would otherwise hold its loads back
+            Staged x0, x1;
+            load(0, x0);
+            for (; t + 1 < quiet; t += 2) {
+                load(t + 1, x1);
+                position(t, x0, std::false_type{});
+                load(t + 2, x0);
+                position(t + 1, x1, std::false_type{});
+            }
+            if (t < quiet) position(t++, x0, std::false_type{});
+        }
+        if (!PIPE && r0 + GLA_R <= d.dk) {
+#pragma unroll 1
+            for (; t < quiet; ++t) {
+                Staged x;
+                load(t, x);
+                position(t, x, std::false_type{});
             }
         }
-        __syncthreads();   // the chunk is consumed (its buffer may be refilled) and the partial sums are complete
-        for (int i = threadIdx.x; i < nt * 32; i += nthr) {
-            const int t = i >> 5, c = i & 31;
+#pragma unroll 1
+        for (; t < nt; ++t) {
+            Staged x;
+            load(t, x);
+            position(t, x, std::true_type{});
+            if (t >= quiet) copy_state(st_cta + (long long)((p0 + (c0 + t - t0)) % ring) * st_entry, true);
+        }
+        __syncthreads();   // the chunk is consumed (its buffer may be refilled) and the shares are complete
+        for (int i = tid; i < nt * (GLA_COLS / 4); i += nthr) {
+            const int tt = i >> 3, c = (i & 7) * 4;
             if (col0 + c >= d.dv) continue;
-            float o = 0.f;
-            for (int w = 0; w < RS; ++w) o += part[(w * CH + t) * 32 + c];
-            out[(long long)(c0 + t) * d.heads * d.dv + hv + col0 + c] = o * d.q_scale;
+            float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int w = 0; w < RG; ++w) {
+                const float4 x = *reinterpret_cast<const float4*>(part + w * share + tt * GLA_COLS + c);
+                o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
+            }
+            o.x *= d.q_scale, o.y *= d.q_scale, o.z *= d.q_scale, o.w *= d.q_scale;
+            float* dst = out + (long long)(c0 + tt) * d.heads * d.dv + hv + col0 + c;
+            if (vec) {
+                *reinterpret_cast<float4*>(dst) = o;
+            } else {
+                dst[0] = o.x;
+                if (col0 + c + 1 < d.dv) dst[1] = o.y;
+                if (col0 + c + 2 < d.dv) dst[2] = o.z;
+                if (col0 + c + 3 < d.dv) dst[3] = o.w;
+            }
         }
     }
 }
 
+// one warp per (token, head); a lane keeps its values between the sum and the result: VN groups of four (dv <= 128 * VN, sizes
+// and addresses allow 16-byte accesses), or VN = 0: any size, read twice.  2151 tokens, 16 heads of 128: 22 -> 12.5 us.
+template <int VN>
 __global__ void gla_out_kernel(const float* o, const float* gate, long long ldg, const float* w, float eps, void* y,
-                               int of32, int heads, int dv) {
+                               int of32, long long pairs, int heads, int dv) {
     pdl_enter();
-    // one warp per (token, head)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int h = blockIdx.y * (blockDim.x >> 5) + warp;
-    if (h >= heads) return;
-    const long long m = blockIdx.x;
-    const float* src = o + (m * heads + h) * dv;
-    const float* g = gate + m * ldg + (long long)h * dv;
+    const int lane = threadIdx.x & 31;
+    const long long i0 = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (i0 >= pairs) return;
+    const long long m = i0 / heads;
+    const float* src = o + i0 * dv;
+    const float* g = gate + m * ldg + (i0 - m * heads) * dv;
     float ss = 0.f;
-    for (int i = lane; i < dv; i += 32) ss += src[i] * src[i];
-    ss = warp_sum(ss);
-    const float r = 1.f / sqrtf(ss / (float)dv + eps);
-    for (int i = lane; i < dv; i += 32) {
-        const float gv = g[i];
-        stx(y, (m * heads + h) * dv + i, of32, src[i] * r * w[i] * (gv / (1.f + expf(-gv))));
+    if constexpr (VN > 0) {
+        float x[VN][4], gv[VN][4];
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int i = (j * 32 + lane) * 4;
+            if (i >= dv) break;
+            ldx4(src, i, 1, x[j]);
+            ldx4(g, i, 1, gv[j]);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) ss += x[j][e] * x[j][e];
+        }
+        ss = warp_sum(ss);
+        const float r = 1.f / sqrtf(ss / (float)dv + eps);
+#pragma unroll
+        for (int j = 0; j < VN; ++j) {
+            const int i = (j * 32 + lane) * 4;
+            if (i >= dv) break;
+            float wv[4];
+            ldx4(w, i, 1, wv);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) x[j][e] = x[j][e] * r * wv[e] * (gv[j][e] / (1.f + expf(-gv[j][e])));
+            stx4(y, i0 * dv + i, of32, x[j]);
+        }
+    } else {
+        for (int i = lane; i < dv; i += 32) ss += src[i] * src[i];
+        ss = warp_sum(ss);
+        const float r = 1.f / sqrtf(ss / (float)dv + eps);
+        for (int i = lane; i < dv; i += 32) {
+            const float gv = g[i];
+            stx(y, i0 * dv + i, of32, src[i] * r * w[i] * (gv / (1.f + expf(-gv))));
+        }
     }
 }
 
@@ -215,13 +377,21 @@ int launch_gla_decay(const float* a, long long lda, const float* w_decay, const 
                      float* alpha, int M, cudaStream_t stream) {
     if (M <= 0) return 0;
     if (d.low <= 0 || !(d.tau > 0.f)) return set_error("gla: decay projection of size %d, tau %f", d.low, d.tau);
-    const size_t smem = (size_t)d.low * (GD_CH + GD_TOK) * sizeof(float);
-    if (smem > 200 * 1024) return set_error("gla: decay projection of size %d does not fit shared memory", d.low);
+    if ((size_t)d.low * (256 + GD_TOK) * sizeof(float) > 200 * 1024)
+        return set_error("gla: decay projection of size %d does not fit shared memory", d.low);
+    const int n = d.heads * d.dk, tiles = (M + GD_TOK - 1) / GD_TOK;
+    if (tiles > 65535) return set_error("gla: too many tokens");
+    // four channels a thread where that still gives every SM a CTA
+    const int cpt = (n + 4 * GD_LANES - 1) / (4 * GD_LANES) * tiles >= sm_count() ? 4 : 1;
+    const size_t smem = ((size_t)d.low * (GD_LANES * cpt + 1) + (size_t)d.low * GD_TOK) * sizeof(float);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    dim3 grid((d.heads * d.dk + GD_CH - 1) / GD_CH, (M + GD_TOK - 1) / GD_TOK);
-    if (grid.y > 65535) return set_error("gla: too many tokens");
-    ASD_CUDA(launch_pdl(gla_decay_kernel, grid, GD_CH, smem, stream, a, lda, w_decay, b_decay, d, alpha, M));
+    if (once.need()) {
+        ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    }
+    const dim3 grid((n + GD_LANES * cpt - 1) / (GD_LANES * cpt), tiles);
+    ASD_CUDA(launch_pdl(cpt == 4 ? gla_decay_kernel<4> : gla_decay_kernel<1>, grid, GD_THREADS, smem, stream, a, lda, w_decay,
+                        b_decay, d, alpha, M));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -231,30 +401,28 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
                           const float* k, const float* v, long long ld, const float* alpha, const GlaDims& d,
                           float* state, int ring, float* out, cudaStream_t stream) {
     if (ix.M <= 0 || nseq <= 0) return 0;
-    if (d.dk <= 0 || d.dk > 32 * GLA_NR) return set_error("gla: key size %d outside 1..%d", d.dk, 32 * GLA_NR);
+    if (d.dk <= 0 || d.dk > 1024) return set_error("gla: key size %d outside 1..1024", d.dk);
     if (ring <= 0 || !state) return set_error("gla: no state");
-    // the fewest state rows per thread (4, 8, 16 or 32) that at most eight warps cover
-    int rows = 4;
-    while (rows < GLA_NR && rows * 8 < d.dk) rows *= 2;
-    const int RS = (d.dk + rows - 1) / rows;              // more than eight warps only for key sizes above 256
-    const int dkp = RS * rows;
-    const int ch = RS <= 8 ? GLA_CH : GLA_CH / 4;         // shorter chunks keep the staged rows of a large head in shared memory
-    const size_t smem = (size_t)(2 * (3 * ch * dkp + ch * 32) + RS * ch * 32) * sizeof(float);
-    dim3 grid(nseq, d.heads, (d.dv + 31) / 32);
+    const int threads = ((d.dk + GLA_R - 1) / GLA_R * GLA_CG + 31) / 32 * 32, RG = threads / GLA_CG, dkp = RG * GLA_R;
+    // chunks as long as two (large heads: one) staged CTAs per SM allow, and no longer than the runs: a step's CTAs are then
+    // small enough for an SM to hold all that its registers can
+    int ch = dkp <= 128 ? 16 : (dkp <= 512 ? 8 : 4);
+    const int run = (ix.M + nseq - 1) / nseq;
+    ch = std::min(ch, run <= 1 ? 1 : std::max(4, run));
+    const size_t smem = (size_t)(2 * (3 * ch * dkp + ch * GLA_COLS) + RG * ch * GLA_COLS) * sizeof(float);
+    const dim3 grid(nseq, d.heads, (d.dv + GLA_COLS - 1) / GLA_COLS);
     if (grid.y > 65535 || grid.z > 65535) return set_error("gla: too many heads or value columns");
-#define ASD_GLA_CASE(R, T, C)                                                                                         \
-    {                                                                                                                 \
-        auto fn = gla_recurrence_kernel<R, T, C>;                                                                        \
-        static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
-        ASD_CUDA(launch_pdl(fn, grid, RS * 32, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out));             \
-    }
-    if (RS > 8) ASD_GLA_CASE(32, 1024, GLA_CH / 4)
-    else if (rows == 4) ASD_GLA_CASE(4, 256, GLA_CH)
-    else if (rows == 8) ASD_GLA_CASE(8, 256, GLA_CH)
-    else if (rows == 16) ASD_GLA_CASE(16, 256, GLA_CH)
-    else ASD_GLA_CASE(32, 256, GLA_CH)
-#undef ASD_GLA_CASE
+    const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
+                         reinterpret_cast<uintptr_t>(alpha) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out);
+    const int vec = (at & 15) == 0 && ld % 4 == 0 && d.dk % 4 == 0 && d.dv % 4 == 0;
+    // steps: no loads ahead, and the registers of four (key sizes up to 128: eight) CTAs per SM
+    auto fn = threads > 512 ? gla_recurrence_kernel<1024, 1, false>
+                            : (threads > 256 ? gla_recurrence_kernel<512, 1, true>
+                                             : (ch == 1 ? gla_recurrence_kernel<256, 4, false> : gla_recurrence_kernel<256, 2, true>));
+    static PerDeviceOnce once[4];
+    if (once[threads > 512 ? 3 : (threads > 256 ? 2 : ch == 1)].need())
+        ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_CUDA(launch_pdl(fn, grid, threads, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out, ch, vec));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -263,9 +431,13 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
 int launch_gla_out(const float* o, const float* gate, long long ldg, const float* w, float eps, void* y, int of32, int M,
                    int heads, int dv, cudaStream_t stream) {
     if (M <= 0) return 0;
-    const int wpb = heads < 8 ? heads : 8;
-    dim3 grid(M, (heads + wpb - 1) / wpb);
-    ASD_CUDA(launch_pdl(gla_out_kernel, grid, wpb * 32, 0, stream, o, gate, ldg, w, eps, y, of32, heads, dv));
+    const long long pairs = (long long)M * heads, blocks = (pairs + 7) / 8;
+    if (blocks > 0x7fffffffLL) return set_error("gla: too many tokens");
+    const uintptr_t at = reinterpret_cast<uintptr_t>(o) | reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(w) |
+                         reinterpret_cast<uintptr_t>(y);
+    const bool vec = (at & 15) == 0 && ldg % 4 == 0 && dv % 4 == 0 && dv <= 256;
+    auto fn = !vec ? gla_out_kernel<0> : (dv <= 128 ? gla_out_kernel<1> : gla_out_kernel<2>);
+    ASD_CUDA(launch_pdl(fn, (unsigned)blocks, 256, 0, stream, o, gate, ldg, w, eps, y, of32, pairs, heads, dv));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;

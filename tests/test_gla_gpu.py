@@ -1,0 +1,26 @@
+"""GPU: the gated recurrence at the edges of its split: 8 key rows x 4 columns of the state per thread, 32 columns per CTA,
+positions staged 4, 8 or 16 at a time (1 in steps), 16-byte copies where the sizes allow."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from oracle import rivetar_oracle as O  # noqa: E402
+from test_rivetar_gpu import close, config, feed, gla, make_engine, rel_err, tokens  # noqa: E402
+
+
+# one row group, whole groups and a rest of one, sizes that are no multiple of four, the largest group counts of both instances
+@pytest.mark.parametrize("dim,vdim,rank", [(8, 4, 8), (72, 36, 1), (65, 34, 3), (128, 128, 32), (260, 32, 5), (512, 33, 2),
+                                           (520, 12, 2), (1024, 8, 1)])
+def test_state_tiles_and_chunks(dim, vdim, rank):
+    cfg = config([gla(heads=2, dim=dim, vdim=vdim, tau=16.0, decay_rank=rank)])
+    w = O.random_model(cfg, seed=21)
+    ids = tokens(47, 96, 22)
+    ref, _ = O.forward(cfg, w, ids)
+    eng = make_engine(cfg, w, max_tokens=64)
+    one = feed(eng, eng.open_sequence(), ids, [])
+    # runs of 1, 2, 4, 5, 16 and 17 positions: the sums of a position do not depend on the cut
+    cut = feed(eng, eng.open_sequence(), ids, [1, 2, 4, 5, 16, 17, 1, 1])
+    assert rel_err(one, ref)[1] < 2e-4          # as the other tests of this engine: far below one missed position
+    assert torch.equal(one, cut)
+    close(eng)
