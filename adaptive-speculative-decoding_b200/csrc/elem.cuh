@@ -104,4 +104,18 @@ __device__ __forceinline__ float block_sum(float v, float* red) {
     return red[32];
 }
 
+// K sums over the block in a fixed order with one barrier; red: K * 32 floats of shared memory of their own
+template <int K>
+__device__ __forceinline__ void block_sums(float (&v)[K], float* red) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        v[k] = warp_sum(v[k]);
+        if (lane == 0) red[k * 32 + warp] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] = warp_sum(lane < nw ? red[k * 32 + lane] : 0.f);
+}
+
 }  // namespace asd
