@@ -5,7 +5,8 @@ import torch
 
 pytestmark = pytest.mark.gpu
 
-from oracle import rivetar_oracle as O  # noqa: E402
+import test_mezilix_gpu as mz  # noqa: E402
+from oracle import mezilix_oracle, rivetar_oracle as O  # noqa: E402
 from test_rivetar_gpu import close, config, feed, gla, latent, make_engine, rel_err, tokens  # noqa: E402
 
 
@@ -23,3 +24,18 @@ def test_closes_norms_and_polynomials_of_odd_widths(width, ff, q_rank):
     assert rel_err(one, ref)[1] < 2e-4          # as the other tests of this engine
     assert torch.equal(one, cut)                # a row's sums do not depend on the rows beside it
     close(eng)
+
+
+@pytest.mark.parametrize("width", [36, 1024, 1028, 2052, 16384, 16388, 1026])
+def test_pair_embedding_shift_and_depth_weighted_close_of_odd_widths(width):
+    cfg = mz.config([mz.layer(heads=1, dim=8, rot_dim=4, vdim=8, kv_rank=12, experts=3, top=2, ff=8),
+                     mz.layer(heads=1, dim=8, rot_dim=4, vdim=8, kv_rank=12, experts=0)], width=width)
+    w = mezilix_oracle.random_model(cfg, seed=33)
+    ids = mz.tokens(9, 96, 34)
+    ref, _ = mezilix_oracle.forward(cfg, w, ids)
+    eng = mz.make_engine(cfg, w)
+    one = mz.feed(eng, eng.open_sequence(), ids, [])
+    cut = mz.feed(eng, eng.open_sequence(), ids, [4, 1])
+    assert mz.rel_err(one, ref)[1] < 2e-4
+    assert torch.equal(one, cut)
+    mz.close(eng)
