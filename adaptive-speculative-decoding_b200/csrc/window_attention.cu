@@ -51,30 +51,47 @@ __device__ __forceinline__ float turned(const float* src, int i, int n, int inte
     return i == a ? u * cs - v * sn : v * cs + u * sn;
 }
 
+// 2151 tokens, 16 + 4 heads of 128: 38 -> 18 us; 16 tokens: 13 -> 7 (a sincosf per coordinate and head, and a copy of the row, before).
 __global__ void window_post_kernel(SeqIndex ix, float* qkv, long long ld, WindowDims d, const float* freq_k,
                                    const float* freq_v, PagedRows cache) {
     pdl_enter();
-    extern __shared__ float row[];   // the token's q | k | v as projected
+    extern __shared__ float2 turn[];   // cos, sin of the token's angles, of keys and of values: once a token, not once a head
     const int m = blockIdx.x;
     const int pos = ix.positions[m], slot = ix.token_slot[m];
-    const int nq = d.heads * d.dk, nk = d.kv_heads * d.dk, nv = d.kv_heads * d.dv;
-    float* src = qkv + (long long)m * ld;
-    for (int i = threadIdx.x; i < nq + nk + nv; i += blockDim.x) row[i] = src[i];
-    __syncthreads();
-    const long long crow = wcache_row(cache, slot, pos) * (nk + nv);
+    const int nq = d.heads * d.dk, nk = d.kv_heads * d.dk, nv = d.kv_heads * d.dv, half = d.rot_dims >> 1, halfv = d.dv >> 1;
     const float p = (float)pos;
-    for (int i = threadIdx.x; i < nq + nk; i += blockDim.x) {
-        const int h = i / d.dk, c = i % d.dk;
-        const float v = turned(row + (long long)h * d.dk, c, d.rot_dims, d.interleaved, p, freq_k, 1.f);
-        if (i < nq)
-            src[i] = v;
-        else
-            stx(cache.pool, crow + (i - nq), cache.f32, v);
+    for (int j = threadIdx.x; j < half + halfv; j += blockDim.x) {
+        float sn, cs;
+        sincosf(p * (j < half ? freq_k[j] : freq_v[j - half]), &sn, &cs);
+        turn[j] = make_float2(cs, sn);
     }
-    for (int i = threadIdx.x; i < nv; i += blockDim.x) {
-        const int h = i / d.dv, c = i % d.dv;
-        stx(cache.pool, crow + nk + i, cache.f32,
-            turned(row + nq + nk + (long long)h * d.dv, c, d.dv, d.interleaved, p, freq_v, 1.f));
+    float* src = qkv + (long long)m * ld;
+    const long long crow = wcache_row(cache, slot, pos) * (nk + nv);
+    __syncthreads();
+    // a pair per step: of query and key heads, then of value heads
+    const int n_qk = (d.heads + d.kv_heads) * half, n_v = d.kv_heads * halfv;
+    for (int t = threadIdx.x; t < n_qk + n_v; t += blockDim.x) {
+        const bool val = t >= n_qk;
+        const int n = val ? halfv : half, i = val ? t - n_qk : t, h = i / n, j = i - h * n;
+        const int a = d.interleaved ? 2 * j : j, b = d.interleaved ? 2 * j + 1 : j + n;
+        float* at = src + (val ? nq + nk + h * d.dv : h * d.dk);
+        const float2 cs = turn[val ? half + j : j];
+        const float x = at[a], y = at[b];
+        const float u = x * cs.x - y * cs.y, w = y * cs.x + x * cs.y;
+        if (!val && h < d.heads) {
+            at[a] = u;
+            at[b] = w;
+        } else {
+            const long long c = crow + (val ? nk + h * d.dv : (h - d.heads) * d.dk);
+            stx(cache.pool, c + a, cache.f32, u);
+            stx(cache.pool, c + b, cache.f32, w);
+        }
+    }
+    // key coordinates that are not turned
+    const int rest = d.dk - d.rot_dims;
+    for (int i = threadIdx.x; i < d.kv_heads * rest; i += blockDim.x) {
+        const int h = i / rest, c = d.rot_dims + i - h * rest;
+        stx(cache.pool, crow + h * d.dk + c, cache.f32, src[nq + h * d.dk + c]);
     }
 }
 
@@ -699,8 +716,9 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
                        const float* freq_v, const PagedRows& cache, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
     if (check_dims(d)) return -1;
-    const size_t smem = (size_t)(d.heads * d.dk + d.kv_heads * (d.dk + d.dv)) * sizeof(float);
-    if (smem > 200 * 1024) return set_error("windowed attention: a token's q | k | v row does not fit shared memory");
+    if ((size_t)(d.heads * d.dk + d.kv_heads * (d.dk + d.dv)) * sizeof(float) > 200 * 1024)
+        return set_error("windowed attention: a token's q | k | v row is too long");
+    const size_t smem = (size_t)(d.rot_dims + d.dv) / 2 * sizeof(float2);
     static PerDeviceOnce once;
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(window_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
     ASD_CUDA(launch_pdl(window_post_kernel, ix.M, 256, smem, stream, ix, qkv, ld, d, freq_k, freq_v, cache));
