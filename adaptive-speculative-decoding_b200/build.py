@@ -27,7 +27,7 @@ COMPONENTS = {
     "latent": ["latent_attention.cu", "latent_attention_tc.cu"],
     "rows": ["norm_ops.cu", "moe.cu"],          # row kernels and the expert router that several families share
     "mezilix": ["mezilix_engine.cu", "stream_ops.cu"],
-    "rivetar": ["rivetar_engine.cu", "gla.cu", "window_attention.cu"],
+    "rivetar": ["rivetar_engine.cu", "gla.cu", "window_attention.cu", "window_attention_tc.cu"],
     "delta": ["delta_rule.cu"],                 # delta rules and short convolutions
     "mixattn": ["mixed_attention.cu", "mixed_attention_tc.cu", "sigmoid_attention.cu",
                 "decode_attention_tc.cu"],

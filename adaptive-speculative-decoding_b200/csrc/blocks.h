@@ -312,16 +312,24 @@ struct WindowDims {
     float scale;
 };
 // qkv fp32 rows (ld floats apart) = [heads * dk | kv_heads * dk | kv_heads * dv].  Rotates the queries in place and
-// appends the rotated keys and values to the cache.  freq_k fp32 [rot_dims / 2], freq_v fp32 [dv / 2].
+// appends the rotated keys and values to the cache.  freq_k fp32 [rot_dims / 2], freq_v fp32 [dv / 2].  turns (optional,
+// [M][dv / 2]): receives cos, sin of every token's value angles.
 int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const WindowDims& d, const float* freq_k,
-                       const float* freq_v, const PagedRows& cache, cudaStream_t stream);
+                       const float* freq_v, const PagedRows& cache, float2* turns, cudaStream_t stream);
 // out[m][heads * dv] in the engine's element type: softmax (denominator + exp(sink[head])) over the visible positions,
 // turned back by the query's position.  sink fp32 [heads] (nullptr: none).  tiled = 0: one warp per (token, head);
 // else bf16 cache rows run on the tensor cores where the sizes allow.  ws (the AttnSplit workspace of the latent
 // kernels; o and ml may be nullptr) holds the partial results when single-token steps cut the keys into shares.
+// turns: what launch_window_post wrote; with it (and ws.tiled 2) calls of enough query rows take the tcgen05 form
+// (window_attention_tc.cu) where the sizes allow.
+bool window_attention_tc_takes(const WindowDims& d, const PagedRows& cache, int max_qlen, const float* q, long long ldq,
+                               const void* out, int of32);
+int launch_window_attention_tc(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen, const float* q,
+                               long long ldq, const WindowDims& d, const float* sink, const float2* turns,
+                               const PagedRows& cache, void* out, cudaStream_t stream);
 int launch_window_attention(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,
                             int max_kv_len, const float* q, long long ldq, const WindowDims& d, const float* sink,
-                            const float* freq_v, const PagedRows& cache, void* out, int of32, int tiled,
+                            const float* freq_v, const float2* turns, const PagedRows& cache, void* out, int of32, int tiled,
                             const AttnSplit& ws, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------- delta_rule.cu

@@ -64,6 +64,7 @@ struct RvEngine : asd_rivetar_engine {
     // owned activations
     float *x = nullptr, *x0 = nullptr, *y = nullptr, *proj = nullptr, *qbuf = nullptr, *qlat = nullptr, *olat = nullptr,
           *alpha = nullptr, *orec = nullptr, *up = nullptr;
+    float2* turns = nullptr;   // cos, sin of the tokens' value angles (windowed attention of bf16 engines)
     void *hn = nullptr, *cq = nullptr, *mixed = nullptr, *act = nullptr, *xsel = nullptr;
     std::vector<void*> owned;
     DenseRunner dn;
@@ -206,14 +207,15 @@ static int mix_window(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
         if (e->dn.run(e->hn, ly.w("w_in"), e->proj, M, ly.n_in, D, ly.n_in, li * 16 + 0, s)) return -1;
     }
     const WindowDims wd{c.heads, c.kv_heads, c.dim, c.vdim, c.rot_dims, c.rot_interleaved, c.window, c.keep_first, c.scale};
-    const PagedRows cache{e->pool + run.cache_off * e->esz, f32, e->page_table, e->max_pages, e->c.page_size};
+    const PagedRows cache{e->pool + run.cache_off * e->esz, f32,           e->page_table,
+                          e->max_pages,                     e->c.page_size, (long long)e->num_pages * e->c.page_size};
     {
         RV_PROF(RV_GLUE);
-        if (launch_window_post(b.ix, e->proj, ly.n_in, wd, ly.freq_k, ly.freq_v, cache, s)) return -1;
+        if (launch_window_post(b.ix, e->proj, ly.n_in, wd, ly.freq_k, ly.freq_v, cache, e->turns, s)) return -1;
     }
     RV_PROF(RV_WINDOW_ATTN);
     return launch_window_attention(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->proj, ly.n_in, wd,
-                                   ly.f("sink"), ly.freq_v, cache, e->mixed, f32, e->fused_attn, e->attn_ws, s);
+                                   ly.f("sink"), ly.freq_v, e->turns, cache, e->mixed, f32, e->fused_attn, e->attn_ws, s);
 }
 
 static int forward(RvEngine* e, const Batch& b, const int* logit_rows, int n_rows, float* logits, long long ld,
@@ -358,7 +360,7 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     e->esz = cfg->dtype ? 4 : 2;
     cudaGetDevice(&e->device);
     const size_t MT = cfg->max_tokens, D = cfg->width;
-    size_t n_in = 1, nq = 1, qlat = 1, olat = 1, hv = 1, qr = 1, nk = 1, ff = 1;
+    size_t n_in = 1, nq = 1, qlat = 1, olat = 1, hv = 1, qr = 1, nk = 1, ff = 1, vh = 0;
     auto fail = [&](const char* what, int l) {
         set_error("asd_rivetar_create: %s (layer %d)", what, l);
         asd_rivetar_destroy(e);
@@ -392,6 +394,7 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
                 return fail("bad windowed attention sizes", l);
             ly.n_in = c.heads * c.dim + c.kv_heads * (c.dim + c.vdim);
             ly.cache_row = c.kv_heads * (c.dim + c.vdim);
+            vh = std::max(vh, (size_t)c.vdim / 2);
             if (upload_freq(e, &ly.freq_k, c.rot_dims, c.rot_base) || upload_freq(e, &ly.freq_v, c.vdim, c.rot_base))
                 return fail("device allocation failed", l);
         }
@@ -427,6 +430,7 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     rc |= dev_alloc(e, (char**)&e->mixed, MT * hv * e->esz);
     rc |= dev_alloc(e, (char**)&e->act, MT * ff * e->esz);
     rc |= dev_alloc(e, (char**)&e->xsel, MT * D * e->esz);
+    if (vh && !e->f32) rc |= dev_alloc(e, &e->turns, MT * vh);
     e->attn_ws.rows = 16384;
     e->attn_ws.o_elems = e->attn_ws.rows * 512;
     rc |= dev_alloc(e, &e->attn_ws.o, (size_t)e->attn_ws.o_elems);

@@ -53,7 +53,7 @@ __device__ __forceinline__ float turned(const float* src, int i, int n, int inte
 
 // 2151 tokens, 16 + 4 heads of 128: 38 -> 18 us; 16 tokens: 13 -> 7 (a sincosf per coordinate and head, and a copy of the row, before).
 __global__ void window_post_kernel(SeqIndex ix, float* qkv, long long ld, WindowDims d, const float* freq_k,
-                                   const float* freq_v, PagedRows cache) {
+                                   const float* freq_v, PagedRows cache, float2* turns) {
     pdl_enter();
     extern __shared__ float2 turn[];   // cos, sin of the token's angles, of keys and of values: once a token, not once a head
     const int m = blockIdx.x;
@@ -64,6 +64,7 @@ __global__ void window_post_kernel(SeqIndex ix, float* qkv, long long ld, Window
         float sn, cs;
         sincosf(p * (j < half ? freq_k[j] : freq_v[j - half]), &sn, &cs);
         turn[j] = make_float2(cs, sn);
+        if (turns && j >= half) turns[(long long)m * halfv + j - half] = make_float2(cs, sn);
     }
     float* src = qkv + (long long)m * ld;
     const long long crow = wcache_row(cache, slot, pos) * (nk + nv);
@@ -713,7 +714,7 @@ int check_dims(const WindowDims& d) {
 }  // namespace
 
 int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const WindowDims& d, const float* freq_k,
-                       const float* freq_v, const PagedRows& cache, cudaStream_t stream) {
+                       const float* freq_v, const PagedRows& cache, float2* turns, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
     if (check_dims(d)) return -1;
     if ((size_t)(d.heads * d.dk + d.kv_heads * (d.dk + d.dv)) * sizeof(float) > 200 * 1024)
@@ -721,7 +722,7 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
     const size_t smem = (size_t)(d.rot_dims + d.dv) / 2 * sizeof(float2);
     static PerDeviceOnce once;
     if (once.need()) ASD_CUDA(cudaFuncSetAttribute(window_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    ASD_CUDA(launch_pdl(window_post_kernel, ix.M, 256, smem, stream, ix, qkv, ld, d, freq_k, freq_v, cache));
+    ASD_CUDA(launch_pdl(window_post_kernel, ix.M, 256, smem, stream, ix, qkv, ld, d, freq_k, freq_v, cache, turns));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
@@ -729,10 +730,12 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
 
 int launch_window_attention(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,
                             int max_kv_len, const float* q, long long ldq, const WindowDims& d, const float* sink,
-                            const float* freq_v, const PagedRows& cache, void* out, int of32, int tiled,
+                            const float* freq_v, const float2* turns, const PagedRows& cache, void* out, int of32, int tiled,
                             const AttnSplit& ws, cudaStream_t stream) {
     if (ix.M <= 0 || nseq <= 0) return 0;
     if (check_dims(d)) return -1;
+    if (tiled && ws.tiled >= 2 && turns && window_attention_tc_takes(d, cache, max_qlen, q, ldq, out, of32))
+        return launch_window_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, q, ldq, d, sink, turns, cache, out, stream);
     if (tiled && mma_supports(d, cache))
         return launch_mma(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q, ldq, d, sink, freq_v, cache, out, of32, ws, stream);
     return cache.f32 ? launch_simple<float>(ix, cu_q, seq_slot, nseq, max_qlen, q, ldq, d, sink, freq_v, cache, out, of32, stream)

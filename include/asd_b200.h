@@ -38,7 +38,7 @@ ASD_API const char* asd_last_error(void);
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
 /* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemv",
- * "attention_tc", "latent_tc", "sampler_draw"; -1 for another name */
+ * "attention_tc", "latent_tc", "window_tc", "sampler_draw"; -1 for another name */
 ASD_API long long asd_kernel_launches(const char* name);
 /* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:
  * engines then refuse every later forward (asd_*_device_error names the kernel), a sampler call is refused once.
