@@ -37,7 +37,7 @@ struct DenseRunner {
                 Entry t;
                 if (make_tmap_bf16(&t.tw, w, N, K, K, 128)) return -1;
                 if (M >= tc_min_rows) {   // above the HBM / tensor ridge: 256 weight rows x MT tokens on a CTA pair
-                    if (gemm_tc_plan(&t.big, M, N, K, GEMM_OUT_F32, 1, 0)) return -1;
+                    if (gemm_tc_plan(&t.big, M, N, K, GEMM_OUT_F32, 1, 0, false)) return -1;
                     if (make_tmap_bf16(&t.tx, x, M, K, K, t.big.MT / 2)) return -1;
                 } else {
                     if (gemm_plan(&t.pl, M, N, K, GEMM_OUT_F32, 0, 0, 1)) return -1;

@@ -154,15 +154,15 @@ static int ensure_plans(Engine* e, int M, Plans** out) {
     if (make_tmap_bf16(&p.x_act, e->act, M, e->c.ffn, e->c.ffn, p.down.MT)) return -1;
     p.use_tc = e->tune.gemm_big && M > 256;
     if (p.use_tc) {
-        if (gemm_tc_plan(&p.gu_tc, M, 2 * e->ffp, h, GEMM_OUT_SWIGLU, 0, e->force_stages)) return -1;
-        if (gemm_tc_plan(&p.down_tc, M, h, e->c.ffn, GEMM_OUT_F32, 0, e->force_stages)) return -1;
+        if (gemm_tc_plan(&p.gu_tc, M, 2 * e->ffp, h, GEMM_OUT_SWIGLU, 0, e->force_stages, true)) return -1;
+        if (gemm_tc_plan(&p.down_tc, M, h, e->c.ffn, GEMM_OUT_F32, 0, e->force_stages, false)) return -1;
         if ((size_t)p.down_tc.ksplit * M * h > e->part_floats) return set_error("engine: split-K workspace too small");
         if (make_tmap_bf16(&p.x_norm_tc, e->fuse_norm ? e->resid_bf : e->xnorm, M, h, h, p.gu_tc.MT / 2)) return -1;
         if (make_tmap_bf16(&p.x_act_tc, e->act, M, e->c.ffn, e->c.ffn, p.down_tc.MT / 2)) return -1;
         // QKV and O as well: at 576 tokens the weight-streaming kernel spends 59 / 120 us per layer on them (72B, TP4
         // shard; its per-thread epilogue loops are serial over the tokens), the CTA-pair kernel runs them at ~900 TFLOP/s
-        if (gemm_tc_plan(&p.qkv_tc, M, e->nqkv, h, GEMM_OUT_F32, 0, e->force_stages)) return -1;
-        if (gemm_tc_plan(&p.o_tc, M, h, e->qdim, GEMM_OUT_F32, 0, e->force_stages)) return -1;
+        if (gemm_tc_plan(&p.qkv_tc, M, e->nqkv, h, GEMM_OUT_F32, 0, e->force_stages, true)) return -1;
+        if (gemm_tc_plan(&p.o_tc, M, h, e->qdim, GEMM_OUT_F32, 0, e->force_stages, false)) return -1;
         if ((size_t)p.qkv_tc.ksplit * M * e->nqkv > e->part_floats || (size_t)p.o_tc.ksplit * M * h > e->part_floats)
             return set_error("engine: split-K workspace too small");
         if (make_tmap_bf16(&p.x_norm_qkv_tc, e->fuse_norm ? e->resid_bf : e->xnorm, M, h, h, p.qkv_tc.MT / 2)) return -1;
@@ -574,7 +574,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         auto jt = e->lm_plans_tc.find(key);
         if (jt == e->lm_plans_tc.end()) {
             std::pair<TcPlan, CUtensorMap> v;
-            if (gemm_tc_plan(&v.first, rows, c.vocab, h, GEMM_OUT_F32, 1, e->force_stages)) return -1;
+            if (gemm_tc_plan(&v.first, rows, c.vocab, h, GEMM_OUT_F32, 1, e->force_stages, true)) return -1;
             if (make_tmap_bf16(&v.second, src, rows, h, h, v.first.MT / 2)) return -1;
             jt = e->lm_plans_tc.emplace(key, v).first;
         }

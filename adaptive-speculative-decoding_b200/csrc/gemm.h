@@ -71,6 +71,9 @@ int gemm_token_tile(int M);
 int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, int reduce);
 int make_tmap_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint64_t row_stride_elems,
                    uint32_t box_rows);
+// [slices][M][ldo] fp32, `cols` columns of a row; box = box_cols x box_rows, no swizzle: what TMA stores name their places by
+int make_tmap_f32_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols, uint64_t slices, uint64_t ldo, uint64_t slice_stride,
+                      uint32_t box_cols, uint32_t box_rows);
 int make_tmap_bf16_planes(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint32_t planes, uint32_t box_rows);
 // out: GEMM_OUT_F32 -> float [ksplit][M][ldo]; GEMM_OUT_BF16 -> bf16 [M][ldo];
 // GEMM_OUT_SWIGLU -> bf16 [M][ldo] with N/2 columns (n_valid = ff)
@@ -82,9 +85,11 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
 struct TcPlan {
     int M, N, K, mode;
     int MT, m_tiles, w_tiles, kblocks, ksplit, stages, smem_bytes, pairs;
+    bool norm;
 };
 constexpr int kTcMaxTokens = 4096;       // of one call
-int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages);
+// norm: launches may scale tokens by a fused RMSNorm (their factors take shared memory)
+int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm);
 // x tensor map: box rows = MT / 2 (each CTA of the pair loads half of the token tile); w tensor map: box rows = 128.
 // GEMM_OUT_F32: out fp32 [ksplit][slice_stride] slices of [M][ldo]; GEMM_OUT_SWIGLU: out bf16 [M][ldo].
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,

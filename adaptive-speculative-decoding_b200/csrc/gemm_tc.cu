@@ -15,6 +15,11 @@
 //     tile fastest, so neighbouring pairs stream the SAME weight tile at the same time and HBM sees it once
 //     (the others hit L2); TMEM holds two accumulators, so the epilogue of tile i overlaps the MMAs of tile i+1;
 //   * K splits write fp32 slices that the glue kernels (add_norm / reduce_slices) sum in order - deterministic.
+//   * fp32 results leave by TMA stores: 16 tokens x 128 weight rows go through shared memory (four buffers, one barrier each) and
+//     one thread sends the box.  A store per lane and token, as before, took 15 us for a tile of 256 x 240 - longer than
+//     its products up to K = 3000 - and the last tile's is exposed: 2151 x 6144 x 2048 61 -> 49 us, 2151 x 2048 x 2048 31 -> 23,
+//     2151 x 2048 x 6144 56 -> 47, 2048 x 7168 x 5120 141 -> 132.  Outputs that a tensor map cannot name (rows that are no
+//     multiple of 16 bytes) and accumulation keep the direct form.
 // Epilogues: fp32 (+ per-token rstd of the fused RMSNorm, + accumulate) and SwiGLU -> bf16 for gate|up weights
 // interleaved 64 gate / 64 up rows per 128-row tile (same layout as gemm.cu).
 //
@@ -37,12 +42,14 @@ constexpr int kTcThreads = 256;          // warp 0 TMA, warp 1 MMA (leader), war
 constexpr int kTcBlockK = 64;
 constexpr int kTcABytes = 128 * kTcBlockK * 2;
 constexpr int kTcAccCols = 256;          // TMEM column stride between the two accumulators
-constexpr int kTcMaxM = kTcMaxTokens;    // per-token rstd table in shared memory
+constexpr int kTcOutTok = 16;            // tokens per TMA store of an fp32 result
+constexpr int kTcOutBufs = 4;
+constexpr int kTcXchgBytes = kTcOutBufs * kTcOutTok * 128 * 4;   // those buffers, or the SwiGLU exchange [2][32][128] floats
 
 struct TcArgs {
     int M, N, K;
     int MT, m_tiles, w_tiles, kblocks, ksplit, stages, mode;
-    int ldo, n_valid, accumulate;
+    int ldo, n_valid, accumulate, tma_out;
     void* out;
     size_t slice_stride;   // elements between the K-split slices of the fp32 output
     NormFusion norm;       // consumer side only (sumsq_in / parts / ld / hidden / eps)
@@ -91,6 +98,17 @@ __device__ __forceinline__ void umma_commit_cg2(uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar_cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_cluster_addr) : "memory");
 }
+// shared memory -> global box of this thread's bulk group
+__device__ __forceinline__ void tma_store_3d(const void* tmap, const void* src_smem, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap), "r"(smem_u32(src_smem)),
+                 "r"(c0), "r"(c1), "r"(c2)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read() {      // at most N of this thread's stores still read shared memory
+    asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ uint64_t policy_evict_normal() {
     uint64_t p;
     asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
@@ -115,19 +133,20 @@ __device__ __forceinline__ TcUnit tc_unit(const TcArgs& a, int u) {
 }
 
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
-    gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const TcArgs a) {
+    gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
+                   const __grid_constant__ CUtensorMap tmap_o, const TcArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int b_bytes = (a.MT / 2) * 128;
     const int stage_bytes = kTcABytes + b_bytes;
-    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + (size_t)a.stages * stage_bytes);
+    float* stage_t = reinterpret_cast<float*>(smem + (size_t)a.stages * stage_bytes);   // kTcXchgBytes, 1024-byte aligned
+    uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + (size_t)a.stages * stage_bytes + kTcXchgBytes);
     uint64_t* empty_bar = full_bar + a.stages;
     uint64_t* tfull_bar = empty_bar + a.stages;   // [2] accumulator ready (per CTA)
     uint64_t* tempty_bar = tfull_bar + 2;         // [2] accumulator drained (leader's copy is the one waited on)
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 2);
     const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 1), a.err, WAIT_GEMM_PAIR << 8};
-    float* rstd_s = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));   // [M]
-    float* stage_t = rstd_s + ((a.norm.sumsq_in != nullptr ? a.M : 0) + 3) / 4 * 4;   // SwiGLU exchange [2][32][128]
+    float* rstd_s = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(tmem_slot + 4) + 15) & ~uintptr_t(15));   // [m_tiles * MT], if the plan has a norm
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_ctarank();
@@ -221,7 +240,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             asm volatile("bar.sync 1, 128;" ::: "memory");
         }
         const uint32_t tempty_leader = mapa(smem_u32(tempty_bar), 0);
-        int tile = 0;
+        int tile = 0, buf = 0;
         for (int u = pair; u < units; u += npairs, ++tile) {
             const TcUnit t = tc_unit(a, u);
             const int acc = tile & 1, use = tile >> 1;
@@ -269,6 +288,32 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                         }
                     }
                 }
+            } else if (a.tma_out) {
+                const int rows = min(a.MT, a.M - m0);
+                if (tile128 * 128 < a.n_valid) {
+#pragma unroll 1
+                    for (int c0 = 0; c0 < rows; c0 += kTcOutTok) {
+                        float* T = stage_t + buf * (kTcOutTok * 128);
+                        uint32_t r[16];
+                        tmem_ld_32x16(taddr + c0, r);
+                        tmem_ld_wait();
+                        if (scale) {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * rstd_s[m0 + c0 + i]);
+                        }
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) T[i * 128 + row] = __uint_as_float(r[i]);
+                        fence_proxy_async_smem();
+                        // behind this barrier the buffer is complete, and the one that comes next is free: its store was the
+                        // third before the last that thread 0 has sent, of which it left two reading at most
+                        asm volatile("bar.sync 1, 128;" ::: "memory");
+                        if (et == 0) {
+                            tma_store_3d(&tmap_o, T, tile128 * 128, m0 + c0, t.ks);      // rows beyond the result are clipped
+                            tma_store_wait_read<kTcOutBufs - 2>();
+                        }
+                        if (++buf == kTcOutBufs) buf = 0;
+                    }
+                }
             } else {
                 float* out = static_cast<float*>(a.out) + (size_t)t.ks * a.slice_stride;
                 const int n = tile128 * 128 + row;
@@ -294,6 +339,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster(tempty_leader + (uint32_t)acc * 8u);
         }
+        if (et == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
     }
     wait_settle(guard);
     tc_fence_before();
@@ -308,7 +354,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 static PerDeviceOnce g_tc_attr;
 static int g_tc_sms = 0, g_tc_smem_optin = 0;
 
-int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages) {
+int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm) {
     if (!g_tc_sms) {
         int dev = 0;
         ASD_CUDA(cudaGetDevice(&dev));
@@ -317,7 +363,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     }
     if (M <= 0 || N <= 0 || K <= 0 || (K & 7)) return set_error("gemm_tc: need M, N, K > 0 and K %% 8 == 0");
     if (mode != GEMM_OUT_F32 && mode != GEMM_OUT_SWIGLU) return set_error("gemm_tc: fp32 and SwiGLU epilogues only");
-    if (M > kTcMaxM) return set_error("gemm_tc: at most %d tokens per call", kTcMaxM);
+    if (M > kTcMaxTokens) return set_error("gemm_tc: at most %d tokens per call", kTcMaxTokens);
     pl->M = M;
     pl->N = N;
     pl->K = K;
@@ -370,7 +416,8 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     if (mode == GEMM_OUT_SWIGLU) best = 1;
     pl->ksplit = best;
     const int stage_bytes = kTcABytes + (mt / 2) * 128;
-    const int fixed = 1024 + 256 + 4 * kTcMaxM + (mode == GEMM_OUT_SWIGLU ? 2 * 32 * 128 * 4 : 0) + 64;
+    const int fixed = 1024 + 256 + kTcXchgBytes + (norm ? 4 * pl->m_tiles * mt : 0) + 64;
+    pl->norm = norm;
     int stages = (g_tc_smem_optin - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
     if (force_stages > 0 && force_stages < stages) stages = force_stages;
@@ -388,6 +435,7 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
         ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
         prefer_max_smem(gemm_tc_kernel);
     }
+    if (norm && !pl.norm) return set_error("gemm_tc: the plan has no place for a norm's factors");
     if (accumulate && (pl.mode != GEMM_OUT_F32 || pl.ksplit != 1))
         return set_error("gemm_tc: accumulate needs the fp32 epilogue without a K split");
     TcArgs a;
@@ -407,10 +455,16 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.out = out;
     a.slice_stride = slice_stride;
     a.norm = norm ? *norm : NormFusion{};
+    CUtensorMap to = tmap_x;                     // (never read unless tma_out)
+    a.tma_out = pl.mode == GEMM_OUT_F32 && !accumulate && ldo % 4 == 0 && (pl.ksplit == 1 || slice_stride % 4 == 0) &&
+                (reinterpret_cast<uintptr_t>(out) & 15) == 0;
+    if (a.tma_out && make_tmap_f32_out(&to, out, pl.M, n_valid, pl.ksplit, ldo, pl.ksplit == 1 ? (size_t)pl.M * ldo : slice_stride,
+                                       128, kTcOutTok))
+        return -1;
     a.err = wait_word();
     // plainly (ptx.cuh); its successor may start early.  Eight prompts of 500 to 1000 tokens through two 32B layers, forwards of
     // 2048 tokens: 13.4 to 13.7 ms launched programmatically, 13.5 to 14.4 so (power cap; boxes differ by as much)
-    gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, a);
+    gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, to, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_PAIR);
     return 0;
@@ -432,7 +486,7 @@ extern "C" int asd_linear_bf16_tc(const void* x, const void* w, void* out, int M
     using namespace asd;
     if (out_mode != 0 && out_mode != 2) return set_error("asd_linear_bf16_tc: out_mode 0 (fp32 slices) or 2 (SwiGLU)");
     TcPlan pl;
-    if (gemm_tc_plan(&pl, M, N, K, out_mode == 2 ? GEMM_OUT_SWIGLU : GEMM_OUT_F32, ksplit, stages)) return -1;
+    if (gemm_tc_plan(&pl, M, N, K, out_mode == 2 ? GEMM_OUT_SWIGLU : GEMM_OUT_F32, ksplit, stages, false)) return -1;
     CUtensorMap tw, tx;
     if (make_tmap_bf16(&tw, w, N, K, K, 128)) return -1;
     if (make_tmap_bf16(&tx, x, M, K, K, pl.MT / 2)) return -1;
