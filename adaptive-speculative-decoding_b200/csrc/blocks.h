@@ -174,6 +174,8 @@ struct MoeRouterInput {
 };
 int launch_moe_route(const float* logits, const MoeRouterInput* in, int M, int E, int top, int* expert_of, float* gate,
                      int* counters, int* group_off, int* sorted_tok, int* slot_of, cudaStream_t stream);
+// dst[i][D] = src[index[i]][D], i < n: bf16 rows of a multiple of eight elements from and to 16-byte aligned places
+int launch_gather_rows_bf16(const void* src, const int* index, void* dst, int n, int D, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------- norm_ops.cu
 // Row kernels of sandwich-normed layers (a norm before and after every sublayer).  "Offset" RMS norms store their

@@ -680,17 +680,19 @@ int make_tmap_bf16_planes(CUtensorMap* map, const void* ptr, uint64_t rows, uint
     return 0;
 }
 
-int make_tmap_f32_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols, uint64_t slices, uint64_t ldo, uint64_t slice_stride,
-                      uint32_t box_cols, uint32_t box_rows) {
+int make_tmap_out(CUtensorMap* map, void* ptr, bool bf16, uint64_t rows, uint64_t cols, uint64_t slices, uint64_t ldo,
+                  uint64_t slice_stride, uint32_t box_cols, uint32_t box_rows) {
     if (load_encode()) return -1;
-    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || ldo * 4 % 16 || slice_stride * 4 % 16)
+    const uint64_t size = bf16 ? 2 : 4;
+    if ((reinterpret_cast<uintptr_t>(ptr) & 15) || ldo * size % 16 || slice_stride * size % 16)
         return set_error("tensor map: base and strides must be 16-byte aligned");
     cuuint64_t gdim[3] = {cols, rows, slices};
-    cuuint64_t gstride[2] = {ldo * 4, slice_stride * 4};
+    cuuint64_t gstride[2] = {ldo * size, slice_stride * size};
     cuuint32_t box[3] = {box_cols, box_rows, 1};
     cuuint32_t estr[3] = {1, 1, 1};
-    CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ptr, gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    CUresult r = g_encode(map, bf16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, ptr, gdim, gstride, box,
+                          estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
+                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return set_error("cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
     return 0;
 }

@@ -6,7 +6,7 @@
 
 namespace asd {
 
-enum GemmOut { GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2, GEMM_OUT_QKV = 3 };
+enum GemmOut { GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2, GEMM_OUT_QKV = 3, GEMM_OUT_RELU2 = 4 };
 
 // Fused RMSNorm.  Producer side (fp32 accumulate epilogue of the O / down projection): besides the fp32
 // residual v it writes x = bf16(v * ln_w[n]) (the next norm's weight applied per column, NOT yet divided by
@@ -71,9 +71,9 @@ int gemm_token_tile(int M);
 int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, int reduce);
 int make_tmap_bf16(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint64_t row_stride_elems,
                    uint32_t box_rows);
-// [slices][M][ldo] fp32, `cols` columns of a row; box = box_cols x box_rows, no swizzle: what TMA stores name their places by
-int make_tmap_f32_out(CUtensorMap* map, void* ptr, uint64_t rows, uint64_t cols, uint64_t slices, uint64_t ldo, uint64_t slice_stride,
-                      uint32_t box_cols, uint32_t box_rows);
+// [slices][M][ldo] fp32 or bf16, `cols` columns of a row; box = box_cols x box_rows, no swizzle: what TMA stores name their places by
+int make_tmap_out(CUtensorMap* map, void* ptr, bool bf16, uint64_t rows, uint64_t cols, uint64_t slices, uint64_t ldo,
+                  uint64_t slice_stride, uint32_t box_cols, uint32_t box_rows);
 int make_tmap_bf16_planes(CUtensorMap* map, const void* ptr, uint64_t rows, uint64_t cols, uint32_t planes, uint32_t box_rows);
 // out: GEMM_OUT_F32 -> float [ksplit][M][ldo]; GEMM_OUT_BF16 -> bf16 [M][ldo];
 // GEMM_OUT_SWIGLU -> bf16 [M][ldo] with N/2 columns (n_valid = ff)
@@ -89,11 +89,18 @@ struct TcPlan {
 };
 constexpr int kTcMaxTokens = 4096;       // of one call
 // norm: launches may scale tokens by a fused RMSNorm (their factors take shared memory)
-int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm);
+int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm, int force_mt = 0);
 // x tensor map: box rows = MT / 2 (each CTA of the pair loads half of the token tile); w tensor map: box rows = 128.
 // GEMM_OUT_F32: out fp32 [ksplit][slice_stride] slices of [M][ldo]; GEMM_OUT_SWIGLU: out bf16 [M][ldo].
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
                    size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm);
+
+// The grouped form of the same kernel for a mixture of experts' linear (SimtLinear with group_off, no gather): rows of A and C in
+// group order, `rows` in all; fp32 results, or relu(y)^2 in bf16.
+// min_rows: rows a group, on average, from which it is wanted (0: where it measured better).
+struct SimtLinear;
+bool gemm_tc_grouped_takes(const SimtLinear& L, int groups, long long rows, int min_rows);
+int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream_t stream);
 
 // ---- one token (gemv.cu): CUDA cores, weight rows straight into registers
 bool gemv_takes(int M, int max_k, size_t max_bytes);

@@ -20,7 +20,11 @@
 //     its products up to K = 3000 - and the last tile's is exposed: 2151 x 6144 x 2048 61 -> 49 us, 2151 x 2048 x 2048 31 -> 23,
 //     2151 x 2048 x 6144 56 -> 47, 2048 x 7168 x 5120 141 -> 132.  Outputs that a tensor map cannot name (rows that are no
 //     multiple of 16 bytes) and accumulation keep the direct form.
-// Epilogues: fp32 (+ per-token rstd of the fused RMSNorm, + accumulate) and SwiGLU -> bf16 for gate|up weights
+//   * grouped form (mixture of experts): rows [off[z], off[z + 1]) of X and Y multiply matrix z of W; the group sizes stand in
+//     device memory, every CTA derives the same list of (matrix, weight tile, token tile) from them.  Before, these products ran
+//     on single CTAs of 128 x 128 whose operands went through registers (linear_tc.cu): 8192 rows in 8 groups, 2048 x 2048 each
+//     184 and 183 us, here 66 and 64.
+// Epilogues: fp32 (+ per-token rstd of the fused RMSNorm, + accumulate), relu(y)^2 -> bf16 (grouped form) and SwiGLU -> bf16 for gate|up weights
 // interleaved 64 gate / 64 up rows per 128-row tile (same layout as gemm.cu).
 //
 // Stands behind Stage.generate's model forward, which the reference delegates to vLLM
@@ -31,8 +35,10 @@
 #include <stdint.h>
 
 #include <algorithm>
+#include <cmath>
 
 #include "asd_internal.h"
+#include "blocks.h"
 #include "gemm.h"
 #include "ptx.cuh"
 
@@ -44,6 +50,7 @@ constexpr int kTcABytes = 128 * kTcBlockK * 2;
 constexpr int kTcAccCols = 256;          // TMEM column stride between the two accumulators
 constexpr int kTcOutTok = 16;            // tokens per TMA store of an fp32 result
 constexpr int kTcOutBufs = 4;
+constexpr int kTcGroups = 512;           // of the grouped form: their table takes the place of a norm's factors
 constexpr int kTcXchgBytes = kTcOutBufs * kTcOutTok * 128 * 4;   // those buffers, or the SwiGLU exchange [2][32][128] floats
 
 struct TcArgs {
@@ -54,6 +61,8 @@ struct TcArgs {
     size_t slice_stride;   // elements between the K-split slices of the fp32 output
     NormFusion norm;       // consumer side only (sumsq_in / parts / ld / hidden / eps)
     int* err;              // where a wait that ran out is reported
+    const int* group_off;  // grouped form: [groups + 1]
+    int groups;
 };
 
 // ---- cta_group::2 flavours of the PTX wrappers
@@ -118,20 +127,37 @@ __device__ __forceinline__ uint64_t policy_evict_normal() {
 __device__ __forceinline__ float tc_silu_mul(float g, float u) { return __fdividef(g, 1.0f + __expf(-g)) * u; }
 
 struct TcUnit {
-    int w_tile, ks, t_tile, kb0, nkb;
+    int w_tile, ks, kb0, nkb;
+    int w_row, m0, m_end;          // first weight row of the tile, its first token row and the end of its rows
 };
 __device__ __forceinline__ TcUnit tc_unit(const TcArgs& a, int u) {
     TcUnit r;
-    r.t_tile = u % a.m_tiles;
+    r.m0 = u % a.m_tiles * a.MT;
+    r.m_end = a.M;
     const int v = u / a.m_tiles;
     r.ks = v % a.ksplit;
     r.w_tile = v / a.ksplit;
+    r.w_row = r.w_tile * 256;
     const int base = a.kblocks / a.ksplit, rem = a.kblocks % a.ksplit;
     r.kb0 = r.ks * base + (r.ks < rem ? r.ks : rem);
     r.nkb = base + (r.ks < rem ? 1 : 0);
     return r;
 }
 
+// the same from the table of the groups in shared memory: first row and first unit of each; z only grows within a role's walk
+__device__ __forceinline__ TcUnit tc_group_unit(const TcArgs& a, const int2* table, int u, int& z) {
+    while (u >= table[z + 1].y) ++z;
+    const int row = table[z].x, end = table[z + 1].x, tiles = (end - row + a.MT - 1) / a.MT, v = u - table[z].y;
+    TcUnit r;
+    r.w_tile = v / tiles;
+    r.ks = 0, r.kb0 = 0, r.nkb = a.kblocks;
+    r.w_row = z * a.N + r.w_tile * 256;
+    r.m0 = row + (v - r.w_tile * tiles) * a.MT;
+    r.m_end = end;
+    return r;
+}
+
+template <bool GROUPED>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const __grid_constant__ CUtensorMap tmap_o, const TcArgs a) {
@@ -152,7 +178,21 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     const uint32_t rank = cluster_ctarank();
     const bool leader = rank == 0;
     const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-    const int units = a.w_tiles * a.ksplit * a.m_tiles;
+    int units = a.w_tiles * a.ksplit * a.m_tiles;
+    int2* table = reinterpret_cast<int2*>(rstd_s);       // grouped form (no norm there): [groups + 1]
+    if (GROUPED) {
+        for (int z = threadIdx.x; z <= a.groups; z += kTcThreads) table[z].x = a.group_off[z];
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int n = 0;
+            for (int z = 0; z <= a.groups; ++z) {
+                table[z].y = n;
+                if (z < a.groups) n += (table[z + 1].x - table[z].x + a.MT - 1) / a.MT * a.w_tiles;
+            }
+        }
+    }
+    int group = 0;
+    auto unit_of = [&](int u) { return GROUPED ? tc_group_unit(a, table, u, group) : tc_unit(a, u); };
 
     if (warp == 0 && lane == 0) {
         tma_prefetch_desc(&tmap_w);
@@ -175,6 +215,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     tc_fence_before();
     cluster_sync();      // both CTAs' barriers are initialised before anything arrives remotely
     tc_fence_after();
+    if (GROUPED) units = table[a.groups].y;
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp == 0) {
@@ -186,16 +227,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             const uint32_t full_leader = mapa(smem_u32(full_bar), 0);
             int it = 0;
             for (int u = pair; u < units; u += npairs) {
-                const TcUnit t = tc_unit(a, u);
+                const TcUnit t = unit_of(u);
                 for (int kb = 0; kb < t.nkb; ++kb, ++it) {
                     const int s = it % a.stages, round = it / a.stages;
                     if (round > 0 && !mbar_wait(&empty_bar[s], (round - 1) & 1, guard)) return;
                     if (leader) mbar_expect_tx(&full_bar[s], 2 * stage_bytes);
                     uint8_t* st = smem + (size_t)s * stage_bytes;
                     const uint32_t bar = full_leader + (uint32_t)s * 8u;
-                    tma_load_2d_cg2(st, &tmap_w, (t.kb0 + kb) * kTcBlockK, t.w_tile * 256 + (int)rank * 128, bar, pol_w);
+                    tma_load_2d_cg2(st, &tmap_w, (t.kb0 + kb) * kTcBlockK, t.w_row + (int)rank * 128, bar, pol_w);
                     tma_load_2d_cg2(st + kTcABytes, &tmap_x, (t.kb0 + kb) * kTcBlockK,
-                                    t.t_tile * a.MT + (int)rank * (a.MT / 2), bar, pol_x);
+                                    t.m0 + (int)rank * (a.MT / 2), bar, pol_x);
                 }
             }
         };
@@ -207,7 +248,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             const uint32_t idesc = umma_idesc_bf16(256, a.MT);
             int it = 0, tile = 0;
             for (int u = pair; u < units; u += npairs, ++tile) {
-                const TcUnit t = tc_unit(a, u);
+                const TcUnit t = unit_of(u);
                 const int acc = tile & 1, use = tile >> 1;
                 if (use > 0 && !mbar_wait(&tempty_bar[acc], (use - 1) & 1, guard)) return;
                 tc_fence_after();
@@ -242,13 +283,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
         const uint32_t tempty_leader = mapa(smem_u32(tempty_bar), 0);
         int tile = 0, buf = 0;
         for (int u = pair; u < units; u += npairs, ++tile) {
-            const TcUnit t = tc_unit(a, u);
+            const TcUnit t = unit_of(u);
             const int acc = tile & 1, use = tile >> 1;
             mbar_wait_timed(&tfull_bar[acc], use & 1, guard, 1);
             tc_fence_after();
             if (tile == 0) grid_dep_launch();
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTcAccCols);
-            const int m0 = t.t_tile * a.MT;
+            const int m0 = t.m0;
             const int tile128 = t.w_tile * 2 + (int)rank;          // 128-row weight tile this CTA holds
             if (a.mode == GEMM_OUT_SWIGLU) {
                 __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
@@ -289,8 +330,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                     }
                 }
             } else if (a.tma_out) {
-                const int rows = min(a.MT, a.M - m0);
+                const int rows = min(a.MT, t.m_end - m0);
                 if (tile128 * 128 < a.n_valid) {
+                    const bool half_out = GROUPED && a.mode == GEMM_OUT_RELU2;
 #pragma unroll 1
                     for (int c0 = 0; c0 < rows; c0 += kTcOutTok) {
                         float* T = stage_t + buf * (kTcOutTok * 128);
@@ -301,8 +343,35 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 #pragma unroll
                             for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * rstd_s[m0 + c0 + i]);
                         }
+                        if (half_out) {
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) T[i * 128 + row] = __uint_as_float(r[i]);
+                            for (int i = 0; i < 16; ++i) r[i] = __float_as_uint(fmaxf(__uint_as_float(r[i]), 0.f));
+                        }
+                        if (GROUPED && c0 + kTcOutTok > rows) {       // the next rows are another group's: no box over them
+                            const int n = tile128 * 128 + row;
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if (c0 + i < rows && n < a.n_valid) {
+                                    const float v = __uint_as_float(r[i]);
+                                    const size_t at = (size_t)(m0 + c0 + i) * a.ldo + n;
+                                    if (half_out)
+                                        static_cast<__nv_bfloat16*>(a.out)[at] = __float2bfloat16(v * v);
+                                    else
+                                        static_cast<float*>(a.out)[at] = v;
+                                }
+                            break;
+                        }
+                        if (half_out) {
+                            __nv_bfloat16* H = reinterpret_cast<__nv_bfloat16*>(T);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                const float v = __uint_as_float(r[i]);
+                                H[i * 128 + row] = __float2bfloat16(v * v);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) T[i * 128 + row] = __uint_as_float(r[i]);
+                        }
                         fence_proxy_async_smem();
                         // behind this barrier the buffer is complete, and the one that comes next is free: its store was the
                         // third before the last that thread 0 has sent, of which it left two reading at most
@@ -354,7 +423,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 static PerDeviceOnce g_tc_attr;
 static int g_tc_sms = 0, g_tc_smem_optin = 0;
 
-int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm) {
+int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm, int force_mt) {
     if (!g_tc_sms) {
         int dev = 0;
         ASD_CUDA(cudaGetDevice(&dev));
@@ -386,7 +455,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     for (int nt = 1; nt <= 16; ++nt) {
         int mt = ((M + nt - 1) / nt + 15) / 16 * 16;
         if (mt < 32) mt = 32;
-        if (mt > 256) continue;
+        if (mt > 256 || (force_mt > 0 && mt != force_mt)) continue;
         if (env_mt >= 32 && nt != (M + env_mt - 1) / env_mt) continue;
         const int m_tiles = (M + mt - 1) / mt;
         const double clk = std::max(2.0 * mt, (16384.0 + 64.0 * mt) / 58.0);
@@ -416,7 +485,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     if (mode == GEMM_OUT_SWIGLU) best = 1;
     pl->ksplit = best;
     const int stage_bytes = kTcABytes + (mt / 2) * 128;
-    const int fixed = 1024 + 256 + kTcXchgBytes + (norm ? 4 * pl->m_tiles * mt : 0) + 64;
+    const int fixed = 1024 + 256 + kTcXchgBytes + (norm ? std::max(4 * pl->m_tiles * mt, 8 * (kTcGroups + 1)) : 0) + 64;
     pl->norm = norm;
     int stages = (g_tc_smem_optin - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
@@ -432,8 +501,8 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
                    size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm) {
     if (g_tc_attr.need()) {
-        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
-        prefer_max_smem(gemm_tc_kernel);
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
+        prefer_max_smem(gemm_tc_kernel<false>);
     }
     if (norm && !pl.norm) return set_error("gemm_tc: the plan has no place for a norm's factors");
     if (accumulate && (pl.mode != GEMM_OUT_F32 || pl.ksplit != 1))
@@ -455,18 +524,61 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.out = out;
     a.slice_stride = slice_stride;
     a.norm = norm ? *norm : NormFusion{};
+    a.group_off = nullptr, a.groups = 0;
     CUtensorMap to = tmap_x;                     // (never read unless tma_out)
     a.tma_out = pl.mode == GEMM_OUT_F32 && !accumulate && ldo % 4 == 0 && (pl.ksplit == 1 || slice_stride % 4 == 0) &&
                 (reinterpret_cast<uintptr_t>(out) & 15) == 0;
-    if (a.tma_out && make_tmap_f32_out(&to, out, pl.M, n_valid, pl.ksplit, ldo, pl.ksplit == 1 ? (size_t)pl.M * ldo : slice_stride,
-                                       128, kTcOutTok))
+    if (a.tma_out && make_tmap_out(&to, out, false, pl.M, n_valid, pl.ksplit, ldo, pl.ksplit == 1 ? (size_t)pl.M * ldo : slice_stride, 128,
+                                   kTcOutTok))
         return -1;
     a.err = wait_word();
     // plainly (ptx.cuh); its successor may start early.  Eight prompts of 500 to 1000 tokens through two 32B layers, forwards of
     // 2048 tokens: 13.4 to 13.7 ms launched programmatically, 13.5 to 14.4 so (power cap; boxes differ by as much)
-    gemm_tc_kernel<<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, to, a);
+    gemm_tc_kernel<false><<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, to, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_PAIR);
+    return 0;
+}
+
+// From how many rows a group, on average, the grouped form is the better one (us of both products of 8 experts and the copy into
+// group order, before -> here).  Matrices of 2048 x 2048 on: 1 (4 x 2048: 57 -> 46, 16: 62 -> 51, 64: 108 -> 57, 512: 210 -> 111;
+// 4096: 1: 114 -> 73, 16: 136 -> 128, 64: 208 -> 135); of 1024 x 1024: 32 (16: 32 -> 34, 32: 36 -> 36, 64: 46 -> 38, 512: 76 -> 48).
+bool gemm_tc_grouped_takes(const SimtLinear& L, int groups, long long rows, int min_rows) {
+    if (min_rows <= 0) min_rows = (long long)L.N * L.K >= (1 << 22) ? 1 : 32;
+    const uintptr_t at = reinterpret_cast<uintptr_t>(L.a) | reinterpret_cast<uintptr_t>(L.w) | reinterpret_cast<uintptr_t>(L.c);
+    if (L.a_f32 || L.w_f32 || (at & 15) || L.K % 8 || L.lda != L.K || L.ldw != L.K || L.w_zs != (long long)L.N * L.K) return false;
+    if (L.ldc % 8 || L.epilogue > 1 || (L.epilogue == 1) != (L.c_f32 == 0) || L.c_terms > 0) return false;
+    if (groups > kTcGroups || (long long)groups * L.N >= (1ll << 31) || rows >= (1ll << 31)) return false;
+    return rows >= (long long)min_rows * groups;
+}
+
+int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream_t stream) {
+    TcPlan pl;
+    // a tile that holds a group of the average size and three standard deviations of an even choice: a second tile would read the
+    // weights again; groups beyond 256 rows take tiles of 256
+    const double avg = (double)rows / groups;
+    const int mt = std::min(256, std::max(32, ((int)std::ceil(avg + 3.0 * std::sqrt(avg)) + 15) / 16 * 16));
+    if (gemm_tc_plan(&pl, mt, L.N, L.K, GEMM_OUT_F32, 1, 0, true, mt)) return -1;       // (sizes of one tile; the kernel makes the list)
+    TcArgs a = {};
+    a.M = rows, a.N = L.N, a.K = L.K, a.MT = mt, a.w_tiles = pl.w_tiles, a.kblocks = pl.kblocks, a.ksplit = 1;
+    a.m_tiles = 2;                 // (several token tiles read a weight tile: it may stay in L2)
+    a.stages = pl.stages;
+    a.mode = L.epilogue == 1 ? GEMM_OUT_RELU2 : GEMM_OUT_F32;
+    a.ldo = (int)L.ldc, a.n_valid = L.N, a.out = L.c, a.tma_out = 1;
+    a.err = wait_word();
+    a.group_off = L.group_off, a.groups = groups;
+    CUtensorMap tw, tx, to;
+    if (make_tmap_bf16(&tw, L.w, (uint64_t)groups * L.N, L.K, L.K, 128)) return -1;
+    if (make_tmap_bf16(&tx, L.a, rows, L.K, L.K, mt / 2)) return -1;
+    if (make_tmap_out(&to, L.c, L.epilogue == 1, rows, L.N, 1, L.ldc, (size_t)rows * L.ldc, 128, kTcOutTok)) return -1;
+    static PerDeviceOnce once;
+    if (once.need()) {
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
+        prefer_max_smem(gemm_tc_kernel<true>);
+    }
+    gemm_tc_kernel<true><<<g_tc_sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
+    ASD_CUDA(cudaGetLastError());
+    count_kernel(KERNEL_GEMM_GROUPED);
     return 0;
 }
 
@@ -474,7 +586,7 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_gemm_tc() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_tc_kernel));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_tc_kernel<false>));
     return 0;
 }
 

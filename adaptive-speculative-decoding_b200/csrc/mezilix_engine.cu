@@ -49,6 +49,7 @@ struct MzEngine : asd_mezilix_engine {
     float *stack = nullptr, *xavg = nullptr, *hn = nullptr, *qd = nullptr, *qlat = nullptr, *olat = nullptr, *mix = nullptr,
           *rlog = nullptr, *gate = nullptr, *eout = nullptr;
     void *h = nullptr, *hs = nullptr, *vout = nullptr, *act = nullptr, *xsel = nullptr;
+    int experts_rows = 0;      // rows an expert, on average, from which its products run on CTA pairs (0: the measured rule)
     int *expert_of = nullptr, *counters = nullptr, *group_off = nullptr, *sorted_tok = nullptr, *slot_of = nullptr;
     std::vector<void*> owned;
     DenseRunner dn;              // dense projections: tcgen05 GEMMs or the CUDA-core kernel, by shape and type
@@ -170,14 +171,25 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
             U.c = e->act, U.c_f32 = f32, U.ldc = c.ff;
             U.M = M, U.N = c.ff, U.K = D, U.Z = c.experts;
             U.group_off = e->group_off, U.gather = e->sorted_tok, U.epilogue = 1;
-            if (linear(e, U, s)) return -1;
             SimtLinear W;
             W.a = e->act, W.a_f32 = f32, W.lda = c.ff;
             W.w = ly.w_down, W.w_f32 = f32, W.ldw = c.ff, W.w_zs = (long long)D * c.ff;
             W.c = e->eout, W.c_f32 = 1, W.ldc = D;
             W.M = M, W.N = D, W.K = c.ff, W.Z = c.experts;
             W.group_off = e->group_off;
-            if (linear(e, W, s)) return -1;
+            // many rows an expert: both products on CTA pairs, from rows copied into group order (they wait where the second
+            // product's results go)
+            const long long rows = (long long)M * c.top;
+            SimtLinear G = U;
+            G.a = e->eout, G.gather = nullptr;
+            if (!f32 && e->dn.tc_linear && D % 8 == 0 && gemm_tc_grouped_takes(G, c.experts, rows, e->experts_rows) &&
+                gemm_tc_grouped_takes(W, c.experts, rows, e->experts_rows)) {
+                if (launch_gather_rows_bf16(e->h, e->sorted_tok, e->eout, (int)rows, D, s) ||
+                    launch_gemm_tc_grouped(G, c.experts, (int)rows, s) || launch_gemm_tc_grouped(W, c.experts, (int)rows, s))
+                    return -1;
+            } else if (linear(e, U, s) || linear(e, W, s)) {
+                return -1;
+            }
         }
         MZ_PROF(MZ_GLUE);
         LayerClose C;
@@ -360,6 +372,10 @@ int asd_mezilix_set_option(asd_mezilix_engine_t* h, const char* name, int value)
     if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
     if (!strcmp(name, "tc_linear")) {
         e->dn.tc_linear = value;
+        return 0;
+    }
+    if (!strcmp(name, "experts_rows")) {
+        e->experts_rows = value;
         return 0;
     }
     if (!strcmp(name, "tc_min_rows")) {

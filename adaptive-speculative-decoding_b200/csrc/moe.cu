@@ -274,6 +274,17 @@ __global__ void moe_scatter_kernel(const int* expert_of, int n, int top, int E, 
     if (slot_gate) slot_gate[slot] = gate[i];
 }
 
+// one warp per row
+__global__ void gather_rows_bf16_kernel(const uint4* src, const int* index, uint4* dst, int n, int per) {
+    pdl_enter();
+    const int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (r >= n) return;
+    const uint4* from = src + (long long)index[r] * per;
+    uint4* to = dst + (long long)r * per;
+#pragma unroll 8
+    for (int i = lane; i < per; i += 32) to[i] = from[i];
+}
+
 template <int NJ, int NTOK>
 void launch_logits_as(const MoeRouterInput& in, int M, int E, int rows, cudaStream_t stream) {
     const uintptr_t at = reinterpret_cast<uintptr_t>(in.x) | reinterpret_cast<uintptr_t>(in.w);
@@ -339,6 +350,16 @@ int launch_moe_route(const float* logits, const MoeRouterInput* in, int M, int E
                         sorted_tok, slot_of,
                                                             gate, c.slot_gate));
     count_launch(3);
+    ASD_CUDA(cudaGetLastError());
+    return 0;
+}
+
+int launch_gather_rows_bf16(const void* src, const int* index, void* dst, int n, int D, cudaStream_t stream) {
+    if (n <= 0) return 0;
+    if (D % 8 || ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15)) return set_error("gather_rows: alignment");
+    ASD_CUDA(launch_pdl(gather_rows_bf16_kernel, (n + 7) / 8, 256, 0, stream, static_cast<const uint4*>(src), index,
+                        static_cast<uint4*>(dst), n, D / 8));
+    count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
 }

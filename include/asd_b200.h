@@ -37,7 +37,7 @@ ASD_API const char* asd_last_error(void);
 /* number of kernels this library has launched since load / since the last reset (bench "gpu_launches") */
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
-/* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemv",
+/* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemm_grouped", "gemv",
  * "attention_tc", "latent_tc", "window_tc", "sampler_draw"; -1 for another name */
 ASD_API long long asd_kernel_launches(const char* name);
 /* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:
