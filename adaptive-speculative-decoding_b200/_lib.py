@@ -159,6 +159,7 @@ def lib() -> ctypes.CDLL:
         "asd_linear_bf16_tc": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp]),
         "asd_linear_plan": (i32, [i32, i32, i32, i32, vp, vp, vp]),
         "asd_engine_create": (vp, [vp]),
+        "asd_engine_create_for_prompts": (vp, [vp, i32]),
         "asd_engine_destroy": (None, [vp]),
         "asd_engine_set_layer": (i32, [vp, i32, vp, vp, vp, vp, vp, vp, vp]),
         "asd_engine_set_globals": (i32, [vp, vp, vp, vp, vp]),

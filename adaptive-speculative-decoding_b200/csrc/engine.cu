@@ -62,6 +62,7 @@ struct Engine {
     float *sumsq = nullptr, *sumsq_sel = nullptr;
     __nv_bfloat16 *xnorm = nullptr, *q = nullptr, *attn = nullptr, *act = nullptr, *xsel = nullptr;
     size_t part_floats = 0, o_part_floats = 0;
+    int scratch_tokens = 0;          // activations fit: max_tokens, or a longer prompt of one sequence
     std::unordered_map<int, Plans> plans;
     std::unordered_map<int, std::pair<GemmPlan, CUtensorMap>> lm_plans;  // keyed by rows (xnorm) / -rows (xsel)
     std::unordered_map<int, std::pair<TcPlan, CUtensorMap>> lm_plans_tc;
@@ -186,7 +187,8 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     const asd_model_config& c = e->c;
     if (M <= 0) return 0;
     TuningScope tuning_scope(&e->tune);
-    if (M > c.max_tokens) return set_error("engine: M = %d exceeds max_tokens = %d", M, c.max_tokens);
+    if (M > c.max_tokens && !(prompt && nseq == 1 && M <= e->scratch_tokens))
+        return set_error("engine: M = %d exceeds max_tokens = %d", M, c.max_tokens);
     if (!e->embed || !e->kv_pool || !e->inv_freq) return set_error("engine: weights / KV pool not set");
     for (auto& L : e->layers)
         if (!L.wqkv) return set_error("engine: a layer has no weights");
@@ -194,7 +196,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     if (fn && !(e->reduce && e->fuse_rope)) return set_error("engine: fuse_norm needs reduce = 1 and fuse_rope = 1");
     Plans* P = nullptr;
     if (ensure_plans(e, M, &P)) return -1;
-    const int h = c.hidden, nh = c.n_heads, nkv = c.n_kv_heads, hd = c.head_dim, Mx = c.max_tokens;
+    const int h = c.hidden, nh = c.n_heads, nkv = c.n_kv_heads, hd = c.head_dim, Mx = e->scratch_tokens;
     const bool tp = c.tp_size > 1;
     if (tp && !e->allreduce && !e->p2p) return set_error("engine: tp_size > 1 but no all-reduce installed");
 
@@ -215,6 +217,10 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     if (nsplit < 1) nsplit = 1;
     int split_keys = ((max_kv_len + nsplit - 1) / nsplit + 127) / 128 * 128;   // whole key tiles of both kernels
     if (split_keys < 128) split_keys = 128;
+    // (a prompt beyond max_tokens finds less workspace a token)
+    while (split_keys < max_kv_len &&
+           (size_t)M * nh * ((max_kv_len + split_keys - 1) / split_keys) * hd > e->o_part_floats)
+        split_keys += 128;
     const int nsplit_max = (max_kv_len + split_keys - 1) / split_keys;
     if ((size_t)M * nh * nsplit_max * hd > e->o_part_floats) return set_error("engine: attention workspace too small");
 
@@ -600,7 +606,9 @@ using namespace asd;
 
 extern "C" {
 
-asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
+asd_engine_t* asd_engine_create(const asd_model_config* cfg) { return asd_engine_create_for_prompts(cfg, 0); }
+
+asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int prompt_tokens) {
     if (!cfg) {
         set_error("asd_engine_create: NULL config");
         return nullptr;
@@ -610,6 +618,11 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
         c.n_heads % c.n_kv_heads || (c.head_dim != 64 && c.head_dim != 128) || c.ffn <= 0 || c.ffn % 8 ||
         c.vocab <= 0 || c.max_tokens <= 0 || c.page_size <= 0 || c.tp_size < 1) {
         set_error("asd_engine_create: unsupported model shape");
+        return nullptr;
+    }
+    if (prompt_tokens > kTcMaxTokens || (prompt_tokens > 0 && c.tp_size > 1)) {
+        set_error("asd_engine_create: prompts of %d tokens a forward; at most %d, and none on tensor-parallel ranks", prompt_tokens,
+                  kTcMaxTokens);
         return nullptr;
     }
     {   // lazy module loading + spinning tensor-parallel kernels in one process = deadlock: load everything now
@@ -625,9 +638,13 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
     e->qdim = c.n_heads * c.head_dim;
     e->ffp = (c.ffn + 63) / 64 * 64;
     e->layers.resize(c.n_layers);
-    const size_t Mx = c.max_tokens;
-    e->part_floats = 16 * Mx * (size_t)std::max(e->nqkv, c.hidden);
-    e->o_part_floats = Mx * c.n_heads * (size_t)e->max_attn_splits * c.head_dim;
+    e->scratch_tokens = std::max(c.max_tokens, prompt_tokens);
+    const size_t Mx = e->scratch_tokens;
+    // K-split slices: up to 16 for a step, 8 for the tokens of a prompt; the same of the attention's key shares, of which a prompt
+    // needs one
+    e->part_floats = std::max(16 * (size_t)c.max_tokens, 8 * Mx) * (size_t)std::max(e->nqkv, c.hidden);
+    const size_t shares = std::max(c.max_tokens * (size_t)e->max_attn_splits, Mx);
+    e->o_part_floats = shares * c.n_heads * c.head_dim;
     bool ok = true;
     auto alloc = [&](void** p, size_t bytes) {
         if (ok && cudaMalloc(p, bytes) != cudaSuccess) {
@@ -638,7 +655,7 @@ asd_engine_t* asd_engine_create(const asd_model_config* cfg) {
     alloc((void**)&e->resid, Mx * c.hidden * 4);
     alloc((void**)&e->part, e->part_floats * 4);
     alloc((void**)&e->o_part, e->o_part_floats * 4);
-    alloc((void**)&e->ml_part, Mx * c.n_heads * (size_t)e->max_attn_splits * 2 * 4);
+    alloc((void**)&e->ml_part, shares * c.n_heads * 2 * 4);
     alloc((void**)&e->rope_cs, Mx * (c.head_dim / 2) * sizeof(float2));
     alloc((void**)&e->resid_bf, Mx * c.hidden * 2);
     // norm statistics: one sum per token and 128 columns, or per block of a one-token projection

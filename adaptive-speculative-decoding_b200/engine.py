@@ -255,8 +255,13 @@ class QwenEngine(_BatchOps):
                               cfg.num_key_value_heads // tp_size, cfg.head_dim, cfg.intermediate_size // tp_size,
                               cfg.vocab_size, cfg.rms_norm_eps, max_tokens, page_size, tp_rank, tp_size)
         self._lock = threading.Lock()
+        # One user's prompt goes through the layers whole, up to 1024 tokens a forward, however few an engine holds for its steps:
+        # in forwards of 256 the weights stream once for each (509 tokens, two 7B layers: 1184 us, whole 766).  Several prompts at
+        # once keep to max_tokens.
+        self.prompt_tokens = max(max_tokens, min(1024, max_seq_len)) if tp_size == 1 else max_tokens
         with torch.cuda.device(self.device):
-            self.h = lib().asd_engine_create(ctypes.byref(self.c))
+            self.h = lib().asd_engine_create_for_prompts(ctypes.byref(self.c),
+                                                         self.prompt_tokens if self.prompt_tokens > max_tokens else 0)
         if not self.h:
             check(-1, "asd_engine_create")
         self.max_pages = (max_seq_len + page_size - 1) // page_size
@@ -378,7 +383,7 @@ class QwenEngine(_BatchOps):
         # tokens a call) allow.  A tensor-parallel rank keeps the short chunk: its exchanges grow with the tokens.
         if self.tp_size > 1:
             return super()._prompt_chunk(nseq)
-        return max(1, min(self.max_tokens, 4096) // nseq)
+        return max(1, min(self.prompt_tokens if nseq == 1 else self.max_tokens, 4096) // nseq)
 
     def _prompt_forward(self, *args):
         return self._forward("asd_engine_forward_prompt", *args)

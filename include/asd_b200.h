@@ -167,6 +167,9 @@ typedef struct asd_model_config {
 typedef struct asd_engine asd_engine_t;
 
 ASD_API asd_engine_t* asd_engine_create(const asd_model_config* cfg); /* NULL on error */
+/* The same with activations for prompts of up to prompt_tokens (at most 4096; single rank): asd_engine_forward_prompt then takes
+ * that many new positions of ONE sequence in a call, whatever max_tokens. */
+ASD_API asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int prompt_tokens);
 ASD_API void asd_engine_destroy(asd_engine_t* e);
 ASD_API int asd_engine_set_layer(asd_engine_t* e, int layer, const void* wqkv, const void* bqkv, const void* wo,
                          const void* wgateup, const void* wdown, const void* ln1, const void* ln2);
@@ -250,7 +253,8 @@ ASD_API int asd_engine_forward(asd_engine_t* e, const int32_t* tokens, const int
                        const int32_t* token_slot, int M, const int32_t* cu_q, const int32_t* seq_slot, int nseq,
                        int max_qlen, int max_kv_len, const int32_t* logit_rows, int n_logit_rows, float* logits_out,
                        long long logits_ld, void* stream);
-/* The same for prompts: a sequence may bring any number of new positions (M <= max_tokens, and 4096 a call); beyond
+/* The same for prompts: a sequence may bring any number of new positions (M <= max_tokens, or the engine's
+ * prompt_tokens for one sequence, and 4096 a call); beyond
  * 128 / (heads per key/value head) of them attention runs in query tiles of that many positions.  At most 128 heads per
  * key/value head. */
 ASD_API int asd_engine_forward_prompt(asd_engine_t* e, const int32_t* tokens, const int32_t* positions,
