@@ -157,6 +157,7 @@ def lib() -> ctypes.CDLL:
         "asd_bayesian_adjustment_host": (f64, [f64, f64, f64, f64]),
         "asd_linear_bf16": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp]),
         "asd_linear_bf16_tc": (i32, [vp, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp]),
+        "asd_linear_bf16_few": (i32, [vp, vp, vp, i32, i32, i32, vp]),
         "asd_linear_plan": (i32, [i32, i32, i32, i32, vp, vp, vp]),
         "asd_engine_create": (vp, [vp]),
         "asd_engine_create_for_prompts": (vp, [vp, i32]),

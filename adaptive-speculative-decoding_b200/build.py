@@ -23,7 +23,7 @@ FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-std=c++17", "-li
 COMPONENTS = {
     "core": ["core.cu"],
     "linear": ["gemm.cu", "gemm_tc.cu"],
-    "blocks": ["linear_simt.cu", "linear_tc.cu"],
+    "blocks": ["linear_simt.cu", "linear_tc.cu", "linear_few.cu"],
     "latent": ["latent_attention.cu", "latent_attention_tc.cu"],
     "rows": ["norm_ops.cu", "moe.cu"],          # row kernels and the expert router that several families share
     "mezilix": ["mezilix_engine.cu", "stream_ops.cu"],

@@ -147,6 +147,11 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
                                int max_kv_len, const __nv_bfloat16* q_terms, const LatentDims& d, const PagedRows& cache,
                                float* out_lat, const AttnSplit& ws, int* err, cudaStream_t stream);
 
+// ---------------------------------------------------------------------------------------------- linear_few.cu
+// y fp32 [M][ldc] = x bf16 [M][K] * w bf16 [N][K]^T for a few tokens (M <= 16)
+bool linear_few_takes(const void* x, const void* w, int M, int N, int K);
+int launch_linear_few(const void* x, const void* w, float* y, int M, int N, int K, int ldc, cudaStream_t stream);
+
 // ---------------------------------------------------------------------------------------------- moe.cu
 // Router: probs = softmax(logits) over all E experts (fp32); the `top` largest are kept with their probabilities as
 // gates (not renormalised; ties go to the lower index).  Then the (token, choice) pairs are grouped by expert:

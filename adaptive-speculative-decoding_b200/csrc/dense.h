@@ -17,6 +17,7 @@ namespace asd {
 struct DenseRunner {
     int f32 = 0;                 // 1: fp32 operands (always the CUDA-core kernel)
     int tc_linear = 1;
+    int few = 1;                 // few tokens on smaller matrices: linear_few.cu
     int tc_min_rows = 257;       // token count from which the tensor-bound CTA-pair GEMM runs
     struct Entry {
         GemmPlan pl;
@@ -31,6 +32,7 @@ struct DenseRunner {
         if (!f32 && tc_linear && (K % 8) == 0 && (ldc % 4) == 0 && K >= 64 && N >= 8 &&
             (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
+            if (few && linear_few_takes(x, w, M, N, K)) return launch_linear_few(x, w, y, M, N, K, ldc, s);
             const unsigned long long k = ((unsigned long long)key << 32) | (unsigned)M;
             auto it = cache.find(k);
             if (it == cache.end()) {

@@ -510,6 +510,10 @@ int asd_rivetar_set_option(asd_rivetar_engine_t* h, const char* name, int value)
         e->dn.tc_linear = value;
         return 0;
     }
+    if (!strcmp(name, "linear_few")) {
+        e->dn.few = value;
+        return 0;
+    }
     if (!strcmp(name, "tc_min_rows")) {
         e->dn.tc_min_rows = value > 0 ? value : 1 << 30;
         e->dn.clear();

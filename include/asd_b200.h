@@ -37,7 +37,7 @@ ASD_API const char* asd_last_error(void);
 /* number of kernels this library has launched since load / since the last reset (bench "gpu_launches") */
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
-/* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemm_grouped", "gemv",
+/* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemm_grouped", "gemv", "linear_few",
  * "attention_tc", "latent_tc", "window_tc", "sampler_draw"; -1 for another name */
 ASD_API long long asd_kernel_launches(const char* name);
 /* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:
@@ -134,6 +134,8 @@ ASD_API int asd_linear_bf16(const void* x, const void* w, void* out, int M, int 
  * accumulators.  out_mode 0: fp32 [ksplit_used, M, N] slices; out_mode 2: SwiGLU bf16 [M, N/2]. */
 ASD_API int asd_linear_bf16_tc(const void* x, const void* w, void* out, int M, int N, int K, int out_mode, int ksplit,
                        int stages, int* ksplit_used, void* stream);
+/* Same contraction for a few tokens (M <= 16, matrices up to 64 MB): out fp32 [M, N] */
+ASD_API int asd_linear_bf16_few(const void* x, const void* w, void* out, int M, int N, int K, void* stream);
 ASD_API int asd_linear_plan(int M, int N, int K, int out_mode, int* ksplit, int* stages, int* token_tile);
 
 /* ---------------------------------------------------------------------------------------------
