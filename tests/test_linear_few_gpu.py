@@ -15,8 +15,9 @@ def few(x, w):
     return out
 
 
-# rows that no group of 16 fills, k that no piece of 32, warp or block of eight pieces fills, several groups a CTA, the longest k
-@pytest.mark.parametrize("N,K", [(1, 8), (16, 40), (25, 256), (100, 1000), (2051, 2048), (6144, 2048), (9000, 264), (48, 3000),
+# rows that no group of 16 fills, k that no piece of 32, warp or block of eight pieces fills, several groups a CTA,
+# both sides of the line between two blocks an SM and one, the longest k
+@pytest.mark.parametrize("N,K", [(1, 8), (16, 40), (25, 256), (100, 1000), (2051, 2048), (6144, 2048), (9000, 264), (48, 3000), (2816, 2816), (4000, 2824), (6000, 4096),
                                  (2048, 6144)])
 def test_few_tokens_match_and_do_not_depend_on_their_number(N, K):
     g = torch.Generator(device="cuda").manual_seed(N + K)
