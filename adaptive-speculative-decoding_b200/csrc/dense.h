@@ -1,6 +1,6 @@
 // Dense projection of an engine's activations, y fp32 [M][ldc] = x [M][K] * w[N][K]^T, routed by shape and element
 // type: the weight-streaming tcgen05 GEMM (gemm.cu) for bf16 operands it accepts, its tensor-bound CTA-pair form
-// (gemm_tc.cu) from `tc_min_rows` tokens on, the CUDA-core kernel (linear_simt.cu) for fp32 engines and every other
+// (gemm_tc.cu) above 256 tokens, of larger matrices above 160, the CUDA-core kernel (linear_simt.cu) for fp32 engines and every other
 // shape.  Plans and tensor maps are cached per (call site, token count); a call site always passes the same buffers.
 #pragma once
 #include <cuda.h>
@@ -18,7 +18,7 @@ struct DenseRunner {
     int f32 = 0;                 // 1: fp32 operands (always the CUDA-core kernel)
     int tc_linear = 1;
     int few = 1;                 // few tokens on smaller matrices: linear_few.cu
-    int tc_min_rows = 257;       // token count from which the tensor-bound CTA-pair GEMM runs
+    int tc_min_rows = 0;         // token count from which the tensor-bound CTA-pair GEMM runs (0: pair_from's rule)
     struct Entry {
         GemmPlan pl;
         TcPlan big;
@@ -27,6 +27,15 @@ struct DenseRunner {
     std::unordered_map<unsigned long long, Entry> cache;
 
     void clear() { cache.clear(); }
+
+    // Above 160 tokens the weight-streaming kernel has room for fewer blocks of its wider tiles (a step of three Rivetar layers of
+    // width 2048, 160 tokens 511 us, 192 590; on CTA pairs 557 and 574, of width 4096 707, 1005 and 892, 919, a Mezilix layer of
+    // width 4096 348, 397 and 362, 370).  Of matrices below 4M elements the pairs gain less than their plain launches cost (Rivetar
+    // of width 1024, 192 tokens: 389 and 416).
+    bool pair_from(int M, int N, int K) const {
+        if (tc_min_rows > 0) return M >= tc_min_rows;
+        return M > 256 || (M > 160 && (long long)N * K >= 1 << 22);
+    }
 
     int run(const void* x, const void* w, float* y, int M, int N, int K, int ldc, int key, cudaStream_t s) {
         if (!f32 && tc_linear && (K % 8) == 0 && (ldc % 4) == 0 && K >= 64 && N >= 8 &&
@@ -38,7 +47,7 @@ struct DenseRunner {
             if (it == cache.end()) {
                 Entry t;
                 if (make_tmap_bf16(&t.tw, w, N, K, K, 128)) return -1;
-                if (M >= tc_min_rows) {   // above the HBM / tensor ridge: 256 weight rows x MT tokens on a CTA pair
+                if (pair_from(M, N, K)) {   // above the HBM / tensor ridge: 256 weight rows x MT tokens on a CTA pair
                     if (gemm_tc_plan(&t.big, M, N, K, GEMM_OUT_F32, 1, 0, false)) return -1;
                     if (make_tmap_bf16(&t.tx, x, M, K, K, t.big.MT / 2)) return -1;
                 } else {
@@ -47,7 +56,7 @@ struct DenseRunner {
                 }
                 it = cache.emplace(k, t).first;
             }
-            if (M >= tc_min_rows)
+            if (pair_from(M, N, K))
                 return gemm_tc_launch(it->second.big, it->second.tw, it->second.tx, y, ldc, N, 0, s, false, nullptr);
             return gemm_launch(it->second.pl, it->second.tw, it->second.tx, y, ldc, N, true, s, false);
         }

@@ -314,8 +314,10 @@ ASD_API size_t asd_mezilix_cache_bytes(const asd_mezilix_engine_t* e, int num_pa
 ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, int32_t* token_ring, float* shift_ring);
 /* options: "tc_linear" (1, default: bf16 projections whose shape the tcgen05 kernels accept run on them; 0: CUDA-core
- * kernel everywhere), "tc_min_rows" (token count from which dense projections use the tensor-bound CTA-pair GEMM, default
- * 257; 0 = never), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
+ * kernel everywhere), "tc_min_rows" (token count from which dense projections use the tensor-bound CTA-pair GEMM; 0 = never;
+ * left alone: 257, 161 for matrices of 4M elements on), "linear_few" (1, default: up to 16 tokens on matrices up to 64 MB run
+ * linear_few.cu), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
+ * rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
  * per (token, head)), "profile" (1: CUDA events around every launch, read with asd_mezilix_profile_read) */
 ASD_API int asd_mezilix_set_option(asd_mezilix_engine_t* e, const char* name, int value);
@@ -398,7 +400,8 @@ ASD_API size_t asd_rivetar_cache_bytes(const asd_rivetar_engine_t* e, int num_pa
 ASD_API size_t asd_rivetar_state_bytes(const asd_rivetar_engine_t* e, int max_seqs);
 ASD_API int asd_rivetar_set_cache(asd_rivetar_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows", "attn_tiled" as for the Mezilix engine; "fused_attn" (1, default: tiled windowed
+/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_tiled" as for the Mezilix engine (attn_tiled 2: windowed attention of
+ * 17 query rows a tile and more on tcgen05 too); "fused_attn" (1, default: tiled windowed
  * attention kernel; 0: one warp per (token, head)); "profile" */
 ASD_API int asd_rivetar_set_option(asd_rivetar_engine_t* e, const char* name, int value);
 /* Same arguments as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [runs][M][width]) receives the

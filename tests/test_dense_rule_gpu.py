@@ -1,0 +1,31 @@
+"""GPU: which dense projections of a family's engine run on CTA pairs, by tokens and matrix size."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from oracle import rivetar_oracle as O  # noqa: E402
+from test_rivetar_gpu import close, config, gla, make_engine, tokens  # noqa: E402
+
+
+@pytest.mark.parametrize("length,pairs", [(160, 0), (161, 2), (256, 2), (257, 3)])
+def test_larger_matrices_take_pairs_from_161_tokens(length, pairs):
+    """up and down projection of 2048 x 2048 (4M elements) and a smaller input projection (the output projection of 16 columns and
+    the head's single row take other kernels)"""
+    from asd_b200._lib import lib
+    cfg = config([gla(heads=1, dim=16, vdim=16, ff=2048)], width=2048)
+    w = O.random_model(cfg, seed=71)
+    ids = tokens(length, 96, 72)
+    outs = []
+    for rows in (0, None):
+        eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512)
+        if rows is not None:
+            eng.set_option("tc_min_rows", rows)         # 0: never
+        slot = eng.open_sequence()
+        eng.reserve(slot, length)
+        before = lib().asd_kernel_launches(b"gemm_pair")
+        outs.append(eng.forward_ragged([(slot, 0, ids, [length - 1])]).double().cpu())
+        assert lib().asd_kernel_launches(b"gemm_pair") - before == (pairs if rows is None else 0)
+        close(eng)
+    # the same bf16 operands, fp32 sums in another order: a rounding of the activations apart
+    assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() < 1e-2
