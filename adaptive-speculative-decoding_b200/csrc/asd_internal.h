@@ -5,6 +5,8 @@
 #include <stdint.h>
 #include <stdlib.h>
 
+#include "per_device.h"
+
 #define ASD_NUM_FEATURES 6
 
 namespace asd {
@@ -95,20 +97,6 @@ struct TuningScope {
 };
 
 int sm_count();      // multiprocessors of the current device
-
-// cudaFuncSetAttribute is per device: remember which devices a kernel's attributes were set on
-struct PerDeviceOnce {
-    unsigned long long mask = 0;
-    bool need(int* dev_out = nullptr) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (dev_out) *dev_out = dev;
-        const unsigned long long bit = 1ull << (dev & 63);
-        if (mask & bit) return false;
-        mask |= bit;
-        return true;
-    }
-};
 
 // sampler.cu
 size_t reject_sample_workspace_bytes(int B, int k);

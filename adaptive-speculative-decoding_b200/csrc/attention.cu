@@ -495,11 +495,11 @@ template <int HD, int KW, int NS>
 static int launch_mma(const AttnArgs& a, const CUtensorMap& pf0, const CUtensorMap& pf1, dim3 grid, int threads,
                       size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(attn_mma_kernel<HD, KW, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       200 * 1024));
         prefer_max_smem(attn_mma_kernel<HD, KW, NS>);
-    }
+    });
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

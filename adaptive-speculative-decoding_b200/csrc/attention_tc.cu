@@ -517,10 +517,10 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     static PerDeviceOnce once;
     const size_t smem = 1024 + 5 * (size_t)kAtOp + 22 * 8 + 16 + 6 * 128 * 4 +
                         ((size_t)L.split_keys / L.page_size + 2) * 4 + 64;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
         prefer_max_smem(attn_tc_kernel<false>);
-    }
+    });
     if (smem > 227 * 1024) return set_error("attention_tc: split of %d keys does not fit the page-table slice", L.split_keys);
     AttnTcArgs a;
     a.q = L.q;

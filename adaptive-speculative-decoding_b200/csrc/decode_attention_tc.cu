@@ -269,7 +269,7 @@ template <int NDV, int NS, int MODE>
 int launch_mode(const MixArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kernel = decode_tc_kernel<NDV, NS, MODE>;
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     kernel<<<grid, NT, smem, stream>>>(a);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

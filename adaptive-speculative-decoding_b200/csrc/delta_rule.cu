@@ -691,8 +691,8 @@ int launch_lowrank_channels(const float* a, long long lda, const LowRankChannels
     const size_t smem = (size_t)p.low * (LC_CH + LC_TOK) * sizeof(float);
     if (smem > 200 * 1024) return set_error("lowrank_channels: inner size %d does not fit shared memory", p.low);
     static PerDeviceOnce once;
-    if (once.need())
-        ASD_CUDA(cudaFuncSetAttribute(lowrank_channels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once,
+             ASD_CUDA(cudaFuncSetAttribute(lowrank_channels_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     dim3 grid((p.n + LC_CH - 1) / LC_CH, (M + LC_TOK - 1) / LC_TOK);
     if (grid.y > 65535) return set_error("lowrank_channels: too many tokens");
     lowrank_channels_kernel<<<grid, LC_CH, smem, stream>>>(a, lda, p, out, M);
@@ -812,7 +812,7 @@ int launch_delta_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_
     {                                                                                                                 \
         auto fn = delta_recurrence_cols_kernel<P_, NVV>;                                                              \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         fn<<<grid, warps * 32, need(ch), stream>>>(ix, cu_q, seq_slot, rv, sc, v, ldv, heads, dk, dv, state, ring, out, \
                                                    ch);                                                               \
     }
@@ -849,7 +849,7 @@ int launch_delta_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_
     {                                                                                                                 \
         auto fn = delta_recurrence_kernel<R, NVV, T>;                                                                  \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         fn<<<grid, RS * 32, smem, stream>>>(ix, cu_q, seq_slot, rv, sc, v, ldv, heads, dk, dv, state, ring, out, ch);  \
     }
 #define ASD_DR_ROWS(NVV)                             \

@@ -627,8 +627,10 @@ asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int pro
     }
     {   // lazy module loading + spinning tensor-parallel kernels in one process = deadlock: load everything now
         static PerDeviceOnce loaded;
-        if (loaded.need() && (preload_layers() || preload_attention() || preload_attention_tc() || preload_gemm() ||
-                              preload_gemm_tc() || preload_gemv()))
+        if (loaded.run([]() -> int {
+                return preload_layers() || preload_attention() || preload_attention_tc() || preload_gemm() || preload_gemm_tc() ||
+                       preload_gemv();
+            }))
             return nullptr;
     }
     Engine* e = new Engine();

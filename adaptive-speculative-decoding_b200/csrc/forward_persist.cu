@@ -1073,10 +1073,10 @@ bool persist_supported(int M, int n_logit_rows, int max_qlen, int nh, int nkv, i
 template <int HD, int KW>
 static int p_launch_t(const CUtensorMap maps[5], const PArgs& a, int grid, size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(fwd_persist_kernel<HD, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_p_smem));
         prefer_max_smem(fwd_persist_kernel<HD, KW>);
-    }
+    });
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;

@@ -821,11 +821,11 @@ void gemm_set_next(const GemmPlan& next, const CUtensorMap* next_w) {
 int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo,
                 int n_valid, bool pdl, cudaStream_t stream, bool accumulate, const QkvEpilogue* qkv,
                 const NormFusion* norm, const TpFusion* tp) {
-    if (g_gemm_attr.need()) {
+    ASD_ONCE(g_gemm_attr, {
         if (device_props()) return -1;
         ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
         prefer_max_smem(gemm_ws_kernel<false>);
-    }
+    });
     GemmArgs a;
     a.M = pl.M;
     a.N = pl.N;

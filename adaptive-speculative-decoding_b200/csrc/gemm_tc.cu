@@ -500,10 +500,10 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
                    size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm) {
-    if (g_tc_attr.need()) {
+    ASD_ONCE(g_tc_attr, {
         ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
         prefer_max_smem(gemm_tc_kernel<false>);
-    }
+    });
     if (norm && !pl.norm) return set_error("gemm_tc: the plan has no place for a norm's factors");
     if (accumulate && (pl.mode != GEMM_OUT_F32 || pl.ksplit != 1))
         return set_error("gemm_tc: accumulate needs the fp32 epilogue without a K split");
@@ -572,10 +572,10 @@ int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream
     if (make_tmap_bf16(&tx, L.a, rows, L.K, L.K, mt / 2)) return -1;
     if (make_tmap_out(&to, L.c, L.epilogue == 1, rows, L.N, 1, L.ldc, (size_t)rows * L.ldc, 128, kTcOutTok)) return -1;
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
         prefer_max_smem(gemm_tc_kernel<true>);
-    }
+    });
     gemm_tc_kernel<true><<<g_tc_sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_GROUPED);

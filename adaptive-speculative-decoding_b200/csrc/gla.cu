@@ -385,10 +385,10 @@ int launch_gla_decay(const float* a, long long lda, const float* w_decay, const 
     const int cpt = (n + 4 * GD_LANES - 1) / (4 * GD_LANES) * tiles >= sm_count() ? 4 : 1;
     const size_t smem = ((size_t)d.low * (GD_LANES * cpt + 1) + (size_t)d.low * GD_TOK) * sizeof(float);
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(gla_decay_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    }
+    });
     const dim3 grid((n + GD_LANES * cpt - 1) / (GD_LANES * cpt), tiles);
     ASD_CUDA(launch_pdl(cpt == 4 ? gla_decay_kernel<4> : gla_decay_kernel<1>, grid, GD_THREADS, smem, stream, a, lda, w_decay,
                         b_decay, d, alpha, M));
@@ -420,8 +420,8 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
                             : (threads > 256 ? gla_recurrence_kernel<512, 1, true>
                                              : (ch == 1 ? gla_recurrence_kernel<256, 4, false> : gla_recurrence_kernel<256, 2, true>));
     static PerDeviceOnce once[4];
-    if (once[threads > 512 ? 3 : (threads > 256 ? 2 : ch == 1)].need())
-        ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once[threads > 512 ? 3 : (threads > 256 ? 2 : ch == 1)],
+             ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(fn, grid, threads, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out, ch, vec));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -920,7 +920,7 @@ int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, 
     if (d.rot_dims < 0 || d.rot_dims > d.dr || (d.rot_dims & 1))
         return set_error("latent attention: rot_dims %d must be even and <= %d", d.rot_dims, d.dr);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(latent_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(latent_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(latent_post_kernel, ix.M, 256, std::max(d.rot_dims / 2, 1) * sizeof(float2), stream, ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq,
                         cache, q_lat, q_terms,
                                                (long long)ix.M * d.heads * (d.R + d.dr)));

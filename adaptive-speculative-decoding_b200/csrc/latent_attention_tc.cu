@@ -29,7 +29,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "asd_internal.h"
 #include "blocks.h"
@@ -567,12 +566,8 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     if (make_tmap_bf16_planes(&mq, q_terms, rows, rw, 3, a.box_rows)) return -1;
     if (make_tmap_bf16(&mk, cache.pool, cache.rows, rw, rw, cache.page_size)) return -1;
     const int smem = 1024 + (kLtVSlots + kLtKSlots + 3 * kLtQSlots) * kLtSlot + (int)sizeof(LtBars);
-    static std::once_flag once[64];     // (a second thread's first launch must not overtake the attribute)
-    int dev = 0;
-    ASD_CUDA(cudaGetDevice(&dev));
-    cudaError_t rc = cudaSuccess;
-    std::call_once(once[dev & 63], [&] { rc = cudaFuncSetAttribute(latent_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem); });
-    ASD_CUDA(rc);
+    static PerDeviceOnce once;
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(latent_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)));
     const dim3 grid(p.q_tiles * p.hgs * p.parts, nseq * a.nsplit);
     latent_attn_tc<<<grid, kLtThreads, smem, stream>>>(mq, mk, a);
     count_kernel(KERNEL_LATENT_TC);

@@ -441,13 +441,15 @@ int launch_gather_rows(const __nv_bfloat16* src, const int* rows, __nv_bfloat16*
 
 static void glue_carveout() {
     static PerDeviceOnce once;
-    if (!once.need()) return;
-    prefer_max_smem(add_norm_kernel);
-    prefer_max_smem(tp_allreduce_norm_kernel);
-    prefer_max_smem(reduce_slices_kernel);
-    prefer_max_smem(qkv_rope_kernel);
-    prefer_max_smem(rope_table_kernel);
-    prefer_max_smem(gather_rows_kernel);
+    once.run([]() {
+        prefer_max_smem(add_norm_kernel);
+        prefer_max_smem(tp_allreduce_norm_kernel);
+        prefer_max_smem(reduce_slices_kernel);
+        prefer_max_smem(qkv_rope_kernel);
+        prefer_max_smem(rope_table_kernel);
+        prefer_max_smem(gather_rows_kernel);
+        return 0;
+    });
 }
 
 // Force the (lazily loaded) kernels of this file into the context now: a first launch that loads a kernel may need a

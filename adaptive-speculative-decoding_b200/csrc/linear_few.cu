@@ -166,7 +166,7 @@ int launch_linear_few(const void* x, const void* w, float* y, int M, int N, int 
     a.row_bytes = (a.pieces | 1) * 64;
     const size_t smem = lf_smem(K);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(linear_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLfSmemMax));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(linear_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLfSmemMax)));
     const int groups = (N + kLfRows - 1) / kLfRows, per_sm = smem <= 96 * 1024 ? 2 : 1;
     ASD_CUDA(launch_pdl(linear_few_kernel, std::min(groups, per_sm * sm_count()), kLfThreads, smem, stream, a));
     ASD_CUDA(cudaGetLastError());

@@ -834,12 +834,12 @@ int launch_mix_post(const SeqIndex& ix, float* qkv, long long ld, const MixDims&
     const int threads = n >= 2048 ? 256 : 128;
     if (smem > 200 * 1024) return set_error("mix_post: a row of %d values does not fit shared memory", n);
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(mix_post_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(mix_post_kernel<float, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(mix_post_kernel<__nv_bfloat16, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(mix_post_kernel<__nv_bfloat16, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    }
+    });
     const uintptr_t at = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(p.bias) |
                          (p.q_only ? 0 : reinterpret_cast<uintptr_t>(cache.pool));
     const bool four = d.dk % 4 == 0 && d.dv % 4 == 0 && ld % 4 == 0 && (at & 15) == 0;
@@ -867,10 +867,10 @@ int launch_mix_merge(const MixArgs& a, cudaStream_t stream, bool stats) {
 template <typename T>
 static int launch_dec(const MixArgs& a, dim3 grid, size_t smem_scores, size_t smem_apply, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(mix_dec_scores_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(mix_dec_apply_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    }
+    });
     mix_dec_scores_kernel<T><<<grid, NT, smem_scores, stream>>>(a);
     mix_dec_apply_kernel<T><<<grid, NT, smem_apply, stream>>>(a);
     count_launch(2);
@@ -915,8 +915,8 @@ int launch_mix_attention_decode(MixArgs a, int nseq, int max_kv_len, const MixWo
 template <typename T, bool APPLY, int CB>
 static int launch_one(const MixArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need())
-        ASD_CUDA(cudaFuncSetAttribute(mix_attn_kernel<T, APPLY, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once,
+             ASD_CUDA(cudaFuncSetAttribute(mix_attn_kernel<T, APPLY, CB>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     mix_attn_kernel<T, APPLY, CB><<<grid, NT, smem, stream>>>(a);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -432,7 +432,7 @@ template <int KT, int NDV, bool APPLY, bool TALK, int MODE, bool CAP = false>
 int launch_tc(const MixArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     auto kernel = mix_tc_kernel<KT, NDV, APPLY, TALK, MODE, CAP>;
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     kernel<<<grid, NT, smem, stream>>>(a);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -350,7 +350,7 @@ int launch_mlstm_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_
     {                                                                                                                 \
         auto fn = mlstm_recurrence_kernel<R, T>;                                                                      \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         fn<<<grid, RS * 32, smem, stream>>>(a);                                                                       \
     }
     if (RS > 8) ASD_ML_CASE(32, 1024)

@@ -614,10 +614,10 @@ int launch_row_close(const RowClose& c, cudaStream_t stream) {
     const size_t smem = (size_t)(c.D + 33 + MAX_NORM_GROUPS) * sizeof(float);
     if (smem > 200 * 1024) return set_error("row_close: width %d does not fit shared memory", c.D);
     static PerDeviceOnce once;
-    if (once.need()) {
+    ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(row_close_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         ASD_CUDA(cudaFuncSetAttribute(row_close_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
-    }
+    });
     if (wide && c.D % 4 == 0 && (c.D / c.groups) % 4 == 0)
         ASD_CUDA(launch_pdl(row_close_kernel<4>, c.M, row_threads(c.D), smem, stream, c));
     else
@@ -635,7 +635,7 @@ int launch_embed_normed(const SeqIndex& ix, const void* embed, int wf32, const f
     const size_t smem = (size_t)(D + 33 + MAX_NORM_GROUPS) * sizeof(float);
     if (smem > 200 * 1024) return set_error("embed_normed: width %d does not fit shared memory", D);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(embed_normed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(embed_normed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(embed_normed_kernel, ix.M, row_threads(D), smem, stream, ix, embed, wf32, w, groups, eps, x, D));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
@@ -715,7 +715,7 @@ int launch_polynorm(const float* z, const float* coeff, float eps, void* out, in
     const int staged = (size_t)F * sizeof(float) <= 96 * 1024;
     const size_t smem = (33 + (staged ? (size_t)F : 0)) * sizeof(float);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(polynorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(polynorm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(polynorm_kernel, M, row_threads(F), smem, stream, z, coeff, eps, out, of32, F, staged));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -1,0 +1,42 @@
+// What host code does once per device and process: kernel attributes, module loads, device limits.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <atomic>
+#include <mutex>
+
+namespace asd {
+
+// cudaFuncSetAttribute and module loads are per device.  `run` calls `set` on the current device until one call of it has returned 0;
+// a thread that meets another's call waits for its end, so that no first launch overtakes the attribute it needs.
+class PerDeviceOnce {
+public:
+    template <typename F>
+    int run(F&& set) {
+        int dev = 0;
+        cudaGetDevice(&dev);
+        const unsigned long long bit = 1ull << (dev & 63);
+        if (done_.load(std::memory_order_acquire) & bit) return 0;
+        std::lock_guard<std::mutex> hold(lock_);
+        if (done_.load(std::memory_order_relaxed) & bit) return 0;
+        const int rc = set();
+        if (rc == 0) done_.fetch_or(bit, std::memory_order_release);
+        return rc;
+    }
+
+private:
+    std::atomic<unsigned long long> done_{0};
+    std::mutex lock_;
+};
+
+// the statements (which may return -1, as ASD_CUDA does) once per device, in a function that returns -1 on failure
+#define ASD_ONCE(once, ...)                  \
+    do {                                     \
+        if ((once).run([&]() -> int {        \
+                __VA_ARGS__;                 \
+                return 0;                    \
+            }))                              \
+            return -1;                       \
+    } while (0)
+
+}  // namespace asd

@@ -99,8 +99,8 @@ int launch_embed_streams(const SeqIndex& ix, const void* embed, const void* pos_
 template <int S_>
 static int launch_close(const StreamClose& c, size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need())
-        ASD_CUDA(cudaFuncSetAttribute(stream_close_kernel<S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once,
+             ASD_CUDA(cudaFuncSetAttribute(stream_close_kernel<S_>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     stream_close_kernel<S_><<<c.M, stream_threads(c.D), smem, stream>>>(c);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

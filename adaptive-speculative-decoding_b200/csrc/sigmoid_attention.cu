@@ -189,8 +189,8 @@ __global__ void __launch_bounds__(NT) sigmoid_decode_kernel(MixArgs a) {
 template <typename T, int VC>
 int launch_sig(const MixArgs& a, dim3 grid, size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
-    if (once.need())
-        ASD_CUDA(cudaFuncSetAttribute(sigmoid_decode_kernel<T, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once,
+             ASD_CUDA(cudaFuncSetAttribute(sigmoid_decode_kernel<T, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     sigmoid_decode_kernel<T, VC><<<grid, NT, smem, stream>>>(a);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

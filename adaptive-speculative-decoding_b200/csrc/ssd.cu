@@ -294,7 +294,7 @@ int launch_ssd_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     {                                                                                                                 \
         auto fn = ssd_recurrence_kernel<R, T>;                                                                        \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         fn<<<grid, RS * 32, smem, stream>>>(a);                                                                       \
     }
     if (RS > 8) ASD_SSD_CASE(32, 1024)

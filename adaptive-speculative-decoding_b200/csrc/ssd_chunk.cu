@@ -294,7 +294,7 @@ template <int NK>
 int launch_nk(const SsdArgs& a, dim3 grid, cudaStream_t stream) {
     const int smem = chunk_smem(16 * NK + 8);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(ssd_chunk_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(ssd_chunk_kernel<NK>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)));
     ssd_chunk_kernel<NK><<<grid, NT, smem, stream>>>(a);
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -792,7 +792,7 @@ int launch_talk_attention(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     {                                                                                                                 \
         auto fn = talk_attention_mma_kernel<N, P>;                                                                    \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         ASD_CUDA(cudaLaunchKernelEx(&lc, fn, ix, cu_q, seq_slot, q, ldq, d, talk, sink, cache, out, of32, ldo, out_scale)); \
     }
 #define ASD_TM_CASE(N)                  \
@@ -902,7 +902,7 @@ int launch_talk_attention(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     {                                                                                                                 \
         auto fn = talk_attention_kernel<L, Q>;                                                                        \
         static PerDeviceOnce once;                                                                                    \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         fn<<<grid, d.heads * 32, smem, stream>>>(ix, cu_q, seq_slot, q, ldq, d, talk, sink, cache, out, of32, ldo,     \
                                                  out_scale, tl, ws.o, nsplit);                                        \
     }

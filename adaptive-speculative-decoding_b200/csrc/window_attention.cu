@@ -230,7 +230,7 @@ int launch_simple(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
     {                                                                                                                \
         auto fn = window_attn_kernel<T, A>;                                                                          \
         static PerDeviceOnce once;                                                                                   \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024))); \
         ASD_CUDA(launch_pdl(fn, grid, warps * 32, smem, stream, ix, cu_q, seq_slot, TQ, hpc, q, ldq, d, sink, freq_v, cache, out, of32)); \
     }
     if (acc <= 1) ASD_WIN_CASE(1)
@@ -670,7 +670,7 @@ int launch_mma(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nse
     {                                                                                                                \
         auto fn = window_attn_mma<N, S, G, Q>;                                                                           \
         static PerDeviceOnce once;   /* the attribute is set once per device: a host call per launch costs microseconds */ \
-        if (once.need()) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem)); \
+        ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxSmem))); \
         ASD_CUDA(launch_pdl(fn, grid, 128, smem, stream, ix, cu_q, seq_slot, TQ, q, ldq, d, sink, freq_v, cache, out, of32, nsplit,   \
                                         ws.o, ws.ml, q_alloc));                                                       \
     }
@@ -721,7 +721,7 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
         return set_error("windowed attention: a token's q | k | v row is too long");
     const size_t smem = (size_t)(d.rot_dims + d.dv) / 2 * sizeof(float2);
     static PerDeviceOnce once;
-    if (once.need()) ASD_CUDA(cudaFuncSetAttribute(window_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(window_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(window_post_kernel, ix.M, 256, smem, stream, ix, qkv, ld, d, freq_k, freq_v, cache, turns));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

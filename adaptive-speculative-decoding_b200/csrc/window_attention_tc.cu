@@ -22,7 +22,6 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
 #include "asd_internal.h"
@@ -477,12 +476,8 @@ int launch_window_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     CUtensorMap mk;
     if (make_tmap_bf16(&mk, cache.pool, cache.rows, rowlen, rowlen, cache.page_size)) return -1;
     const int smem = 1024 + (4 * kc + 2 * vc) * kWtSlot + (int)sizeof(WtBars);
-    static std::once_flag once[64];     // (a second thread's first launch must not overtake the attribute)
-    int dev = 0;
-    ASD_CUDA(cudaGetDevice(&dev));
-    cudaError_t rc = cudaSuccess;
-    std::call_once(once[dev & 63], [&] { rc = cudaFuncSetAttribute(window_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024); });
-    ASD_CUDA(rc);
+    static PerDeviceOnce once;
+    ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(window_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     window_attn_tc<<<grid, kWtThreads, smem, stream>>>(mk, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_WINDOW_TC);
