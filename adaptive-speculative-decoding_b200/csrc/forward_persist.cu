@@ -1045,19 +1045,10 @@ __global__ void __launch_bounds__(kPThreads, 1)
 }
 
 // ------------------------------------------------------------------------------------------------------- host
-static int g_p_sms = 0, g_p_smem = 0;
-static int p_props() {
-    if (g_p_sms) return 0;
-    int dev = 0;
-    ASD_CUDA(cudaGetDevice(&dev));
-    ASD_CUDA(cudaDeviceGetAttribute(&g_p_sms, cudaDevAttrMultiProcessorCount, dev));
-    ASD_CUDA(cudaDeviceGetAttribute(&g_p_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    return 0;
-}
-
 int persist_num_ctas() {
-    if (p_props()) return 0;
-    return g_p_sms < 256 ? g_p_sms : 256;
+    DeviceLimits dev;
+    if (device_limits(&dev)) return 0;
+    return dev.sms < 256 ? dev.sms : 256;
 }
 size_t persist_part_ws_bytes() { return (size_t)persist_num_ctas() * 2 * kPTile * 128 * sizeof(float); }
 
@@ -1074,7 +1065,9 @@ template <int HD, int KW>
 static int p_launch_t(const CUtensorMap maps[5], const PArgs& a, int grid, size_t smem, cudaStream_t stream) {
     static PerDeviceOnce once;
     ASD_ONCE(once, {
-        ASD_CUDA(cudaFuncSetAttribute(fwd_persist_kernel<HD, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_p_smem));
+        DeviceLimits dev;
+        if (device_limits(&dev)) return -1;
+        ASD_CUDA(cudaFuncSetAttribute(fwd_persist_kernel<HD, KW>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
         prefer_max_smem(fwd_persist_kernel<HD, KW>);
     });
     cudaLaunchConfig_t cfg = {};
@@ -1092,7 +1085,8 @@ static int p_launch_t(const CUtensorMap maps[5], const PArgs& a, int grid, size_
 }
 
 int persist_launch(const PersistLaunch& L, cudaStream_t stream) {
-    if (p_props()) return -1;
+    DeviceLimits dev;
+    if (device_limits(&dev)) return -1;
     if (!persist_supported(L.M, L.n_logit_rows, L.max_qlen, L.nh, L.nkv, L.hd, L.page_size, L.h, L.n_layers))
         return set_error("persist: unsupported shape");
     PArgs a;
@@ -1122,7 +1116,7 @@ int persist_launch(const PersistLaunch& L, cudaStream_t stream) {
     aux = (aux + 1023) / 1024 * 1024;
     a.aux_bytes = (int)aux;
     const int small = 2048;
-    int stages = (int)((g_p_smem - 1024 - (int)aux - small) / a.stage_bytes);
+    int stages = (int)((dev.smem_optin - 1024 - (int)aux - small) / a.stage_bytes);
     if (stages > 12) stages = 12;
     if (stages < 2) return set_error("persist: shared memory does not fit a two-stage ring");
     a.stages = stages;

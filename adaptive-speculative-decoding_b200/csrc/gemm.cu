@@ -701,18 +701,7 @@ thread_local NextPrefetch g_gemm_next;   // set by the caller right before gemm_
 unsigned long long* g_gemm_trace = nullptr;   // diagnostics buffer [max launches][kTraceCtas][kTraceSlots]
 int g_gemm_trace_max = 0, g_gemm_trace_next = 0;
 constexpr int kTraceCtas = 1024;   // the caller marked it (the GEMM that follows the latency-bound attention kernel)
-static int g_num_sms = 0;
-static int g_smem_optin = 0;
 static PerDeviceOnce g_gemm_attr;
-
-static int device_props() {
-    if (g_num_sms) return 0;
-    int dev = 0;
-    ASD_CUDA(cudaGetDevice(&dev));
-    ASD_CUDA(cudaDeviceGetAttribute(&g_num_sms, cudaDevAttrMultiProcessorCount, dev));
-    ASD_CUDA(cudaDeviceGetAttribute(&g_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    return 0;
-}
 
 static inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
@@ -724,7 +713,8 @@ int gemm_token_tile(int M) {
 
 // Choose the split so that all CTAs fit in one co-resident wave and there are enough bytes in flight.
 int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, int reduce) {
-    if (device_props()) return -1;
+    DeviceLimits dev;
+    if (device_limits(&dev)) return -1;
     pl->reduce = ((reduce && mode == GEMM_OUT_F32) || mode == GEMM_OUT_QKV) ? 1 : 0;
     if (M <= 0 || N <= 0 || K <= 0 || (K & 7)) return set_error("gemm: need M, N, K > 0 and K %% 8 == 0");
     pl->M = M;
@@ -748,7 +738,7 @@ int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int
     if (mode != GEMM_OUT_SWIGLU && mode != GEMM_OUT_BF16) {
         // largest split that keeps every CTA co-resident in one wave with >= 4 k-blocks each; with the
         // in-cluster reduction it is a power of two <= 8 (cluster sizes that tile the GPCs evenly)
-        const int slots = g_num_sms * max_ctas_per_sm;
+        const int slots = dev.sms * max_ctas_per_sm;
         ksplit = slots / tiles;
         if (ksplit < 1) ksplit = 1;
         const int max_by_k = pl->kblocks / 4 > 0 ? pl->kblocks / 4 : 1;
@@ -762,7 +752,7 @@ int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int
     }
     if (force_ksplit > 0) ksplit = force_ksplit;
     // pipeline depth from the expected residency: fewer CTAs per SM -> deeper ring per CTA
-    int ctas_per_sm = (tiles * ksplit + g_num_sms - 1) / g_num_sms;
+    int ctas_per_sm = (tiles * ksplit + dev.sms - 1) / dev.sms;
     if (ctas_per_sm > max_ctas_per_sm) ctas_per_sm = max_ctas_per_sm;
     if (ctas_per_sm < 1) ctas_per_sm = 1;
     // headroom: leave shared memory for that many CTAs of the NEXT kernel (programmatic launch + early trigger)
@@ -796,7 +786,7 @@ int gemm_plan(GemmPlan* pl, int M, int N, int K, int mode, int force_ksplit, int
     pl->stages = stages;
     if (ksplit == 1 && mode != GEMM_OUT_QKV) pl->reduce = 0;
     pl->smem_bytes = fixed + recv_extra + stages * stage_bytes;
-    if (pl->smem_bytes > g_smem_optin) return set_error("gemm: tile does not fit in shared memory");
+    if (pl->smem_bytes > dev.smem_optin) return set_error("gemm: tile does not fit in shared memory");
     uint32_t cols = 32;
     while ((int)cols < pl->MT) cols <<= 1;
     pl->tmem_cols = cols;
@@ -822,8 +812,9 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
                 int n_valid, bool pdl, cudaStream_t stream, bool accumulate, const QkvEpilogue* qkv,
                 const NormFusion* norm, const TpFusion* tp) {
     ASD_ONCE(g_gemm_attr, {
-        if (device_props()) return -1;
-        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
+        DeviceLimits dev;
+        if (device_limits(&dev)) return -1;
+        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
         prefer_max_smem(gemm_ws_kernel<false>);
     });
     GemmArgs a;
@@ -869,7 +860,9 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
         ++g_gemm_trace_next;
     }
     if (a.trace) {      // (not before it is asked for: setting an attribute loads the kernel)
-        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_smem_optin));
+        DeviceLimits dev;
+        if (device_limits(&dev)) return -1;
+        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
         prefer_max_smem(gemm_ws_kernel<true>);
     }
     if (a.norm.sumsq_out != nullptr) {

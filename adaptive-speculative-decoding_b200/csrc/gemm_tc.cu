@@ -421,15 +421,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
 
 // ------------------------------------------------------------------------------------------- host
 static PerDeviceOnce g_tc_attr;
-static int g_tc_sms = 0, g_tc_smem_optin = 0;
 
 int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, int force_stages, bool norm, int force_mt) {
-    if (!g_tc_sms) {
-        int dev = 0;
-        ASD_CUDA(cudaGetDevice(&dev));
-        ASD_CUDA(cudaDeviceGetAttribute(&g_tc_sms, cudaDevAttrMultiProcessorCount, dev));
-        ASD_CUDA(cudaDeviceGetAttribute(&g_tc_smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-    }
+    DeviceLimits dev;
+    if (device_limits(&dev)) return -1;
     if (M <= 0 || N <= 0 || K <= 0 || (K & 7)) return set_error("gemm_tc: need M, N, K > 0 and K %% 8 == 0");
     if (mode != GEMM_OUT_F32 && mode != GEMM_OUT_SWIGLU) return set_error("gemm_tc: fp32 and SwiGLU epilogues only");
     if (M > kTcMaxTokens) return set_error("gemm_tc: at most %d tokens per call", kTcMaxTokens);
@@ -439,7 +434,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     pl->mode = mode;
     pl->w_tiles = (N + 255) / 256;
     pl->kblocks = (K + kTcBlockK - 1) / kTcBlockK;
-    const int npairs = g_tc_sms / 2;
+    const int npairs = dev.sms / 2;
     static const int env_mt = []() {
         const char* v = getenv("ASD_TC_MT");     // experiments: force the token tile
         return v ? atoi(v) : 0;
@@ -487,7 +482,7 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
     const int stage_bytes = kTcABytes + (mt / 2) * 128;
     const int fixed = 1024 + 256 + kTcXchgBytes + (norm ? std::max(4 * pl->m_tiles * mt, 8 * (kTcGroups + 1)) : 0) + 64;
     pl->norm = norm;
-    int stages = (g_tc_smem_optin - fixed) / stage_bytes;
+    int stages = (dev.smem_optin - fixed) / stage_bytes;
     if (stages > 8) stages = 8;
     if (force_stages > 0 && force_stages < stages) stages = force_stages;
     if (stages < 2) return set_error("gemm_tc: tile does not fit in shared memory");
@@ -501,7 +496,9 @@ int gemm_tc_plan(TcPlan* pl, int M, int N, int K, int mode, int force_ksplit, in
 int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap& tmap_x, void* out, int ldo, int n_valid,
                    size_t slice_stride, cudaStream_t stream, bool accumulate, const NormFusion* norm) {
     ASD_ONCE(g_tc_attr, {
-        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
+        DeviceLimits dev;
+        if (device_limits(&dev)) return -1;
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
         prefer_max_smem(gemm_tc_kernel<false>);
     });
     if (norm && !pl.norm) return set_error("gemm_tc: the plan has no place for a norm's factors");
@@ -571,12 +568,14 @@ int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream
     if (make_tmap_bf16(&tw, L.w, (uint64_t)groups * L.N, L.K, L.K, 128)) return -1;
     if (make_tmap_bf16(&tx, L.a, rows, L.K, L.K, mt / 2)) return -1;
     if (make_tmap_out(&to, L.c, L.epilogue == 1, rows, L.N, 1, L.ldc, (size_t)rows * L.ldc, 128, kTcOutTok)) return -1;
+    DeviceLimits dev;
+    if (device_limits(&dev)) return -1;
     static PerDeviceOnce once;
     ASD_ONCE(once, {
-        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, g_tc_smem_optin));
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
         prefer_max_smem(gemm_tc_kernel<true>);
     });
-    gemm_tc_kernel<true><<<g_tc_sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
+    gemm_tc_kernel<true><<<dev.sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_GROUPED);
     return 0;

@@ -7,6 +7,8 @@
 
 namespace asd {
 
+int set_error(const char* fmt, ...);     // records the message, returns -1
+
 // cudaFuncSetAttribute and module loads are per device.  `run` calls `set` on the current device until one call of it has returned 0;
 // a thread that meets another's call waits for its end, so that no first launch overtakes the attribute it needs.
 class PerDeviceOnce {
@@ -38,5 +40,27 @@ private:
             }))                              \
             return -1;                       \
     } while (0)
+
+struct DeviceLimits {
+    int sms = 0, smem_optin = 0;         // multiprocessors; shared memory that a block may ask for
+};
+
+// of the current device: no thread sees one of them without the other
+inline int device_limits(DeviceLimits* out) {
+    static PerDeviceOnce once;
+    static DeviceLimits known[64];
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    DeviceLimits& d = known[dev & 63];
+    if (e == cudaSuccess)
+        once.run([&]() -> int {
+            e = cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&d.smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+            return e == cudaSuccess ? 0 : -1;
+        });
+    if (e != cudaSuccess) return set_error("the device's limits cannot be read: %s", cudaGetErrorString(e));
+    *out = d;
+    return 0;
+}
 
 }  // namespace asd

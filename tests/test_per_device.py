@@ -2,6 +2,8 @@
 import os
 import subprocess
 
+import pytest
+
 CSRC = os.path.join(os.path.dirname(__file__), "..", "adaptive-speculative-decoding_b200", "csrc")
 
 PROGRAM = r"""
@@ -13,6 +15,8 @@ PROGRAM = r"""
 
 static thread_local int device = 0;
 extern "C" cudaError_t cudaGetDevice(int* d) { *d = device; return cudaSuccess; }
+extern "C" const char* cudaGetErrorString(cudaError_t) { return "fake"; }
+namespace asd { int set_error(const char*, ...) { return -1; } }
 static void slowly() { std::this_thread::sleep_for(std::chrono::milliseconds(20)); }
 
 static std::atomic<int> calls{0}, ready[2], overtook{0};
@@ -31,24 +35,53 @@ static int fails_once() {
     ASD_ONCE(failing, if (++tries == 1) return -1);
     return 0;
 }
-int main() {
+static std::atomic<int> asked{0}, half{0};
+extern "C" cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr attr, int dev) {
+    asked.fetch_add(1);
+    slowly();
+    if (dev == 2 && half.load() < 2) return cudaErrorUnknown;       // a device that cannot be read at first
+    *v = (attr == cudaDevAttrMultiProcessorCount ? 100 : 1000) + dev;
+    return cudaSuccess;
+}
+static void limits() {
+    asd::DeviceLimits d;
+    if (asd::device_limits(&d) || d.sms != 100 + device || d.smem_optin != 1000 + device) half.fetch_add(1);
+}
+template <typename F>
+static void threads(F f) {
     std::vector<std::thread> all;
-    for (int i = 0; i < 16; ++i) all.emplace_back([i] { device = i & 1; launch(once); });
+    for (int i = 0; i < 16; ++i) all.emplace_back([i, f] { device = i & 1; f(); });
     for (auto& t : all) t.join();
+}
+int main() {
+    threads([] { launch(once); });
     const int first = fails_once(), second = fails_once(), third = fails_once();
     printf("%d %d %d %d %d %d\n", calls.load(), overtook.load(), first, second, third, tries);
+    threads(limits);
+    printf("%d %d", asked.load(), half.load());
+    half = 0;
+    device = 2;
+    for (int i = 0; i < 4; ++i) limits();
+    printf(" %d\n", half.load());
 }
 """
 
 
-def run(tmp_path, program):
-    src, exe = tmp_path / "t.cpp", tmp_path / "t"
-    src.write_text(program)
+@pytest.fixture(scope="module")
+def lines(tmp_path_factory):
+    tmp = tmp_path_factory.mktemp("per_device")
+    src, exe = tmp / "t.cpp", tmp / "t"
+    src.write_text(PROGRAM)
     include = os.path.join(os.environ.get("CUDA_HOME", "/usr/local/cuda"), "include")
     subprocess.run(["g++", "-std=c++17", "-pthread", "-I", include, "-I", CSRC, str(src), "-o", str(exe)], check=True)
-    return subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=60).stdout.split()
+    return subprocess.run([str(exe)], check=True, capture_output=True, text=True, timeout=60).stdout.splitlines()
 
 
-def test_no_thread_goes_on_before_the_first_has_finished(tmp_path):
+def test_no_thread_goes_on_before_the_first_has_finished(lines):
     """one call per device, nobody ahead of it; a call that failed is made again"""
-    assert run(tmp_path, PROGRAM) == ["2", "0", "-1", "0", "0", "2"]
+    assert lines[0].split() == ["2", "0", "-1", "0", "0", "2"]
+
+
+def test_no_thread_sees_half_of_a_devices_limits(lines):
+    """two questions a device, both answers for everyone; a device that could not be read is asked again"""
+    assert lines[1].split() == ["4", "0", "2"]
