@@ -551,8 +551,11 @@ int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     if (g_attn_trace && g_attn_trace_next < g_attn_trace_max && (long long)tiles * L.nseq * L.nkv * L.nsplit_max <= 1024)
         a.trace = g_attn_trace + (size_t)(g_attn_trace_next++) * 1024 * 16;
     if (a.trace) {      // (not before it is asked for: setting an attribute loads the kernel)
-        ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-        prefer_max_smem(attn_tc_kernel<true>);
+        static PerDeviceOnce traced;
+        ASD_ONCE(traced, {
+            if (allow_max_smem(attn_tc_kernel<true>)) return -1;
+            prefer_max_smem(attn_tc_kernel<true>);
+        });
     }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];

@@ -860,10 +860,11 @@ int gemm_launch(const GemmPlan& pl, const CUtensorMap& tmap_w, const CUtensorMap
         ++g_gemm_trace_next;
     }
     if (a.trace) {      // (not before it is asked for: setting an attribute loads the kernel)
-        DeviceLimits dev;
-        if (device_limits(&dev)) return -1;
-        ASD_CUDA(cudaFuncSetAttribute(gemm_ws_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
-        prefer_max_smem(gemm_ws_kernel<true>);
+        static PerDeviceOnce traced;
+        ASD_ONCE(traced, {
+            if (allow_max_smem(gemm_ws_kernel<true>)) return -1;
+            prefer_max_smem(gemm_ws_kernel<true>);
+        });
     }
     if (a.norm.sumsq_out != nullptr) {
         if (!pl.reduce || pl.mode != GEMM_OUT_F32)

@@ -784,7 +784,8 @@ int launch_tiled_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int
         if (nsplit > 64) nsplit = 64;
     }
     auto fn = latent_attn_tiled<T, RPT, RC>;
-    ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static PerDeviceOnce once;
+    ASD_ONCE(once, if (allow_max_smem(fn)) return -1);
     dim3 grid(q_tiles, nseq * nsplit, hgs);
     const int vec = sizeof(T) == 2 && (rw & 7) == 0 && (reinterpret_cast<uintptr_t>(cache.pool) & 15) == 0;
     ASD_CUDA(launch_pdl(fn, grid, 256, smem, stream, ix, cu_q, seq_slot, TQ, HG, nsplit, vec, q_lat, d, cache, out_lat,
@@ -826,7 +827,8 @@ int launch_mma_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int n
         if (nsplit < 1) nsplit = 1;
         if (nsplit > 64) nsplit = 64;
     }
-    ASD_CUDA(cudaFuncSetAttribute(latent_attn_mma<MT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static PerDeviceOnce once;
+    ASD_ONCE(once, if (allow_max_smem(latent_attn_mma<MT>)) return -1);
     dim3 grid(q_tiles, nseq * nsplit, hgs);
     ASD_CUDA(launch_pdl(latent_attn_mma<MT>, grid, 256, smem, stream, ix, cu_q, seq_slot, TQ, HG, nsplit, q_lat, d, cache,
                         out_lat, ws.o, ws.ml));
@@ -884,7 +886,8 @@ int launch_attn_t(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int 
 #define ASD_LAT_CASE(A)                                                                                              \
     {                                                                                                                \
         auto fn = latent_attn_kernel<T, A>;                                                                          \
-        if (smem > 48 * 1024) ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); \
+        static PerDeviceOnce once;                                                                                   \
+        ASD_ONCE(once, if (allow_max_smem(fn)) return -1);                                                           \
         ASD_CUDA(launch_pdl(fn, grid, warps * 32, smem, stream, ix, cu_q, seq_slot, TQ, HG, q_lat, d, cache, out_lat));                \
     }
     if (smem > 220 * 1024) return set_error("latent attention: latent + rotated size %d does not fit shared memory", rw);

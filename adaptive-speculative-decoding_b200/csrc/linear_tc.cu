@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kThreads) tc_linear_kernel(SimtLinear L, int M
 template <typename TA, typename TC>
 int launch_t(const SimtLinear& L, dim3 grid, int MT, uint32_t cols, size_t smem, int* err, cudaStream_t s) {
     auto fn = tc_linear_kernel<TA, TC>;
-    ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static PerDeviceOnce once;
+    ASD_ONCE(once, if (allow_max_smem(fn)) return -1);
     fn<<<grid, kThreads, smem, s>>>(L, MT, cols, err);
     return 0;
 }

@@ -63,4 +63,17 @@ inline int device_limits(DeviceLimits* out) {
     return 0;
 }
 
+// lets launches of fn ask for all the shared memory that its static part leaves.  Once per device: set to each launch's own size, a
+// smaller launch on another thread takes it back before a larger one has started.
+template <typename F>
+int allow_max_smem(F* fn) {
+    DeviceLimits dev;
+    cudaFuncAttributes fa;
+    if (device_limits(&dev)) return -1;
+    cudaError_t e = cudaFuncGetAttributes(&fa, fn);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin - (int)fa.sharedSizeBytes);
+    return e == cudaSuccess ? 0 : set_error("shared memory of a kernel: %s", cudaGetErrorString(e));
+}
+
 }  // namespace asd

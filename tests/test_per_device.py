@@ -1,5 +1,6 @@
 """What host code does once per device (csrc/per_device.h), under several host threads: built with g++ against fake runtime calls."""
 import os
+import re
 import subprocess
 
 import pytest
@@ -85,3 +86,18 @@ def test_no_thread_goes_on_before_the_first_has_finished(lines):
 def test_no_thread_sees_half_of_a_devices_limits(lines):
     """two questions a device, both answers for everyone; a device that could not be read is asked again"""
     assert lines[1].split() == ["4", "0", "2"]
+
+
+def test_every_size_of_shared_memory_is_allowed_once():
+    """no launch sets the attribute to its own size: a smaller launch on another thread would take it back in between"""
+    for name in sorted(os.listdir(CSRC)):
+        if not name.endswith((".cu", ".cuh", ".h")) or name == "per_device.h":
+            continue
+        text = open(os.path.join(CSRC, name)).read()
+        for m in re.finditer(r"cudaFuncSetAttribute\([^;]*MaxDynamicSharedMemorySize|allow_max_smem\(", text):
+            before = text[:m.start()]
+            opened = max(before.rfind(word) for word in ("ASD_ONCE(", "call_once("))
+            depth = 0
+            for ch in before[opened:]:
+                depth += (ch == "(") - (ch == ")")
+            assert opened >= 0 and depth > 0, (name, text.count("\n", 0, m.start()) + 1)
