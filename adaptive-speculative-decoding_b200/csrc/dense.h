@@ -1,6 +1,6 @@
 // Dense projection of an engine's activations, y fp32 [M][ldc] = x [M][K] * w[N][K]^T, routed by shape and element
 // type: the weight-streaming tcgen05 GEMM (gemm.cu) for bf16 operands it accepts, its tensor-bound CTA-pair form
-// (gemm_tc.cu) above 256 tokens, of larger matrices above 160, the CUDA-core kernel (linear_simt.cu) for fp32 engines and every other
+// (gemm_tc.cu) above 256 tokens, of larger matrices whose rows are not too long above 160, the CUDA-core kernel (linear_simt.cu) for fp32 engines and every other
 // shape.  Plans and tensor maps are cached per (call site, token count); a call site always passes the same buffers.
 #pragma once
 #include <cuda.h>
@@ -28,13 +28,15 @@ struct DenseRunner {
 
     void clear() { cache.clear(); }
 
-    // Above 160 tokens the weight-streaming kernel has room for fewer blocks of its wider tiles (a step of three Rivetar layers of
-    // width 2048, 160 tokens 511 us, 192 590; on CTA pairs 557 and 574, of width 4096 707, 1005 and 892, 919, a Mezilix layer of
-    // width 4096 348, 397 and 362, 370).  Of matrices below 4M elements the pairs gain less than their plain launches cost (Rivetar
-    // of width 1024, 192 tokens: 389 and 416).
+    // Above 160 tokens the weight-streaming kernel has room for fewer blocks of its wider tiles, and CTA pairs are the better form of
+    // a matrix of 4M elements whose rows are no longer than it has of them.  The pairs take K in one slice here, 5.4 us per 1024 of it
+    // however few their tiles are: longer rows stay with the weight-streaming kernel, which splits them over a cluster.  161 tokens, us
+    // alone, weight-streaming and pairs: 2048 x 2048 22.6, 18.5; 6144 x 2048 28.6, 18.5; 4096 x 4096 39.5, 29.1; 12288 x 4096 51.3,
+    // 30.9; but 1024 x 4096 14.4, 28.8; 2048 x 6144 28.8, 39.6; 512 x 8192 16.5, 51.2; 4096 x 12288 60.0, 73.9 (256 tokens 70.6, 74.1).
+    // Below 4M elements the pairs gain less than their plain launches cost in a step.
     bool pair_from(int M, int N, int K) const {
         if (tc_min_rows > 0) return M >= tc_min_rows;
-        return M > 256 || (M > 160 && (long long)N * K >= 1 << 22);
+        return M > 256 || (M > 160 && (long long)N * K >= 1 << 22 && K <= N);
     }
 
     int run(const void* x, const void* w, float* y, int M, int N, int K, int ldc, int key, cudaStream_t s) {

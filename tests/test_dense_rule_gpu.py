@@ -29,3 +29,19 @@ def test_larger_matrices_take_pairs_from_161_tokens(length, pairs):
         close(eng)
     # the same bf16 operands, fp32 sums in another order: a rounding of the activations apart
     assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() < 1e-2
+
+
+@pytest.mark.parametrize("length,pairs", [(161, 1), (256, 1), (257, 3)])
+def test_long_rows_stay_with_the_weight_streaming_kernel(length, pairs):
+    """up projection 4096 x 1024 on pairs, down projection 1024 x 4096 (as many elements, four times the K of one slice) not before
+    257 tokens"""
+    from asd_b200._lib import lib
+    cfg = config([gla(heads=1, dim=16, vdim=16, ff=4096)], width=1024)
+    w = O.random_model(cfg, seed=73)
+    eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512)
+    slot = eng.open_sequence()
+    eng.reserve(slot, length)
+    before = lib().asd_kernel_launches(b"gemm_pair")
+    eng.forward_ragged([(slot, 0, tokens(length, 96, 74), [length - 1])])
+    assert lib().asd_kernel_launches(b"gemm_pair") - before == pairs
+    close(eng)
