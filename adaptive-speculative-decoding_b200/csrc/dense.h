@@ -6,6 +6,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <unordered_map>
 
@@ -28,6 +29,21 @@ struct DenseRunner {
 
     void clear() { cache.clear(); }
 
+    // the engines' options that are this runner's; false: another's
+    bool set_option(const char* name, int value) {
+        if (!strcmp(name, "tc_linear")) {
+            tc_linear = value;
+        } else if (!strcmp(name, "linear_few")) {
+            few = value;
+        } else if (!strcmp(name, "tc_min_rows")) {
+            tc_min_rows = value > 0 ? value : 1 << 30;
+            clear();
+        } else {
+            return false;
+        }
+        return true;
+    }
+
     // Above 160 tokens the weight-streaming kernel has room for fewer blocks of its wider tiles, and CTA pairs are the better form of
     // a matrix of 4M elements whose rows are no longer than it has of them.  The pairs take K in one slice here, 5.4 us per 1024 of it
     // however few their tiles are: longer rows stay with the weight-streaming kernel, which splits them over a cluster.  161 tokens, us
@@ -43,7 +59,8 @@ struct DenseRunner {
         if (!f32 && tc_linear && (K % 8) == 0 && (ldc % 4) == 0 && K >= 64 && N >= 8 &&
             (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-            if (few && linear_few_takes(x, w, M, N, K)) return launch_linear_few(x, w, y, M, N, K, ldc, s);
+            const bool asked_for_pairs = tc_min_rows > 0 && M >= tc_min_rows;
+            if (few && !asked_for_pairs && linear_few_takes(x, w, M, N, K)) return launch_linear_few(x, w, y, M, N, K, ldc, s);
             const unsigned long long k = ((unsigned long long)key << 32) | (unsigned)M;
             auto it = cache.find(k);
             if (it == cache.end()) {

@@ -355,15 +355,7 @@ int asd_lukopel_set_option(asd_lukopel_engine_t* h, const char* name, int value)
     LkEngine* e = static_cast<LkEngine*>(h);
     if (!e || !name) return set_error("asd_lukopel_set_option: NULL argument");
     if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
-    if (!strcmp(name, "tc_linear")) {
-        e->dn.tc_linear = value;
-        return 0;
-    }
-    if (!strcmp(name, "tc_min_rows")) {
-        e->dn.tc_min_rows = value > 0 ? value : 1 << 30;
-        e->dn.clear();
-        return 0;
-    }
+    if (e->dn.set_option(name, value)) return 0;
     if (!strcmp(name, "attn_general")) {
         e->attn_ws.mode = value ? 1 : 0;
         return 0;

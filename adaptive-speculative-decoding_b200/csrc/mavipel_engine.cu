@@ -582,15 +582,7 @@ int asd_mavipel_set_option(asd_mavipel_engine_t* h, const char* name, int value)
     MvEngine* e = static_cast<MvEngine*>(h);
     if (!e || !name) return set_error("asd_mavipel_set_option: NULL argument");
     if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
-    if (!strcmp(name, "tc_linear")) {
-        e->dn.tc_linear = value;
-        return 0;
-    }
-    if (!strcmp(name, "tc_min_rows")) {
-        e->dn.tc_min_rows = value > 0 ? value : 1 << 30;
-        e->dn.clear();
-        return 0;
-    }
+    if (e->dn.set_option(name, value)) return 0;
     if (!strcmp(name, "attn_mma")) {
         e->attn_ws.tiled = value;
         return 0;

@@ -578,15 +578,7 @@ int asd_nobonex_set_option(asd_nobonex_engine_t* h, const char* name, int value)
     NbEngine* e = static_cast<NbEngine*>(h);
     if (!e || !name) return set_error("asd_nobonex_set_option: NULL argument");
     if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
-    if (!strcmp(name, "tc_linear")) {
-        e->dn.tc_linear = value;
-        return 0;
-    }
-    if (!strcmp(name, "tc_min_rows")) {
-        e->dn.tc_min_rows = value > 0 ? value : 1 << 30;
-        e->dn.clear();
-        return 0;
-    }
+    if (e->dn.set_option(name, value)) return 0;
     if (!strcmp(name, "attn_general")) {
         e->attn_ws.mode = value;
         return 0;

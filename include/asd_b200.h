@@ -316,7 +316,7 @@ ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_p
 /* options: "tc_linear" (1, default: bf16 projections whose shape the tcgen05 kernels accept run on them; 0: CUDA-core
  * kernel everywhere), "tc_min_rows" (token count from which dense projections use the tensor-bound CTA-pair GEMM; 0 = never;
  * left alone: 257, 161 for matrices of 4M elements on with no more columns than rows), "linear_few" (1, default: up to 16 tokens on matrices up to 64 MB run
- * linear_few.cu), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
+ * linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
  * rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
  * per (token, head)), "profile" (1: CUDA events around every launch, read with asd_mezilix_profile_read) */
@@ -485,7 +485,7 @@ ASD_API size_t asd_mavipel_cache_bytes(const asd_mavipel_engine_t* e, int num_pa
 ASD_API size_t asd_mavipel_state_bytes(const asd_mavipel_engine_t* e, int max_seqs);
 ASD_API int asd_mavipel_set_cache(asd_mavipel_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows" as for the Mezilix engine; "attn_mma" (1, default: prompts and portions of a bf16
+/* options: "tc_linear", "tc_min_rows", "linear_few" as for the Mezilix engine; "attn_mma" (1, default: prompts and portions of a bf16
  * engine take the tensor-core window attention where the sizes allow; 0: always the CUDA-core kernel); "profile" */
 ASD_API int asd_mavipel_set_option(asd_mavipel_engine_t* e, const char* name, int value);
 /* Same arguments as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [runs][M][width]) receives the
@@ -552,7 +552,7 @@ ASD_API size_t asd_lukopel_cache_bytes(const asd_lukopel_engine_t* e, int num_pa
 ASD_API size_t asd_lukopel_state_bytes(const asd_lukopel_engine_t* e, int max_seqs);   /* 0: the cache is all */
 ASD_API int asd_lukopel_set_cache(asd_lukopel_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows" as for the Mezilix engine; "attn_general" (1: every attention runs the general
+/* options: "tc_linear", "tc_min_rows", "linear_few" as for the Mezilix engine; "attn_general" (1: every attention runs the general
  * CUDA-core kernels; 0, default: steps of few tokens and, in a bf16 engine, prompts on the tensor cores take kernels of
  * their own where the sizes allow); "profile" */
 ASD_API int asd_lukopel_set_option(asd_lukopel_engine_t* e, const char* name, int value);
@@ -635,7 +635,7 @@ ASD_API size_t asd_dikopel_cache_bytes(const asd_dikopel_engine_t* e, int num_pa
 ASD_API size_t asd_dikopel_state_bytes(const asd_dikopel_engine_t* e, int max_seqs);
 ASD_API int asd_dikopel_set_cache(asd_dikopel_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows" as for the Mezilix engine; "attn_general" as for the Lukopel engine; "profile" */
+/* options: "tc_linear", "tc_min_rows", "linear_few" as for the Mezilix engine; "attn_general" as for the Lukopel engine; "profile" */
 ASD_API int asd_dikopel_set_option(asd_dikopel_engine_t* e, const char* name, int value);
 /* Same arguments as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [n_layers][M][width]) receives the
  * stream that leaves every layer. */
@@ -712,7 +712,7 @@ ASD_API size_t asd_nobonex_cache_bytes(const asd_nobonex_engine_t* e, int num_pa
 ASD_API size_t asd_nobonex_state_bytes(const asd_nobonex_engine_t* e, int max_seqs);
 ASD_API int asd_nobonex_set_cache(asd_nobonex_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows", "attn_general", "profile" as for the Dikopel engine; "ssd_mode" 0: prompts of a bf16
+/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_general", "profile" as for the Dikopel engine; "ssd_mode" 0: prompts of a bf16
  * engine run the recurrence chunk by chunk on the tensor cores, 1: position by position in fp32 */
 ASD_API int asd_nobonex_set_option(asd_nobonex_engine_t* e, const char* name, int value);
 /* Same arguments as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [n_layers][M][width]) receives the

@@ -1,4 +1,4 @@
-"""GPU: which dense projections of a family's engine run on CTA pairs, by tokens and matrix size."""
+"""GPU: which kernel a dense projection of a family's engine runs on, by tokens, matrix size and options."""
 import pytest
 import torch
 
@@ -45,3 +45,35 @@ def test_long_rows_stay_with_the_weight_streaming_kernel(length, pairs):
     eng.forward_ragged([(slot, 0, tokens(length, 96, 74), [length - 1])])
     assert lib().asd_kernel_launches(b"gemm_pair") - before == pairs
     close(eng)
+
+
+@pytest.mark.parametrize("family", ["Mezilix", "Rivetar", "Mavipel", "Lukopel", "Dikopel", "Nobonex"])
+def test_options_of_dense_projections_hold_for_few_tokens(family):
+    """8 tokens of every family's engine: the few-token kernel, without it, and CTA pairs where they are asked for"""
+    import importlib
+    from asd_b200 import engine
+    from asd_b200._lib import lib
+    model = importlib.import_module(f"asd_b200.models.{family.lower()}")
+    cfg = model.sized_config(256, 3, 2, vocab=512)
+    eng = getattr(engine, family + "Engine")(cfg, max_seqs=8, max_seq_len=64, max_tokens=64).load_random(seed=5)
+    slots = torch.arange(8, dtype=torch.int32, device="cuda")
+    ids = torch.randint(0, 512, (8, 1), generator=torch.Generator().manual_seed(6), dtype=torch.int32).cuda()
+
+    def launches(**options):
+        for name, value in options.items():
+            eng.set_option(name, value)
+        names = (b"linear_few", b"gemm", b"gemm_pair")
+        before = [lib().asd_kernel_launches(n) for n in names]
+        out = eng.forward_uniform(ids, torch.zeros(8, dtype=torch.int32, device="cuda"), slots, 1).double()
+        return [lib().asd_kernel_launches(n) - b for n, b in zip(names, before)], out
+    (few, stream, pairs), a = launches()
+    assert few > 0 and pairs == 0
+    count, b = launches(linear_few=0)
+    assert count == [0, stream + few, 0]
+    count, c = launches(linear_few=1, tc_min_rows=9)
+    assert count == [few, stream, 0]
+    count, d = launches(tc_min_rows=8)
+    assert count == [0, 0, stream + few]
+    # the same bf16 operands, fp32 sums in another order: a rounding of the activations apart
+    assert max(((x - a).norm() / a.norm()).item() for x in (b, c, d)) < 2e-2
+    eng.close()
