@@ -1,9 +1,9 @@
 // Gated linear attention: a recurrence with a [dk][dv] state per head and a decay per key channel,
 //   S_t = diag(alpha_t) S_(t-1) + k_t v_t^T,   o_t = S_t^T q_t,   alpha_t = sigmoid(z_t)^(1 / tau).
 // gla_decay_kernel:  alpha from the inner decay projection (a thread has 1 or 4 channels of 8 tokens, fp32).
-// gla_recurrence_kernel: one CTA per (sequence, head, 32 value columns).  Columns of S never mix, so a CTA owns its
+// gla_recurrence_kernel: one CTA per (sequence, head, 32 value columns, or 16).  Columns of S never mix, so a CTA owns its
 //   columns for the whole run of new positions: a thread keeps 8 key rows x 4 columns of the state in registers.  The
-//   new positions are staged CH at a time in shared memory (q, k, decay rows and the CTA's 32 value columns) by
+//   new positions are staged CH at a time in shared memory (q, k, decay rows and the CTA's value columns) by
 //   cp.async, one chunk ahead; per position every thread updates its part and forms its rows' share of o, and after the
 //   chunk the shares are added in index order.  The arithmetic per position is the same whatever the chunking or the
 //   batch, so a sequence's outputs do not depend on how its tokens were cut into forwards.
@@ -25,8 +25,6 @@ namespace {
 
 constexpr int GLA_R = 8;     // key rows of the state per thread
 constexpr int GLA_C = 4;     // and columns
-constexpr int GLA_COLS = 32; // value columns per CTA
-constexpr int GLA_CG = GLA_COLS / GLA_C;
 
 __device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
     const unsigned addr = (unsigned)__cvta_generic_to_shared(dst);
@@ -129,24 +127,30 @@ struct Staged {                         // one position's values for a thread: i
 // brought 12 bytes per element into registers, 780 clocks on an SM with two CTAs; with 8 rows x 4 columns it is 3.5, below the
 // arithmetic, which runs on packed pairs of rows.  3 prompts of up to 777 positions, 16 heads of 128 x 128: 321 -> 174 us
 // (436 clocks a position where an SM has two of the 192 CTAs, 245 where it has one; fp32 pipe 0.54 busy on the former).
-// Rows beyond dk are staged as zeros and take no k v^T (an infinite v times zero would be NaN): they add nothing.  `vec`: sizes and addresses allow 16-byte
-// copies.  MAXT: threads at most (8 per 8 key rows); PIPE: loads a position ahead.
-template <int MAXT, int MINB, bool PIPE>
+// Rows beyond dk are staged as zeros and take no k v^T (an infinite v times zero would be NaN): they add nothing.  A thread that has
+// nothing but such rows does what its warp does, and nobody reads its share: had it a loop of its own, a warp of key size 16 or 24
+// would walk every position twice (2 sequences of 500, 4 heads of 24 x 40: 162 us so, now 101).  `vec`: sizes and addresses allow
+// 16-byte copies.  MAXT: threads at most (COLS / 4 per 8 key rows); PIPE: loads a position ahead.
+template <int MAXT, int MINB, bool PIPE, int COLS = 32>
 __global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix, const int* cu_q, const int* seq_slot, const float* q,
                                                               const float* k, const float* v, long long ld, const float* alpha,
                                                               GlaDims d, float* state, int ring, float* out, int CH, int vec) {
     pdl_enter();
+    constexpr int CG = COLS / GLA_C;                    // column groups
     extern __shared__ __align__(16) float sm[];
-    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * GLA_COLS;
+    const int seq = blockIdx.x, head = blockIdx.y, col0 = blockIdx.z * COLS;
     const int t0 = cu_q[seq], t1 = cu_q[seq + 1];
     if (t0 >= t1) return;
-    const int tid = threadIdx.x, nthr = blockDim.x, RG = nthr / GLA_CG;
+    const int tid = threadIdx.x, nthr = blockDim.x, RG = nthr / CG;
     const int dkp = RG * GLA_R;                         // padded key size
-    const int rg = tid / GLA_CG, r0 = rg * GLA_R, ca = tid % GLA_CG * GLA_C;   // the thread's rows and columns
+    const int rg = tid / CG, r0 = rg * GLA_R, ca = tid % CG * GLA_C;   // the thread's rows and columns
+    const int live = (d.dk + GLA_R - 1) / GLA_R;        // row groups that hold a row; what the others compute is used by nobody
+    // no thread of the warp has rows on both sides of dk
+    const bool whole = __all_sync(0xffffffffu, r0 + GLA_R <= d.dk || r0 >= d.dk);
     const int slot = seq_slot[seq];
     const int p0 = ix.positions[t0];
-    // shared: two buffers of { q, k, decay [CH][dkp] each, v [CH][32] }, then the shares of o [RG][CH][32]
-    const int buf_elems = 3 * CH * dkp + CH * GLA_COLS, share = CH * GLA_COLS;
+    // shared: two buffers of { q, k, decay [CH][dkp] each, v [CH][COLS] }, then the shares of o [RG][CH][COLS]
+    const int buf_elems = 3 * CH * dkp + CH * COLS, share = CH * COLS;
     float* part = sm + 2 * buf_elems;
     const long long st_entry = (long long)d.heads * d.dk * d.dv;
     float* st_cta = state + (long long)slot * ring * st_entry + (long long)head * d.dk * d.dv + col0;
@@ -200,14 +204,14 @@ __global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix,
     auto fetch_w = [&](int buf, int c0, auto width) {
         constexpr int W = decltype(width)::value;
         const int nt = min(CH, t1 - c0), per = dkp / W;
-        for (int i = tid; i < 3 * per + GLA_COLS / W; i += nthr) {
+        for (int i = tid; i < 3 * per + COLS / W; i += nthr) {
             const int arr = i >= 2 * per ? (i >= 3 * per ? 3 : 2) : (i >= per ? 1 : 0);
             const int c = (i - arr * per) * W;
             const bool ok = arr == 3 ? col0 + c < d.dv : c < d.dk;
             const long long step = arr == 2 ? n_alpha : ld;
             const float* src = arr == 0 ? q : (arr == 1 ? k : (arr == 2 ? alpha : v));
             if (ok) src += c0 * step + (arr == 3 ? hv + col0 + c : hq + c);
-            const int width_s = arr == 3 ? GLA_COLS : dkp;
+            const int width_s = arr == 3 ? COLS : dkp;
             float* dst = sm + buf * buf_elems + arr * CH * dkp + c;
             for (int t = 0; t < nt; ++t) {              // places beyond the chunk's positions are never read
                 if constexpr (W == 4)
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix,
                 *reinterpret_cast<float4*>(&x.k[2 * i]) = *reinterpret_cast<const float4*>(qs + CH * dkp + t * dkp + 4 * i);
                 *reinterpret_cast<float4*>(&x.q[2 * i]) = *reinterpret_cast<const float4*>(qs + t * dkp + 4 * i);
             }
-            *reinterpret_cast<float4*>(x.v) = *reinterpret_cast<const float4*>(vs + t * GLA_COLS + ca);
+            *reinterpret_cast<float4*>(x.v) = *reinterpret_cast<const float4*>(vs + t * COLS + ca);
         };
         auto position = [&](int t, const Staged& x, auto beyond) {
             float o[GLA_C];
@@ -268,32 +272,38 @@ __global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix,
                 }
                 o[c] = s.x + s.y;
             }
-            *reinterpret_cast<float4*>(ps + t * GLA_COLS + ca) = make_float4(o[0], o[1], o[2], o[3]);
+            *reinterpret_cast<float4*>(ps + t * COLS + ca) = make_float4(o[0], o[1], o[2], o[3]);
         };
         // the last `ring` new positions leave their state behind
         const int quiet = min(nt, max(0, t1 - ring - c0));
         int t = 0;
-        if (PIPE && r0 + GLA_R <= d.dk && quiet > 0) {
-            // the next position's values are on their way while this one's are used (one past the last reads what is there, in
-            // bounds, for nothing); a share's store would otherwise hold its loads back
-            Staged x0, x1;
-            load(0, x0);
-            for (; t + 1 < quiet; t += 2) {
-                load(t + 1, x1);
-                position(t, x0, std::false_type{});
-                load(t + 2, x0);
-                position(t + 1, x1, std::false_type{});
-            }
-            if (t < quiet) position(t++, x0, std::false_type{});
-        }
-        if (!PIPE && r0 + GLA_R <= d.dk) {
+        auto run = [&](auto beyond) {
+            if constexpr (PIPE) {
+                // the next position's values are on their way while this one's are used (one past the last reads what is there, in
+                // bounds, for nothing); a share's store would otherwise hold its loads back
+                if (quiet <= 0) return;
+                Staged x0, x1;
+                load(0, x0);
+                for (; t + 1 < quiet; t += 2) {
+                    load(t + 1, x1);
+                    position(t, x0, beyond);
+                    load(t + 2, x0);
+                    position(t + 1, x1, beyond);
+                }
+                if (t < quiet) position(t++, x0, beyond);
+            } else {
 #pragma unroll 1
-            for (; t < quiet; ++t) {
-                Staged x;
-                load(t, x);
-                position(t, x, std::false_type{});
+                for (; t < quiet; ++t) {
+                    Staged x;
+                    load(t, x);
+                    position(t, x, beyond);
+                }
             }
-        }
+        };
+        if (whole)
+            run(std::false_type{});
+        else
+            run(std::true_type{});
 #pragma unroll 1
         for (; t < nt; ++t) {
             Staged x;
@@ -302,12 +312,12 @@ __global__ void __launch_bounds__(MAXT, MINB) gla_recurrence_kernel(SeqIndex ix,
             if (t >= quiet) copy_state(st_cta + (long long)((p0 + (c0 + t - t0)) % ring) * st_entry, true);
         }
         __syncthreads();   // the chunk is consumed (its buffer may be refilled) and the shares are complete
-        for (int i = tid; i < nt * (GLA_COLS / 4); i += nthr) {
-            const int tt = i >> 3, c = (i & 7) * 4;
+        for (int i = tid; i < nt * CG; i += nthr) {
+            const int tt = i / CG, c = i % CG * GLA_C;
             if (col0 + c >= d.dv) continue;
             float4 o = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int w = 0; w < RG; ++w) {
-                const float4 x = *reinterpret_cast<const float4*>(part + w * share + tt * GLA_COLS + c);
+            for (int w = 0; w < live; ++w) {
+                const float4 x = *reinterpret_cast<const float4*>(part + w * share + tt * COLS + c);
                 o.x += x.x, o.y += x.y, o.z += x.z, o.w += x.w;
             }
             o.x *= d.q_scale, o.y *= d.q_scale, o.z *= d.q_scale, o.w *= d.q_scale;
@@ -403,25 +413,32 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     if (ix.M <= 0 || nseq <= 0) return 0;
     if (d.dk <= 0 || d.dk > 1024) return set_error("gla: key size %d outside 1..1024", d.dk);
     if (ring <= 0 || !state) return set_error("gla: no state");
-    const int threads = ((d.dk + GLA_R - 1) / GLA_R * GLA_CG + 31) / 32 * 32, RG = threads / GLA_CG, dkp = RG * GLA_R;
+    const int groups = (d.dk + GLA_R - 1) / GLA_R, run = (ix.M + nseq - 1) / nseq;
+    // 32 columns a CTA; steps of large heads 16, so that an SM holds several (64 single tokens, 4 heads of 512 x 512: one CTA of 512
+    // threads per SM 252 us, two 150, four of 256 threads 136; 1 head of 1024 x 1024: one of 1024 threads 177, two of 512 152)
+    const int cols = groups > 32 && run <= 1 ? 16 : 32, cg = cols / GLA_C;
+    const int threads = (groups * cg + 31) / 32 * 32, RG = threads / cg, dkp = RG * GLA_R;
     // chunks as long as two (large heads: one) staged CTAs per SM allow, and no longer than the runs: a step's CTAs are then
     // small enough for an SM to hold all that its registers can
     int ch = dkp <= 128 ? 16 : (dkp <= 512 ? 8 : 4);
-    const int run = (ix.M + nseq - 1) / nseq;
     ch = std::min(ch, run <= 1 ? 1 : std::max(4, run));
-    const size_t smem = (size_t)(2 * (3 * ch * dkp + ch * GLA_COLS) + RG * ch * GLA_COLS) * sizeof(float);
-    const dim3 grid(nseq, d.heads, (d.dv + GLA_COLS - 1) / GLA_COLS);
+    const size_t smem = (size_t)(2 * (3 * ch * dkp + ch * cols) + RG * ch * cols) * sizeof(float);
+    const dim3 grid(nseq, d.heads, (d.dv + cols - 1) / cols);
     if (grid.y > 65535 || grid.z > 65535) return set_error("gla: too many heads or value columns");
     const uintptr_t at = reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) | reinterpret_cast<uintptr_t>(v) |
                          reinterpret_cast<uintptr_t>(alpha) | reinterpret_cast<uintptr_t>(state) | reinterpret_cast<uintptr_t>(out);
     const int vec = (at & 15) == 0 && ld % 4 == 0 && d.dk % 4 == 0 && d.dv % 4 == 0;
-    // steps: no loads ahead, and the registers of four (key sizes up to 128: eight) CTAs per SM
-    auto fn = threads > 512 ? gla_recurrence_kernel<1024, 1, false>
-                            : (threads > 256 ? gla_recurrence_kernel<512, 1, true>
-                                             : (ch == 1 ? gla_recurrence_kernel<256, 4, false> : gla_recurrence_kernel<256, 2, true>));
-    static PerDeviceOnce once[4];
-    ASD_ONCE(once[threads > 512 ? 3 : (threads > 256 ? 2 : ch == 1)],
-             ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
+    // steps and short runs of large heads wait for the state, not for their positions: no loads ahead, and the registers of as many
+    // CTAs per SM as there can be (64 runs of 5, 4 heads of 512 x 512: one 295 us, two 191)
+    const int form = cols == 16 ? (threads > 256 ? 0 : 1)
+                                : (threads > 512 ? 2 : (threads > 256 ? (2 * smem <= 220 * 1024 ? 3 : 4) : (ch == 1 ? 5 : 6)));
+    const decltype(&gla_recurrence_kernel<256, 2, true>) forms[] = {
+        gla_recurrence_kernel<512, 2, false, 16>, gla_recurrence_kernel<256, 4, false, 16>, gla_recurrence_kernel<1024, 1, false>,
+        gla_recurrence_kernel<512, 2, false>,     gla_recurrence_kernel<512, 1, true>,      gla_recurrence_kernel<256, 4, false>,
+        gla_recurrence_kernel<256, 2, true>};
+    auto fn = forms[form];
+    static PerDeviceOnce once[7];
+    ASD_ONCE(once[form], ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(fn, grid, threads, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out, ch, vec));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());

@@ -1,5 +1,5 @@
-"""GPU: the gated recurrence at the edges of its split: 8 key rows x 4 columns of the state per thread, 32 columns per CTA,
-positions staged 4, 8 or 16 at a time (1 in steps), 16-byte copies where the sizes allow."""
+"""GPU: the gated recurrence at the edges of its split: 8 key rows x 4 columns of the state per thread, 32 or 16 columns per CTA,
+positions staged 4 to 16 at a time (as many as the forward's average run; 1 in steps), 16-byte copies where the sizes allow."""
 import pytest
 import torch
 
@@ -22,5 +22,20 @@ def test_state_tiles_and_chunks(dim, vdim, rank):
     # runs of 1, 2, 4, 5, 16 and 17 positions: the sums of a position do not depend on the cut
     cut = feed(eng, eng.open_sequence(), ids, [1, 2, 4, 5, 16, 17, 1, 1])
     assert rel_err(one, ref)[1] < 2e-4          # as the other tests of this engine: far below one missed position
+    assert torch.equal(one, cut)
+    close(eng)
+
+
+# warps with row groups beyond the key size, whole and in part; steps of 16 columns a CTA that the values do not fill
+@pytest.mark.parametrize("dim,vdim", [(16, 8), (24, 40), (20, 33), (264, 36), (300, 20), (516, 44)])
+def test_row_groups_beyond_the_key_size(dim, vdim):
+    cfg = config([gla(heads=2, dim=dim, vdim=vdim, tau=16.0, decay_rank=4)])
+    w = O.random_model(cfg, seed=23)
+    ids = tokens(24, 96, 24)
+    ref, _ = O.forward(cfg, w, ids)
+    eng = make_engine(cfg, w, max_tokens=64)
+    one = feed(eng, eng.open_sequence(), ids, [])
+    cut = feed(eng, eng.open_sequence(), ids, [1, 1, 5, 1, 9, 1])
+    assert rel_err(one, ref)[1] < 2e-4          # as above
     assert torch.equal(one, cut)
     close(eng)
