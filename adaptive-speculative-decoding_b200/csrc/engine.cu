@@ -141,12 +141,18 @@ static int ensure_plans(Engine* e, int M, Plans** out) {
     }
     Plans p;
     const int h = e->c.hidden;
-    if (gemm_plan(&p.qkv, M, e->nqkv, h, (e->reduce && e->fuse_rope) ? GEMM_OUT_QKV : GEMM_OUT_F32, e->force_ksplit,
-                  e->force_stages, e->reduce))
-        return -1;
-    if (gemm_plan(&p.o, M, h, e->qdim, GEMM_OUT_F32, e->force_ksplit, e->force_stages, e->reduce)) return -1;
+    // A prompt beyond max_tokens finds room for 8 slices a token instead of 16 (asd_engine_create_for_prompts): a plan that would
+    // take more, without the in-cluster reduction, takes what fits.
+    auto plan = [&](GemmPlan* pl, int N, int K, int mode) {
+        if (gemm_plan(pl, M, N, K, mode, e->force_ksplit, e->force_stages, e->reduce)) return -1;
+        const size_t fit = e->part_floats / ((size_t)M * N);
+        if (M <= e->c.max_tokens || (size_t)pl->ksplit <= fit || fit == 0) return 0;
+        return gemm_plan(pl, M, N, K, mode, (int)fit, e->force_stages, e->reduce);
+    };
+    if (plan(&p.qkv, e->nqkv, h, (e->reduce && e->fuse_rope) ? GEMM_OUT_QKV : GEMM_OUT_F32)) return -1;
+    if (plan(&p.o, h, e->qdim, GEMM_OUT_F32)) return -1;
     if (gemm_plan(&p.gu, M, 2 * e->ffp, h, GEMM_OUT_SWIGLU, 0, e->force_stages, 0)) return -1;
-    if (gemm_plan(&p.down, M, h, e->c.ffn, GEMM_OUT_F32, e->force_ksplit, e->force_stages, e->reduce)) return -1;
+    if (plan(&p.down, h, e->c.ffn, GEMM_OUT_F32)) return -1;
     const size_t need = (size_t)M * std::max(std::max((size_t)p.qkv.ksplit * e->nqkv, (size_t)p.o.ksplit * h),
                                              (size_t)p.down.ksplit * h);
     if (need > e->part_floats) return set_error("engine: split-K workspace too small for M = %d", M);

@@ -35,3 +35,22 @@ def test_one_prompt_goes_through_whole(length):
             small._uniform(small._prompt_forward, ids[:, :17], torch.zeros(2, dtype=torch.int32, device="cuda"), slots, 17, True, True)
     small.close()
     large.close()
+
+
+@pytest.mark.parametrize("length,max_tokens,max_seq_len,options", [
+    (509, 64, 517, {}), (768, 256, 1024, {}), (768, 256, 1024, {"gemm_big": 0}), (1000, 32, 1024, {"ksplit": 16})])
+def test_whole_prompts_without_the_in_cluster_reduction(length, max_tokens, max_seq_len, options):
+    """plans of up to 16 K slices, the workspace of a prompt beyond max_tokens holds 8: widths of the 0.5B model"""
+    from asd_b200.engine import QwenEngine
+    from asd_b200.models.qwen2 import Qwen2Config
+    cfg = Qwen2Config(896, 1, 14, 2, 4864, 512, head_dim=64, name="0.5b-layer")
+    ids = torch.randint(0, cfg.vocab_size, (1, length), generator=torch.Generator().manual_seed(8), dtype=torch.int32).cuda()
+    slots = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out = []
+    for held, opts in ((max_tokens, {"reduce": 0, **options}), (1024, {})):
+        eng = QwenEngine(cfg, max_seqs=1, max_seq_len=max_seq_len, max_tokens=held, fuse_norm=False).load_random(seed=4)
+        for name, value in opts.items():
+            eng.set_option(name, value)
+        out.append(eng.prefill(ids, slots).double().cpu())
+        eng.close()
+    assert _rel(out[0], out[1]) < 2e-2      # the same products, their fp32 slices added in another order
