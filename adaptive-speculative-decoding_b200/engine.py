@@ -236,12 +236,26 @@ class _BatchOps:
         return out
 
 
+def whole_prompt_tokens(max_tokens: int, max_seq_len: int, tp_size: int = 1, prompt_tokens: Optional[int] = None) -> int:
+    """new positions that a forward of one sequence's prompt takes (``QwenEngine``'s ``prompt_tokens``)"""
+    if prompt_tokens is None:
+        prompt_tokens = min(1024, max_seq_len) if tp_size == 1 else 0
+    return max(max_tokens, prompt_tokens)
+
+
 class QwenEngine(_BatchOps):
-    """One model on one tensor-parallel rank: wraps an ``asd_engine_t`` handle."""
+    """One model on one tensor-parallel rank: wraps an ``asd_engine_t`` handle.
+
+    ``max_tokens`` bounds the tokens of a forward.  ``prompt_tokens`` (at most 4096; one rank) bounds those of a forward that brings
+    one sequence's prompt and nothing else, which ``prefill`` and ``prefill_ragged`` make for a single prompt: the weights then stream
+    once where forwards of ``max_tokens`` stream them for each (509 tokens, two 7B layers: 1184 us in forwards of 256, whole 766).
+    Left alone it is min(1024, max_seq_len).  The engine holds
+    activations for as many tokens: between 256 and 1024, 0.22 GB at the 32B widths, 0.14 at 7B, 0.04 at 0.5B.  An engine that
+    never sees a long prompt saves them with ``prompt_tokens=0``.  Several prompts at once, and steps, keep to ``max_tokens``."""
 
     def __init__(self, cfg: Qwen2Config, max_seqs: int, max_seq_len: int, max_tokens: int = 256, page_size: int = 16,
                  tp_rank: int = 0, tp_size: int = 1, device="cuda", shuffle_pages: bool = True,
-                 fuse_norm: bool = True):
+                 fuse_norm: bool = True, prompt_tokens: Optional[int] = None):
         if not torch.cuda.is_available():
             raise AsdError("QwenEngine needs a CUDA device (there is no CPU fallback)")
         dev = torch.device(device)
@@ -255,10 +269,7 @@ class QwenEngine(_BatchOps):
                               cfg.num_key_value_heads // tp_size, cfg.head_dim, cfg.intermediate_size // tp_size,
                               cfg.vocab_size, cfg.rms_norm_eps, max_tokens, page_size, tp_rank, tp_size)
         self._lock = threading.Lock()
-        # One user's prompt goes through the layers whole, up to 1024 tokens a forward, however few an engine holds for its steps:
-        # in forwards of 256 the weights stream once for each (509 tokens, two 7B layers: 1184 us, whole 766).  Several prompts at
-        # once keep to max_tokens.
-        self.prompt_tokens = max(max_tokens, min(1024, max_seq_len)) if tp_size == 1 else max_tokens
+        self.prompt_tokens = whole_prompt_tokens(max_tokens, max_seq_len, tp_size, prompt_tokens)
         with torch.cuda.device(self.device):
             self.h = lib().asd_engine_create_for_prompts(ctypes.byref(self.c),
                                                          self.prompt_tokens if self.prompt_tokens > max_tokens else 0)

@@ -54,3 +54,28 @@ def test_whole_prompts_without_the_in_cluster_reduction(length, max_tokens, max_
         out.append(eng.prefill(ids, slots).double().cpu())
         eng.close()
     assert _rel(out[0], out[1]) < 2e-2      # the same products, their fp32 slices added in another order
+
+
+def test_prompt_tokens_of_an_engine_are_the_callers():
+    """0: forwards of max_tokens and no memory beyond; a number of its own; more than a call of the CTA-pair GEMM takes is refused"""
+    from asd_b200._lib import AsdError
+    from asd_b200.engine import QwenEngine
+    cfg = tiny_config(num_hidden_layers=1, intermediate_size=16384)
+    ids = torch.randint(0, cfg.vocab_size, (1, 300), generator=torch.Generator().manual_seed(9), dtype=torch.int32).cuda()
+    slots = torch.zeros(1, dtype=torch.int32, device="cuda")
+    held, outs = [], []
+    for asked, largest in ((0, 32), (64, 64), (None, 300)):
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        eng = QwenEngine(cfg, max_seqs=1, max_seq_len=1200, max_tokens=32, prompt_tokens=asked)
+        held.append(free - torch.cuda.mem_get_info()[0])
+        eng.load_random(seed=3)
+        forwards, entry = [], eng._forward
+        eng._forward = lambda name, tokens, *a: (forwards.append(tokens.numel()), entry(name, tokens, *a))[1]
+        outs.append(eng.prefill(ids, slots).double().cpu())
+        assert max(forwards) == largest
+        eng.close()
+    assert held[2] - held[0] > 24 << 20             # 992 tokens of 16384 bf16 activations, at least
+    assert max(_rel(o, outs[2]) for o in outs) < 2e-2
+    with pytest.raises(AsdError, match="at most 4096"):
+        QwenEngine(cfg, max_seqs=1, max_seq_len=1200, max_tokens=32, prompt_tokens=4097)
