@@ -236,10 +236,17 @@ class _BatchOps:
         return out
 
 
-def whole_prompt_tokens(max_tokens: int, max_seq_len: int, tp_size: int = 1, prompt_tokens: Optional[int] = None) -> int:
+# Pages of a sequence up to which its prompts go through whole.  A whole prompt's attention walks all keys in one piece, and a block
+# stages that piece's page numbers beside 168 KB of tiles: 16062 of them fit.
+WHOLE_PROMPT_PAGES = 8192
+
+
+def whole_prompt_tokens(max_tokens: int, max_seq_len: int, page_size: int, tp_size: int = 1,
+                        prompt_tokens: Optional[int] = None) -> int:
     """new positions that a forward of one sequence's prompt takes (``QwenEngine``'s ``prompt_tokens``)"""
     if prompt_tokens is None:
-        prompt_tokens = min(1024, max_seq_len) if tp_size == 1 else 0
+        whole = tp_size == 1 and -(-max_seq_len // page_size) <= WHOLE_PROMPT_PAGES
+        prompt_tokens = min(1024, max_seq_len) if whole else 0
     return max(max_tokens, prompt_tokens)
 
 
@@ -249,7 +256,7 @@ class QwenEngine(_BatchOps):
     ``max_tokens`` bounds the tokens of a forward.  ``prompt_tokens`` (at most 4096; one rank) bounds those of a forward that brings
     one sequence's prompt and nothing else, which ``prefill`` and ``prefill_ragged`` make for a single prompt: the weights then stream
     once where forwards of ``max_tokens`` stream them for each (509 tokens, two 7B layers: 1184 us in forwards of 256, whole 766).
-    Left alone it is min(1024, max_seq_len).  The engine holds
+    Left alone it is min(1024, max_seq_len), or ``max_tokens`` where a sequence may have more than 8192 pages.  The engine holds
     activations for as many tokens: between 256 and 1024, 0.22 GB at the 32B widths, 0.14 at 7B, 0.04 at 0.5B.  An engine that
     never sees a long prompt saves them with ``prompt_tokens=0``.  Several prompts at once, and steps, keep to ``max_tokens``."""
 
@@ -269,7 +276,7 @@ class QwenEngine(_BatchOps):
                               cfg.num_key_value_heads // tp_size, cfg.head_dim, cfg.intermediate_size // tp_size,
                               cfg.vocab_size, cfg.rms_norm_eps, max_tokens, page_size, tp_rank, tp_size)
         self._lock = threading.Lock()
-        self.prompt_tokens = whole_prompt_tokens(max_tokens, max_seq_len, tp_size, prompt_tokens)
+        self.prompt_tokens = whole_prompt_tokens(max_tokens, max_seq_len, page_size, tp_size, prompt_tokens)
         with torch.cuda.device(self.device):
             self.h = lib().asd_engine_create_for_prompts(ctypes.byref(self.c),
                                                          self.prompt_tokens if self.prompt_tokens > max_tokens else 0)
