@@ -45,14 +45,17 @@ struct DenseRunner {
     }
 
     // Above 160 tokens the weight-streaming kernel has room for fewer blocks of its wider tiles, and CTA pairs are the better form of
-    // a matrix of 4M elements whose rows are no longer than it has of them.  The pairs take K in one slice here, 5.4 us per 1024 of it
+    // larger matrices whose rows are no longer than they have of them.  The pairs take K in one slice here, 5.4 us per 1024 of it
     // however few their tiles are: longer rows stay with the weight-streaming kernel, which splits them over a cluster.  161 tokens, us
     // alone, weight-streaming and pairs: 2048 x 2048 22.6, 18.5; 6144 x 2048 28.6, 18.5; 4096 x 4096 39.5, 29.1; 12288 x 4096 51.3,
     // 30.9; but 1024 x 4096 14.4, 28.8; 2048 x 6144 28.8, 39.6; 512 x 8192 16.5, 51.2; 4096 x 12288 60.0, 73.9 (256 tokens 70.6, 74.1).
-    // Below 4M elements the pairs gain less than their plain launches cost in a step.
+    // Their plain launches cost a step some 4 us each: 4096 x 1024 (14.4, 12.4) made steps of 168 and 192 tokens of width 1024 slower
+    // (Rivetar 324 -> 329 and 335 -> 340, Mavipel 457 -> 462).  Steps of 168 tokens of width 2048 with and without pairs: Mavipel 682,
+    // 746, Lukopel 714, 727, Dikopel 558, 633, Nobonex 591, 685, Rivetar 477, 513, Mezilix 214, 236; of width 4096 4 to 12 % faster.
     bool pair_from(int M, int N, int K) const {
         if (tc_min_rows > 0) return M >= tc_min_rows;
-        return M > 256 || (M > 160 && (long long)N * K >= 1 << 22 && K <= N);
+        const long long elements = (long long)N * K;
+        return M > 256 || (M > 160 && K <= N && (elements >= 8 << 20 || (elements >= 4 << 20 && K >= 2048)));
     }
 
     int run(const void* x, const void* w, float* y, int M, int N, int K, int ldc, int key, cudaStream_t s) {

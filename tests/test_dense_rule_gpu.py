@@ -31,12 +31,15 @@ def test_larger_matrices_take_pairs_from_161_tokens(length, pairs):
     assert ((outs[0] - outs[1]).norm() / outs[0].norm()).item() < 1e-2
 
 
-@pytest.mark.parametrize("length,pairs", [(161, 1), (256, 1), (257, 3)])
-def test_long_rows_stay_with_the_weight_streaming_kernel(length, pairs):
-    """up projection 4096 x 1024 on pairs, down projection 1024 x 4096 (as many elements, four times the K of one slice) not before
-    257 tokens"""
+@pytest.mark.parametrize("width,ff,length,pairs", [
+    (2048, 4096, 161, 1), (2048, 4096, 256, 1), (2048, 4096, 257, 3),       # up projection 4096 x 2048 on pairs, down 2048 x 4096 not
+    (1024, 4096, 161, 0), (1024, 4096, 256, 0), (1024, 4096, 257, 3),       # 4096 x 1024: K too short for the plain launch it costs
+    (1024, 8192, 161, 1),                                                   # 8M elements
+])
+def test_long_rows_stay_with_the_weight_streaming_kernel(width, ff, length, pairs):
+    """matrices of more columns than rows, which the pairs would take in one slice, not before 257 tokens"""
     from asd_b200._lib import lib
-    cfg = config([gla(heads=1, dim=16, vdim=16, ff=4096)], width=1024)
+    cfg = config([gla(heads=1, dim=16, vdim=16, ff=ff)], width=width)
     w = O.random_model(cfg, seed=73)
     eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512)
     slot = eng.open_sequence()
