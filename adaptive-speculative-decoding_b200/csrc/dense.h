@@ -58,12 +58,18 @@ struct DenseRunner {
         return M > 256 || (M > 160 && K <= N && (elements >= 8 << 20 || (elements >= 4 << 20 && K >= 2048)));
     }
 
+    // Few tokens: linear_few.cu, of rows up to 4096.  Its blocks stage all of a token's K, 196 KB at 6144 and hence one block an SM, and in
+    // a step the weight-streaming kernel's launches overlap: 16 tokens, width 2048, down projections of 2048 x 6144 here and there,
+    // Rivetar 226 and 220 us, Lukopel 289 and 283, Mavipel 373 and 368; Mavipel of width 4096, output projections of 4096 x 6144, 588
+    // and 579 (580 without linear_few.cu at all).  Steps of 1 to 16 tokens with it and without: width 1024 4 to 11 % faster in all six
+    // families, 2048 3 to 8 %, 4096 0 to 5 %.
+    bool few_from(int M, int K) const { return few && K <= 4096 && !(tc_min_rows > 0 && M >= tc_min_rows); }
+
     int run(const void* x, const void* w, float* y, int M, int N, int K, int ldc, int key, cudaStream_t s) {
         if (!f32 && tc_linear && (K % 8) == 0 && (ldc % 4) == 0 && K >= 64 && N >= 8 &&
             (reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0 &&
             (reinterpret_cast<uintptr_t>(y) & 15) == 0) {
-            const bool asked_for_pairs = tc_min_rows > 0 && M >= tc_min_rows;
-            if (few && !asked_for_pairs && linear_few_takes(x, w, M, N, K)) return launch_linear_few(x, w, y, M, N, K, ldc, s);
+            if (few_from(M, K) && linear_few_takes(x, w, M, N, K)) return launch_linear_few(x, w, y, M, N, K, ldc, s);
             const unsigned long long k = ((unsigned long long)key << 32) | (unsigned)M;
             auto it = cache.find(k);
             if (it == cache.end()) {

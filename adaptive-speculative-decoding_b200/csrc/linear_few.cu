@@ -11,8 +11,8 @@
 //   * the warps' sums meet in shared memory, added in warp order, one barrier per group.
 // The sums of a token depend on neither M nor the other tokens.
 // 16 tokens, cold matrices, us (gemm.cu before): 2048 x 2048 10.3 -> 5.6, 6144 x 2048 12.4 -> 9.4, 8224 x 2048 13.1 -> 9.8,
-// 3072 x 1024 8.3 -> 5.4, 4096 x 4096 14.2 -> 10.2, 6720 x 4096 22.3 -> 13.4.  In a step gemm.cu's launches overlap: 16 x 1 of three
-// Rivetar layers of width 2048 312 -> 302, of a Mezilix layer of width 4096 309 -> 299.
+// 3072 x 1024 8.3 -> 5.4, 4096 x 4096 14.2 -> 10.2, 6720 x 4096 22.3 -> 13.4; 2048 x 6144 13.8 -> 12.1,
+// 128 x 6144 10.3 -> 10.4.  In a step gemm.cu's launches overlap; dense.h says which matrices a step leaves to them.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>

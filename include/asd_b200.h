@@ -315,8 +315,8 @@ ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_p
                                   int max_seqs, int max_pages_per_seq, int32_t* token_ring, float* shift_ring);
 /* options: "tc_linear" (1, default: bf16 projections whose shape the tcgen05 kernels accept run on them; 0: CUDA-core
  * kernel everywhere), "tc_min_rows" (token count from which dense projections use the tensor-bound CTA-pair GEMM; 0 = never;
- * left alone: 257, 161 for larger matrices with no more columns than rows), "linear_few" (1, default: up to 16 tokens on matrices up to 64 MB run
- * linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
+ * left alone: 257, 161 for larger matrices with no more columns than rows), "linear_few" (1, default: up to 16 tokens on matrices up to 64 MB of up to
+ * 4096 columns run linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
  * rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
  * per (token, head)), "profile" (1: CUDA events around every launch, read with asd_mezilix_profile_read) */

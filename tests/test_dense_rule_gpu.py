@@ -50,6 +50,22 @@ def test_long_rows_stay_with_the_weight_streaming_kernel(width, ff, length, pair
     close(eng)
 
 
+@pytest.mark.parametrize("ff,few", [(4096, 3), (4104, 2)])
+def test_few_tokens_of_long_rows_stay_with_the_weight_streaming_kernel(ff, few):
+    """input, up and down projection (2048 x ff) and the head for 8 tokens: a block of the few-token kernel would stage all of ff"""
+    from asd_b200._lib import lib
+    cfg = config([gla(heads=1, dim=16, vdim=16, ff=ff)], width=2048)
+    w = O.random_model(cfg, seed=75)
+    eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=64)
+    slot = eng.open_sequence()
+    eng.reserve(slot, 8)
+    names = (b"linear_few", b"gemm")
+    before = [lib().asd_kernel_launches(n) for n in names]
+    eng.forward_ragged([(slot, 0, tokens(8, 96, 76), [7])])
+    assert [lib().asd_kernel_launches(n) - b for n, b in zip(names, before)] == [few + 1, 3 - few]
+    close(eng)
+
+
 @pytest.mark.parametrize("family", ["Mezilix", "Rivetar", "Mavipel", "Lukopel", "Dikopel", "Nobonex"])
 def test_options_of_dense_projections_hold_for_few_tokens(family):
     """8 tokens of every family's engine: the few-token kernel, without it, and CTA pairs where they are asked for"""
