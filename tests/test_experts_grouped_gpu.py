@@ -38,3 +38,24 @@ def test_experts_on_cta_pairs(width, ff, experts, top, tokens, alone):
         mz.close(eng)
     e_pair, e_one = mz.rel_err(outs[0], ref)[0], mz.rel_err(outs[1], ref)[0]
     assert e_one < 4e-2 and e_pair < 1.1 * e_one + 1e-4, (e_pair, e_one)
+
+
+@pytest.mark.parametrize("width,top,tokens,pairs", [
+    (2048, 1, 3, False), (2048, 1, 4, True),            # 4M elements: a row an expert, on average
+    (1024, 2, 63, False), (1024, 2, 64, True),          # 1M: 32
+])
+def test_rows_an_expert_from_which_pairs_are_taken(width, top, tokens, pairs):
+    """four experts of width x width, the rule's own border on either side; the same result as without pairs"""
+    from asd_b200._lib import lib
+    cfg = mz.config([mz.layer(heads=1, dim=16, rot_dim=8, vdim=16, kv_rank=24, experts=4, top=top, ff=width)], width=width)
+    w = O.random_model(cfg, seed=63)
+    ids = mz.tokens(tokens, 96, 64)
+    outs = []
+    for rows in (0, 1 << 20):
+        eng = mz.make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=64, max_seq_len=64)
+        eng.set_option("experts_rows", rows)
+        before = lib().asd_kernel_launches(b"gemm_grouped")
+        outs.append(mz.feed(eng, eng.open_sequence(), ids, []).double().cpu())
+        assert lib().asd_kernel_launches(b"gemm_grouped") - before == (2 if pairs and rows == 0 else 0)
+        mz.close(eng)
+    assert ((outs[0] - outs[1]).norm() / outs[1].norm()).item() < 1e-2      # fp32 sums in another order, one bf16 rounding between

@@ -39,3 +39,25 @@ def test_row_groups_beyond_the_key_size(dim, vdim):
     assert rel_err(one, ref)[1] < 2e-4          # as above
     assert torch.equal(one, cut)
     close(eng)
+
+
+def test_chunks_of_an_unequal_batch():
+    """one run of 100 positions beside nine single tokens: chunks of the average run (11), which no run of its own has, then a step of
+    all of them; bit for bit what every sequence gets alone"""
+    cfg = config([gla(heads=2, dim=72, vdim=36, tau=16.0, decay_rank=4)])
+    w = O.random_model(cfg, seed=25)
+    lens = [1, 1, 1, 100, 1, 1, 1, 1, 1, 1]
+    ids = [tokens(n + 7, 96, 26 + i) for i, n in enumerate(lens)]       # six positions before, one after
+    eng = make_engine(cfg, w, max_tokens=128, max_seqs=20)
+    alone, slots = [], []
+    for t, n in zip(ids, lens):
+        alone.append(feed(eng, eng.open_sequence(), t, [6, n, 1]))
+    for t in ids:
+        slots.append(eng.open_sequence())
+        eng.reserve(slots[-1], len(t))
+        eng.forward_ragged([(slots[-1], 0, t[:6], [5])])
+    got = eng.forward_ragged([(s, 6, t[6:6 + n], list(range(n))) for s, t, n in zip(slots, ids, lens)])
+    step = eng.forward_ragged([(s, 6 + n, t[6 + n:], [0]) for s, t, n in zip(slots, ids, lens)])
+    assert torch.equal(got, torch.cat([a[6:6 + n] for a, n in zip(alone, lens)]))
+    assert torch.equal(step, torch.cat([a[6 + n:] for a, n in zip(alone, lens)]))
+    close(eng)
