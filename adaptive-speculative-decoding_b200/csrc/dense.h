@@ -1,7 +1,8 @@
 // Dense projection of an engine's activations, y fp32 [M][ldc] = x [M][K] * w[N][K]^T, routed by shape and element
-// type: the weight-streaming tcgen05 GEMM (gemm.cu) for bf16 operands it accepts, its tensor-bound CTA-pair form
-// (gemm_tc.cu) above 256 tokens, of larger matrices whose rows are not too long above 160, the CUDA-core kernel (linear_simt.cu) for fp32 engines and every other
-// shape.  Plans and tensor maps are cached per (call site, token count); a call site always passes the same buffers.
+// type: the weight-streaming tcgen05 GEMM (gemm.cu) for bf16 operands it accepts, its tensor-bound CTA-pair form (gemm_tc.cu)
+// above 256 tokens, of larger matrices whose rows are not too long above 160, the few-token kernel (linear_few.cu) up to 16, the
+// CUDA-core kernel (linear_simt.cu) for fp32 engines and every other shape.  Plans and tensor maps are cached per (call site,
+// token count); a call site always passes the same buffers.
 #pragma once
 #include <cuda.h>
 #include <cuda_runtime.h>

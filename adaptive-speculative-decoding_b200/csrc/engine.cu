@@ -210,9 +210,10 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     // pass (~4 us, more than ten 64-key tiles of the key loop), so a sequence is only split into pieces of
     // at least attn_min_split_keys keys
     // A prompt whose new positions x group are more rows than the 128 lanes of a query tile runs in tiles of 128 / group
-    // positions, so that one forward takes as many positions as max_tokens allows: a chunk limited to 128 rows streamed all
-    // weights once per 128 / group positions (one 509-token prompt through two 7B layers: 29 forwards, 6.9 ms; now two,
-    // 1.2 ms; eight prompts of 500 to 1000 tokens through two 32B layers: 40 forwards, 27.8 ms; now four, 13.5 to 14.4 ms).
+    // positions, so that one forward takes as many positions as the activations allow (max_tokens; scratch_tokens of one sequence's):
+    // a chunk limited to 128 rows streamed all weights once per 128 / group positions (one 509-token prompt through two 7B layers:
+    // 29 forwards, 6.9 ms; now one, 0.75 to 0.79; eight prompts of 500 to 1000 tokens through two 32B layers: 40 forwards, 27.8 ms;
+    // now four, 13 to 13.9).
     const int group = nh / nkv;
     const int q_tile = prompt && max_qlen * group > 128 && group <= 128 ? 128 / group : 0;
     const int items = nseq * nkv * (q_tile > 0 ? (max_qlen + q_tile - 1) / q_tile : 1);

@@ -1,5 +1,5 @@
 // Tensor-bound bf16 GEMM for the large verify steps:  Y[m, n] = sum_k X[m, k] * W[n, k]  with M above the
-// HBM/tensor ridge (~211 tokens on B200: 72B verify of 64 x 9 = 576 tokens, and prefill).
+// HBM/tensor ridge (~211 tokens on B200: the 72B verification of 64 x 9 = 576 tokens, and prefill).
 //
 // The weight-streaming kernel (gemm.cu) gives every CTA one 128-row weight tile and ALL its k-blocks once; with
 // several token tiles it re-reads the weights per token tile and its 128 x MT tile moves 2 * (128 + MT) bytes per

@@ -19,8 +19,8 @@
 //     below 2^8 and the sums exact in fp32.
 //   * A thread needs ~200 clocks to wait for a barrier and issue one box or four products, so boxes are as large as the
 //     layout allows, a query slot feeds twelve products, three warps load, and the issuing warp walks its loops whole (a
-//     first form with 16 KB slots, one loader and one issuing thread took 666 us where this one takes 366).
-// Four prompts of 1024 tokens, 16 heads, latent 512 + 64: 1350 us on mma.sync, 366 here (185 GFLOP: 0.5 PFLOP/s).
+//     first form with 16 KB slots, one loader and one issuing thread took 666 us where the next took 366).
+// Four prompts of 1024 tokens, 16 heads, latent 512 + 64: 1350 us on mma.sync, 354 here (185 GFLOP: 0.52 PFLOP/s).
 // Every wait is bounded: on expiry the kernel raises the caller's error flag, lets its copies land, frees its TMEM and ends.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -49,8 +49,8 @@ constexpr int kLtMaxV = 4;                 // chunks of 64 result columns per CT
 constexpr float kLtSlack = 8.0f;           // log2 growth of a row maximum that the weights tolerate before a rescale
 constexpr uint32_t kLtSpin = 1u << 20;
 // Query rows of a tile from which this kernel is the better one.  A tile costs what 128 rows cost, however many are real:
-// 64 single tokens of 32 heads at 1024 positions: 146 us on mma.sync, 111 us here; 16 of 16 heads at 1500: 58 us there, 72
-// here (4096 prompt tokens of 16 heads, 128 rows a tile: 1350 and 366).
+// 64 single tokens of 32 heads at 1024 positions: 146 us on mma.sync, 96 us here; 16 of 16 heads at 1500: 58 us there, 72 here
+// when the line was drawn (4096 prompt tokens of 16 heads, 128 rows a tile: 1350 and 354).
 constexpr int kLtMinRows = 32;
 
 struct LtArgs {

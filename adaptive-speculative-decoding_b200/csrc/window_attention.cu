@@ -717,6 +717,8 @@ int launch_window_post(const SeqIndex& ix, float* qkv, long long ld, const Windo
                        const float* freq_v, const PagedRows& cache, float2* turns, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
     if (check_dims(d)) return -1;
+    // no longer for the row's sake, which stays in global memory: it bounds the angles (rot_dims <= dk) below what a block may hold, and
+    // rows that were refused stay refused
     if ((size_t)(d.heads * d.dk + d.kv_heads * (d.dk + d.dv)) * sizeof(float) > 200 * 1024)
         return set_error("windowed attention: a token's q | k | v row is too long");
     const size_t smem = (size_t)(d.rot_dims + d.dv) / 2 * sizeof(float2);

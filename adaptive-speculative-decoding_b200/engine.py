@@ -397,8 +397,10 @@ class QwenEngine(_BatchOps):
                              logit_rows, logits_out, want_logits, logits_ld)
 
     def _prompt_chunk(self, nseq: int) -> int:
-        # Attention tiles any number of new positions, so a forward is as large as max_tokens and the CTA-pair GEMM (4096
-        # tokens a call) allow.  A tensor-parallel rank keeps the short chunk: its exchanges grow with the tokens.
+        # Attention tiles any number of new positions, so a forward is as large as the activations and the CTA-pair GEMM (4096
+        # tokens a call) allow: prompt_tokens for one sequence, max_tokens for several (nothing in the kernels asks for that; forwards of
+        # several prompts beyond max_tokens have not been measured).  A tensor-parallel rank keeps the short chunk: its exchanges
+        # grow with the tokens.
         if self.tp_size > 1:
             return super()._prompt_chunk(nseq)
         return max(1, min(self.prompt_tokens if nseq == 1 else self.max_tokens, 4096) // nseq)

@@ -129,8 +129,8 @@ ASD_API double asd_bayesian_adjustment_host(double p_hat, double n_obs, double a
  */
 ASD_API int asd_linear_bf16(const void* x, const void* w, void* out, int M, int N, int K, int out_mode, int ksplit,
                     int stages, int* ksplit_used, void* stream);
-/* Same contraction on the tensor-bound kernel used above the HBM/tensor ridge (M > 256 tokens: BASELINE configs[4],
- * prefill): CTA pairs (tcgen05 cta_group::2, 256 weight rows x <= 256 tokens per tile), persistent, two TMEM
+/* Same contraction on the tensor-bound kernel used above the HBM/tensor ridge (prompts, verifications of more than 256 tokens, larger
+ * projections of the families from 161): CTA pairs (tcgen05 cta_group::2, 256 weight rows x <= 256 tokens per tile), persistent, two TMEM
  * accumulators.  out_mode 0: fp32 [ksplit_used, M, N] slices; out_mode 2: SwiGLU bf16 [M, N/2]. */
 ASD_API int asd_linear_bf16_tc(const void* x, const void* w, void* out, int M, int N, int K, int out_mode, int ksplit,
                        int stages, int* ksplit_used, void* stream);
@@ -315,9 +315,9 @@ ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_p
                                   int max_seqs, int max_pages_per_seq, int32_t* token_ring, float* shift_ring);
 /* options: "tc_linear" (1, default: bf16 projections whose shape the tcgen05 kernels accept run on them; 0: CUDA-core
  * kernel everywhere), "tc_min_rows" (token count from which dense projections use the tensor-bound CTA-pair GEMM; 0 = never;
- * left alone: 257, 161 for larger matrices with no more columns than rows), "linear_few" (1, default: up to 16 tokens on matrices up to 64 MB of up to
- * 4096 columns run linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an expert, on average, from which its products run on CTA pairs; 0, default: the measured
- * rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
+ * left alone: 257, 161 for larger matrices with no more columns than rows), "linear_few" (1, default: up to 16 tokens on
+ * matrices up to 64 MB of up to 4096 columns run linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an
+ * expert, on average, from which its products run on CTA pairs; 0, default: the measured rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
  * per (token, head)), "profile" (1: CUDA events around every launch, read with asd_mezilix_profile_read) */
 ASD_API int asd_mezilix_set_option(asd_mezilix_engine_t* e, const char* name, int value);
