@@ -1,5 +1,5 @@
 """Stop-rule policy seam: same names, arguments and error behaviour as the reference's
-``src/algorithms/dp_solver.py`` (/root/reference/src/algorithms/dp_solver.py:12-289), with
+``src/algorithms/dp_solver.py`` (:12-289), with
 the arithmetic executed by libasd_b200.so (``asd_stop_rule_host`` for the scalar API the
 pipeline calls per request, ``asd_stop_rule`` on the device for batches - see ``stop_rule_batch``).
 Results are bit-exact with the reference (tests/test_stop_rule.py)."""
@@ -57,7 +57,7 @@ def bayesian_adjustment(p_hat: float, n_obs: int, alpha: float = 1.0, beta: floa
 
 def stop_rule_batch(p, C, lam: float, risk_adjustment: bool = False, alpha: float = 1.0, beta: float = 1.0):
     """Device form: p, C are CUDA float64 tensors [n, L]; returns (k_star int32 [n], J float64 [n, L+1])
-    without leaving the GPU (north-star item 3)."""
+    without leaving the GPU."""
     import torch
     assert p.is_cuda and C.is_cuda and p.dtype == torch.float64 and C.dtype == torch.float64
     p, C = p.contiguous(), C.contiguous()
@@ -204,8 +204,8 @@ class AdaptiveStopping:
 
 
 class DynamicProgrammingSolver:
-    """Imported by real_model_pipeline.py:39 but never defined by the reference
-    (SURVEY.md Appendix A).  ``should_stop`` asks the DP whether stopping at ``stage_id`` is
+    """Imported by real_model_pipeline.py:39 but never defined by the
+    reference.  ``should_stop`` asks the DP whether stopping at ``stage_id`` is
     optimal given the quality estimate as this stage's acceptance probability and 1.0 for the
     later stages (the pipeline's own convention that the last stage always accepts,
     pipeline.py:241-242); the reference's stated fallback ``quality > 0.8 or last stage``

@@ -1,4 +1,4 @@
-"""Lambda tuning around the cascade (SURVEY.md 8 f1): same names, arguments and search procedures as the
+"""Lambda tuning around the cascade: same names, arguments and search procedures as the
 reference's src/algorithms/optimizer.py (``OptimizationResult`` :15-21, ``LambdaOptimizer`` :24-205,
 ``find_optimal_lambda`` :208-258, ``GridSearchOptimizer`` :261-353).  Pure host control flow that calls
 ``pipeline.process_request`` - which runs on the B200 engine - and reads the result like a dict and

@@ -1,6 +1,6 @@
 // Paged-KV verify attention on tcgen05 / TMEM (head_dim 128): the Blackwell-native replacement of the mma.sync
-// kernel in attention.cu, which is bound by legacy-HMMA issue once the context is long (
-// 72B verify at a 4096-token prefix spent 28 of 78 ms there at 0.23 of HBM) and by per-tile latency when it is short.
+// kernel in attention.cu, which is bound by legacy-HMMA issue once the context is long (a
+// 72B verification at a 4096-token prefix spent 28 of 78 ms there at 0.23 of HBM) and by per-tile latency when it is short.
 //
 // Work item = (sequence, kv head, kv split) as before: the query tile is all new positions x the GQA group
 // (rows = q_len * G <= 128, padded to the 128 TMEM lanes), so each K/V byte is read once per sequence.
@@ -12,8 +12,8 @@
 //                   head-dim elements per page and half, gathered through the page table);
 //   softmax         warps 0-3, thread = query row = TMEM lane: row maximum and exp2 over two tcgen05.ld passes
 //                   (straight-line, select-based masking, four independent accumulators: the first version's
-//                   per-pair branches serialised one MUFU latency after the other - 5.2 us per tile, measured with
-//                   tools/trace_attn.py); the bf16 probabilities go straight back into TMEM (tcgen05.st over the
+//                   per-pair branches serialised one MUFU latency after the other - 5.2 us per tile by
+//                   asd_debug_attn_trace); the bf16 probabilities go straight back into TMEM (tcgen05.st over the
 //                   first 64 columns of the S buffer they came from), never through shared memory;
 //   O_t = P V       tcgen05.mma with A = P from TMEM and V as an MN-major B operand (the pool stores
 //                   [position][head_dim], so keys are the contraction dimension: no transpose, no ldmatrix.trans);
@@ -22,7 +22,7 @@
 // S/P and O_t are double-buffered in TMEM (4 x 128 columns): QK^T of tile j+1 runs while the softmax of tile j is
 // in flight, P V of tile j while the softmax of tile j+1 runs (P lives in the other S buffer: the second version
 // kept P in ONE shared-memory buffer and its softmax warps spent a quarter of their time waiting for P V to release
-// it, profiles/ncu_attn_tc_r02.txt).  Warp 8 streams K, warp 9 streams V (2-deep rings), one thread of warp 10
+// it, profiles/ncu_attn_tc.txt).  Warp 8 streams K, warp 9 streams V (2-deep rings), one thread of warp 10
 // issues all MMAs.  Warps whose 32 rows are all padding sit the loop out (the barrier counts are the number of
 // active warps).  Long contexts are split over the KV length (flash decoding) with the same ticket merge as
 // attention.cu.

@@ -74,7 +74,7 @@ struct Engine {
         attn_target_ctas = 148, fuse_rope = 1, fuse_norm = 0, attn_min_split_keys = 1024, tp_fused = 1, tp_two_shot = 0;
     Tuning tune;   // per-engine knobs, installed for the calling thread by forward()
     // persistent forward kernel (forward_persist.cu): one cooperative launch per forward when the shape allows
-    // measured on B200 (tools/trace_persist.py): the persistent kernel streams every GEMM at 87-95 % of HBM speed, but a
+    // measured on B200: the persistent kernel streams every GEMM at 87-95 % of HBM speed, but a
     // phase boundary through global memory (partials -> flags -> reduce -> epilogue -> counter -> X load) costs 15-18 us
     // against 10-12 us for a kernel boundary under programmatic dependent launch, so it is opt-in (option persist = 1)
     int persist = 0, persist_ahead = 0;

@@ -30,7 +30,7 @@
 // Replaces (reference): per-token softmax + log(probs[token]) with a host sync per token,
 // src/training/generate_training_data.py:128-134, and the logprob feature
 // reductions of docs/guides/RESEARCH_PROTOCOL.md:379-398.  The accept/resample rule itself has no
-// reference implementation (SURVEY.md Appendix C).
+// reference implementation.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>

@@ -90,7 +90,7 @@ __global__ void stop_rule_kernel(const double* __restrict__ p, const double* __r
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Scorer -> stop decision on the device (north star 3): one CTA per request turns the per-token features the
+// Scorer -> stop decision on the device: one CTA per request turns the per-token features the
 // sampling kernel left in device memory (entropy / max-prob / margin / emitted-token log-prob over the FULL vocabulary)
 // into the predictor's feature vector, runs the 256 -> 128 -> 1 MLP, the Bayesian shrinkage and the optimal-stopping
 // DP, and emits (acceptance probability, stop?, k*).  The host only reads those three numbers per request: no logits,

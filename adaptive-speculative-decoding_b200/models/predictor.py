@@ -1,6 +1,6 @@
 """Scorer seam.  ``QualityPredictor`` / ``FeatureExtractor`` are imported by the reference
 (src/serving/pipeline.py:15,225-231; src/serving/server.py:24,168-179) from ``src/models/predictor.py``,
-which it does not ship; reconstructed from docs/guides/RESEARCH_PROTOCOL.md:308-409 (SURVEY.md App. A).
+which it does not ship; reconstructed from docs/guides/RESEARCH_PROTOCOL.md:308-409.
 
 The feature vector keeps the listing's 5 live dimensions in the listing's order (entropy, prompt length
 / 2048, output length / 512, mean max-logprob, stage / 4, zero-padded to 256).  When the logprobs come

@@ -1,4 +1,4 @@
-"""Qwen2.5 shapes (public HF config.json values; SURVEY.md Appendix D), random initialisation and the
+"""Qwen2.5 shapes (public HF config.json values), random initialisation and the
 packing of HF-named weights into the layouts ``asd_engine_set_layer`` expects (include/asd_b200.h)."""
 from __future__ import annotations
 
@@ -30,7 +30,7 @@ class Qwen2Config:
         return L * per + h + self.vocab_size * h * (1 if self.tie_word_embeddings else 2)
 
     def streamed_bytes(self) -> int:
-        """bf16 weight bytes one forward step must read (embedding gather excluded; SURVEY.md 8d)."""
+        """bf16 weight bytes one forward step must read (embedding gather excluded)."""
         h, L = self.hidden_size, self.num_hidden_layers
         qkv = (self.num_attention_heads + 2 * self.num_key_value_heads) * self.head_dim
         per = qkv * h + self.num_attention_heads * self.head_dim * h + 3 * h * self.intermediate_size
@@ -64,10 +64,9 @@ def tiny_config(**kw) -> Qwen2Config:
 
 def random_hf_weights(cfg: Qwen2Config, seed: int, device="cpu", std: float = 0.02,
                       dtype=torch.bfloat16, logit_std: float = None) -> Dict[str, torch.Tensor]:
-    """HF-named state dict with N(0, std^2) weights (norm weights 1 + N(0, std^2)), one seed per model
-    (SURVEY.md 8d synthetic inputs).  ``logit_std`` rescales the output embedding so that the logits have that
+    """HF-named state dict with N(0, std^2) weights (norm weights 1 + N(0, std^2)), one seed per model.  ``logit_std`` rescales the output embedding so that the logits have that
     standard deviation (the final RMSNorm leaves unit-RMS activations, so logit std = head std * sqrt(hidden)):
-    the north-star tolerance "max-abs <= 2e-2" is an absolute bound stated for logits of ordinary magnitude,
+    the tolerance "max-abs <= 2e-2" is an absolute bound stated for logits of ordinary magnitude,
     and logit_std = 0.4 keeps |logit| < ~2 over a 152K vocabulary."""
     g = torch.Generator(device=device).manual_seed(seed)
     h, nh, nkv, hd, ff = (cfg.hidden_size, cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim,

@@ -1,7 +1,7 @@
 """Engine seam.  ``Stage`` / ``StageManager`` / ``StageConfig`` are imported by the reference
 (src/serving/pipeline.py:14, src/serving/server.py:23,151-164) from ``src/models/stage.py``, a file the
 reference does not ship; the signatures below are reconstructed from those call sites and from the
-listing in docs/guides/RESEARCH_PROTOCOL.md:233-304 (SURVEY.md Appendix A).  Where the reference's
+listing in docs/guides/RESEARCH_PROTOCOL.md:233-304.  Where the reference's
 Stage wraps ``vllm.LLM`` this one wraps a B200 engine chosen by the model registry (``QwenEngine`` for the Qwen2
 family, ``MezilixEngine`` / ``RivetarEngine`` for the Mezilix / Rivetar families), optionally accelerated by a smaller draft engine through chain
 draft-then-verify (``SpecDecoder``)."""
@@ -412,7 +412,7 @@ class StageManager:
         return list(self.order)
 
     def calibrate_costs(self, prompts: Optional[List[str]] = None, max_tokens: int = 32) -> Dict[str, float]:
-        """SURVEY.md 8 f3 (RealModelPipeline._calibrate_costs, real_model_pipeline.py:313-362): replace the
+        """As RealModelPipeline._calibrate_costs (real_model_pipeline.py:313-362): replace the
         hard-coded cost table by measured per-token generation time on this machine, normalised so that the
         first stage costs 1.0; updates ``stage.cost_per_token`` in place and returns the new table."""
         prompts = prompts or ["Hello, how are you today?", "What is the capital of France?",

@@ -1,2 +1,2 @@
 """Mirror of the reference's ``src.serving`` package for the hot path (pipeline, cache manager,
-real-model pipeline).  The FastAPI shell (server.py) is out of scope."""
+real-model pipeline) and its HTTP front end (server.py)."""

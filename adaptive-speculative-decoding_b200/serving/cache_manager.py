@@ -1,5 +1,5 @@
 """``KVCacheManager``: the reference's per-(request, stage) result store with byte accounting, LRU
-eviction and a TTL sweep (/root/reference/src/serving/cache_manager.py:26-387).  Despite its name it
+eviction and a TTL sweep (src/serving/cache_manager.py:26-387).  Despite its name it
 never held K/V tensors; the paged K/V pool of the B200 engine lives in ``asd_b200.engine.QwenEngine``.
 Same public API; unlike the reference it tolerates the non-tensor payloads the pipeline stores
 (the reference calls ``.is_cuda`` on ``str`` / ``ndarray`` and crashes, cache_manager.py:176-178,213-215)."""

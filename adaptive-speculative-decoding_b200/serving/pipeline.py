@@ -3,7 +3,7 @@
 B200 engine behind the stage seam.  Per stage: generate -> predict acceptance probability -> Bayesian
 shrinkage -> DP stop rule -> stop or escalate (pipeline.py:184-266).
 
-Reference quirks (SURVEY.md Appendix E) are decided explicitly, not inherited silently:
+Reference quirks are decided explicitly, not inherited silently:
   * ``start_time`` is an undefined global in the reference (:269): here it is passed to ``_process_stages``.
   * The reference evaluates the DP on the PREFIX of probabilities seen so far (:248-256); with the
     last-index rule of dp_solver.py:69 that always stops at stage 0.  ``reference_compat=True``

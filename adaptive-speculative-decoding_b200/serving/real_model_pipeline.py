@@ -2,8 +2,8 @@
 (``StageConfig`` :44-52, ``InferenceRequest`` :54-62, ``StageInferenceResult`` :64-76, ``RealModelStage``
 :78-190, ``RealModelPipeline`` :192-520, ``create_real_pipeline`` :522-526).  Names and argument meaning are
 kept; the body runs on the B200 engine instead of ``vllm.LLM`` (:98-108).  ``SamplingParams``,
-``PipelineResult`` and ``DynamicProgrammingSolver`` are names the reference imports but never defines
-(SURVEY.md Appendix A); minimal definitions live here / in algorithms.dp_solver."""
+``PipelineResult`` and ``DynamicProgrammingSolver`` are names the reference imports but never defines;
+minimal definitions live here / in algorithms.dp_solver."""
 from __future__ import annotations
 
 import logging

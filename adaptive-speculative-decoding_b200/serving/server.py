@@ -1,4 +1,4 @@
-"""HTTP front end of the cascade, mirroring the reference's FastAPI surface
+"""HTTP front end of the cascade mirroring the reference's FastAPI surface
 (`src/serving/server.py:40-84` schemas, `:223-376` endpoints) on top of `asd_b200.serving.pipeline`:
 
     GET  /health         POST /generate        POST /batch_generate   GET /stats

@@ -1,7 +1,7 @@
 """Threshold variant of the stop rule: same names and results as the reference's
 src/theory/optimal_stopping.py:15-91 (``derive_optimal_policy``), bit-exact in binary64
 (tests/test_api_surface.py against goldens generated from the reference).  The regret / sample
-complexity formulas of the same file are paper mathematics with no runtime role (SURVEY.md section 2 row 7)."""
+complexity formulas of the same file are paper mathematics with no runtime role."""
 from __future__ import annotations
 
 from dataclasses import dataclass

@@ -1,1 +1,1 @@
-"""Predictor training-data path (SURVEY.md 8 f4)."""
+"""Predictor training-data path."""

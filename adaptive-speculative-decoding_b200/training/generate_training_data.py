@@ -1,4 +1,4 @@
-"""Training rows for the quality predictor, emitted from what the B200 engine computes (SURVEY.md 8 f4).
+"""Training rows for the quality predictor, emitted from what the B200 engine computes.
 
 Mirrors the on-disk format of the reference's src/training/generate_training_data.py: a JSON list of
 ``TrainingSample`` records (:35-47, written at :348-356) plus ``feature_stats.json`` (:361-371), and its 64-d

@@ -1,5 +1,5 @@
 """Training of the quality predictor on the rows `generate_training_data.save_training_data` writes
-(SURVEY.md 8 f4; mirrors the surface of the reference's `scripts/train_predictor.py`: model :57-91, trainer
+(mirrors the surface of the reference's `scripts/train_predictor.py`: model :57-91, trainer
 :261-466, result dictionary :420-458).
 
 Same recipe - standardised features, K-fold cross-validation (shuffle, seed 42), AdamW + cosine schedule, MSE

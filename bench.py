@@ -1,7 +1,7 @@
 #!/usr/bin/env python
-"""bench.py - accepted tok/s of the draft-then-verify step (BASELINE.json metric).
+"""bench.py - accepted tok/s of the draft-then-verify step.
 
-Workload (BASELINE.json configs[2]): Qwen2.5-7B draft -> Qwen2.5-32B target, bf16, chain k = 5,
+Workload: Qwen2.5-7B draft -> Qwen2.5-32B target, bf16, chain k = 5,
 batch 16, 512-token prefix, temperature 0.7, random-init weights, synthetic prompts.
   --gpus 1 : both models on one B200.
   --gpus N : the 32B target tensor-parallel over N ranks (NCCL all-reduce on the two row-parallel
@@ -140,10 +140,10 @@ def config_dict(wl, n_gpus, extra=None):
 
 # ------------------------------------------------------------------------------------------- reference arm
 def run_reference(args):
-    """CPU arm.  The line's ``value`` is the same metric on the same config as our arm (configs[2]); a full
+    """CPU arm.  The line's ``value`` is the same metric on the same config as our arm; a full
     7B -> 32B step on CPU takes minutes, so it is a bounded sample multiplied out (``"extrapolated": true``).
     Next to it ``cpu_baselines`` holds three MEASURED, un-extrapolated baselines: the stop
-    rule over 10^5 triples in CPython, the C sampler oracle on two config-2 grid points, and configs[0] end to end
+    rule over 10^5 triples in CPython, the C sampler oracle on two points of its grid, and the smallest pair end to end
     (HF Qwen2ForCausalLM fp32, 0.5B -> 1.5B, k = 4, greedy) - our arm reports the same three on the GPU."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -213,7 +213,7 @@ def tp_check(torch, dist, rank, world, dev, dec, target, tcfg):
     1. every rank's verify logits of the last timed step must be bit-identical (ranks stay in lock step without
        exchanging tokens only if they are), 2. no rank may have timed out waiting for a peer
        (asd_engine_tp_error), 3. a 2-layer model of the target's width is run on M = 96 tokens by the N-way sharded
-       engine and by a single-GPU engine on rank 0; their logits must agree within the north-star tolerance
+       engine and by a single-GPU engine on rank 0; their logits must agree within the tolerance of the engine tests
        (max-abs <= 2e-2 at logit std 0.25; they differ by fp32 summation order, which flips bf16 roundings)."""
     from dataclasses import replace
     from asd_b200.engine import QwenEngine
@@ -262,9 +262,9 @@ def tp_check(torch, dist, rank, world, dev, dec, target, tcfg):
 
 
 def config5(torch, dist, rank, world, dev, args, peaks):
-    """BASELINE configs[4]: Qwen2.5-72B verify-only at TP = N, batch 64, 4096-token prefix, k = 8 (576 tokens per
-    forward), paged KV.  The KV prefix is N(0,1) bf16 written straight into the paged pool (SURVEY 8d allows it
-    for the verify-only sweep: a real 64 x 4096-token prefill is 38 PFLOP); everything timed is the real forward."""
+    """Qwen2.5-72B verify-only at TP = N, batch 64, 4096-token prefix, k = 8 (576 tokens per
+    forward), paged KV.  The KV prefix is N(0,1) bf16 written straight into the paged pool (a real
+    64 x 4096-token prefill is 38 PFLOP); everything timed is the real forward."""
     from asd_b200.engine import QwenEngine
     from asd_b200.models.qwen2 import QWEN25
     cfg = QWEN25["72b"]
@@ -389,7 +389,7 @@ def companions(torch, dev, peak):
         del tl, dl, flush
     out["sampler"] = {"grid": grid, "what": "asd_reject_sample, L2 flushed between launches, median of 5"}
     torch.cuda.empty_cache()
-    # 0.5B -> 1.5B, k = 4, batch 1, greedy
+    # the smallest pair: 0.5B -> 1.5B, k = 4, batch 1, greedy
     t = QwenEngine(QWEN25["1.5b"], max_seqs=1, max_seq_len=1024, max_tokens=64, device=dev).load_random(seed=1)
     d = QwenEngine(QWEN25["0.5b"], max_seqs=1, max_seq_len=1024, max_tokens=64, device=dev).load_random(seed=0)
     dec = SpecDecoder(t, d, 1, 4, 0.0)
@@ -1060,7 +1060,7 @@ def main():
     ap.add_argument("--no-cpu-baseline", action="store_true")
     ap.add_argument("--no-companions", action="store_true", help="skip the stop-rule / sampler-grid / config-1 / Stage.generate records")
     ap.add_argument("--config5-only", action="store_true", help="N > 1: only the 72B verify-only record")
-    ap.add_argument("--no-config5", action="store_true", help="N > 1: skip the 72B verify-only record (BASELINE configs[4])")
+    ap.add_argument("--no-config5", action="store_true", help="N > 1: skip the 72B verify-only record")
     ap.add_argument("--no-fuse-norm", action="store_true", help="separate add+RMSNorm kernels instead of the fused epilogues")
     ap.add_argument("--nccl-only", action="store_true", help="TP boundaries through ncclAllReduce instead of the fused kernel")
     ap.add_argument("--opt", action="append", help="engine option name=value (e.g. pdl=0, attn_impl=0)")

@@ -53,7 +53,7 @@ ASD_API int asd_debug_wait_expiry(void* stream);
  * Replaces the per-token softmax/log + .item() loop of
  * src/training/generate_training_data.py:128-134 and the logprob reductions of
  * FeatureExtractor.extract (docs/guides/RESEARCH_PROTOCOL.md:379-398); the accept/resample rule is
- * the canonical speculative sampling of SURVEY.md Appendix C (no reference implementation).
+ * canonical speculative sampling (no reference implementation).
  *
  *   target_logits fp32 [B, k+1, V]   draft_logits fp32 [B, k, V] (may be NULL if k == 0 or T <= 0)
  *   draft_tokens  i32  [B, k]        u_accept fp64 [B, k]        u_resid fp64 [B]
@@ -91,7 +91,7 @@ ASD_API int asd_stop_rule_rows(const double* p, const double* C, const double* l
                        double alpha, double beta, int32_t* k_star, double* J, void* stream);
 ASD_API int asd_stop_rule_rows_host(const double* p, const double* C, const double* lam, int n, int L, int risk_adjustment,
                             double alpha, double beta, int32_t* k_star, double* J);
-/* Scorer -> stop decision in ONE launch, all on the device (north star 3; replaces the chain
+/* Scorer -> stop decision in ONE launch, all on the device (replaces the chain
  * FeatureExtractor.extract -> QualityPredictor.predict -> bayesian_adjustment -> optimal_stopping_rule of
  * src/serving/pipeline.py:225-256 for n requests that have just finished stage `stage_idx`):
  *   features fp32 [n, T, ASD_NUM_FEATURES]: the rows asd_reject_sample wrote for each request's generated tokens (still

@@ -1,11 +1,11 @@
-"""ORACLE-side CPU baseline for BASELINE configs[0]: Qwen2.5-0.5B draft -> Qwen2.5-1.5B target, random-init,
+"""ORACLE-side CPU baseline of the smallest pair: Qwen2.5-0.5B draft -> Qwen2.5-1.5B target, random-init,
 chain k = 4, batch 1, greedy, on the host cores (``bench.py --impl reference`` only).
 
 The reference's Stage is ``vllm.LLM`` / HF ``generate`` (src/serving/real_model_pipeline.py:98-108,
 src/training/generate_training_data.py:110-119): the CPU path it can actually run is HF ``Qwen2ForCausalLM``
 in fp32, so that is what is timed - the installed ``transformers`` model with its own KV cache, driven by a plain
-draft-then-verify loop (k draft forwards of 1 token, one (k+1)-token verify forward, greedy accept rule of
-SURVEY App. C).  A bounded number of steps; nothing here is extrapolated."""
+draft-then-verify loop (k draft forwards of 1 token, one (k+1)-token verify forward, greedy accept
+rule).  A bounded number of steps; nothing here is extrapolated."""
 from __future__ import annotations
 
 import os

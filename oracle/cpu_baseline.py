@@ -5,7 +5,7 @@ workload: ``sample_layers`` decoder layers of the target shape at M = B*(k+1) to
 shape at M = B tokens (fp32 math on bf16-valued weights, torch CPU with all host threads), both
 lm_heads, and the C sampler oracle on real-sized logits; the per-layer time is then multiplied out to
 the full depth.  The reference itself has no runnable CPU implementation of this path (its Stage is
-vLLM on GPU; SURVEY.md section 0), so the kind reported is "port"."""
+vLLM on GPU), so the kind reported is "port"."""
 from __future__ import annotations
 
 import math

@@ -5,7 +5,7 @@ src/algorithms/dp_solver.py and src/theory/optimal_stopping.py by file path, eva
 on seeded inputs and on the documented example (docs/guides/GETTING_STARTED.md:61-65), and
 stores inputs + outputs as C99 hex floats so the comparison is bit-exact.  Also drives the
 reference's UNMODIFIED src/serving/pipeline.py through stub stage/predictor modules
- and records the resulting RequestResult fields.
+and records the resulting RequestResult fields.
 """
 from __future__ import annotations
 

@@ -1,6 +1,6 @@
 """Golden vectors that pin oracle/sampler_oracle.c to an INDEPENDENT implementation of speculative rejection
 sampling: vLLM's ``vllm/v1/sample/rejection_sampler.py`` (the engine the reference's Stage wraps,
-/root/reference/src/serving/real_model_pipeline.py:98-108; the reference itself has no token-level sampler).
+src/serving/real_model_pipeline.py:98-108; the reference itself has no token-level sampler).
 
 vLLM's sampler is a set of Triton kernels; this script runs them ON THE CPU through the Triton interpreter
 (``TRITON_INTERPRET=1``) with OUR uniforms and records, per case, what vLLM decided:

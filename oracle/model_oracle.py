@@ -1,9 +1,9 @@
 """ORACLE (test infrastructure only): CPU fp32 restatement of the Qwen2 decoder forward.
 
 The reference never implements the model forward: Stage.generate delegates to vLLM
-(/root/reference/src/serving/real_model_pipeline.py:98-108,135; docs/guides/RESEARCH_PROTOCOL.md:233-304)
+(src/serving/real_model_pipeline.py:98-108,135; docs/guides/RESEARCH_PROTOCOL.md:233-304)
 and data generation to HF ``model.generate`` (src/training/generate_training_data.py:110-119).
-The arithmetic therefore lives in third-party code absent from /root/reference:
+The arithmetic therefore lives in third-party code absent from the reference:
 ``transformers>=4.40,<5`` (requirements.txt:5-6; docs pin transformers==4.40.0), class
 ``Qwen2ForCausalLM``.  This file restates its published algorithm (RMSNorm with eps inside rsqrt,
 rotate_half RoPE with theta = 1e6, GQA attention with QKV bias and 1/sqrt(head_dim) scale, SwiGLU MLP)
@@ -38,7 +38,7 @@ def qwen2_forward(w: dict, cfg, input_ids: torch.Tensor, positions: torch.Tensor
     """w: HF-named state dict (any float dtype, used in fp32); cfg has hidden_size, num_hidden_layers,
     num_attention_heads, num_key_value_heads, head_dim, rms_norm_eps, rope_theta.
     input_ids [B, T] -> logits fp32 [B, T, V] (``last_n``: only the last n positions, [B, n, V] - the lm_head
-    of a 152K vocabulary over every prefix position is most of the oracle's time at the BASELINE shapes)."""
+    of a 152K vocabulary over every prefix position is most of the oracle's time at the 32B shapes)."""
     B, T = input_ids.shape
     nh, nkv, hd = cfg.num_attention_heads, cfg.num_key_value_heads, cfg.head_dim
     f = lambda name: w[name].float()

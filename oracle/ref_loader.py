@@ -1,9 +1,8 @@
 """Load pieces of the reference by file path (ORACLE tooling; container-only).
 
-/root/reference cannot be imported as a package (``import src`` raises TypeError at
-src/core/interfaces.py:466) and does not exist on the GPU box, so
-this module is used only by ``oracle/gen_golden.py`` and by CPU tests that skip when
-the reference tree is absent.
+The reference cannot be imported as a package (``import src`` raises TypeError at
+src/core/interfaces.py:466) and is not everywhere these tests run, so this module is
+used only by ``oracle/gen_golden.py`` and by CPU tests that skip when the reference tree is absent.
 """
 from __future__ import annotations
 
@@ -40,8 +39,8 @@ def optimal_stopping():
 
 def pipeline_module(stage_module, predictor_module):
     """The reference's UNMODIFIED src/serving/pipeline.py, importable through a synthetic
-    parent package whose ``models.stage`` / ``models.predictor`` are the given modules
-    (SURVEY.md Appendix F).  ``start_time`` (pipeline.py:269 reads an undefined global)
+    parent package whose ``models.stage`` / ``models.predictor`` are the given modules.
+    ``start_time`` (pipeline.py:269 reads an undefined global)
     is injected so a request can complete."""
     for pkg in ("refsrc", "refsrc.models", "refsrc.algorithms", "refsrc.serving"):
         m = types.ModuleType(pkg)

@@ -1,7 +1,7 @@
 /*
  * ORACLE (test infrastructure only - never imported by the product path).
  *
- * Pinning.  The reference contains no token-level rejection sampler (SURVEY.md section 0 fact 2, section 8c): it
+ * Pinning.  The reference contains no token-level rejection sampler: it
  * delegates generation to vLLM (requirements.txt:10 "vllm>=0.8.3"; src/serving/real_model_pipeline.py:98-108), so
  * there is no reference implementation, test or golden vector of its own to pin this file to - against the REFERENCE
  * the parity is unpinned.  It is pinned to that third-party dependency instead: tests/golden/sampler_vllm_golden.json
@@ -9,7 +9,7 @@
  * and our uniforms - accepted lengths under rejection_random_sample_kernel, whole output rows under
  * rejection_greedy_sample_kernel - generated by oracle/gen_sampler_golden.py (Triton interpreter, CPU) and replayed
  * through this file by tests/test_oracle_sampler_vllm.py in the CPU suite.  The rule restated is the canonical one the
- * reference cites (docs/papers/FINAL_PAPER.md:22,285; SURVEY.md Appendix C):
+ * reference cites (docs/papers/FINAL_PAPER.md:22,285):
  *     accept x_i  iff  u_i <= min(1, p_i(x_i)/q_i(x_i));
  *     on the first reject resample from normalise(max(0, p - q)); bonus token from p_{k+1};
  * plus the reference's only vocab-wide arithmetic, softmax + log(probs[token])
@@ -19,8 +19,8 @@
  * distribution, not token by token) and tests/test_sampler_vllm_gpu.py (the CUDA kernel against the same vLLM
  * kernels on the GPU).
  *
- * Because fp32 sums are order dependent, the ARITHMETIC CONTRACT below is part of the definition
- * (SURVEY.md section 7 hard part 2).  The CUDA kernels (csrc/sampler.cu) implement the same contract;
+ * Because fp32 sums are order dependent, the ARITHMETIC CONTRACT below is part of the definition.
+ * The CUDA kernels (csrc/sampler.cu) implement the same contract;
  * this file states it with plain loops.  Contract v2 ("chunked streaming": every logit is read from
  * HBM once by an independent 4096-element chunk, no vocabulary-wide exchange before the exponentials):
  *

@@ -2,10 +2,10 @@
  * ORACLE (test infrastructure only - never imported by the product path).
  *
  * CPU restatement, in plain C, of the reference's optimal-stopping policy:
- *   optimal_stopping_rule      /root/reference/src/algorithms/dp_solver.py:12-71
- *   compute_expected_cost      /root/reference/src/algorithms/dp_solver.py:74-103
- *   bayesian_adjustment        /root/reference/src/algorithms/dp_solver.py:106-130
- *   derive_optimal_policy      /root/reference/src/theory/optimal_stopping.py:45-91
+ *   optimal_stopping_rule      src/algorithms/dp_solver.py:12-71
+ *   compute_expected_cost      src/algorithms/dp_solver.py:74-103
+ *   bayesian_adjustment        src/algorithms/dp_solver.py:106-130
+ *   derive_optimal_policy      src/theory/optimal_stopping.py:45-91
  *
  * CPython floats are IEEE binary64 and every operation below is a single
  * correctly-rounded binary64 add / sub / mul / div, so replaying the same

@@ -1,9 +1,8 @@
 """ORACLE (test infrastructure / CPU baseline only): the stop rule exactly as the reference executes it - CPython
-floats, one request at a time - restated from /root/reference/src/algorithms/dp_solver.py:12-71 (backward induction)
+floats, one request at a time - restated from src/algorithms/dp_solver.py:12-71 (backward induction)
 and :106-130 (Beta-posterior shrinkage).  Pinned by tests/golden/stop_rule_golden.json (reference-generated, hex
 floats).  ``bench.py --impl reference`` times it over 10^5 (p, C, lambda) triples on one core, which is what
-the reference's own per-request call costs; /root/reference itself does not exist on the
-GPU box."""
+the reference's own per-request call costs."""
 from __future__ import annotations
 
 import time
@@ -38,7 +37,7 @@ def optimal_stopping_rule(p, C, lam, risk_adjustment=False, alpha=1.0, beta=1.0)
 
 
 def make_triples(n=100_000, seed=7):
-    """BASELINE.md section 4: L in {3, 4}, C = [1, 4.5, 10] / [1, 2, 4.5, 10], lambda in {0.1 .. 10}"""
+    """L in {3, 4}, C = [1, 4.5, 10] / [1, 2, 4.5, 10], lambda in {0.1 .. 10}"""
     import numpy as np
     rng = np.random.default_rng(seed)
     lams = rng.choice([0.1, 0.5, 1.0, 2.0, 5.0, 10.0], n)

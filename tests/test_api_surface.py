@@ -150,7 +150,7 @@ def test_feature_extractor_and_predictor_follow_the_listing():
     p = QualityPredictor(feature_dim=256)
     v = p.predict(prompt="a b", draft_output="c", draft_logprobs=flp, stage_id=0, feature_extractor=FeatureExtractor())
     assert 0.0 < v < 1.0
-    assert sum(x.numel() for x in p.parameters()) == 33025     # SURVEY.md 8(a6)
+    assert sum(x.numel() for x in p.parameters()) == 33025
     assert 0.0 < QualityPredictor({"feature_dim": 128}).predict(np.zeros(128, np.float32)) < 1.0
 
 
@@ -209,7 +209,7 @@ def test_training_feature_vector_matches_the_reference_layout(tmp_path):
 
 
 def test_http_server_mirrors_the_reference_endpoints():
-    """SURVEY 8 (f2): same routes, schemas, validation bounds and status codes as src/serving/server.py:223-376"""
+    """same routes, schemas, validation bounds and status codes as src/serving/server.py:223-376"""
     from fastapi.testclient import TestClient
     from asd_b200.serving.server import create_app
 
@@ -285,7 +285,7 @@ def test_batched_cascade_matches_the_sequential_decisions():
 
 
 def test_predictor_training_on_saved_rows(tmp_path):
-    """SURVEY 8 (f4): rows written by save_training_data train the reference's MLP recipe (K-fold, AdamW, MSE)"""
+    """rows written by save_training_data train the reference's MLP recipe (K-fold, AdamW, MSE)"""
     import json
     import torch
     from asd_b200.training.generate_training_data import TrainingSample, extract_features, save_training_data

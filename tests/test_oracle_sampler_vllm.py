@@ -1,4 +1,4 @@
-"""The sampler ORACLE against an independent implementation, in the CPU suite (SURVEY 8c: the reference has no
+"""The sampler ORACLE against an independent implementation, in the CPU suite (the reference has no
 token-level sampler, so the restatement is pinned to the one public implementation of canonical speculative
 sampling in this image): tests/golden/sampler_vllm_golden.json holds what vLLM's rejection-sampler kernels
 (vllm/v1/sample/rejection_sampler.py, run on the CPU through the Triton interpreter by

@@ -16,7 +16,7 @@ def test_stopping_rule_golden(stop_rule_golden):
 
 
 def test_documented_example(stop_rule_golden):
-    # docs/guides/GETTING_STARTED.md:61-65 (SURVEY.md Appendix B row 1)
+    # docs/guides/GETTING_STARTED.md:61-65
     k, J = oracle.optimal_stopping_rule([0.3, 0.5, 0.7, 0.9], [1.0, 1.6, 4.2, 8.8], 1.0)
     assert k == 0 and J == [1.7, 2.45, 5.095000000000001, 8.8, 0.0]
     k, J = oracle.optimal_stopping_rule([0.6, 1.0], [1.0, 4.5], 12.0)
@@ -47,7 +47,7 @@ def test_length_mismatch_raises():
         oracle.optimal_stopping_rule([0.5], [1.0, 2.0], 1.0)
 
 
-@pytest.mark.skipif(not ref_loader.available(), reason="/root/reference not present (GPU box)")
+@pytest.mark.skipif(not ref_loader.available(), reason="the reference is not present")
 def test_oracle_matches_live_reference():
     import random
     dp = ref_loader.dp_solver()

@@ -1,6 +1,6 @@
 """The persistent forward kernel (engine option persist = 1: the whole forward in ONE cooperative launch, stream-K split
 of every GEMM over all SMs, phase counters instead of kernel boundaries) against the per-kernel path and the CPU
-oracle: same north-star bar (max-abs <= 2e-2), and no device-side wait may have run into its bound."""
+oracle: same bar (max-abs <= 2e-2), and no device-side wait may have run into its bound."""
 import pytest
 import torch
 

@@ -102,7 +102,7 @@ def test_parity_row_sampling_k0_and_host_entry():
 
 
 def test_first_reject_prefix_property_full_size():
-    """size-independent property at the BASELINE config-2 maximum (B=256, k=8): accepted prefix
+    """size-independent property at the largest batch (B=256, k=8): accepted prefix
     is a prefix, emitted tokens = draft prefix + one token, rest -1; draft == target accepts all."""
     import torch
     from asd_b200.ops import RejectionSampler
@@ -134,7 +134,7 @@ def test_first_reject_prefix_property_full_size():
 
 @pytest.mark.parametrize("B", [64, 128, 256])
 def test_full_batch_every_row_against_oracle(B):
-    """BASELINE config-2 batch sizes at k = 8, V = 152064: EVERY sequence compared with the C oracle"""
+    """batch sizes of the sampler grid at k = 8, V = 152064: EVERY sequence compared with the C oracle"""
     k, V, T = 8, 152064, 0.7
     tl, dl, dt, ua, ur = make_case(B, k, V, seed=500 + B, T=T)
     compare(run_gpu(tl, dl, dt, ua, ur, T), oracle.reject_sample(tl, dl, dt, ua, ur, T))

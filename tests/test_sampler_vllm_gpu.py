@@ -1,4 +1,4 @@
-"""Independent pin of the fused rejection sampler (SURVEY 8c): the reference has no token-level sampler, so
+"""Independent pin of the fused rejection sampler: the reference has no token-level sampler, so
 the accept rule is checked against the one public implementation of canonical speculative sampling installed
 in this image, vLLM's ``vllm/v1/sample/rejection_sampler.py`` (the engine the reference's Stage wraps,
 src/serving/real_model_pipeline.py:98-108): its Triton kernels are called directly with OUR uniforms -

@@ -69,7 +69,7 @@ def test_real_model_pipeline_surface():
 
 
 def test_calibrate_costs_replaces_the_cost_table():
-    """SURVEY 8 f3 (real_model_pipeline.py:313-362): measured per-token time, normalised to the first stage"""
+    """(real_model_pipeline.py:313-362): measured per-token time, normalised to the first stage"""
     from asd_b200.models.stage import StageConfig, StageManager
     scs = [StageConfig("tiny-a", "7b", config=tiny_config(num_hidden_layers=1)),
            StageConfig("tiny-b", "32b", config=tiny_config(num_hidden_layers=2))]

@@ -58,7 +58,7 @@ def test_table_and_adaptive_match_live_reference():
     """OptimalStoppingTable (one batched call) and AdaptiveStopping against the reference's own classes"""
     from oracle import ref_loader
     if not ref_loader.available():
-        pytest.skip("/root/reference not present (GPU box)")
+        pytest.skip("the reference is not present")
     ref = ref_loader.dp_solver()
     rng = np.random.default_rng(11)
     lams = [0.1, 0.5, 1.0, 2.0, 5.0, 10.0]

@@ -1,6 +1,6 @@
-"""In-process tensor parallelism behind the reference-facing seam (SURVEY 8 rows a11 / n2): ``TPQwenEngine`` and
+"""In-process tensor parallelism behind the reference-facing seam: ``TPQwenEngine`` and
 ``Stage(tensor_parallel_size=t, gpu_ids=[...])`` - t rank engines on t GPUs of ONE process, row-parallel
-boundaries over peer-mapped memory - against the CPU oracle, against the single-GPU engine at the BASELINE
+boundaries over peer-mapped memory - against the CPU oracle, against the single-GPU engine at full
 widths, and through ``StageManager`` + ``AdaptiveSpeculativePipeline`` with the reference's placement
 (7B on its own GPU, 32B TP=2, 72B TP=4; configs/qwen3_models.yaml:10-51).  Skipped below the GPU count needed."""
 from dataclasses import replace
@@ -49,9 +49,9 @@ def test_tp2_inprocess_matches_oracle(mode):
 @pytest.mark.skipif(NGPU < 2, reason="needs 2 GPUs")
 @pytest.mark.parametrize("tp", [2, 4, 8])
 def test_tp_inprocess_32b_width_matches_single_gpu(tp):
-    """2 layers of the 32B shape at M = 96 (the verify shape of BASELINE configs[2]): the sharded engine must
+    """2 layers of the 32B shape at M = 96 (the verify shape of the benchmark): the sharded engine must
     agree with the single-GPU engine (itself checked against the oracle in test_engine_baseline_shapes_gpu.py)
-    within the north-star tolerance.  The two differ only in the fp32 summation order of the row-parallel partials,
+    within the tolerance of the engine tests.  The two differ only in the fp32 summation order of the row-parallel partials,
     but an fp32 difference in the last bit flips bf16 roundings of the next GEMM's operand, so the worst of the
     14.6 million compared logits sits at about half the bf16-vs-fp32 error (measured 0.012 at max|logit| 2.1)."""
     if NGPU < tp:
@@ -83,7 +83,7 @@ def test_tp_inprocess_32b_width_matches_single_gpu(tp):
 @pytest.mark.skipif(NGPU < 2, reason="needs 2 GPUs")
 @pytest.mark.parametrize("tp,two_shot", [(2, 0), (2, 1), (4, 0), (4, -1), (8, 0)])
 def test_tp_inprocess_large_verify_matches_single_gpu(tp, two_shot):
-    """M = 320 tokens (> 256: the tensor-bound CTA-pair GEMM, BASELINE configs[4]'s regime; 6.5 MB per boundary): O
+    """M = 320 tokens (> 256: the tensor-bound CTA-pair GEMM; 6.5 MB per boundary): O
     through the weight-streaming kernel with the fused exchange (two ranks) or the all-reduce kernel, down through the
     CTA-pair kernel + slice reduction + all-reduce kernel (one-shot / two-shot, tp_two_shot forces either).  All must
     agree with one GPU."""
@@ -127,7 +127,7 @@ def _cascade_placement():
 
 @pytest.mark.skipif(NGPU < 3, reason="needs >= 3 GPUs (7B on GPU 0, 32B TP=2 on GPUs 1-2; 72B TP=4 with >= 7)")
 def test_stage_manager_cascade_with_tensor_parallel_stages():
-    """BASELINE configs[3]: 7B -> 32B (TP=2) -> 72B (TP=4) on disjoint GPUs through StageManager and the pipeline,
+    """7B -> 32B (TP=2) -> 72B (TP=4) on disjoint GPUs through StageManager and the pipeline,
     layer-truncated (2 layers each) at the real widths and vocabulary."""
     from asd_b200.models.predictor import FeatureExtractor, QualityPredictor
     from asd_b200.models.stage import StageConfig, StageManager

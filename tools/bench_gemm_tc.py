@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Times the 72B shard GEMM shapes of BASELINE configs[4] (576 tokens) on both kernels:
+"""Times the 72B shard GEMM shapes of a verification of 576 tokens on both kernels:
 the weight-streaming kernel (asd_linear_bf16) and the tensor-bound CTA-pair kernel (asd_linear_bf16_tc)."""
 import ctypes
 import json

@@ -1,4 +1,4 @@
-"""One rank's share of BASELINE configs[4] on ONE GPU (72B sharded t ways as local dims, 2 layers, no exchange):
+"""One rank's share of the 72B verification on ONE GPU (72B sharded t ways as local dims, 2 layers, no exchange):
 for ncu launch lists of the per-rank GEMM / attention shapes."""
 import os, sys
 from dataclasses import replace
