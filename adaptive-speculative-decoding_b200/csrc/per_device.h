@@ -10,7 +10,8 @@ namespace asd {
 int set_error(const char* fmt, ...);     // records the message, returns -1
 
 // cudaFuncSetAttribute and module loads are per device.  `run` calls `set` on the current device until one call of it has returned 0;
-// a thread that meets another's call waits for its end, so that no first launch overtakes the attribute it needs.
+// a thread that meets another's call on its device waits for its end, so that no first launch overtakes the attribute it needs.
+// Devices do not wait for one another: a module load may wait for its device, whose kernels may wait for a rank on another one.
 class PerDeviceOnce {
 public:
     template <typename F>
@@ -19,7 +20,7 @@ public:
         cudaGetDevice(&dev);
         const unsigned long long bit = 1ull << (dev & 63);
         if (done_.load(std::memory_order_acquire) & bit) return 0;
-        std::lock_guard<std::mutex> hold(lock_);
+        std::lock_guard<std::mutex> hold(lock_[dev & 63]);
         if (done_.load(std::memory_order_relaxed) & bit) return 0;
         const int rc = set();
         if (rc == 0) done_.fetch_or(bit, std::memory_order_release);
@@ -28,7 +29,7 @@ public:
 
 private:
     std::atomic<unsigned long long> done_{0};
-    std::mutex lock_;
+    std::mutex lock_[64];
 };
 
 // the statements (which may return -1, as ASD_CUDA does) once per device, in a function that returns -1 on failure

@@ -36,6 +36,16 @@ static int fails_once() {
     ASD_ONCE(failing, if (++tries == 1) return -1);
     return 0;
 }
+static asd::PerDeviceOnce apart;
+static std::atomic<int> second_done{0}, waited{0};
+static int across() {                                   // device 0's work ends only after device 1's
+    ASD_ONCE(apart, {
+        if (device == 1) second_done.store(1);
+        for (int i = 0; device == 0 && i < 500 && !second_done.load(); ++i) std::this_thread::sleep_for(std::chrono::milliseconds(10));
+        if (device == 0 && !second_done.load()) waited.store(1);
+    });
+    return 0;
+}
 static std::atomic<int> asked{0}, half{0};
 extern "C" cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr attr, int dev) {
     asked.fetch_add(1);
@@ -64,6 +74,11 @@ int main() {
     device = 2;
     for (int i = 0; i < 4; ++i) limits();
     printf(" %d\n", half.load());
+    std::thread a([] { device = 0; across(); });
+    std::this_thread::sleep_for(std::chrono::milliseconds(50));
+    std::thread b([] { device = 1; across(); });
+    a.join(), b.join();
+    printf("%d %d\n", second_done.load(), waited.load());
 }
 """
 
@@ -86,6 +101,11 @@ def test_no_thread_goes_on_before_the_first_has_finished(lines):
 def test_no_thread_sees_half_of_a_devices_limits(lines):
     """two questions a device, both answers for everyone; a device that could not be read is asked again"""
     assert lines[1].split() == ["4", "0", "2"]
+
+
+def test_devices_do_not_wait_for_one_another(lines):
+    """a rank's first launch on one device, held up by kernels that wait for a rank on another, whose first launch is still to come"""
+    assert lines[2].split() == ["1", "0"]
 
 
 def test_every_size_of_shared_memory_is_allowed_once():
