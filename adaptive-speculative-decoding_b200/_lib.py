@@ -181,6 +181,7 @@ def lib() -> ctypes.CDLL:
         "asd_mezilix_destroy": (None, [vp]),
         "asd_mezilix_set_globals": (i32, [vp, vp, vp, vp, vp]),
         "asd_mezilix_set_layer": (i32, [vp, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp]),
+        "asd_mezilix_set_latent_up": (i32, [vp, i32, vp]),
         "asd_mezilix_cache_bytes": (sz, [vp, i32]),
         "asd_mezilix_set_cache": (i32, [vp, vp, i32, vp, i32, i32, vp, vp]),
         "asd_mezilix_set_option": (i32, [vp, c.c_char_p, i32]),

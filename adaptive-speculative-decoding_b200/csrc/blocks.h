@@ -121,6 +121,10 @@ int launch_latent_post(const SeqIndex& ix, const float* qd, const LatentDims& d,
 int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv,
                              const LatentDims& d, const void* c_norm, int wf32, float eps, const float* inv_freq,
                              const PagedRows& cache, float* q_lat, cudaStream_t stream, __nv_bfloat16* q_terms = nullptr);
+// The same for launch_latent_prompt: the queries' rotated parts are turned where they are.
+int launch_latent_post_inplace(const SeqIndex& ix, float* q, long long ldq, const float* kv, long long ldkv, const LatentDims& d,
+                               const void* c_norm, int wf32, float eps, const float* inv_freq, const PagedRows& cache,
+                               cudaStream_t stream);
 // Workspace of the register-tiled kernel when it cuts a long key range into shares (few query rows, long context):
 // o [o_elems] floats, ml [2 * rows] floats; (token, head) pairs x shares must fit `rows`.  tiled = 0 forces the
 // one-warp-per-pair kernel, which takes any latent size; 1 the register-tiled fp32 kernel where the sizes allow; 2 (default)
@@ -146,6 +150,22 @@ bool latent_attention_tc_takes(const LatentDims& d, const PagedRows& cache, int 
 int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen,
                                int max_kv_len, const __nv_bfloat16* q_terms, const LatentDims& d, const PagedRows& cache,
                                float* out_lat, const AttnSplit& ws, int* err, cudaStream_t stream);
+
+// ---------------------------------------------------------------------------------------------- latent_prompt_tc.cu
+// The same from the queries as they are (no head products before or behind): out bf16 [M][heads * dv] = the softmax's sum carried
+// through the value up-projection, for calls whose sequences bring about as many tokens as they see positions (`takes`).
+struct LatentPromptWs {
+    const void* w = nullptr;             // bf16 [heads * (dn + dv)][R]: rows of the heads' key up-projections, then of their value up-projections
+    void* rows = nullptr;                // scratch for the visible cache rows, and for two bf16 terms of what they become
+    __nv_bfloat16* planes = nullptr;
+    long long row_elems = 0, plane_elems = 0;
+    int mode = 1;                        // 0 never, 1 where it measured better, 2 wherever the sizes allow
+};
+bool latent_prompt_takes(const LatentDims& d, const PagedRows& cache, int M, int nseq, int max_qlen, int max_kv_len, const float* q,
+                         long long ldq, const LatentPromptWs& ws, int tiled);
+int launch_latent_prompt(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen, int max_kv_len,
+                         const float* q, long long ldq, const LatentDims& d, const PagedRows& cache, const LatentPromptWs& ws,
+                         void* out, int* err, cudaStream_t stream);
 
 // ---------------------------------------------------------------------------------------------- linear_few.cu
 // y fp32 [M][ldc] = x bf16 [M][K] * w bf16 [N][K]^T for a few tokens (M <= 16)

@@ -6,7 +6,7 @@
 
 namespace asd {
 
-enum GemmOut { GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2, GEMM_OUT_QKV = 3, GEMM_OUT_RELU2 = 4 };
+enum GemmOut { GEMM_OUT_F32 = 0, GEMM_OUT_BF16 = 1, GEMM_OUT_SWIGLU = 2, GEMM_OUT_QKV = 3, GEMM_OUT_RELU2 = 4, GEMM_OUT_TERMS = 5 };
 
 // Fused RMSNorm.  Producer side (fp32 accumulate epilogue of the O / down projection): besides the fp32
 // residual v it writes x = bf16(v * ln_w[n]) (the next norm's weight applied per column, NOT yet divided by
@@ -101,6 +101,10 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
 struct SimtLinear;
 bool gemm_tc_grouped_takes(const SimtLinear& L, int groups, long long rows, int min_rows);
 int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream_t stream);
+
+// The same kernel with results as two bf16 terms (y = high + low to 16 bits) in two planes: out [2][M][N] from x rows ldx elements apart,
+// any number of rows; N a multiple of 8.
+int launch_gemm_tc_terms(const void* x, long long ldx, const void* w, int M, int N, int K, void* out, cudaStream_t stream);
 
 // ---- one token (gemv.cu): CUDA cores, weight rows straight into registers
 bool gemv_takes(int M, int max_k, size_t max_bytes);

@@ -112,8 +112,8 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, const void* src_s
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(tmap), "r"(smem_u32(src_smem)),
                  "r"(c0), "r"(c1), "r"(c2)
                  : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void tma_store_wait_read() {      // at most N of this thread's stores still read shared memory
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
@@ -157,10 +157,13 @@ __device__ __forceinline__ TcUnit tc_group_unit(const TcArgs& a, const int2* tab
     return r;
 }
 
-template <bool GROUPED>
+enum TcForm { TC_PLAIN, TC_GROUPED, TC_TERMS };      // instances: what the others do costs none of their instructions
+
+template <TcForm FORM>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
     gemm_tc_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                    const __grid_constant__ CUtensorMap tmap_o, const TcArgs a) {
+    constexpr bool GROUPED = FORM == TC_GROUPED, TERMS = FORM == TC_TERMS;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int b_bytes = (a.MT / 2) * 128;
@@ -291,7 +294,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * kTcAccCols);
             const int m0 = t.m0;
             const int tile128 = t.w_tile * 2 + (int)rank;          // 128-row weight tile this CTA holds
-            if (a.mode == GEMM_OUT_SWIGLU) {
+            if (!TERMS && a.mode == GEMM_OUT_SWIGLU) {
                 __nv_bfloat16* out = static_cast<__nv_bfloat16*>(a.out);
                 const bool wide = (a.ldo & 7) == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0;
 #pragma unroll 1
@@ -329,7 +332,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                         }
                     }
                 }
-            } else if (a.tma_out) {
+            } else if (TERMS || a.tma_out) {
                 const int rows = min(a.MT, t.m_end - m0);
                 if (tile128 * 128 < a.n_valid) {
                     const bool half_out = GROUPED && a.mode == GEMM_OUT_RELU2;
@@ -361,7 +364,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                                 }
                             break;
                         }
-                        if (half_out) {
+                        if constexpr (TERMS) {         // half a buffer a term
+                            __nv_bfloat16* H = reinterpret_cast<__nv_bfloat16*>(T);
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                const float v = __uint_as_float(r[i]);
+                                const __nv_bfloat16 hi = __float2bfloat16(v);
+                                H[i * 128 + row] = hi;
+                                H[(kTcOutTok + i) * 128 + row] = __float2bfloat16(v - __bfloat162float(hi));
+                            }
+                        } else if (half_out) {
                             __nv_bfloat16* H = reinterpret_cast<__nv_bfloat16*>(T);
 #pragma unroll
                             for (int i = 0; i < 16; ++i) {
@@ -378,6 +390,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kTcThreads, 1)
                         asm volatile("bar.sync 1, 128;" ::: "memory");
                         if (et == 0) {
                             tma_store_3d(&tmap_o, T, tile128 * 128, m0 + c0, t.ks);      // rows beyond the result are clipped
+                            if (TERMS) tma_store_3d(&tmap_o, T + kTcOutTok * 64, tile128 * 128, m0 + c0, 1);
+                            tma_store_commit();
                             tma_store_wait_read<kTcOutBufs - 2>();
                         }
                         if (++buf == kTcOutBufs) buf = 0;
@@ -498,8 +512,8 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     ASD_ONCE(g_tc_attr, {
         DeviceLimits dev;
         if (device_limits(&dev)) return -1;
-        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
-        prefer_max_smem(gemm_tc_kernel<false>);
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<TC_PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
+        prefer_max_smem(gemm_tc_kernel<TC_PLAIN>);
     });
     if (norm && !pl.norm) return set_error("gemm_tc: the plan has no place for a norm's factors");
     if (accumulate && (pl.mode != GEMM_OUT_F32 || pl.ksplit != 1))
@@ -531,7 +545,7 @@ int gemm_tc_launch(const TcPlan& pl, const CUtensorMap& tmap_w, const CUtensorMa
     a.err = wait_word();
     // plainly (ptx.cuh); its successor may start early.  Eight prompts of 500 to 1000 tokens through two 32B layers, forwards of
     // 2048 tokens: 13.4 to 13.7 ms launched programmatically, 13.5 to 14.4 so (power cap; boxes differ by as much)
-    gemm_tc_kernel<false><<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, to, a);
+    gemm_tc_kernel<TC_PLAIN><<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tmap_w, tmap_x, to, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_PAIR);
     return 0;
@@ -572,12 +586,42 @@ int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream
     if (device_limits(&dev)) return -1;
     static PerDeviceOnce once;
     ASD_ONCE(once, {
-        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
-        prefer_max_smem(gemm_tc_kernel<true>);
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<TC_GROUPED>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
+        prefer_max_smem(gemm_tc_kernel<TC_GROUPED>);
     });
-    gemm_tc_kernel<true><<<dev.sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
+    gemm_tc_kernel<TC_GROUPED><<<dev.sms / 2 * 2, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_GEMM_GROUPED);
+    return 0;
+}
+
+int launch_gemm_tc_terms(const void* x, long long ldx, const void* w, int M, int N, int K, void* out, cudaStream_t stream) {
+    DeviceLimits dev;
+    if (device_limits(&dev)) return -1;
+    static PerDeviceOnce once;
+    ASD_ONCE(once, {
+        ASD_CUDA(cudaFuncSetAttribute(gemm_tc_kernel<TC_TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, dev.smem_optin));
+        prefer_max_smem(gemm_tc_kernel<TC_TERMS>);
+    });
+    if (N % 8) return set_error("gemm_tc: rows of terms must be multiples of 16 bytes");
+    __nv_bfloat16* const planes = static_cast<__nv_bfloat16*>(out);
+    for (int m = 0; m < M; m += kTcMaxTokens) {
+        const int rows = std::min(kTcMaxTokens, M - m);
+        TcPlan pl;
+        if (gemm_tc_plan(&pl, rows, N, K, GEMM_OUT_F32, 1, 0, false)) return -1;
+        TcArgs a = {};
+        a.M = rows, a.N = N, a.K = K, a.MT = pl.MT, a.m_tiles = pl.m_tiles, a.w_tiles = pl.w_tiles, a.kblocks = pl.kblocks, a.ksplit = 1;
+        a.stages = pl.stages, a.mode = GEMM_OUT_TERMS;
+        a.ldo = N, a.n_valid = N, a.out = planes + (size_t)m * N, a.tma_out = 1;
+        a.err = wait_word();
+        CUtensorMap tw, tx, to;
+        if (make_tmap_bf16(&tw, w, N, K, K, 128)) return -1;
+        if (make_tmap_bf16(&tx, static_cast<const __nv_bfloat16*>(x) + (size_t)m * ldx, rows, K, ldx, pl.MT / 2)) return -1;
+        if (make_tmap_out(&to, a.out, true, rows, N, 2, N, (size_t)M * N, 128, kTcOutTok)) return -1;
+        gemm_tc_kernel<TC_TERMS><<<2 * pl.pairs, kTcThreads, pl.smem_bytes, stream>>>(tw, tx, to, a);       // plainly (ptx.cuh)
+        ASD_CUDA(cudaGetLastError());
+        count_kernel(KERNEL_GEMM_PAIR);
+    }
     return 0;
 }
 
@@ -585,7 +629,7 @@ int launch_gemm_tc_grouped(const SimtLinear& L, int groups, int rows, cudaStream
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_gemm_tc() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_tc_kernel<false>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, gemm_tc_kernel<TC_PLAIN>));
     return 0;
 }
 

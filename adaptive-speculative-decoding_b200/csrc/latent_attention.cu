@@ -30,7 +30,7 @@ __device__ __forceinline__ long long cache_row(const PagedRows& c, int slot, int
 // 4096 tokens, 16 heads, latent 512 + 64: 36 -> 30 us; 16 tokens: 13 -> 7 (a sincosf per coordinate and head before).
 __global__ void latent_post_kernel(SeqIndex ix, const float* q, long long ldq, const float* kvp, long long ldkv,
                                    LatentDims d, const void* c_norm, int wf32, float eps, const float* inv_freq,
-                                   PagedRows cache, float* q_lat, __nv_bfloat16* q_terms, long long plane) {
+                                   PagedRows cache, float* q_lat, __nv_bfloat16* q_terms, long long plane, float* q_own) {
     pdl_enter();
     extern __shared__ float2 turn[];   // cos, sin of the token's angles: once a token, not once a head and coordinate
     __shared__ float red[32];
@@ -69,6 +69,8 @@ __global__ void latent_post_kernel(SeqIndex ix, const float* q, long long ldq, c
     auto put = [&](int vec, int i, float x) {
         if (vec == 0) {
             stx(cache.pool, crow + d.R + i, cache.f32, x);
+        } else if (q_own) {                // (a pair is this thread's alone)
+            q_own[(long long)m * ldq + (long long)(vec - 1) * qw + d.dn + i] = x;
         } else {
             const long long at = ((long long)m * d.heads + (vec - 1)) * rw + d.R + i;
             if (q_terms)
@@ -916,20 +918,31 @@ int launch_latent_combine(const float* ws_o, const float* ws_ml, int nsplit, int
     return 0;
 }
 
-int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv,
-                             const LatentDims& d, const void* c_norm, int wf32, float eps, const float* inv_freq,
-                             const PagedRows& cache, float* q_lat, cudaStream_t stream, __nv_bfloat16* q_terms) {
+static int latent_post(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv, const LatentDims& d,
+                       const void* c_norm, int wf32, float eps, const float* inv_freq, const PagedRows& cache, float* q_lat,
+                       __nv_bfloat16* q_terms, float* q_own, cudaStream_t stream) {
     if (ix.M <= 0) return 0;
     if (d.rot_dims < 0 || d.rot_dims > d.dr || (d.rot_dims & 1))
         return set_error("latent attention: rot_dims %d must be even and <= %d", d.rot_dims, d.dr);
     static PerDeviceOnce once;
     ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(latent_post_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
-    ASD_CUDA(launch_pdl(latent_post_kernel, ix.M, 256, std::max(d.rot_dims / 2, 1) * sizeof(float2), stream, ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq,
-                        cache, q_lat, q_terms,
-                                               (long long)ix.M * d.heads * (d.R + d.dr)));
+    ASD_CUDA(launch_pdl(latent_post_kernel, ix.M, 256, std::max(d.rot_dims / 2, 1) * sizeof(float2), stream, ix, q, ldq, kv, ldkv, d,
+                        c_norm, wf32, eps, inv_freq, cache, q_lat, q_terms, (long long)ix.M * d.heads * (d.R + d.dr), q_own));
     count_launch(1);
     ASD_CUDA(cudaGetLastError());
     return 0;
+}
+
+int launch_latent_post_split(const SeqIndex& ix, const float* q, long long ldq, const float* kv, long long ldkv,
+                             const LatentDims& d, const void* c_norm, int wf32, float eps, const float* inv_freq,
+                             const PagedRows& cache, float* q_lat, cudaStream_t stream, __nv_bfloat16* q_terms) {
+    return latent_post(ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq, cache, q_lat, q_terms, nullptr, stream);
+}
+
+int launch_latent_post_inplace(const SeqIndex& ix, float* q, long long ldq, const float* kv, long long ldkv, const LatentDims& d,
+                               const void* c_norm, int wf32, float eps, const float* inv_freq, const PagedRows& cache,
+                               cudaStream_t stream) {
+    return latent_post(ix, q, ldq, kv, ldkv, d, c_norm, wf32, eps, inv_freq, cache, nullptr, nullptr, q, stream);
 }
 
 int launch_latent_post(const SeqIndex& ix, const float* qd, const LatentDims& d, const void* c_norm, int wf32, float eps,

@@ -28,7 +28,7 @@ namespace asd {
 struct MzLayer {
     asd_mezilix_layer_config c;
     const void *gain = nullptr, *shift = nullptr, *coeff = nullptr, *wqd = nullptr, *latent_gain = nullptr, *wuk = nullptr,
-               *wuv = nullptr, *wo = nullptr, *router = nullptr, *w_up = nullptr, *w_down = nullptr;
+               *wukv = nullptr, *wuv = nullptr, *wo = nullptr, *router = nullptr, *w_up = nullptr, *w_down = nullptr;
     float* inv_freq = nullptr;   // owned, [rot_dims / 2]
     size_t cache_off = 0;        // elements from the pool start (set by set_cache)
     int nq, nqd, rw;
@@ -54,6 +54,7 @@ struct MzEngine : asd_mezilix_engine {
     std::vector<void*> owned;
     DenseRunner dn;              // dense projections: tcgen05 GEMMs or the CUDA-core kernel, by shape and type
     EventProfiler prof;
+    LatentPromptWs prompt_ws;    // scratch of prompts' attention in head space: where latent-space calls keep queries and results
     AttnSplit attn_ws;           // partial sums of the attention kernel's key-range shares
     int* dev_error = nullptr;    // raised by a kernel whose bounded wait ran out
     int device = 0;
@@ -120,37 +121,49 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
         ql.c = e->qlat, ql.c_f32 = 1, ql.ldc = (long long)c.heads * ly.rw, ql.c_zs = ly.rw;
         ql.M = M, ql.N = c.kv_rank, ql.K = c.dim, ql.Z = c.heads;
         __nv_bfloat16* q_terms = nullptr;
-        if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
+        LatentPromptWs lp = e->prompt_ws;
+        lp.w = ly.wukv;
+        const bool head_space = !f32 && e->dn.tc_linear && latent_prompt_takes(dm, cache, M, nseq, max_qlen, max_kv_len, e->qd, ly.nqd, lp,
+                                                                               e->attn_ws.tiled);
+        if (!head_space && !f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
             latent_attention_tc_takes(dm, cache, max_qlen, e->attn_ws.tiled)) {
             q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
             ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
         }
         {
             MZ_PROF(MZ_GLUE);
-            if (launch_latent_post(ix, e->qd, dm, ly.latent_gain, f32, e->c.eps, ly.inv_freq, cache, e->qlat, s,
-                                   q_terms))
+            if (head_space ? launch_latent_post_inplace(ix, e->qd, ly.nqd, e->qd + ly.nq, ly.nqd, dm, ly.latent_gain, f32, e->c.eps,
+                                                        ly.inv_freq, cache, s)
+                           : launch_latent_post(ix, e->qd, dm, ly.latent_gain, f32, e->c.eps, ly.inv_freq, cache, e->qlat, s,
+                                                q_terms))
                 return -1;
         }
-        {
-            MZ_PROF(MZ_HEADS);
-            if (linear(e, ql, s)) return -1;
-        }
-        {
+        if (head_space) {
             MZ_PROF(MZ_ATTN);
-            if (q_terms ? launch_latent_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache,
-                                                     e->olat, e->attn_ws, e->dev_error, s)
-                        : launch_latent_attention(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qlat, dm, cache,
-                                                  e->olat, e->attn_ws, s))
+            if (launch_latent_prompt(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qd, ly.nqd, dm, cache, lp, e->vout, e->dev_error, s))
                 return -1;
-        }
-        {   // v[m][h][:] = Wuv[h] * out_lat[m][h][:]
-            MZ_PROF(MZ_HEADS);
-            SimtLinear L;
-            L.a = e->olat, L.a_f32 = 1, L.lda = (long long)c.heads * c.kv_rank, L.a_zs = c.kv_rank;
-            L.w = ly.wuv, L.w_f32 = f32, L.ldw = c.kv_rank, L.w_zs = (long long)c.vdim * c.kv_rank;
-            L.c = e->vout, L.c_f32 = f32, L.ldc = (long long)c.heads * c.vdim, L.c_zs = c.vdim;
-            L.M = M, L.N = c.vdim, L.K = c.kv_rank, L.Z = c.heads;
-            if (linear(e, L, s)) return -1;
+        } else {
+            {
+                MZ_PROF(MZ_HEADS);
+                if (linear(e, ql, s)) return -1;
+            }
+            {
+                MZ_PROF(MZ_ATTN);
+                if (q_terms ? launch_latent_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache,
+                                                         e->olat, e->attn_ws, e->dev_error, s)
+                            : launch_latent_attention(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qlat, dm, cache,
+                                                      e->olat, e->attn_ws, s))
+                    return -1;
+            }
+            {   // v[m][h][:] = Wuv[h] * out_lat[m][h][:]
+                MZ_PROF(MZ_HEADS);
+                SimtLinear L;
+                L.a = e->olat, L.a_f32 = 1, L.lda = (long long)c.heads * c.kv_rank, L.a_zs = c.kv_rank;
+                L.w = ly.wuv, L.w_f32 = f32, L.ldw = c.kv_rank, L.w_zs = (long long)c.vdim * c.kv_rank;
+                L.c = e->vout, L.c_f32 = f32, L.ldc = (long long)c.heads * c.vdim, L.c_zs = c.vdim;
+                L.M = M, L.N = c.vdim, L.K = c.kv_rank, L.Z = c.heads;
+                if (linear(e, L, s)) return -1;
+            }
         }
         {
             MZ_PROF(MZ_DENSE);
@@ -278,10 +291,12 @@ asd_mezilix_engine_t* asd_mezilix_create(const asd_mezilix_config* cfg, const as
     rc |= dev_alloc(e, &e->hn, MT * D);
     rc |= dev_alloc(e, &e->qd, MT * nqd);
     rc |= dev_alloc(e, &e->qlat, (MT * qlat * 3 + 1) / 2);      // fp32, or three bf16 planes
+    e->prompt_ws.planes = reinterpret_cast<__nv_bfloat16*>(e->qlat), e->prompt_ws.plane_elems = (long long)(MT * qlat * 3);
     {   // the attention's result is read before the experts write: one region for it and for their buffers (the query's third
         // plane is paid for by that)
         const size_t eout = (MT * top * D + 63) & ~(size_t)63, act = (MT * top * ff * e->esz + 3) / 4;
         rc |= dev_alloc(e, &e->olat, std::max(MT * olat, eout + act));
+        e->prompt_ws.rows = e->olat, e->prompt_ws.row_elems = 2 * (long long)(MT * olat);
         e->eout = e->olat;
         e->act = reinterpret_cast<char*>(e->olat + eout);
     }
@@ -336,8 +351,15 @@ int asd_mezilix_set_layer(asd_mezilix_engine_t* h, int layer, const void* gain, 
         return set_error("asd_mezilix_set_layer: NULL weight");
     if (ly.c.experts > 0 && (!router || !w_up || !w_down)) return set_error("asd_mezilix_set_layer: NULL expert weight");
     ly.gain = gain, ly.shift = shift, ly.coeff = depth_coeff, ly.wqd = wqd, ly.latent_gain = latent_gain, ly.wuk = wuk;
-    ly.wuv = wuv, ly.wo = wo, ly.router = router, ly.w_up = w_up, ly.w_down = w_down;
+    ly.wukv = nullptr, ly.wuv = wuv, ly.wo = wo, ly.router = router, ly.w_up = w_up, ly.w_down = w_down;
     e->dn.clear();
+    return 0;
+}
+
+int asd_mezilix_set_latent_up(asd_mezilix_engine_t* h, int layer, const void* wukv) {
+    MzEngine* e = static_cast<MzEngine*>(h);
+    if (!e || layer < 0 || layer >= (int)e->layers.size()) return set_error("asd_mezilix_set_latent_up: bad layer");
+    e->layers[layer].wukv = wukv;
     return 0;
 }
 
@@ -373,6 +395,10 @@ int asd_mezilix_set_option(asd_mezilix_engine_t* h, const char* name, int value)
     if (e->dn.set_option(name, value)) return 0;
     if (!strcmp(name, "experts_rows")) {
         e->experts_rows = value;
+        return 0;
+    }
+    if (!strcmp(name, "latent_prompt")) {
+        e->prompt_ws.mode = value;
         return 0;
     }
     if (!strcmp(name, "attn_tiled")) {

@@ -69,6 +69,7 @@ struct RvEngine : asd_rivetar_engine {
     std::vector<void*> owned;
     DenseRunner dn;
     EventProfiler prof;
+    LatentPromptWs prompt_ws;  // scratch of prompts' attention in head space: where latent-space calls keep queries and results
     AttnSplit attn_ws;
     int fused_attn = 1;
     int* dev_error = nullptr;
@@ -140,6 +141,19 @@ static int mix_latent(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
     ql.c = e->qlat, ql.c_f32 = 1, ql.ldc = (long long)c.heads * rw, ql.c_zs = rw;
     ql.M = M, ql.N = c.kv_rank, ql.K = c.dim, ql.Z = c.heads;
     __nv_bfloat16* q_terms = nullptr;
+    LatentPromptWs lp = e->prompt_ws;
+    lp.w = ly.w("w_ukv");
+    if (!f32 && e->dn.tc_linear && latent_prompt_takes(dm, cache, M, b.nseq, b.max_qlen, b.max_kv_len, e->qbuf, nq, lp, e->attn_ws.tiled)) {
+        {
+            RV_PROF(RV_GLUE);
+            if (launch_latent_post_inplace(b.ix, e->qbuf, nq, e->proj + c.q_rank, ly.n_in, dm, ly.f("kv_norm"), 1, e->c.eps, ly.freq_k,
+                                           cache, s))
+                return -1;
+        }
+        RV_PROF(RV_LATENT_ATTN);
+        return launch_latent_prompt(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qbuf, nq, dm, cache, lp, e->mixed,
+                                    e->dev_error, s);
+    }
     if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) && latent_attention_tc_takes(dm, cache, b.max_qlen, e->attn_ws.tiled)) {
         q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
         ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
@@ -324,7 +338,7 @@ static size_t pool_elems(const RvEngine* e, const RvRun& r, int num_pages) {
 }
 
 static const char* const kLayerNames[] = {"norm1", "norm1b", "norm2", "norm2b", "w_up", "w_down", "act", "w_o", "w_in",
-                                          "q_norm", "kv_norm", "w_uq", "w_uk", "w_uv", "w_decay", "b_decay", "out_norm",
+                                          "q_norm", "kv_norm", "w_uq", "w_uk", "w_uv", "w_ukv", "w_decay", "b_decay", "out_norm",
                                           "sink"};
 static const char* const kGlobalNames[] = {"embed", "final_norm", "head", "loop_in", "loop_step"};
 
@@ -423,6 +437,8 @@ asd_rivetar_engine_t* asd_rivetar_create(const asd_rivetar_config* cfg, const as
     // the attention's result is read before the feed-forward writes: one region (the query's third plane is paid for by that)
     rc |= dev_alloc(e, &e->olat, std::max(MT * olat, MT * ff));
     e->up = e->olat;
+    e->prompt_ws.planes = reinterpret_cast<__nv_bfloat16*>(e->qlat), e->prompt_ws.plane_elems = (long long)(MT * qlat * 3);
+    e->prompt_ws.rows = e->olat, e->prompt_ws.row_elems = 2 * (long long)(MT * olat);
     rc |= dev_alloc(e, &e->alpha, MT * nk);
     rc |= dev_alloc(e, &e->orec, MT * hv);
     rc |= dev_alloc(e, (char**)&e->hn, MT * 2 * D * e->esz);
@@ -461,7 +477,11 @@ int asd_rivetar_set_tensor(asd_rivetar_engine_t* h, int layer, const char* name,
         if (known) e->g[name] = data;
     } else {
         for (const char* n : kLayerNames) known |= !strcmp(n, name);
-        if (known) e->layers[layer].t[name] = data;
+        if (known) {
+            auto& t = e->layers[layer].t;
+            if (!strcmp(name, "w_uk") || !strcmp(name, "w_uv")) t.erase("w_ukv");
+            t[name] = data;
+        }
     }
     if (!known) return set_error("asd_rivetar_set_tensor: unknown tensor %s (layer %d)", name, layer);
     e->dn.clear();
@@ -507,6 +527,10 @@ int asd_rivetar_set_option(asd_rivetar_engine_t* h, const char* name, int value)
     if (!e || !name) return set_error("asd_rivetar_set_option: NULL argument");
     if (!strcmp(name, "debug_wait")) return launch_wait_expiry(e->dev_error, nullptr);
     if (e->dn.set_option(name, value)) return 0;
+    if (!strcmp(name, "latent_prompt")) {
+        e->prompt_ws.mode = value;
+        return 0;
+    }
     if (!strcmp(name, "attn_tiled")) {
         e->attn_ws.tiled = value;
         return 0;

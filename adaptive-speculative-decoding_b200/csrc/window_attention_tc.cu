@@ -29,6 +29,7 @@
 #include "elem.cuh"
 #include "gemm.h"
 #include "ptx.cuh"
+#include "softmax_tile.cuh"
 
 namespace asd {
 
@@ -36,7 +37,6 @@ namespace {
 
 constexpr int kWtThreads = 256;            // warps 0-3 softmax (thread = query row), 4 keys, 5 products, 6 values
 constexpr int kWtKeys = 128;               // keys per tile
-constexpr int kWtSlot = 128 * 128;         // bytes of 128 rows x 64 bf16
 constexpr float kWtSlack = 8.0f;           // log2 growth of a row maximum that the weights tolerate before a rescale
 // Query rows of a tile from which this kernel is the better one: all that the single-token form of the mma.sync kernel (up to 16
 // rows) does not take.  20 rows: 16 sequences at 900 positions 86 us there, 29 here; 64 at 200 41 and 33; one at 64 25 and 15.
@@ -65,60 +65,15 @@ struct WtBars {
     int failed;
 };
 
-// MN-major SW128 operand (keys along rows of 128 B = 64 columns, 8-key atoms 1024 B apart, the next 64 columns a slot further)
-__device__ __forceinline__ uint64_t wt_desc_mn(uint32_t addr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
-    d |= (uint64_t)(kWtSlot >> 4) << 16;
-    d |= (uint64_t)(1024 >> 4) << 32;
-    d |= (uint64_t)1 << 46;
-    d |= (uint64_t)2 << 61;
-    return d;
-}
-__device__ __forceinline__ float wt_ex2(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-// element i of a tile is visible to a row iff i <= hi and (i >= lo or i < kept): as bits of 32 elements from i0 on, so that a test
-// of one costs an instruction (as comparisons the compiler branched on every element: 14000 to 29000 clocks a tile)
-struct WtSeen {
-    int lo, hi, kept;
-    __device__ __forceinline__ static uint32_t below(int n) {          // bits 0 .. n - 1
-        return n <= 0 ? 0u : (n >= 32 ? 0xffffffffu : (1u << n) - 1u);
-    }
-    __device__ __forceinline__ uint32_t bits(int i0) const { return below(hi + 1 - i0) & (~below(lo - i0) | below(kept - i0)); }
-};
-// weights of 32 scores -> 16 packed pairs of their high terms and 16 of what is left
-template <bool MASKED>
-__device__ __forceinline__ void wt_weights(const uint32_t (&v)[32], uint32_t seen, float scale, float nref,
-                                           uint32_t (&ph)[16], uint32_t (&pl)[16], float (&sum)[4]) {
-#pragma unroll
-    for (int i = 0; i < 32; i += 2) {
-        float p0 = wt_ex2(fmaf(__uint_as_float(v[i]), scale, nref));
-        float p1 = wt_ex2(fmaf(__uint_as_float(v[i + 1]), scale, nref));
-        if (MASKED) {
-            p0 = seen & (1u << i) ? p0 : 0.0f;
-            p1 = seen & (2u << i) ? p1 : 0.0f;
-        }
-        sum[(i >> 1) & 3] += p0 + p1;
-        const __nv_bfloat162 h = __floats2bfloat162_rn(p0, p1);
-        const float2 f = __bfloat1622float2(h);
-        const __nv_bfloat162 r = __floats2bfloat162_rn(p0 - f.x, p1 - f.y);
-        ph[i >> 1] = *reinterpret_cast<const uint32_t*>(&h);
-        pl[i >> 1] = *reinterpret_cast<const uint32_t*>(&r);
-    }
-}
-
 __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_constant__ CUtensorMap map_kv, const WtArgs a) {
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const WindowDims& d = a.d;
     const int kc = d.dk >> 6, vc = d.dv >> 6;                  // chunks of 64 columns
     uint8_t* sQ = smem;                                        // [2 terms][kc]
-    uint8_t* sK = sQ + 2 * kc * kWtSlot;                       // [2 tiles][kc]
-    uint8_t* sV = sK + 2 * kc * kWtSlot;                       // [2 tiles][vc]
-    WtBars* B = reinterpret_cast<WtBars*>(sV + 2 * vc * kWtSlot);
+    uint8_t* sK = sQ + 2 * kc * kStSlot;                       // [2 tiles][kc]
+    uint8_t* sV = sK + 2 * kc * kStSlot;                       // [2 tiles][vc]
+    WtBars* B = reinterpret_cast<WtBars*>(sV + 2 * vc * kStSlot);
     const WaitGuard guard{reinterpret_cast<volatile int*>(&B->failed), a.err, WAIT_WINDOW << 8};
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -189,9 +144,9 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
                     hi[e] = *reinterpret_cast<const uint32_t*>(&h);
                     lo[e] = *reinterpret_cast<const uint32_t*>(&l);
                 }
-                uint8_t* dst = sQ + (c >> 3) * kWtSlot + r * 128 + (((c & 7) ^ (r & 7)) << 4);
+                uint8_t* dst = sQ + (c >> 3) * kStSlot + r * 128 + (((c & 7) ^ (r & 7)) << 4);
                 *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
-                *reinterpret_cast<uint4*>(dst + kc * kWtSlot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+                *reinterpret_cast<uint4*>(dst + kc * kStSlot) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
             }
         }
         fence_proxy_async_smem();
@@ -214,11 +169,11 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
             const int page = next, s = j & 1;
             if (j + 1 < nt) next = page_of(j + 1);
             if (j >= 2 && !__all_sync(0xffffffffu, mbar_wait(&freed[s], ((j >> 1) - 1) & 1, guard))) break;
-            if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(nc * kWtSlot));
+            if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(nc * kStSlot));
             __syncwarp();
             if (lane < pages)
                 for (int c = 0; c < nc; ++c)
-                    tma_load_2d(ring + (s * nc + c) * kWtSlot + ((size_t)lane << (psh + 7)), &map_kv, col + c * 64, page << psh,
+                    tma_load_2d(ring + (s * nc + c) * kStSlot + ((size_t)lane << (psh + 7)), &map_kv, col + c * 64, page << psh,
                                 &full[s]);
             __syncwarp();
         }
@@ -236,7 +191,7 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
             if (!ok) return;
             tc_fence_after();
             const uint32_t p = tmem + (uint32_t)(s * 128);
-            const uint64_t vd = wt_desc_mn(uV + (uint32_t)(s * vc * kWtSlot));
+            const uint64_t vd = st_desc_mn(uV + (uint32_t)(s * vc * kStSlot));
             if (lead) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {                  // 16 keys; their high and low terms lie 32 columns apart
@@ -258,8 +213,8 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
             if (lead) {
                 for (int u = 1; u >= 0; --u)                   // the low term first
                     for (int c = 0; c < kc; ++c) {
-                        const uint64_t qd = umma_desc_sw128(uQ + (uint32_t)((u * kc + c) * kWtSlot));
-                        const uint64_t kd = umma_desc_sw128(uK + (uint32_t)((s * kc + c) * kWtSlot));
+                        const uint64_t qd = umma_desc_sw128(uQ + (uint32_t)((u * kc + c) * kStSlot));
+                        const uint64_t kd = umma_desc_sw128(uK + (uint32_t)((s * kc + c) * kStSlot));
 #pragma unroll
                         for (int k = 0; k < 4; ++k)
                             umma_f16(tmem + (uint32_t)(s * 128), qd + 2 * k, kd + 2 * k, id_s, u != 1 || c != 0 || k != 0);
@@ -284,7 +239,7 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
         auto tile = [&](int j, auto masked_tag) {
             constexpr bool MASKED = decltype(masked_tag)::value;
             const int key0 = first_key(j);
-            const WtSeen seen{pos - d.window + 1 - key0, pos - key0, d.keep_first - key0};
+            const StSeen seen{pos - d.window + 1 - key0, pos - key0, d.keep_first - key0};
             const uint32_t tS = lanes + (uint32_t)((j & 1) * 128);
             float m4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll 1
@@ -304,7 +259,7 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
             const float top = fmaxf(fmaxf(m4[0], m4[1]), fmaxf(m4[2], m4[3])) * a.scale2;
             const bool grow = real && (top > ref + kWtSlack || (ref == -INFINITY && top > -INFINITY));
             if (__any_sync(0xffffffffu, grow)) {
-                const float corr = grow ? wt_ex2(ref - top) : 1.0f;        // ref = -inf: 0, of a row that is 0 so far
+                const float corr = grow ? st_ex2(ref - top) : 1.0f;        // ref = -inf: 0, of a row that is 0 so far
                 if (j > 0) {
                     mbar_wait_timed(&B->pv_done[(j - 1) & 1], ((j - 1) >> 1) & 1, guard, 2);
                     tc_fence_after();
@@ -333,10 +288,10 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
                 tmem_ld_32x32(tS + (uint32_t)(h * 64), x0);
                 tmem_ld_32x32(tS + (uint32_t)(h * 64 + 32), x1);
                 tmem_ld_wait();
-                wt_weights<MASKED>(x0, MASKED ? seen.bits(h * 64) : 0u, a.scale2, nref, ph, pl, sum);
+                st_weights<MASKED>(x0, MASKED ? seen.bits(h * 64) : 0u, a.scale2, nref, ph, pl, sum);
                 tmem_st_32x16(tS + (uint32_t)(h * 64), ph);
                 tmem_st_32x16(tS + (uint32_t)(h * 64 + 32), pl);
-                wt_weights<MASKED>(x1, MASKED ? seen.bits(h * 64 + 32) : 0u, a.scale2, nref, ph, pl, sum);
+                st_weights<MASKED>(x1, MASKED ? seen.bits(h * 64 + 32) : 0u, a.scale2, nref, ph, pl, sum);
                 tmem_st_32x16(tS + (uint32_t)(h * 64 + 16), ph);
                 tmem_st_32x16(tS + (uint32_t)(h * 64 + 48), pl);
             }
@@ -358,7 +313,7 @@ __global__ void __launch_bounds__(kWtThreads, 1) window_attn_tc(const __grid_con
                 mbar_wait_timed(&B->v_full[s], (j >> 1) & 1, guard, 3);
                 if (kp > p_last || (kp < j_lo && kp >= d.keep_first))
                     for (int c = 0; c < vc; ++c) {
-                        uint4* dst = reinterpret_cast<uint4*>(sV + (s * vc + c) * kWtSlot + tid * 128);
+                        uint4* dst = reinterpret_cast<uint4*>(sV + (s * vc + c) * kStSlot + tid * 128);
 #pragma unroll
                         for (int i = 0; i < 8; ++i) dst[i] = make_uint4(0, 0, 0, 0);
                     }
@@ -475,7 +430,7 @@ int launch_window_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
     if (grid.y > 65535 || (long long)nseq * d.kv_heads >= (1ll << 31)) return set_error("windowed attention: too many tokens, sequences or heads");
     CUtensorMap mk;
     if (make_tmap_bf16(&mk, cache.pool, cache.rows, rowlen, rowlen, cache.page_size)) return -1;
-    const int smem = 1024 + (4 * kc + 2 * vc) * kWtSlot + (int)sizeof(WtBars);
+    const int smem = 1024 + (4 * kc + 2 * vc) * kStSlot + (int)sizeof(WtBars);
     static PerDeviceOnce once;
     ASD_ONCE(once, ASD_CUDA(cudaFuncSetAttribute(window_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     window_attn_tc<<<grid, kWtThreads, smem, stream>>>(mk, a);

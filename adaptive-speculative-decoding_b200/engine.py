@@ -584,6 +584,7 @@ class MezilixEngine(_SlotOps, _BatchOps):
             check(lib().asd_mezilix_set_layer(self.h, i, ptr("gain"), ptr("shift"), ptr("coeff"), ptr("wqd"),
                                               ptr("latent_gain"), ptr("wuk"), ptr("wuv"), ptr("wo"), ptr("router"),
                                               ptr("w_up"), ptr("w_down")), "asd_mezilix_set_layer")
+            check(lib().asd_mezilix_set_latent_up(self.h, i, ptr("wukv")), "asd_mezilix_set_latent_up")
         for k, shape in (("embed", (self.cfg.vocab_size, self.cfg.width)),
                          ("bigram", (self.cfg.buckets + 1, self.cfg.width)), ("head", (self.cfg.vocab_size, self.cfg.width))):
             if k not in w or tuple(w[k].shape) != shape:

@@ -212,8 +212,11 @@ def pack_layer(w: Dict[str, torch.Tensor], cfg: MezilixConfig, i: int, device, d
            "wqd": dev(torch.cat([w[p + "mix.q"], w[p + "mix.dkv"]], 0)), "latent_gain": dev(w[p + "mix.dkv.norm"]),
            # per head [kv_rank, dim]: the query is carried into latent space as a product with rows of this matrix
            "wuk": dev(w[p + "mix.uk"].reshape(l.heads, l.dim, l.kv_rank).transpose(1, 2)),
-           "wuv": dev(w[p + "mix.uv"]), "wo": dev(w[p + "mix.o"]),
+           "wukv": None, "wuv": dev(w[p + "mix.uv"]), "wo": dev(w[p + "mix.o"]),
            "router": None, "w_up": None, "w_down": None}
+    if dtype == torch.bfloat16:      # prompts carry the positions through both up-projections; one buffer for both value forms
+        out["wukv"] = dev(torch.cat([w[p + "mix.uk"], w[p + "mix.uv"]], 0))
+        out["wuv"] = out["wukv"][l.heads * l.dim:]
     if l.experts:
         out["router"] = dev(w[p + "mlp.router"])
         out["w_up"] = dev(torch.stack([w[p + f"mlp.e{e}.up"] for e in range(l.experts)], 0))

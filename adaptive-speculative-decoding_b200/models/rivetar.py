@@ -301,6 +301,9 @@ def pack(w: Dict[str, torch.Tensor], cfg: RivetarConfig, device, dtype) -> Dict[
             out[(i, "w_uq")] = mat(w[p + "mix.uq"])
             out[(i, "w_uk")] = mat(w[p + "mix.uk"].reshape(l.heads, l.dim, l.kv_rank).transpose(1, 2))
             out[(i, "w_uv")] = mat(w[p + "mix.uv"])
+            if dtype == torch.bfloat16:      # prompts carry the positions through both up-projections; one buffer for both value forms
+                ukv = mat(torch.cat([w[p + "mix.uk"], w[p + "mix.uv"]], 0))
+                out[(i, "w_uv")], out[(i, "w_ukv")] = ukv[l.heads * l.dim:], ukv
         elif l.type == "gla":
             out[(i, "w_in")] = mat(torch.cat([w[p + x] for x in ("mix.q", "mix.k", "mix.v", "mix.g", "mix.a1")], 0))
             out[(i, "w_decay")], out[(i, "b_decay")] = vec(w[p + "mix.a2"]), vec(w[p + "mix.a2.b"])

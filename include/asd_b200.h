@@ -310,6 +310,10 @@ ASD_API int asd_mezilix_set_layer(asd_mezilix_engine_t* e, int layer, const void
                                   const void* depth_coeff, const void* wqd, const void* latent_gain, const void* wuk,
                                   const void* wuv, const void* wo, const void* router, const void* w_up,
                                   const void* w_down);
+/* Optional, after asd_mezilix_set_layer (which drops it), bf16 engines: wukv [heads * (dim + vdim), kv_rank] = the rows of the key
+ * up-projection (not transposed), then those of wuv.  With it prompts of heads of 128 + 64 carry the positions they see through
+ * these rows instead of every query and result (NULL: they do not). */
+ASD_API int asd_mezilix_set_latent_up(asd_mezilix_engine_t* e, int layer, const void* wukv);
 ASD_API size_t asd_mezilix_cache_bytes(const asd_mezilix_engine_t* e, int num_pages);
 ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, int32_t* token_ring, float* shift_ring);
@@ -319,7 +323,9 @@ ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_p
  * matrices up to 64 MB of up to 4096 columns run linear_few.cu, unless tc_min_rows asks for pairs), "experts_rows" (rows an
  * expert, on average, from which its products run on CTA pairs; 0, default: the measured rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
- * per (token, head)), "profile" (1: CUDA events around every launch, read with asd_mezilix_profile_read) */
+ * per (token, head)), "latent_prompt" (attention of prompts in head space, which needs asd_mezilix_set_latent_up; 1, default:
+ * where it measured better, 2: wherever the sizes allow, 0: never), "profile" (1: CUDA events around every launch, read with
+ * asd_mezilix_profile_read) */
 ASD_API int asd_mezilix_set_option(asd_mezilix_engine_t* e, const char* name, int value);
 /* Same contract as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [n_layers][M][width]) receives
  * the stream that leaves every layer. */
@@ -391,7 +397,8 @@ ASD_API void asd_rivetar_destroy(asd_rivetar_engine_t* e);
  * Every layer: "norm1", "norm1b" (and "norm2", "norm2b", "w_up" [ff, width], "w_down" [width, ff], "act" [4] when
  * ff > 0), "w_o" [width, heads * vdim], "w_in" = the matrices that read the mixer input stacked by rows:
  *   type 0: [q_rank | kv_rank + rot_dim]; also "q_norm" [q_rank], "kv_norm" [kv_rank], "w_uq" [heads * (dim + rot_dim),
- *           q_rank], "w_uk" [heads][kv_rank][dim] (transposed per head), "w_uv" [heads * vdim, kv_rank];
+ *           q_rank], "w_uk" [heads][kv_rank][dim] (transposed per head), "w_uv" [heads * vdim, kv_rank],
+ *           optionally after these two (either drops it) "w_ukv" as asd_mezilix_set_latent_up's wukv;
  *   type 1: [q | k | v | gate | decay-in]; also "w_decay" fp32 [heads * dim, decay_rank], "b_decay" [heads * dim],
  *           "out_norm" [vdim];
  *   type 2: [q | k | v]; also "sink" [heads]. */
@@ -400,7 +407,7 @@ ASD_API size_t asd_rivetar_cache_bytes(const asd_rivetar_engine_t* e, int num_pa
 ASD_API size_t asd_rivetar_state_bytes(const asd_rivetar_engine_t* e, int max_seqs);
 ASD_API int asd_rivetar_set_cache(asd_rivetar_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_tiled" as for the Mezilix engine (attn_tiled 2: windowed attention of
+/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_tiled", "latent_prompt" as for the Mezilix engine (attn_tiled 2: windowed attention of
  * 17 query rows a tile and more on tcgen05 too); "fused_attn" (1, default: tiled windowed
  * attention kernel; 0: one warp per (token, head)); "profile" */
 ASD_API int asd_rivetar_set_option(asd_rivetar_engine_t* e, const char* name, int value);
