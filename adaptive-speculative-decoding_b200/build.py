@@ -24,7 +24,7 @@ COMPONENTS = {
     "core": ["core.cu"],
     "linear": ["gemm.cu", "gemm_tc.cu"],
     "blocks": ["linear_simt.cu", "linear_tc.cu", "linear_few.cu"],
-    "latent": ["latent_attention.cu", "latent_attention_tc.cu", "latent_prompt_tc.cu"],
+    "latent": ["latent_attention.cu", "latent_attention_tc.cu", "latent_prompt_tc.cu", "latent_step_tc.cu"],
     "rows": ["norm_ops.cu", "moe.cu"],          # row kernels and the expert router that several families share
     "mezilix": ["mezilix_engine.cu", "stream_ops.cu"],
     "rivetar": ["rivetar_engine.cu", "gla.cu", "window_attention.cu", "window_attention_tc.cu"],

@@ -151,6 +151,13 @@ int launch_latent_attention_tc(const SeqIndex& ix, const int* cu_q, const int* s
                                int max_kv_len, const __nv_bfloat16* q_terms, const LatentDims& d, const PagedRows& cache,
                                float* out_lat, const AttnSplit& ws, int* err, cudaStream_t stream);
 
+// ---------------------------------------------------------------------------------------------- latent_step_tc.cu
+// The same, from the same planes, for up to 32 query rows a CTA.
+bool latent_step_takes(const LatentDims& d, const PagedRows& cache, int max_qlen, int max_kv_len, int tiled);
+int launch_latent_step(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen, int max_kv_len,
+                       const __nv_bfloat16* q_terms, const LatentDims& d, const PagedRows& cache, float* out_lat, const AttnSplit& ws,
+                       int* err, cudaStream_t stream);
+
 // ---------------------------------------------------------------------------------------------- latent_prompt_tc.cu
 // The same from the queries as they are (no head products before or behind): out bf16 [M][heads * dv] = the softmax's sum carried
 // through the value up-projection, for calls whose sequences bring about as many tokens as they see positions (`takes`).

@@ -29,8 +29,9 @@ int set_error(const char* fmt, ...) {
 }
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 static std::atomic<long long> g_kernels[KERNEL_COUNTED];
+void note_kernel(CountedKernel k) { g_kernels[k].fetch_add(1, std::memory_order_relaxed); }
 void count_kernel(CountedKernel k) {
-    g_kernels[k].fetch_add(1, std::memory_order_relaxed);
+    note_kernel(k);
     count_launch(1);
 }
 
@@ -83,7 +84,8 @@ int wait_word_check(const int* word, const char* who) {
     const int v = word ? *static_cast<const volatile int*>(word) : 0;
     if (v == 0) return 0;
     static const char* const kernels[] = {"diagnostic kernel", "weight-streaming GEMM", "CTA-pair GEMM", "paged attention",
-                                          "sampler", "tcgen05 linear", "latent attention", "persistent forward", "windowed attention", "latent attention of prompts"};
+                                          "sampler", "tcgen05 linear", "latent attention", "persistent forward", "windowed attention", "latent attention of prompts",
+                                          "latent attention of few rows"};
     const int k = v >> 8;
     return set_error("%s: a bounded wait of an earlier launch ran out (%s, place %d); its results are not valid", who,
                      kernels[k >= 1 && k <= 8 ? k : 0], v & 255);
@@ -126,7 +128,7 @@ const char* asd_last_error(void) { return g_err; }
 long long asd_launch_count(void) { return g_launches.load(); }
 void asd_reset_launch_count(void) { g_launches.store(0); }
 long long asd_kernel_launches(const char* name) {
-    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "linear_few", "attention_tc", "latent_tc", "latent_prompt", "window_tc", "sampler_draw"};
+    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "linear_few", "attention_tc", "latent_tc", "latent_prompt", "latent_step", "window_tc", "sampler_draw"};
     for (int i = 0; name && i < KERNEL_COUNTED; ++i)
         if (!strcmp(name, names[i])) return g_kernels[i].load();
     return set_error("asd_kernel_launches: unknown kernel %s", name ? name : "(null)");

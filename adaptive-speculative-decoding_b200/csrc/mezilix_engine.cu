@@ -125,8 +125,9 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
         lp.w = ly.wukv;
         const bool head_space = !f32 && e->dn.tc_linear && latent_prompt_takes(dm, cache, M, nseq, max_qlen, max_kv_len, e->qd, ly.nqd, lp,
                                                                                e->attn_ws.tiled);
+        const bool few_rows = latent_step_takes(dm, cache, max_qlen, max_kv_len, e->attn_ws.tiled);
         if (!head_space && !f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
-            latent_attention_tc_takes(dm, cache, max_qlen, e->attn_ws.tiled)) {
+            (few_rows || latent_attention_tc_takes(dm, cache, max_qlen, e->attn_ws.tiled))) {
             q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
             ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
         }
@@ -149,7 +150,9 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
             }
             {
                 MZ_PROF(MZ_ATTN);
-                if (q_terms ? launch_latent_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache,
+                if (q_terms && few_rows ? launch_latent_step(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache, e->olat,
+                                                     e->attn_ws, e->dev_error, s)
+                    : q_terms ? launch_latent_attention_tc(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, q_terms, dm, cache,
                                                          e->olat, e->attn_ws, e->dev_error, s)
                             : launch_latent_attention(ix, cu_q, seq_slot, nseq, max_qlen, max_kv_len, e->qlat, dm, cache,
                                                       e->olat, e->attn_ws, s))

@@ -154,7 +154,9 @@ static int mix_latent(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
         return launch_latent_prompt(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qbuf, nq, dm, cache, lp, e->mixed,
                                     e->dev_error, s);
     }
-    if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) && latent_attention_tc_takes(dm, cache, b.max_qlen, e->attn_ws.tiled)) {
+    const bool few_rows = latent_step_takes(dm, cache, b.max_qlen, b.max_kv_len, e->attn_ws.tiled);
+    if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
+        (few_rows || latent_attention_tc_takes(dm, cache, b.max_qlen, e->attn_ws.tiled))) {
         q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
         ql.c_f32 = 0, ql.c_terms = (long long)M * ql.ldc;
     }
@@ -170,7 +172,9 @@ static int mix_latent(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
     }
     {
         RV_PROF(RV_LATENT_ATTN);
-        if (q_terms ? launch_latent_attention_tc(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, q_terms, dm, cache,
+        if (q_terms && few_rows ? launch_latent_step(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, q_terms, dm, cache,
+                                                 e->olat, e->attn_ws, e->dev_error, s)
+            : q_terms ? launch_latent_attention_tc(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, q_terms, dm, cache,
                                                  e->olat, e->attn_ws, e->dev_error, s)
                     : launch_latent_attention(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qlat, dm, cache,
                                               e->olat, e->attn_ws, s))
