@@ -14,7 +14,7 @@ namespace asd {
 int set_error(const char* fmt, ...);  // records the message, returns -1
 void count_launch(int n);
 // launches of the kernels that a rule chooses between, by name (asd_kernel_launches): what the tests of those rules look at
-enum CountedKernel { KERNEL_GEMM, KERNEL_GEMM_PAIR, KERNEL_GEMM_GROUPED, KERNEL_GEMV, KERNEL_LINEAR_FEW, KERNEL_ATTENTION_TC, KERNEL_LATENT_TC, KERNEL_LATENT_PROMPT, KERNEL_LATENT_STEP, KERNEL_WINDOW_TC, KERNEL_SAMPLER_DRAW, KERNEL_COUNTED };
+enum CountedKernel { KERNEL_GEMM, KERNEL_GEMM_PAIR, KERNEL_GEMM_GROUPED, KERNEL_GEMV, KERNEL_ONE_STEP, KERNEL_LINEAR_FEW, KERNEL_ATTENTION_TC, KERNEL_LATENT_TC, KERNEL_LATENT_PROMPT, KERNEL_LATENT_STEP, KERNEL_WINDOW_TC, KERNEL_SAMPLER_DRAW, KERNEL_COUNTED };
 void count_kernel(CountedKernel k);                     // count_launch(1) too
 void note_kernel(CountedKernel k);                      // of a launch that is counted by another name as well
 
@@ -28,7 +28,7 @@ void note_kernel(CountedKernel k);                      // of a launch that is c
 // ---- Bounded device waits.  A kernel whose barrier does not complete gives up after some seconds (ptx.cuh, mbar_wait), writes
 // (kernel << 8 | place) into a word of mapped host memory and ends.  The host reads that word without touching the device: every
 // entry point of an engine does before it launches anything, and so does whoever hands results to the host.
-enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, WAIT_LINEAR, WAIT_LATENT, WAIT_PERSIST, WAIT_WINDOW, WAIT_LATENT_PROMPT, WAIT_LATENT_STEP };
+enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, WAIT_LINEAR, WAIT_LATENT, WAIT_PERSIST, WAIT_WINDOW, WAIT_LATENT_PROMPT, WAIT_LATENT_STEP, WAIT_ONE_STEP };
 int* wait_word_alloc();                                 // a zeroed word that every device and stream can write, or nullptr
 void wait_word_free(int* word);
 int wait_word_check(const int* word, const char* who);  // 0, or the error that names the kernel and the place

@@ -85,7 +85,7 @@ int wait_word_check(const int* word, const char* who) {
     if (v == 0) return 0;
     static const char* const kernels[] = {"diagnostic kernel", "weight-streaming GEMM", "CTA-pair GEMM", "paged attention",
                                           "sampler", "tcgen05 linear", "latent attention", "persistent forward", "windowed attention", "latent attention of prompts",
-                                          "latent attention of few rows"};
+                                          "latent attention of few rows", "one-token step"};
     const int k = v >> 8;
     return set_error("%s: a bounded wait of an earlier launch ran out (%s, place %d); its results are not valid", who,
                      kernels[k >= 1 && k <= 8 ? k : 0], v & 255);
@@ -128,7 +128,7 @@ const char* asd_last_error(void) { return g_err; }
 long long asd_launch_count(void) { return g_launches.load(); }
 void asd_reset_launch_count(void) { g_launches.store(0); }
 long long asd_kernel_launches(const char* name) {
-    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "linear_few", "attention_tc", "latent_tc", "latent_prompt", "latent_step", "window_tc", "sampler_draw"};
+    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "one_step", "linear_few", "attention_tc", "latent_tc", "latent_prompt", "latent_step", "window_tc", "sampler_draw"};
     for (int i = 0; name && i < KERNEL_COUNTED; ++i)
         if (!strcmp(name, names[i])) return g_kernels[i].load();
     return set_error("asd_kernel_launches: unknown kernel %s", name ? name : "(null)");

@@ -19,6 +19,7 @@
 #include "asd_internal.h"
 #include "gemm.h"
 #include "layers.h"
+#include "one_step.h"
 #include "persist.h"
 
 namespace asd {
@@ -82,7 +83,8 @@ struct Engine {
     int attn_prefetch_mb = 0;
     // token counts above 256: QKV and O also run on the CTA-pair kernel (0 = weight-streaming kernel as for small steps)
     int tc_qkvo = 1;
-    // a step of one token of a small model runs its projections on the CUDA cores (gemv.cu); 0: weight-streaming kernel
+    // a step of one token of a small model runs in one launch (one_step.cu) or, where that does not take its sizes and with 2, has its
+    // projections on the CUDA cores (gemv.cu); 0: weight-streaming kernel
     int one_token = 1;
     PLayer* p_layers = nullptr;      // device array, rebuilt lazily after set_layer / set_kv
     bool p_layers_ok = false;
@@ -96,6 +98,7 @@ struct Engine {
     float* tp_buf[2] = {nullptr, nullptr};
     uint32_t* tp_flags = nullptr;
     int* tp_error = nullptr;
+    void* one_work = nullptr;        // of one_step.cu (nullptr: a model that it does not take)
     size_t sumsq_floats = 0;         // of sumsq and of sumsq_sel
     int* wait_err = nullptr;         // a bounded wait of one of this engine's kernels ran out (mapped host memory)
     const float* peer_buf[2][8] = {};
@@ -288,6 +291,32 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         cons.eps = c.rms_eps;
         return &cons;
     };
+    if (one && e->one_token == 1 && e->one_work && e->attn_impl == 2 && !e->profile && c.n_layers <= kOneMaxLayers) {
+        // all layers in one launch
+        if (n_logit_rows > 0 && !logits_out) return set_error("engine: logits_out is NULL");
+        OneStep st = {};
+        for (int l = 0; l < c.n_layers; ++l) {
+            const Layer& Ly = e->layers[l];
+            __nv_bfloat16* kc = e->kv_pool + (size_t)(2 * l) * e->kv_half;
+            st.layers[l] = OneLayer{Ly.wqkv, Ly.bqkv, Ly.wo, Ly.wgu, Ly.wdown, Ly.ln1, Ly.ln2, kc, kc + e->kv_half};
+        }
+        st.n_layers = c.n_layers, st.h = h, st.nh = nh, st.nkv = nkv, st.hd = hd, st.nqkv = e->nqkv, st.qdim = e->qdim, st.ffn = c.ffn;
+        st.page_size = c.page_size, st.max_pages = e->max_pages, st.eps = c.rms_eps;
+        st.embed = e->embed, st.final_norm = e->final_norm, st.inv_freq = e->inv_freq;
+        st.page_table = e->page_table, st.tokens = tokens, st.positions = positions, st.token_slot = token_slot;
+        st.x_out = e->resid_bf, st.sums_out = e->sumsq;
+        st.work = e->one_work, st.err = e->wait_err;
+        if (one_step_takes(st)) {
+            const int rc = one_step_launch(st, max_kv_len, s);
+            if (rc < 0) return rc;
+            parts = one_step_sums();
+            if (rc == 0)
+                return n_logit_rows > 0 ? gemv_launch(GEMM_OUT_F32, e->resid_bf, e->lm_head, h, c.vocab, logits_out, nullptr, consumer(e->sumsq), 0,
+                                                      nullptr, s)
+                                        : 0;
+            parts = 1;
+        }
+    }
     {
         PROF(PROF_GLUE);
         if (launch_add_norm(e->resid, nullptr, 0, 0, tokens, e->embed, e->layers[0].ln1, fn ? nullptr : e->xnorm, M, h,
@@ -636,7 +665,7 @@ asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int pro
         static PerDeviceOnce loaded;
         if (loaded.run([]() -> int {
                 return preload_layers() || preload_attention() || preload_attention_tc() || preload_gemm() || preload_gemm_tc() ||
-                       preload_gemv();
+                       preload_gemv() || preload_one_step();
             }))
             return nullptr;
     }
@@ -696,6 +725,11 @@ asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int pro
         alloc((void**)&e->p_sync, sizeof(unsigned) * kPersistSyncWords);
         alloc((void**)&e->p_ws, persist_part_ws_bytes());
     }
+    if (c.tp_size == 1 && gemv_takes(1, std::max(std::max(c.hidden, e->qdim), c.ffn), (size_t)2 * e->ffp * c.hidden * 2)) {
+        const size_t bytes = one_step_bytes(c.hidden, e->nqkv, e->qdim, c.ffn);
+        alloc(&e->one_work, bytes);
+        if (ok && cudaMemset(e->one_work, 0, bytes) != cudaSuccess) ok = false;
+    }
     alloc((void**)&e->xnorm, Mx * c.hidden * 2);
     alloc((void**)&e->xsel, Mx * c.hidden * 2);
     alloc((void**)&e->q, Mx * e->qdim * 2);
@@ -714,7 +748,7 @@ void asd_engine_destroy(asd_engine_t* h) {
     if (!e) return;
     void* bufs[] = {e->resid, e->part, e->o_part, e->ml_part, e->tickets, e->rope_cs, e->resid_bf, e->sumsq,
                     e->sumsq_sel, e->tp_buf[0], e->tp_buf[1], e->tp_flags, e->tp_error, e->xnorm, e->xsel, e->q, e->attn, e->act,
-                    e->p_layers, e->p_sync, e->p_ws};
+                    e->p_layers, e->p_sync, e->p_ws, e->one_work};
     for (void* b : bufs)
         if (b) cudaFree(b);
     wait_word_free(e->wait_err);
