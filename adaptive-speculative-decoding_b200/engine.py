@@ -6,8 +6,10 @@ from __future__ import annotations
 import ctypes
 import math
 import threading
+from array import array
 from typing import Dict, Optional
 
+import numpy as np
 import torch
 
 from ._lib import (AsdError, DikopelConfigC, DikopelLayerC, LukopelConfigC, LukopelLayerC, MavipelConfigC, MavipelLayerC, MezilixConfigC, MezilixLayerC, ModelConfigC,
@@ -212,28 +214,41 @@ class _BatchOps:
         if chunk <= 0:
             forward = self._prompt_forward
             chunk = self._prompt_chunk(nseq)
-        out = torch.empty(nseq, self.cfg.vocab_size, dtype=torch.float32, device=dev)
-        slots_h = slots.cpu().tolist()
+        # Each forward's indices travel in one copy, and slots stay on the device: nothing here waits for the GPU, so that a call is
+        # prepared while the one before runs (3 Rivetar prompts of up to 777 tokens, three layers of width 2048: 1475 -> 1120 us a call).
+        ids = [_token_ids(p) for p in prompts]
+        slots = slots.reshape(-1).to(device=dev, dtype=torch.int32)
+        out = None
         for s0 in range(0, max(lens), chunk):
-            toks, pos, tslot, cu, sslot, rows, owners = [], [], [], [0], [], [], []
-            for b in range(nseq):
-                e = min(lens[b], s0 + chunk)
-                if e <= s0:
-                    continue
-                toks += prompts[b][s0:e]
-                pos += list(range(s0, e))
-                tslot += [slots_h[b]] * (e - s0)
-                cu.append(len(toks))
-                sslot.append(slots_h[b])
-                if e == lens[b]:
-                    rows.append(len(toks) - 1)
-                    owners.append(b)
-            mk = lambda x: torch.tensor(x, dtype=torch.int32).to(dev, non_blocking=True)
-            lg = forward(mk(toks), mk(pos), mk(tslot), mk(cu), mk(sslot), min(chunk, max(lens) - s0),
-                         min(max(lens), s0 + chunk), mk(rows) if rows else None, None, bool(rows))
-            if rows:
-                out[torch.tensor(owners, device=dev)] = lg
+            here = [b for b in range(nseq) if lens[b] > s0]
+            n = [min(lens[b] - s0, chunk) for b in here]
+            ends = np.cumsum(n)
+            done = [i for i, b in enumerate(here) if s0 + n[i] == lens[b]]
+            parts = [np.concatenate([ids[b][s0:s0 + k] for b, k in zip(here, n)]),              # tokens
+                     s0 + np.concatenate([np.arange(k, dtype=np.int32) for k in n]),             # positions
+                     np.repeat(np.array(here, dtype=np.int32), n),                               # sequence of each token
+                     np.concatenate([[0], ends]), ends[done] - 1, np.array(here)[done], here]
+            packed = torch.from_numpy(np.concatenate(parts).astype(np.int32, copy=False)).to(dev, non_blocking=True)
+            toks, pos, of, cu, rows, owners, seqs = packed.split([len(p) for p in parts])
+            lg = forward(toks, pos, slots[of], cu, slots if len(here) == nseq else slots[seqs], min(chunk, max(lens) - s0),
+                         min(max(lens), s0 + chunk), rows if done else None, None, bool(done))
+            if len(done) == nseq:
+                return lg
+            if done:
+                if out is None:
+                    out = torch.empty(nseq, self.cfg.vocab_size, dtype=torch.float32, device=dev)
+                out[owners] = lg
         return out
+
+
+def _token_ids(prompt) -> np.ndarray:
+    """a prompt's tokens as int32 on the host; what does not fit raises"""
+    if isinstance(prompt, torch.Tensor):
+        prompt = prompt.tolist()
+    try:
+        return np.frombuffer(array("i", prompt if type(prompt) in (list, tuple) else list(prompt)), dtype=np.int32)
+    except TypeError:                      # elements that are no integers by themselves (tensors on a device, floats)
+        return torch.tensor(list(prompt), dtype=torch.int32).numpy()
 
 
 # Pages of a sequence up to which its prompts go through whole.  A whole prompt's attention walks all keys in one piece, and a block
