@@ -416,8 +416,14 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     const int groups = (d.dk + GLA_R - 1) / GLA_R, run = (ix.M + nseq - 1) / nseq;
     // 32 columns a CTA; steps of large heads 16, so that an SM holds several (64 single tokens, 4 heads of 512 x 512: one CTA of 512
     // threads per SM 252 us, two 150, four of 256 threads 136; 1 head of 1024 x 1024: one of 1024 threads 177, two of 512 152)
-    const int cols = groups > 32 && run <= 1 ? 16 : 32, cg = cols / GLA_C;
-    const int threads = (groups * cg + 31) / 32 * 32, RG = threads / cg, dkp = RG * GLA_R;
+    int cols = groups > 32 && run <= 1 ? 16 : 32;
+    // 48 columns where 32 leave some SMs with two CTAs, which are then the last, and these give every CTA an SM of its own: 436 clocks a
+    // position there, 390 here (3 prompts of up to 777 positions, 16 heads of 128 x 128: 167 -> 158 us; four warps of 8 rows x 6 columns
+    // a CTA instead of six of 8 x 4: 225)
+    const long long heads_all = (long long)nseq * d.heads, sms = sm_count();
+    if (run > 1 && groups <= 16 && heads_all * ((d.dv + 31) / 32) > sms && heads_all * ((d.dv + 47) / 48) <= sms) cols = 48;
+    const int cg = cols / GLA_C, whole = cols == 48 ? 96 : 32;         // threads: whole warps, and whole rows of column groups
+    const int threads = (groups * cg + whole - 1) / whole * whole, RG = threads / cg, dkp = RG * GLA_R;
     // chunks as long as two (large heads: one) staged CTAs per SM allow, and no longer than the runs: a step's CTAs are then
     // small enough for an SM to hold all that its registers can
     int ch = dkp <= 128 ? 16 : (dkp <= 512 ? 8 : 4);
@@ -431,13 +437,14 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     // steps and short runs of large heads wait for the state, not for their positions: no loads ahead, and the registers of as many
     // CTAs per SM as there can be (64 runs of 5, 4 heads of 512 x 512: one 295 us, two 191)
     const int form = cols == 16 ? (threads > 256 ? 0 : 1)
+                : cols == 48 ? 7
                                 : (threads > 512 ? 2 : (threads > 256 ? (2 * smem <= 220 * 1024 ? 3 : 4) : (ch == 1 ? 5 : 6)));
     const decltype(&gla_recurrence_kernel<256, 2, true>) forms[] = {
         gla_recurrence_kernel<512, 2, false, 16>, gla_recurrence_kernel<256, 4, false, 16>, gla_recurrence_kernel<1024, 1, false>,
         gla_recurrence_kernel<512, 2, false>,     gla_recurrence_kernel<512, 1, true>,      gla_recurrence_kernel<256, 4, false>,
-        gla_recurrence_kernel<256, 2, true>};
+        gla_recurrence_kernel<256, 2, true>,      gla_recurrence_kernel<192, 1, true, 48>};
     auto fn = forms[form];
-    static PerDeviceOnce once[7];
+    static PerDeviceOnce once[8];
     ASD_ONCE(once[form], ASD_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024)));
     ASD_CUDA(launch_pdl(fn, grid, threads, smem, stream, ix, cu_q, seq_slot, q, k, v, ld, alpha, d, state, ring, out, ch, vec));
     count_launch(1);

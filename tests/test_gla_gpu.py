@@ -61,3 +61,21 @@ def test_chunks_of_an_unequal_batch():
     assert torch.equal(got, torch.cat([a[6:6 + n] for a, n in zip(alone, lens)]))
     assert torch.equal(step, torch.cat([a[6 + n:] for a, n in zip(alone, lens)]))
     close(eng)
+
+
+# two sequences: 192, 180 and 160 CTAs of 32 columns, 144, 120 and 80 of 48
+@pytest.mark.parametrize("heads,dim,vdim", [(24, 128, 128), (30, 20, 66), (40, 72, 48)])
+def test_wider_column_tiles(heads, dim, vdim):
+    """as many heads and sequences as take 48 columns a CTA: bit for bit what each sequence gets alone, by 32"""
+    cfg = config([gla(heads=heads, dim=dim, vdim=vdim, tau=16.0, decay_rank=4)])
+    w = O.random_model(cfg, seed=31)
+    ids = [tokens(n, 96, 32 + n) for n in (41, 19)]
+    eng = make_engine(cfg, w, max_tokens=64, max_seqs=4)
+    alone = [feed(eng, eng.open_sequence(), t, []) for t in ids]
+    slots = [eng.open_sequence() for _ in ids]
+    for s, t in zip(slots, ids):
+        eng.reserve(s, len(t))
+    got = eng.forward_ragged([(s, 0, t, list(range(len(t)))) for s, t in zip(slots, ids)])
+    assert rel_err(got[:41], O.forward(cfg, w, ids[0])[0])[1] < 2e-4        # as above
+    assert torch.equal(got, torch.cat(alone))
+    close(eng)
