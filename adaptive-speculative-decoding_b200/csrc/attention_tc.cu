@@ -26,6 +26,9 @@
 // issues all MMAs.  Warps whose 32 rows are all padding sit the loop out (the barrier counts are the number of
 // active warps).  Long contexts are split over the KV length (flash decoding) with the same ticket merge as
 // attention.cu.
+// Parity waits are only unambiguous while nobody arrives two phases ahead of a waiter: the weights have a barrier for each
+// buffer (the softmax may finish a tile before the MMA thread has looked for the one before; with one barrier it then waited
+// until its limit), the final sums one of their own.
 //
 // The reference has no attention code (vLLM does it: src/serving/real_model_pipeline.py:98-108);
 // semantics are HF Qwen2 GQA attention with softmax scale 1/sqrt(head_dim), causal among the new positions.
@@ -153,9 +156,9 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
     uint8_t* sV = sK + 2 * kAtOp;          // [2 stages]
     uint64_t* bars = reinterpret_cast<uint64_t*>(sV + 2 * kAtOp);
     uint64_t *k_full = bars, *k_empty = bars + 2, *v_full = bars + 4, *v_empty = bars + 6, *s_full = bars + 8,
-             *s_empty = bars + 10, *o_full = bars + 12, *o_empty = bars + 14, *p_full = bars + 16, *q_full = bars + 17,
-             *c_full = bars + 18;   // c_full[4]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 22);
+             *s_empty = bars + 10, *o_full = bars + 12, *o_empty = bars + 14, *p_full = bars + 16, *q_full = bars + 18,
+             *fin_full = bars + 19, *c_full = bars + 20;   // p_full[2], c_full[4]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 24);
     int* s_last = reinterpret_cast<int*>(tmem_slot + 1);
     const WaitGuard guard{reinterpret_cast<volatile int*>(tmem_slot + 2), a.err, WAIT_ATTENTION << 8};
     float* corr_s = reinterpret_cast<float*>(tmem_slot + 4);   // [4][128] rescale factor of tile j (ring j & 3)
@@ -204,8 +207,10 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             mbar_init(&o_full[i], 1);
             mbar_init(&o_empty[i], nact);
         }
-        mbar_init(p_full, nact);
+        mbar_init(&p_full[0], nact);
+        mbar_init(&p_full[1], nact);
         mbar_init(q_full, 4);
+        mbar_init(fin_full, nact);
         for (int i = 0; i < 4; ++i) mbar_init(&c_full[i], nact);
         *guard.failed = 0;
         fence_mbar_init();
@@ -279,7 +284,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             for (int j = 0; j < nt; ++j) {
                 const int st = j & 1, use = j >> 1;
                 if (j + 1 < nt) issue_qk(j + 1);
-                ok = ok && mbar_wait_far(p_full, j & 1, guard, 4) && mbar_wait_far(&v_full[st], use & 1, guard, 5) &&
+                ok = ok && mbar_wait_far(&p_full[st], use & 1, guard, 4) && mbar_wait_far(&v_full[st], use & 1, guard, 5) &&
                      (use == 0 || mbar_wait_far(&o_empty[st], (use - 1) & 1, guard, 6));
                 if (!ok) break;
                 tc_fence_after();
@@ -335,7 +340,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) {
-                        mbar_arrive(p_full);
+                        mbar_arrive(&p_full[st]);
                         mbar_arrive(&c_full[j & 3]);
                     }
                     return;
@@ -384,7 +389,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive(p_full);
+                    mbar_arrive(&p_full[st]);
                     mbar_arrive(&c_full[j & 3]);
                 }
                 if (r == 0 && j < 2) at_stamp<TRACE>(a, j == 0 ? 3 : 5);
@@ -404,7 +409,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
             fin_s[r] = mx;
             fin_s[128 + r] = l;
             __syncwarp();
-            if (lane == 0) mbar_arrive(&c_full[nt & 3]);
+            if (lane == 0) mbar_arrive(fin_full);
             if (r == 0) at_stamp<TRACE>(a, 8);
         }
     } else {
@@ -437,7 +442,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
                 if (lane == 0) mbar_arrive(&o_empty[st]);
                 if (r == 0 && j == 0) at_stamp<TRACE>(a, 6);
             }
-            mbar_wait(&c_full[nt & 3], (nt >> 2) & 1, guard);
+            mbar_wait(fin_full, 0, guard);
             const float mx = fin_s[r], l = fin_s[128 + r];
             if (r == 0) at_stamp<TRACE>(a, 9);
             // ---- results: final output when the sequence has a single split, else partials + last-CTA combine
@@ -515,7 +520,7 @@ __global__ void __launch_bounds__(kAtThreads, 1) attn_tc_kernel(const __grid_con
 // ------------------------------------------------------------------------------------------- host
 int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream) {
     static PerDeviceOnce once;
-    const size_t smem = 1024 + 5 * (size_t)kAtOp + 22 * 8 + 16 + 6 * 128 * 4 +
+    const size_t smem = 1024 + 5 * (size_t)kAtOp + 24 * 8 + 16 + 6 * 128 * 4 +
                         ((size_t)L.split_keys / L.page_size + 2) * 4 + 64;
     ASD_ONCE(once, {
         ASD_CUDA(cudaFuncSetAttribute(attn_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
