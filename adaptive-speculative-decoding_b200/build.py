@@ -35,7 +35,7 @@ COMPONENTS = {
     "lukopel": ["lukopel_engine.cu", "residual_streams.cu"],
     "dikopel": ["dikopel_engine.cu", "mlstm.cu"],
     "nobonex": ["nobonex_engine.cu", "ssd.cu", "ssd_chunk.cu"],
-    "qwen": ["engine.cu", "layers.cu", "attention.cu", "attention_tc.cu", "forward_persist.cu", "gemv.cu", "one_step.cu"],
+    "qwen": ["engine.cu", "layers.cu", "attention.cu", "attention_tc.cu", "attention_few.cu", "forward_persist.cu", "gemv.cu", "one_step.cu"],
     "sampling": ["api.cu", "sampler.cu", "stop_rule.cu"],
 }
 REQUIRES = {"mezilix": ("linear", "blocks", "latent", "rows"), "rivetar": ("linear", "blocks", "latent", "rows"),

@@ -529,7 +529,8 @@ int launch_attention(const AttnLaunch& L, cudaStream_t stream) {
     const int G = L.nh / L.nkv;
     const int rows = (L.q_tile > 0 ? L.q_tile : L.max_qlen) * G;
     const int tiles = L.q_tile > 0 ? (L.max_qlen + L.q_tile - 1) / L.q_tile : 1;
-    if (L.impl == 2 && L.kv_map != nullptr && L.hd == 128 && rows <= 128 && L.split_keys % 128 == 0)
+    if (L.few) return launch_attention_few(L, stream);
+    if (L.impl >= 2 && L.kv_map != nullptr && L.hd == 128 && rows <= 128 && L.split_keys % 128 == 0)
         return launch_attention_tc(L, stream);
     const int rg = (rows + 15) / 16;
     if (rg > 8) return set_error("attention: q_len * group = %d rows exceeds 128; chunk the query", rows);

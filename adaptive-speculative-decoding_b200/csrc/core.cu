@@ -128,7 +128,7 @@ const char* asd_last_error(void) { return g_err; }
 long long asd_launch_count(void) { return g_launches.load(); }
 void asd_reset_launch_count(void) { g_launches.store(0); }
 long long asd_kernel_launches(const char* name) {
-    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "one_step", "linear_few", "attention_tc", "latent_tc", "latent_prompt", "latent_step", "window_tc", "sampler_draw"};
+    static const char* const names[KERNEL_COUNTED] = {"gemm", "gemm_pair", "gemm_grouped", "gemv", "one_step", "linear_few", "attention_tc", "attention_few", "latent_tc", "latent_prompt", "latent_step", "window_tc", "sampler_draw"};
     for (int i = 0; name && i < KERNEL_COUNTED; ++i)
         if (!strcmp(name, names[i])) return g_kernels[i].load();
     return set_error("asd_kernel_launches: unknown kernel %s", name ? name : "(null)");

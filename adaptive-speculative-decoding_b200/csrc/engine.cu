@@ -68,10 +68,10 @@ struct Engine {
     std::unordered_map<int, std::pair<GemmPlan, CUtensorMap>> lm_plans;  // keyed by rows (xnorm) / -rows (xsel)
     std::unordered_map<int, std::pair<TcPlan, CUtensorMap>> lm_plans_tc;
     // options
-    // attn_impl: 2 = tcgen05 kernel (attention_tc.cu; default: faster on every bench shape since P moved into TMEM -
+    // attn_impl: 3 (default) = attention_few.cu where it takes the step, else as 2; 2 = tcgen05 kernel (attention_tc.cu: against 1
     // 18.7 vs 22.8 us at 32B/prefix 512, 64 vs 180 us at 72B-TP4/prefix 4096, tools/bench_attn.py), 1 = mma.sync kernel
     // (also the fallback for head_dim 64 or more than 128 query rows), 0 = one-warp cross-check kernel
-    int attn_impl = 2, pdl = 1, force_ksplit = 0, force_stages = 0, max_attn_splits = 16, reduce = 1,
+    int attn_impl = 3, pdl = 1, force_ksplit = 0, force_stages = 0, max_attn_splits = 16, reduce = 1,
         attn_target_ctas = 148, fuse_rope = 1, fuse_norm = 0, attn_min_split_keys = 1024, tp_fused = 1, tp_two_shot = 0;
     Tuning tune;   // per-engine knobs, installed for the calling thread by forward()
     // persistent forward kernel (forward_persist.cu): one cooperative launch per forward when the shape allows
@@ -275,6 +275,11 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         PROF(PROF_GEMM);
         return persist_launch(PL, s);
     }
+    // few query rows a key/value head: shares of any whole pages
+    int few_keys = e->attn_impl >= 3 && e->kv_map_ok && q_tile == 0
+                       ? attention_few_split(nseq, nkv, hd, c.page_size, max_qlen * group, max_kv_len) : 0;
+    int few_shares = few_keys > 0 ? (max_kv_len + few_keys - 1) / few_keys : 0;
+    if (few_shares > 1 && (size_t)M * nh * few_shares * hd > e->o_part_floats) few_keys = 0;
     int parts = 1;   // rows of e->sumsq that currently describe the residual (fused-norm mode)
     // one token: every projection through gemv.cu (its norm statistics are one sum per block, side by side)
     const bool one = e->one_token && fn && !tp && e->force_ksplit == 0 && e->force_stages == 0 && n_logit_rows <= 1 &&
@@ -291,7 +296,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         cons.eps = c.rms_eps;
         return &cons;
     };
-    if (one && e->one_token == 1 && e->one_work && e->attn_impl == 2 && !e->profile && c.n_layers <= kOneMaxLayers) {
+    if (one && e->one_token == 1 && e->one_work && e->attn_impl >= 2 && !e->profile && c.n_layers <= kOneMaxLayers) {
         // all layers in one launch
         if (n_logit_rows > 0 && !logits_out) return set_error("engine: logits_out is NULL");
         OneStep st = {};
@@ -526,8 +531,9 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         A.hd = hd;
         A.page_size = c.page_size;
         A.max_pages = e->max_pages;
-        A.split_keys = split_keys;
-        A.nsplit_max = nsplit_max;
+        A.few = few_keys > 0;
+        A.split_keys = A.few ? few_keys : split_keys;
+        A.nsplit_max = A.few ? few_shares : nsplit_max;
         A.impl = e->attn_impl;
         A.q_tile = q_tile;
         A.kv_map = e->kv_map_ok ? &e->kv_map : nullptr;
@@ -664,7 +670,7 @@ asd_engine_t* asd_engine_create_for_prompts(const asd_model_config* cfg, int pro
     {   // lazy module loading + spinning tensor-parallel kernels in one process = deadlock: load everything now
         static PerDeviceOnce loaded;
         if (loaded.run([]() -> int {
-                return preload_layers() || preload_attention() || preload_attention_tc() || preload_gemm() || preload_gemm_tc() ||
+                return preload_layers() || preload_attention() || preload_attention_tc() || preload_attention_few() || preload_gemm() || preload_gemm_tc() ||
                        preload_gemv() || preload_one_step();
             }))
             return nullptr;

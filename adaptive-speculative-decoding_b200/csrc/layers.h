@@ -42,6 +42,7 @@ struct AttnLaunch {
     float* ml_part;
     int* tickets;           // [M * nkv] zero-initialised, self-resetting (one per query tile and kv head: its first token's)
     int M, nseq, max_qlen, nh, nkv, hd, page_size, max_pages, split_keys, nsplit_max, impl;
+    bool few = false;       // attention_few.cu: split_keys from attention_few_split
     int q_tile = 0;         // > 0: new positions per query tile, a sequence's positions spread over ceil(max_qlen / q_tile) CTAs
     // impl 2 (tcgen05 kernel, attention_tc.cu): 2-D TMA map over the whole paged pool viewed as rows of head_dim
     // elements (box = 64 elements x 16 positions) and the first row of this layer's K / V
@@ -59,6 +60,10 @@ struct AttnLaunch {
 // 16-position pages, query tile * group <= 128), else 1
 int launch_attention(const AttnLaunch& L, cudaStream_t stream);
 int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream);
+// few query rows a key/value head (attention_few.cu): keys of a share, or 0 where it does not apply
+int attention_few_split(int nseq, int nkv, int hd, int page_size, int rows, int max_kv_len);
+int launch_attention_few(const AttnLaunch& L, cudaStream_t stream);
+int preload_attention_few();
 
 // load every kernel of the forward into the current context (see layers.cu: preload_layers)
 int preload_layers();

@@ -38,7 +38,7 @@ ASD_API const char* asd_last_error(void);
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
 /* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemm_grouped",
- * "gemv" (projections of one token: launches, or phases of a one_step), "one_step", "linear_few", "attention_tc", "latent_tc" (calls of at
+ * "gemv" (projections of one token: launches, or phases of a one_step), "one_step", "linear_few", "attention_tc", "attention_few", "latent_tc" (calls of at
  * least 32 query rows a tile in latent space), "latent_step", "latent_prompt", "window_tc", "sampler_draw"; -1 for another name */
 ASD_API long long asd_kernel_launches(const char* name);
 /* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:

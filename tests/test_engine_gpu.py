@@ -468,3 +468,36 @@ def test_forward_prompt_limits():
     assert lib().asd_launch_count() == before
     assert torch.isfinite(eng.prefill(ids[None], slot)).all()          # prefill cuts it itself
     eng.close()
+
+
+@pytest.mark.parametrize("nh,nkv,q,lens", [
+    (8, 4, 8, [1, 16, 17, 127, 128, 40]),          # 16 rows; contexts at the edges of pages
+    (17, 1, 1, [15, 143, 144]),                    # 17 rows: two tiles
+    (8, 2, 3, [129, 1140, 765]),                   # 12 rows; several shares, an empty one
+    (16, 2, 4, [1300, 300]),                       # 32 rows, several shares
+    (2, 2, 1, [3300, 5]),                          # one row
+    (9, 3, 6, [9] * 14),                           # 18 rows of too many items
+])
+def test_few_query_rows(nh, nkv, q, lens):
+    """steps of few rows a key/value head: the kernel that takes pages a warp, against the oracle and the tcgen05 kernel"""
+    from asd_b200.engine import QwenEngine
+    cfg = Qwen2Config(512, 2, nh, nkv, 1024, 2048, head_dim=128, name="few")
+    w = random_hf_weights(cfg, seed=23, logit_std=0.4)
+    g = torch.Generator().manual_seed(12)
+    ids = [torch.randint(0, cfg.vocab_size, (1, n + q), generator=g) for n in lens]
+    refs = torch.stack([qwen2_forward(w, cfg, t)[0, -q:] for t in ids])
+    eng = QwenEngine(cfg, max_seqs=len(lens), max_seq_len=max(lens) + 32, max_tokens=512).load_hf_weights(w)
+    slots = torch.arange(len(lens), dtype=torch.int32, device="cuda")
+    eng.prefill_ragged([t[0, :n].tolist() for t, n in zip(ids, lens)], slots)
+    new = torch.cat([t[:, n:] for t, n in zip(ids, lens)]).to(torch.int32).cuda()
+    start = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    takes = q * nh // nkv <= 16 or len(lens) * nkv <= torch.cuda.get_device_properties(0).multi_processor_count // 4
+    got = []
+    for impl in (3, 2):
+        eng.set_option("attn_impl", impl)
+        step = lambda: got.append(eng.forward_uniform(new, start, slots, max(lens) + q).view(len(lens), q, -1).cpu())
+        assert _launched("attention_few", step) == (2 if impl == 3 and takes else 0)
+        check(got[-1], refs)
+    eng.close()
+    # both round queries, keys, values and weights to bf16 and differ in the order of fp32 sums; a flipped rounding moves a logit by less
+    assert (got[0] - got[1]).abs().max().item() <= MAX_ABS / 2
