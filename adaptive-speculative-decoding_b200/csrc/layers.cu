@@ -35,7 +35,11 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
     return t;
 }
 
-// one CTA per token row
+// One CTA per token row.  The norm's weights come before the wait, all loads of a slice before the first of them is added (with a slice
+// after the other inside each element, and the weights behind the row's sum, the kernel ended 7.3 us after the CTA-pair GEMM of an O
+// projection of 509 tokens, hidden size 3584, and 11.6 after the down projection's more slices; now 5.8 and 10).
+// VEC: float4 per thread, so that the registers of an 8192-wide row do not cost narrower ones their CTAs.
+template <int VEC>
 __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restrict__ resid, const float* __restrict__ part,
                                                                  int nslices, size_t slice_stride,
                                                                  const int* __restrict__ tokens,
@@ -45,45 +49,74 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
                                                                  __nv_bfloat16* __restrict__ resid_bf,
                                                                  float* __restrict__ sumsq0) {
     __shared__ float scratch[kNormThreads / 32];
+    const int m = blockIdx.x, nvec = h >> 2;
+    uint32_t wt[VEC][2];        // the norm's weights never change
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = threadIdx.x + i * kNormThreads;
+        if (w != nullptr && c < nvec) {
+            wt[i][0] = __ldg(reinterpret_cast<const uint32_t*>(w) + 2 * c);
+            wt[i][1] = __ldg(reinterpret_cast<const uint32_t*>(w) + 2 * c + 1);
+        }
+    }
+    auto weight = [&](int i, int k) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&wt[i][k])); };
     grid_dep_wait();    // launched programmatically: the upstream kernel's results are needed from here on
     grid_dep_launch();  // lets the next GEMM start streaming its weights (it waits before reading x)
-    const int m = blockIdx.x, nvec = h >> 2;
-    float4 v[kNormMaxVec];
+    float4 v[VEC];
     float ss = 0.0f;
     float4* rrow = reinterpret_cast<float4*>(resid + (size_t)m * h);
+    if (tokens) {
+        const __nv_bfloat162* row = reinterpret_cast<const __nv_bfloat162*>(emb + (size_t)tokens[m] * h);
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
-        const int c = threadIdx.x + i * kNormThreads;
-        if (c < nvec) {
-            float4 x;
-            if (tokens) {
-                const __nv_bfloat162* e =
-                    reinterpret_cast<const __nv_bfloat162*>(emb + (size_t)tokens[m] * h) + 2 * c;
-                const float2 a = __bfloat1622float2(e[0]), b = __bfloat1622float2(e[1]);
-                x = make_float4(a.x, a.y, b.x, b.y);
-            } else {
-                x = rrow[c];
-                for (int s = 0; s < nslices; ++s) {
-                    const float4 p = reinterpret_cast<const float4*>(part + s * slice_stride + (size_t)m * h)[c];
-                    x.x += p.x;
-                    x.y += p.y;
-                    x.z += p.z;
-                    x.w += p.w;
+        for (int i = 0; i < VEC; ++i) {
+            const int c = threadIdx.x + i * kNormThreads;
+            if (c < nvec) {
+                const float2 a = __bfloat1622float2(row[2 * c]), b = __bfloat1622float2(row[2 * c + 1]);
+                v[i] = make_float4(a.x, a.y, b.x, b.y);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) {
+            const int c = threadIdx.x + i * kNormThreads;
+            if (c < nvec) v[i] = rrow[c];
+        }
+        const float4* prow = reinterpret_cast<const float4*>(part + (size_t)m * h);
+#pragma unroll 2
+        for (int s = 0; s < nslices; ++s) {
+            float4 p[VEC];
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                const int c = threadIdx.x + i * kNormThreads;
+                if (c < nvec) p[i] = prow[s * (slice_stride >> 2) + c];
+            }
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) {
+                if (threadIdx.x + i * kNormThreads < nvec) {
+                    v[i].x += p[i].x;
+                    v[i].y += p[i].y;
+                    v[i].z += p[i].z;
+                    v[i].w += p[i].w;
                 }
             }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) {
+        const int c = threadIdx.x + i * kNormThreads;
+        if (c < nvec) {
+            const float4 x = v[i];
             rrow[c] = x;
-            v[i] = x;
             ss += x.x * x.x + x.y * x.y + x.z * x.z + x.w * x.w;
         }
     }
     const float tot = block_sum(ss, scratch);
     if (resid_bf != nullptr) {   // fused-norm mode: the consumer GEMM normalises; publish bf16(resid) and sum x^2
 #pragma unroll
-        for (int i = 0; i < kNormMaxVec; ++i) {
+        for (int i = 0; i < VEC; ++i) {
             const int c = threadIdx.x + i * kNormThreads;
             if (c < nvec) {
-                const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(w) + 2 * c;
-                const float2 w0 = __bfloat1622float2(wp[0]), w1 = __bfloat1622float2(wp[1]);
+                const float2 w0 = weight(i, 0), w1 = weight(i, 1);
                 __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(resid_bf + (size_t)m * h) + 2 * c;
                 op[0] = __floats2bfloat162_rn(v[i].x * w0.x, v[i].y * w0.y);
                 op[1] = __floats2bfloat162_rn(v[i].z * w1.x, v[i].w * w1.y);
@@ -94,11 +127,10 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
     const float inv = rsqrtf(tot / (float)h + eps);
     if (xnorm == nullptr) return;
 #pragma unroll
-    for (int i = 0; i < kNormMaxVec; ++i) {
+    for (int i = 0; i < VEC; ++i) {
         const int c = threadIdx.x + i * kNormThreads;
         if (c < nvec) {
-            const __nv_bfloat162* wp = reinterpret_cast<const __nv_bfloat162*>(w) + 2 * c;
-            const float2 w0 = __bfloat1622float2(wp[0]), w1 = __bfloat1622float2(wp[1]);
+            const float2 w0 = weight(i, 0), w1 = weight(i, 1);
             __nv_bfloat162 o0 = __floats2bfloat162_rn(v[i].x * inv * w0.x, v[i].y * inv * w0.y);
             __nv_bfloat162 o1 = __floats2bfloat162_rn(v[i].z * inv * w1.x, v[i].w * inv * w1.y);
             __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(xnorm + (size_t)m * h) + 2 * c;
@@ -114,6 +146,8 @@ int launch_add_norm(float* resid, const float* part, int nslices, size_t slice_s
     if (h % 4 || h > kNormThreads * kNormMaxVec * 4) return set_error("add_norm: hidden must be %%4 and <= 8192");
     if (M <= 0) return 0;
     glue_carveout();
+    const int vecs = (h / 4 + kNormThreads - 1) / kNormThreads;
+    auto* kernel = vecs <= 2 ? add_norm_kernel<2> : vecs <= 4 ? add_norm_kernel<4> : vecs <= 6 ? add_norm_kernel<6> : add_norm_kernel<8>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -123,7 +157,7 @@ int launch_add_norm(float* resid, const float* part, int nslices, size_t slice_s
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = tuning().glue_pdl ? 1 : 0;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, add_norm_kernel, resid, part, nslices, slice_stride, tokens, emb, w, xnorm, h, eps,
+    ASD_CUDA(cudaLaunchKernelEx(&cfg, kernel, resid, part, nslices, slice_stride, tokens, emb, w, xnorm, h, eps,
                                 resid_bf, sumsq0));
     count_launch(1);
     return 0;
@@ -327,60 +361,89 @@ int launch_reduce_slices(float* part, int nslices, size_t slice_stride, size_t n
     return 0;
 }
 
-// one CTA per token: bias, RoPE, q store, paged K/V append
-__global__ void __launch_bounds__(256) qkv_rope_kernel(const float* __restrict__ part, int nslices, size_t slice_stride,
-                                                        const __nv_bfloat16* __restrict__ bias,
-                                                        const int* __restrict__ positions,
-                                                        const int* __restrict__ token_slot,
-                                                        const int* __restrict__ page_table, int max_pages,
-                                                        const float* __restrict__ inv_freq,
-                                                        __nv_bfloat16* __restrict__ q_out,
-                                                        __nv_bfloat16* __restrict__ k_cache,
-                                                        __nv_bfloat16* __restrict__ v_cache, int nh, int nkv, int hd,
-                                                        int page_size) {
-    extern __shared__ float cs[];  // cos[hd/2], sin[hd/2]
-    grid_dep_launch();
+// One CTA per token: bias, RoPE, q store, paged K/V append.  An item is four rotary pairs of a query or key head, or eight values: two
+// float4 of the row, of which a thread requests three items' before it needs the first.  Angles and page come before the wait.  (A scalar at
+// a time and launched plainly it ended 17.8 us after the GEMM of 509 tokens of 28 + 8 heads; now 5.4.)
+constexpr int kRopeThreads = 256, kRopeItems = 3;
+__device__ __forceinline__ void rope_store4(__nv_bfloat16* p, float a, float b, float c, float d) {
+    __nv_bfloat162 v[2] = {__floats2bfloat162_rn(a, b), __floats2bfloat162_rn(c, d)};
+    *reinterpret_cast<uint2*>(p) = *reinterpret_cast<const uint2*>(v);
+}
+__global__ void __launch_bounds__(kRopeThreads) qkv_rope_kernel(const float* __restrict__ part, int nslices, size_t slice_stride,
+                                                                const __nv_bfloat16* __restrict__ bias,
+                                                                const int* __restrict__ positions,
+                                                                const int* __restrict__ token_slot,
+                                                                const int* __restrict__ page_table, int max_pages,
+                                                                const float* __restrict__ inv_freq,
+                                                                __nv_bfloat16* __restrict__ q_out,
+                                                                __nv_bfloat16* __restrict__ k_cache,
+                                                                __nv_bfloat16* __restrict__ v_cache, int nh, int nkv, int hd,
+                                                                int page_size) {
+    extern __shared__ __align__(16) float cs[];  // cos[hd/2], sin[hd/2]
     const int m = blockIdx.x, half = hd >> 1;
     const int pos = positions[m];
     const int nqkv = (nh + 2 * nkv) * hd;
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
+    for (int i = threadIdx.x; i < half; i += kRopeThreads) {
         float s, c;
         sincosf((float)pos * inv_freq[i], &s, &c);
         cs[i] = c;
         cs[half + i] = s;
     }
-    __syncthreads();
     const int slot = token_slot[m];
     const int page = page_table[(size_t)slot * max_pages + pos / page_size];
     const int in_page = pos % page_size;
     const float* row = part + (size_t)m * nqkv;
-    auto val = [&](int c) {
-        float x = row[c];
-        for (int s = 1; s < nslices; ++s) x += row[s * slice_stride + c];
-        return x + __bfloat162float(bias[c]);
-    };
-    // rotary pairs of q and k heads
-    const int npairs = (nh + nkv) * half;
-    for (int t = threadIdx.x; t < npairs; t += blockDim.x) {
-        const int head = t / half, i = t - head * half;
-        const float x1 = val(head * hd + i), x2 = val(head * hd + i + half);
-        const float c = cs[i], s = cs[half + i];
-        const __nv_bfloat16 o1 = __float2bfloat16(x1 * c - x2 * s), o2 = __float2bfloat16(x2 * c + x1 * s);
-        if (head < nh) {
-            __nv_bfloat16* q = q_out + (size_t)m * nh * hd + head * hd;
-            q[i] = o1;
-            q[i + half] = o2;
-        } else {
-            const int g = head - nh;
-            __nv_bfloat16* k = k_cache + (((size_t)page * nkv + g) * page_size + in_page) * hd;
-            k[i] = o1;
-            k[i + half] = o2;
+    const int quads = half >> 2, nrot = (nh + nkv) * quads, items = nrot + nkv * (hd >> 3);
+    const int v0 = (nh + nkv) * hd;
+    grid_dep_wait();
+    grid_dep_launch();
+    __syncthreads();
+    for (int base = threadIdx.x; base < items; base += kRopeThreads * kRopeItems) {
+        int c1[kRopeItems], c2[kRopeItems];
+        float4 x1[kRopeItems], x2[kRopeItems];
+#pragma unroll
+        for (int u = 0; u < kRopeItems; ++u) {
+            const int t = base + u * kRopeThreads;
+            if (t < nrot) {
+                const int head = t / quads;
+                c1[u] = head * hd + (t - head * quads) * 4, c2[u] = c1[u] + half;
+            } else {
+                c1[u] = v0 + (t - nrot) * 8, c2[u] = c1[u] + 4;
+            }
+            if (t < items) x1[u] = *reinterpret_cast<const float4*>(row + c1[u]), x2[u] = *reinterpret_cast<const float4*>(row + c2[u]);
         }
-    }
-    const int nv = nkv * hd;
-    for (int t = threadIdx.x; t < nv; t += blockDim.x) {
-        const int g = t / hd, d = t - g * hd;
-        v_cache[(((size_t)page * nkv + g) * page_size + in_page) * hd + d] = __float2bfloat16(val((nh + nkv) * hd + t));
+        for (int s = 1; s < nslices; ++s) {
+            const float* sl = row + s * slice_stride;
+#pragma unroll
+            for (int u = 0; u < kRopeItems; ++u)
+                if (base + u * kRopeThreads < items) {
+                    const float4 p1 = *reinterpret_cast<const float4*>(sl + c1[u]), p2 = *reinterpret_cast<const float4*>(sl + c2[u]);
+                    x1[u].x += p1.x, x1[u].y += p1.y, x1[u].z += p1.z, x1[u].w += p1.w;
+                    x2[u].x += p2.x, x2[u].y += p2.y, x2[u].z += p2.z, x2[u].w += p2.w;
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < kRopeItems; ++u) {
+            const int t = base + u * kRopeThreads;
+            if (t >= items) continue;
+            const __nv_bfloat16 *b1 = bias + c1[u], *b2 = bias + c2[u];
+            float4 a = x1[u], b = x2[u];
+            a.x += __bfloat162float(b1[0]), a.y += __bfloat162float(b1[1]), a.z += __bfloat162float(b1[2]), a.w += __bfloat162float(b1[3]);
+            b.x += __bfloat162float(b2[0]), b.y += __bfloat162float(b2[1]), b.z += __bfloat162float(b2[2]), b.w += __bfloat162float(b2[3]);
+            if (t < nrot) {
+                const int head = t / quads, i = (t - head * quads) * 4;
+                const float4 c = *reinterpret_cast<const float4*>(cs + i), s = *reinterpret_cast<const float4*>(cs + half + i);
+                __nv_bfloat16* o = head < nh ? q_out + ((size_t)m * nh + head) * hd + i
+                                             : k_cache + (((size_t)page * nkv + head - nh) * page_size + in_page) * hd + i;
+                rope_store4(o, a.x * c.x - b.x * s.x, a.y * c.y - b.y * s.y, a.z * c.z - b.z * s.z, a.w * c.w - b.w * s.w);
+                rope_store4(o + half, b.x * c.x + a.x * s.x, b.y * c.y + a.y * s.y, b.z * c.z + a.z * s.z, b.w * c.w + a.w * s.w);
+            } else {
+                const int e = (t - nrot) * 8, g = e / hd, d = e - g * hd;
+                __nv_bfloat16* o = v_cache + (((size_t)page * nkv + g) * page_size + in_page) * hd + d;
+                rope_store4(o, a.x, a.y, a.z, a.w);
+                rope_store4(o + 4, b.x, b.y, b.z, b.w);
+            }
+        }
     }
 }
 
@@ -389,10 +452,19 @@ int launch_qkv_rope(const float* part, int nslices, size_t slice_stride, const _
                     const float* inv_freq, __nv_bfloat16* q_out, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, int M,
                     int nh, int nkv, int hd, int page_size, cudaStream_t stream) {
     if (M <= 0) return 0;
-    qkv_rope_kernel<<<M, 256, hd * sizeof(float), stream>>>(part, nslices, slice_stride, bias, positions, token_slot,
-                                                             page_table, max_pages, inv_freq, q_out, k_cache, v_cache,
-                                                             nh, nkv, hd, page_size);
-    ASD_CUDA(cudaGetLastError());
+    if (hd % 8) return set_error("qkv_rope: head_dim must be a multiple of 8");
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(M);
+    cfg.blockDim = dim3(kRopeThreads);
+    cfg.dynamicSmemBytes = hd * sizeof(float);
+    cfg.stream = stream;
+    cfg.attrs = attr;
+    cfg.numAttrs = tuning().glue_pdl ? 1 : 0;
+    ASD_CUDA(cudaLaunchKernelEx(&cfg, qkv_rope_kernel, part, nslices, slice_stride, bias, positions, token_slot, page_table, max_pages,
+                                inv_freq, q_out, k_cache, v_cache, nh, nkv, hd, page_size));
     count_launch(1);
     return 0;
 }
@@ -442,7 +514,10 @@ int launch_gather_rows(const __nv_bfloat16* src, const int* rows, __nv_bfloat16*
 static void glue_carveout() {
     static PerDeviceOnce once;
     once.run([]() {
-        prefer_max_smem(add_norm_kernel);
+        prefer_max_smem(add_norm_kernel<2>);
+        prefer_max_smem(add_norm_kernel<4>);
+        prefer_max_smem(add_norm_kernel<6>);
+        prefer_max_smem(add_norm_kernel<8>);
         prefer_max_smem(tp_allreduce_norm_kernel);
         prefer_max_smem(reduce_slices_kernel);
         prefer_max_smem(qkv_rope_kernel);
@@ -456,7 +531,10 @@ static void glue_carveout() {
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_layers() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<2>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<4>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<6>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<8>));
     ASD_CUDA(cudaFuncGetAttributes(&fa, tp_allreduce_norm_kernel));
     ASD_CUDA(cudaFuncGetAttributes(&fa, reduce_slices_kernel));
     ASD_CUDA(cudaFuncGetAttributes(&fa, qkv_rope_kernel));

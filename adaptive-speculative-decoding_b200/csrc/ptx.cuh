@@ -300,9 +300,10 @@ __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol
 // Programmatic launch and TMEM.  A grid may become resident once every CTA of its predecessor has triggered (or ended), so
 //   * no CTA triggers (griddepcontrol.launch_dependents) before its own tcgen05.alloc has returned: otherwise the successor's CTA
 //     may take the columns and then wait for a grid that waits for those columns.  gemm.cu, gemm_tc.cu and attention_tc.cu
-//     allocate, synchronise the CTA (the pair), and trigger later; latent_attention_tc.cu and linear_tc.cu never trigger;
+//     allocate, synchronise the CTA (the pair), and trigger later; latent_attention_tc.cu, latent_prompt_tc.cu,
+//     latent_step_tc.cu and linear_tc.cu never trigger;
 //   * a kernel that allocates for a CTA pair (gemm_tc.cu) is launched plainly: its columns then never depend on another grid's;
-//   * nobody triggers before it waits, unless it was launched plainly itself (qkv_rope_kernel, sampler_stats_kernel): otherwise
+//   * nobody triggers before it waits, unless it was launched plainly itself (sampler_stats_kernel): otherwise
 //     chains of grids hold their places while the first one runs.
 // Kernels of different streams are outside of these rules: generations that share a device are serialised by the caller.
 //
