@@ -24,6 +24,8 @@
 //     device memory, every CTA derives the same list of (matrix, weight tile, token tile) from them.  Before, these products ran
 //     on single CTAs of 128 x 128 whose operands went through registers (linear_tc.cu): 8192 rows in 8 groups, 2048 x 2048 each
 //     184 and 183 us, here 66 and 64.
+//   * terms form (keys and values of a prompt's latent attention, latent_prompt_tc.cu): every fp32 result leaves as two bf16 terms, a
+//     plane each, 16 of its bits.
 // Epilogues: fp32 (+ per-token rstd of the fused RMSNorm, + accumulate), relu(y)^2 -> bf16 (grouped form) and SwiGLU -> bf16 for gate|up weights
 // interleaved 64 gate / 64 up rows per 128-row tile (same layout as gemm.cu).
 //
