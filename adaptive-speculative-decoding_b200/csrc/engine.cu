@@ -277,7 +277,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
     }
     // few query rows a key/value head: shares of any whole pages
     int few_keys = e->attn_impl >= 3 && e->kv_map_ok && q_tile == 0
-                       ? attention_few_split(nseq, nkv, hd, c.page_size, max_qlen * group, max_kv_len) : 0;
+                       ? attention_few_split(M, nseq, nkv, hd, c.page_size, max_qlen * group, max_kv_len) : 0;
     int few_shares = few_keys > 0 ? (max_kv_len + few_keys - 1) / few_keys : 0;
     if (few_shares > 1 && (size_t)M * nh * few_shares * hd > e->o_part_floats) few_keys = 0;
     int parts = 1;   // rows of e->sumsq that currently describe the residual (fused-norm mode)

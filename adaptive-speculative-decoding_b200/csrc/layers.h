@@ -61,7 +61,7 @@ struct AttnLaunch {
 int launch_attention(const AttnLaunch& L, cudaStream_t stream);
 int launch_attention_tc(const AttnLaunch& L, cudaStream_t stream);
 // few query rows a key/value head (attention_few.cu): keys of a share, or 0 where it does not apply
-int attention_few_split(int nseq, int nkv, int hd, int page_size, int rows, int max_kv_len);
+int attention_few_split(int M, int nseq, int nkv, int hd, int page_size, int rows, int max_kv_len);
 int launch_attention_few(const AttnLaunch& L, cudaStream_t stream);
 int preload_attention_few();
 

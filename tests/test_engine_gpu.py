@@ -476,7 +476,10 @@ def test_forward_prompt_limits():
     (8, 2, 3, [129, 1140, 765]),                   # 12 rows; several shares, an empty one
     (16, 2, 4, [1300, 300]),                       # 32 rows, several shares
     (2, 2, 1, [3300, 5]),                          # one row
-    (9, 3, 6, [9] * 14),                           # 18 rows of too many items
+    (9, 3, 6, [9] * 14),                           # 18 rows
+    (11, 1, 3, [40, 7]),                           # 33 rows: too many
+    (17, 1, 1, [250] * 257),                       # 17 rows, more than 256 tokens
+    (17, 1, 1, [256] * 257),                       # ... of more than 256 keys
 ])
 def test_few_query_rows(nh, nkv, q, lens):
     """steps of few rows a key/value head: the kernel that takes pages a warp, against the oracle and the tcgen05 kernel"""
@@ -491,7 +494,8 @@ def test_few_query_rows(nh, nkv, q, lens):
     eng.prefill_ragged([t[0, :n].tolist() for t, n in zip(ids, lens)], slots)
     new = torch.cat([t[:, n:] for t, n in zip(ids, lens)]).to(torch.int32).cuda()
     start = torch.tensor(lens, dtype=torch.int32, device="cuda")
-    takes = q * nh // nkv <= 16 or len(lens) * nkv <= torch.cuda.get_device_properties(0).multi_processor_count // 4
+    rows = q * nh // nkv
+    takes = rows <= 16 or (rows <= 32 and (len(lens) * q <= 256 or max(lens) + q <= 256))
     got = []
     for impl in (3, 2):
         eng.set_option("attn_impl", impl)
