@@ -123,7 +123,7 @@ __global__ void __launch_bounds__(256 * RT, 1) attn_few_kernel(const __grid_cons
     for (int p = warp; p < pages; p += kAfWarps) {
         const int slot = p % kAfSlots, key0 = kbeg + p * kAfPage;
         uint8_t* pg = ring + slot * kAfSlot;
-        mbar_wait_timed(&full[slot], (p / kAfSlots) & 1, guard, 6);
+        mbar_wait_timed(&full[slot], (p / kAfSlots) & 1, guard, 16);
         if (key0 + kAfPage > kend) {   // places that nobody wrote must not meet the zero weights
             for (int i = lane; i < (key0 + kAfPage - kend) * 16; i += 32) {
                 const int r = kend - key0 + (i >> 4), c = i & 15;

@@ -322,12 +322,14 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
             parts = 1;
         }
     }
+    const bool tc_qkv = P->use_tc && e->tune.gemm_big >= 1 && e->tc_qkvo;        // tensor-bound step: CTA-pair GEMM + one glue kernel
     {
         PROF(PROF_GLUE);
+        const bool table = !tc_qkv && P->qkv.mode == GEMM_OUT_QKV;       // of rotary angles, for the fused QKV epilogue
         if (launch_add_norm(e->resid, nullptr, 0, 0, tokens, e->embed, e->layers[0].ln1, fn ? nullptr : e->xnorm, M, h,
-                            c.rms_eps, s, fn ? e->resid_bf : nullptr, fn ? e->sumsq : nullptr))
+                            c.rms_eps, s, fn ? e->resid_bf : nullptr, fn ? e->sumsq : nullptr, positions, e->inv_freq,
+                            table ? e->rope_cs : nullptr, hd / 2))
             return -1;
-        if (P->qkv.mode == GEMM_OUT_QKV && launch_rope_table(positions, e->inv_freq, e->rope_cs, M, hd / 2, s)) return -1;
     }
     // residual update after a row-parallel projection: fused into the GEMM when possible, else glue kernel
     // one kernel: all-reduce of the partials in tp_buf[epoch & 1] over NVLink peer memory + residual add + norm stats
@@ -463,7 +465,7 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         Layer& L = e->layers[l];
         __nv_bfloat16* kc = e->kv_pool + (size_t)(2 * l) * e->kv_half;
         __nv_bfloat16* vc = kc + e->kv_half;
-        if (P->use_tc && e->tune.gemm_big >= 1 && e->tc_qkvo) {   // tensor-bound step: CTA-pair GEMM + one glue kernel
+        if (tc_qkv) {
             {
                 PROF(PROF_GEMM);
                 if (gemm_tc_launch(P->qkv_tc, L.t_qkv, P->x_norm_qkv_tc, e->part, e->nqkv, e->nqkv, (size_t)M * e->nqkv, s,

@@ -39,7 +39,10 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // after the other inside each element, and the weights behind the row's sum, the kernel ended 7.3 us after the CTA-pair GEMM of an O
 // projection of 509 tokens, hidden size 3584, and 11.6 after the down projection's more slices; now 5.8 and 10).
 // VEC: float4 per thread, so that the registers of an 8192-wide row do not cost narrower ones their CTAs.
-template <int VEC>
+// EMBED: the forward's first launch.  It also fills the table of rotary angles that the fused QKV epilogue reads.  As a kernel of its own
+// that stood between the gather and the QKV projection, which can now request its weights meanwhile: a drafted token through four 7B layers
+// 564 -> 559 us, a verification of 16 x 6 tokens through three 32B layers 935 -> 931.
+template <int VEC, bool EMBED>
 __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restrict__ resid, const float* __restrict__ part,
                                                                  int nslices, size_t slice_stride,
                                                                  const int* __restrict__ tokens,
@@ -47,7 +50,8 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
                                                                  const __nv_bfloat16* __restrict__ w,
                                                                  __nv_bfloat16* __restrict__ xnorm, int h, float eps,
                                                                  __nv_bfloat16* __restrict__ resid_bf,
-                                                                 float* __restrict__ sumsq0) {
+                                                                 float* __restrict__ sumsq0, const int* __restrict__ positions,
+                                                                 const float* __restrict__ inv_freq, float2* __restrict__ cs, int half) {
     __shared__ float scratch[kNormThreads / 32];
     const int m = blockIdx.x, nvec = h >> 2;
     uint32_t wt[VEC][2];        // the norm's weights never change
@@ -65,7 +69,7 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
     float4 v[VEC];
     float ss = 0.0f;
     float4* rrow = reinterpret_cast<float4*>(resid + (size_t)m * h);
-    if (tokens) {
+    if (EMBED) {
         const __nv_bfloat162* row = reinterpret_cast<const __nv_bfloat162*>(emb + (size_t)tokens[m] * h);
 #pragma unroll
         for (int i = 0; i < VEC; ++i) {
@@ -73,6 +77,14 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
             if (c < nvec) {
                 const float2 a = __bfloat1622float2(row[2 * c]), b = __bfloat1622float2(row[2 * c + 1]);
                 v[i] = make_float4(a.x, a.y, b.x, b.y);
+            }
+        }
+        if (cs != nullptr) {
+            const float pos = (float)positions[m];
+            for (int i = threadIdx.x; i < half; i += kNormThreads) {
+                float sn, c;
+                sincosf(pos * inv_freq[i], &sn, &c);
+                cs[(size_t)m * half + i] = make_float2(c, sn);
             }
         }
     } else {
@@ -142,12 +154,17 @@ __global__ void __launch_bounds__(kNormThreads) add_norm_kernel(float* __restric
 
 int launch_add_norm(float* resid, const float* part, int nslices, size_t slice_stride, const int* tokens,
                     const __nv_bfloat16* emb, const __nv_bfloat16* w, __nv_bfloat16* xnorm, int M, int h, float eps,
-                    cudaStream_t stream, __nv_bfloat16* resid_bf, float* sumsq0) {
+                    cudaStream_t stream, __nv_bfloat16* resid_bf, float* sumsq0, const int* positions, const float* inv_freq, float2* cs,
+                    int half) {
     if (h % 4 || h > kNormThreads * kNormMaxVec * 4) return set_error("add_norm: hidden must be %%4 and <= 8192");
     if (M <= 0) return 0;
     glue_carveout();
     const int vecs = (h / 4 + kNormThreads - 1) / kNormThreads;
-    auto* kernel = vecs <= 2 ? add_norm_kernel<2> : vecs <= 4 ? add_norm_kernel<4> : vecs <= 6 ? add_norm_kernel<6> : add_norm_kernel<8>;
+    auto* kernel = vecs <= 2   ? tokens ? add_norm_kernel<2, true> : add_norm_kernel<2, false>
+                   : vecs <= 4 ? tokens ? add_norm_kernel<4, true> : add_norm_kernel<4, false>
+                   : vecs <= 6 ? tokens ? add_norm_kernel<6, true> : add_norm_kernel<6, false>
+                   : tokens    ? add_norm_kernel<8, true>
+                               : add_norm_kernel<8, false>;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -158,7 +175,7 @@ int launch_add_norm(float* resid, const float* part, int nslices, size_t slice_s
     cfg.attrs = attr;
     cfg.numAttrs = tuning().glue_pdl ? 1 : 0;
     ASD_CUDA(cudaLaunchKernelEx(&cfg, kernel, resid, part, nslices, slice_stride, tokens, emb, w, xnorm, h, eps,
-                                resid_bf, sumsq0));
+                                resid_bf, sumsq0, positions, inv_freq, cs, half));
     count_launch(1);
     return 0;
 }
@@ -469,27 +486,6 @@ int launch_qkv_rope(const float* part, int nslices, size_t slice_stride, const _
     return 0;
 }
 
-// (cos, sin) of every token's rotary angles, once per forward (consumed by the fused QKV epilogue)
-__global__ void rope_table_kernel(const int* __restrict__ positions, const float* __restrict__ inv_freq,
-                                  float2* __restrict__ cs, int half) {
-    const int m = blockIdx.x;
-    const float pos = (float)positions[m];
-    for (int i = threadIdx.x; i < half; i += blockDim.x) {
-        float s, c;
-        sincosf(pos * inv_freq[i], &s, &c);
-        cs[(size_t)m * half + i] = make_float2(c, s);
-    }
-}
-
-int launch_rope_table(const int* positions, const float* inv_freq, float2* cs, int M, int half, cudaStream_t stream) {
-    if (M <= 0) return 0;
-    glue_carveout();
-    rope_table_kernel<<<M, 64, 0, stream>>>(positions, inv_freq, cs, half);
-    ASD_CUDA(cudaGetLastError());
-    count_launch(1);
-    return 0;
-}
-
 __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ src, const int* __restrict__ rows,
                                    __nv_bfloat16* __restrict__ dst, int h, const float* __restrict__ ss_src,
                                    float* __restrict__ ss_dst, int parts, int ld) {
@@ -514,14 +510,17 @@ int launch_gather_rows(const __nv_bfloat16* src, const int* rows, __nv_bfloat16*
 static void glue_carveout() {
     static PerDeviceOnce once;
     once.run([]() {
-        prefer_max_smem(add_norm_kernel<2>);
-        prefer_max_smem(add_norm_kernel<4>);
-        prefer_max_smem(add_norm_kernel<6>);
-        prefer_max_smem(add_norm_kernel<8>);
+        prefer_max_smem(add_norm_kernel<2, false>);
+        prefer_max_smem(add_norm_kernel<2, true>);
+        prefer_max_smem(add_norm_kernel<4, false>);
+        prefer_max_smem(add_norm_kernel<4, true>);
+        prefer_max_smem(add_norm_kernel<6, false>);
+        prefer_max_smem(add_norm_kernel<6, true>);
+        prefer_max_smem(add_norm_kernel<8, false>);
+        prefer_max_smem(add_norm_kernel<8, true>);
         prefer_max_smem(tp_allreduce_norm_kernel);
         prefer_max_smem(reduce_slices_kernel);
         prefer_max_smem(qkv_rope_kernel);
-        prefer_max_smem(rope_table_kernel);
         prefer_max_smem(gather_rows_kernel);
         return 0;
     });
@@ -531,14 +530,17 @@ static void glue_carveout() {
 // context synchronisation, which deadlocks when another rank of the same process is spinning for this rank's launch.
 int preload_layers() {
     cudaFuncAttributes fa;
-    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<2>));
-    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<4>));
-    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<6>));
-    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<8>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<2, false>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<2, true>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<4, false>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<4, true>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<6, false>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<6, true>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<8, false>));
+    ASD_CUDA(cudaFuncGetAttributes(&fa, add_norm_kernel<8, true>));
     ASD_CUDA(cudaFuncGetAttributes(&fa, tp_allreduce_norm_kernel));
     ASD_CUDA(cudaFuncGetAttributes(&fa, reduce_slices_kernel));
     ASD_CUDA(cudaFuncGetAttributes(&fa, qkv_rope_kernel));
-    ASD_CUDA(cudaFuncGetAttributes(&fa, rope_table_kernel));
     ASD_CUDA(cudaFuncGetAttributes(&fa, gather_rows_kernel));
     return 0;
 }

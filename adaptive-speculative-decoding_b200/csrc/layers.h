@@ -11,7 +11,8 @@ namespace asd {
 
 int launch_add_norm(float* resid, const float* part, int nslices, size_t slice_stride, const int* tokens,
                     const __nv_bfloat16* emb, const __nv_bfloat16* w, __nv_bfloat16* xnorm, int M, int h, float eps,
-                    cudaStream_t stream, __nv_bfloat16* resid_bf = nullptr, float* sumsq0 = nullptr);
+                    cudaStream_t stream, __nv_bfloat16* resid_bf = nullptr, float* sumsq0 = nullptr,
+                    const int* positions = nullptr, const float* inv_freq = nullptr, float2* cs = nullptr, int half = 0);   // tokens: (cos, sin) too
 int launch_tp_allreduce_norm(const float* const* peer_bufs, uint32_t* const* peer_flags, int rank, int world,
                              uint32_t epoch, int* error, float* resid, const __nv_bfloat16* w, __nv_bfloat16* xnorm,
                              int M, int h, float eps, __nv_bfloat16* resid_bf, float* sumsq0, cudaStream_t stream,
@@ -23,7 +24,6 @@ int launch_qkv_rope(const float* part, int nslices, size_t slice_stride, const _
                     const int* positions, const int* token_slot, const int* page_table, int max_pages,
                     const float* inv_freq, __nv_bfloat16* q_out, __nv_bfloat16* k_cache, __nv_bfloat16* v_cache, int M,
                     int nh, int nkv, int hd, int page_size, cudaStream_t stream);
-int launch_rope_table(const int* positions, const float* inv_freq, float2* cs, int M, int half, cudaStream_t stream);
 int launch_gather_rows(const __nv_bfloat16* src, const int* rows, __nv_bfloat16* dst, int n, int h,
                        cudaStream_t stream, const float* ss_src = nullptr, float* ss_dst = nullptr, int parts = 0,
                        int ld = 0);

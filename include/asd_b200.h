@@ -202,7 +202,7 @@ ASD_API int asd_engine_device_error(asd_engine_t* e);
  * ONE process, rank r on its own device.  Enables peer access between the devices and wires every rank's receive
  * buffers and flags into the others (no IPC, no torchrun).  engines[r] must be rank r of a t-way group. */
 ASD_API int asd_engine_peer_connect(asd_engine_t** engines, int n);
-/* options: "attn_impl" (2 tcgen05 / TMEM kernel - default; 1 mma.sync kernel, also the fallback for head_dim 64 or more
+/* options: "attn_impl" (3, default: the few-row kernel where it takes a step, else as 2; 2 tcgen05 / TMEM kernel; 1 mma.sync kernel, also the fallback for head_dim 64 or more
  * than 128 query rows; 0 one-warp cross-check kernel), "tc_qkvo" (1, default: above 256 tokens QKV and O run on the
  * CTA-pair tensor-bound GEMM like gate|up / down / lm_head; 0: weight-streaming kernel), "gemm_big" (0: never use the
  * CTA-pair GEMM), "attn_prefetch_mb" (L2 prefetch of the following GEMMs' weights from the attention kernel, measured
