@@ -11,7 +11,7 @@
 //     the warps' sums meet in shared memory, one thread a row adds them in order and runs the epilogue.
 //   * A hand-over is one trip through L2: every 64-bit word of an activation carries its phase's number beside the value, the reader
 //     polls the words it needs, and no fence, flag or grid-wide barrier stands between them.  A word is written again only by a CTA that
-//     has seen results of all its readers.
+//     has seen results of all its readers, so every CTA must have results of its own (one_step_sizes).
 //   * A row of the residual belongs to the same thread in both of its projections and stays in a register.
 //   * Attention runs on a CTA per query head and share of the keys, cache rows requested before the query is there, one worker of eight
 //     (sixteen) lanes a key; shares meet at the head's first CTA.
@@ -38,9 +38,7 @@ namespace asd {
 namespace {
 
 constexpr int kOsWarps = 16, kOsThreads = (kOsWarps + 1) * 32;        // warps that multiply, and one that streams
-constexpr int kOsPanel = 16;                                         // weight rows of a panel
 constexpr int kOsMaxPiece = 1024;                                    // k elements of a panel
-constexpr int kOsMaxPanels = 8;                                      // of a phase
 constexpr int kOsArrivals = 240;                                     // of a panel's readers together: 1, 2, 3, 4, 5, 8 or 16 warps
 constexpr int kOsWords = 5;                                          // words a thread asks for at once
 constexpr int kOsLine = 16;                                          // words of a line: what all CTAs poll stands alone in one
@@ -593,12 +591,7 @@ size_t one_step_bytes(int h, int nqkv, int qdim, int ffn) { return 64 + 8 * os_w
 bool one_step_takes(const OneStep& s) {
     DeviceLimits dev;
     if (device_limits(&dev)) return false;
-    const int grid = dev.sms;
-    if (s.n_layers <= 0 || s.n_layers > kOneMaxLayers || (s.hd != 64 && s.hd != 128) || s.nkv <= 0 || s.nh % s.nkv || s.nh > grid) return false;
-    if (s.h % 16 || s.qdim % 16 || s.ffn % 16 || s.h < grid || grid > 256) return false;
-    auto most = [&](int n) { return (n + grid - 1) / grid; };
-    if (most(s.h) > 32 || 2 * most(s.nqkv / 2) > kOsMaxPanels * kOsPanel || 4 * most(s.ffn / 2) > kOsMaxPanels * kOsPanel) return false;
-    return one_step_bytes(s.h, s.nqkv, s.qdim, s.ffn) > 0 && s.work;
+    return one_step_sizes(s, dev.sms) && one_step_bytes(s.h, s.nqkv, s.qdim, s.ffn) > 0 && s.work;
 }
 
 int one_step_launch(const OneStep& s, int max_kv_len, cudaStream_t stream) {

@@ -11,7 +11,7 @@ from test_engine_gpu import MAX_ABS, Qwen2Config, _launched, check, qwen2_forwar
     (Qwen2Config(896, 3, 14, 2, 4864, 1531, head_dim=64, name="step-896"), 16, (0, 1, 63, 254, 256, 700)),     # one share of keys, two, three
     (Qwen2Config(1536, 2, 12, 2, 8960, 999, head_dim=128, name="step-1536"), 24, (5, 126, 127, 128, 300)),     # two pieces of k, eight panels
     (Qwen2Config(960, 2, 5, 5, 1232, 515, head_dim=64, name="step-odd"), 8, (40, 129)),      # pieces of 960 and 272, no grouping, few rows
-    (Qwen2Config(160, 2, 8, 1, 512, 300, head_dim=128, name="step-least"), 16, (17, 300)),   # one or two rows a CTA, some CTAs without any
+    (Qwen2Config(160, 2, 8, 1, 512, 300, head_dim=128, name="step-least"), 16, (17, 300)),   # one or two rows a CTA
 ])
 def test_one_token_in_one_launch(cfg, page, contexts):
     """three steps in a row behind every context, so that each reads what the ones before appended: against the oracle and the chain of
@@ -37,6 +37,28 @@ def test_one_token_in_one_launch(cfg, page, contexts):
             eng.close()
         check(got[1], ref[0, n:n + 3])
         assert (got[1] - got[2]).abs().max().item() <= MAX_ABS
+
+
+@pytest.mark.parametrize("cfg", [
+    Qwen2Config(256, 2, 4, 2, 256, 300, head_dim=64, name="step-narrow-ffn"),      # 128 pairs of gate and up rows: fewer than CTAs
+])
+def test_narrow_models_stay_a_chain(cfg):
+    """a model whose matrices leave CTAs without rows takes a kernel a projection, as larger steps do"""
+    from asd_b200.engine import QwenEngine
+    w = random_hf_weights(cfg, seed=37, logit_std=0.4)
+    ids = torch.randint(0, cfg.vocab_size, (1, 20), generator=torch.Generator().manual_seed(9))
+    ref = qwen2_forward(w, cfg, ids)
+    eng = QwenEngine(cfg, max_seqs=1, max_seq_len=32, max_tokens=16).load_hf_weights(w)
+    idc, slot, got = ids.cuda().to(torch.int32), torch.zeros(1, dtype=torch.int32, device="cuda"), []
+
+    def steps():
+        for i in range(20):
+            got.append(eng.forward_uniform(idc[:, i:i + 1].contiguous(), slot + i, slot, i + 1))
+
+    assert _launched("one_step", steps) == 0
+    check(torch.cat(got).cpu(), ref[0])
+    eng.check_device()
+    eng.close()
 
 
 def test_one_launch_again_and_again():
