@@ -26,13 +26,15 @@ struct OneStep {
     int* err;                              // where a wait that ran out is reported
 };
 
-// Sizes that one_step.cu takes on `grid` CTAs.  Every CTA signs that it has read its input by publishing rows of its own, and every CTA
-// waits for all signs before it overwrites what they read: each must have rows of the hidden size and of gate | up (pairs).
+// Sizes that one_step.cu takes on `grid` CTAs.  Every CTA shows that it has read its input by publishing rows of its own, and the others
+// wait for all of these before they overwrite what it read: each must have rows of the hidden size, of gate | up and of QKV (pairs of
+// rows).  Of QKV because the O projection overwrites the residual that the QKV projection reads: it has waited for the heads, and the
+// heads for every row of QKV.
 constexpr int kOsPanel = 16;               // weight rows of a panel
 constexpr int kOsMaxPanels = 8;            // of a phase
 inline bool one_step_sizes(const OneStep& s, int grid) {
     if (s.n_layers <= 0 || s.n_layers > kOneMaxLayers || (s.hd != 64 && s.hd != 128) || s.nkv <= 0 || s.nh % s.nkv || s.nh > grid) return false;
-    if (s.h % 16 || s.qdim % 16 || s.ffn % 16 || s.h < grid || s.ffn / 2 < grid || grid > 256) return false;
+    if (s.h % 16 || s.qdim % 16 || s.ffn % 16 || s.h < grid || s.ffn / 2 < grid || s.nqkv / 2 < grid || grid > 256) return false;
     auto most = [&](int n) { return (n + grid - 1) / grid; };
     return most(s.h) <= 32 && 2 * most(s.nqkv / 2) <= kOsMaxPanels * kOsPanel && 4 * most(s.ffn / 2) <= kOsMaxPanels * kOsPanel;
 }

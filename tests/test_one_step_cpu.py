@@ -53,6 +53,7 @@ def test_every_cta_has_rows_to_publish(takes, grid):
         if yes:
             took += 1
             assert min(shares(h, grid)) > 0 and min(shares(ffn // 2, grid)) > 0, size
+            assert min(shares((nh + 2 * nkv) * hd // 2, grid)) > 0, size
     assert took > 20
 
 

@@ -41,6 +41,7 @@ def test_one_token_in_one_launch(cfg, page, contexts):
 
 @pytest.mark.parametrize("cfg", [
     Qwen2Config(256, 2, 4, 2, 256, 300, head_dim=64, name="step-narrow-ffn"),      # 128 pairs of gate and up rows: fewer than CTAs
+    Qwen2Config(256, 2, 2, 1, 512, 300, head_dim=64, name="step-narrow-qkv"),      # 128 pairs of query, key and value rows
 ])
 def test_narrow_models_stay_a_chain(cfg):
     """a model whose matrices leave CTAs without rows takes a kernel a projection, as larger steps do"""
