@@ -135,7 +135,7 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_step_kernel(const __grid
             mbar_init(&B->r_empty[i], 1);
         }
         mbar_init(&B->s_full, 1);
-        mbar_init(&B->s_read, 3);
+        mbar_init(&B->s_read, 4);                              // every warp that waits for s_full: none of them may be lapped
         mbar_init(&B->p_full, 4);
         mbar_init(&B->pv_done, 1);
         B->failed = 0;
@@ -319,6 +319,8 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_step_kernel(const __grid
                     const uint32_t* v = &x[i >> 3][(i & 7) * 4];
                     dst[i] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
                 }
+            } else if (lane == 0) {
+                mbar_arrive(&B->s_read);                       // has no scores to read, and has seen that they are there
             }
             if (key0 + kLsKeys > p_last + 1 || key0 < j_lo) {
                 // keys that no row may see: whatever the pool holds there must not meet the zero weights (the scores have read them)

@@ -71,3 +71,28 @@ def test_few_rows_of_unequal_sequences():
         assert mz.rel_err(got[at:at + b], O.forward(cfg, w, t)[0][a:])[0] < 4e-2
         at += b
     mz.close(eng)
+
+
+def test_many_tiles_of_the_narrowest_latent():
+    """128 latent columns leave the least time between the scores of two tiles (12 products): 64 sequences of 40 tiles, again and again with
+    the same bits, and no wait ran out"""
+    from asd_b200._lib import lib
+    cfg = _config(16, 128, 1 << 20, 0.3)
+    w = O.random_model(cfg, seed=85, scale=1.5)
+    n, prompt = 64, 2560
+    eng = mz.make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512, max_seq_len=prompt + 16, max_seqs=n)
+    ids = mz.tokens(prompt + 1, 96, 86)
+    slots = [eng.open_sequence() for _ in range(n)]
+    for s in slots:
+        eng.reserve(s, prompt + 1)
+        eng.forward_ragged([(s, 0, ids[:prompt], [])])
+    tok = torch.full((n, 1), ids[prompt], dtype=torch.int32, device="cuda")
+    at, slot = torch.full((n,), prompt, dtype=torch.int32, device="cuda"), torch.tensor(slots, dtype=torch.int32, device="cuda")
+    before = lib().asd_kernel_launches(b"latent_step")
+    first = eng.forward_uniform(tok, at, slot, prompt + 1).clone()
+    for _ in range(100):
+        assert torch.equal(eng.forward_uniform(tok, at, slot, prompt + 1), first)
+    assert lib().asd_kernel_launches(b"latent_step") - before == 101
+    eng.check_device()
+    assert mz.rel_err(first[:1].cpu(), O.forward(cfg, w, ids)[0][-1:])[0] < 4e-2
+    mz.close(eng)
