@@ -273,7 +273,8 @@ static int forward(Engine* e, const int* tokens, const int* positions, const int
         PL.prefetch_ahead = e->persist_ahead;
         PL.sync = e->p_sync, PL.part_ws = e->p_ws, PL.error = e->wait_err, PL.trace = e->p_trace;
         PROF(PROF_GEMM);
-        return persist_launch(PL, s);
+        const int rc = persist_launch(PL, s);
+        if (rc <= 0) return rc;
     }
     // few query rows a key/value head: shares of any whole pages
     int few_keys = e->attn_impl >= 3 && e->kv_map_ok && q_tile == 0

@@ -38,6 +38,7 @@
 
 #include "asd_internal.h"
 #include "gemm.h"
+#include "grid_turn.h"
 #include "mma_sync.cuh"
 #include "persist.h"
 #include "ptx.cuh"
@@ -1080,8 +1081,10 @@ static int p_launch_t(const CUtensorMap maps[5], const PArgs& a, int grid, size_
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, fwd_persist_kernel<HD, KW>, maps[0], maps[1], maps[2], maps[3], maps[4], a));
-    return 0;
+    return grid_in_turn(stream, [&] {
+        const cudaError_t e = cudaMemsetAsync(a.L.sync, 0, sizeof(unsigned) * kPersistSyncWords, stream);
+        return e ? e : cudaLaunchKernelEx(&cfg, fwd_persist_kernel<HD, KW>, maps[0], maps[1], maps[2], maps[3], maps[4], a);
+    });
 }
 
 int persist_launch(const PersistLaunch& L, cudaStream_t stream) {
@@ -1134,7 +1137,6 @@ int persist_launch(const PersistLaunch& L, cudaStream_t stream) {
     }
     if (make_tmap_bf16(&maps[4], L.lm_head, L.vocab, L.h, L.h, 128)) return -1;
     const int grid = persist_num_ctas();
-    ASD_CUDA(cudaMemsetAsync(L.sync, 0, sizeof(unsigned) * kPersistSyncWords, stream));
     int rc;
 #define ASD_P(HD_)                                                                                    \
     (a.rg_count == 1 ? p_launch_t<HD_, 16>(maps, a, grid, smem, stream)                               \

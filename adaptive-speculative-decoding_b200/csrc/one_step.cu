@@ -25,10 +25,10 @@
 #include <stdint.h>
 
 #include <algorithm>
-#include <mutex>
 
 #include "asd_internal.h"
 #include "gemm.h"
+#include "grid_turn.h"
 #include "mma_sync.cuh"
 #include "one_step.h"
 #include "ptx.cuh"
@@ -571,13 +571,6 @@ __global__ void __launch_bounds__(kOsThreads, 1) one_step_kernel(const __grid_co
     }
 }
 
-constexpr int kOsDevices = 64;
-struct OsTurn {
-    std::mutex m;
-    cudaEvent_t done = nullptr;                // behind the last launch on the device; lives as long as the process
-};
-OsTurn g_turns[kOsDevices];
-
 size_t os_words(int h, int nqkv, int qdim, int ffn, int grid) {
     return (size_t)nqkv / 2 + qdim / 2 + (size_t)grid * 130 + h + ffn / 2 + 4 * grid * kOsLine + 3 * kOsLine;
 }
@@ -628,17 +621,6 @@ int one_step_launch(const OneStep& s, int max_kv_len, cudaStream_t stream) {
     const int smem = a.slots * a.slot_bytes + a.x_bytes + (int)sizeof(OsShared);
     auto fn = s.hd == 64 ? one_step_kernel<64> : one_step_kernel<128>;
     if (preload_one_step()) return -1;
-    // Its CTAs wait for one another, and two such grids would share the SMs between them: one at a time on a device, whatever the streams.
-    // A captured step could not keep to that when it is replayed and stays a chain of kernels.
-    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-    ASD_CUDA(cudaStreamIsCapturing(stream, &capturing));
-    int device = 0;
-    ASD_CUDA(cudaGetDevice(&device));
-    if (capturing != cudaStreamCaptureStatusNone || device >= kOsDevices) return 1;
-    OsTurn& turn = g_turns[device];
-    std::lock_guard<std::mutex> lock(turn.m);
-    if (!turn.done) ASD_CUDA(cudaEventCreateWithFlags(&turn.done, cudaEventDisableTiming));
-    ASD_CUDA(cudaStreamWaitEvent(stream, turn.done, 0));       // (nothing recorded yet: no wait)
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;       // all CTAs resident, or an error
@@ -649,8 +631,7 @@ int one_step_launch(const OneStep& s, int max_kv_len, cudaStream_t stream) {
     cfg.stream = stream;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    ASD_CUDA(cudaLaunchKernelEx(&cfg, fn, a));
-    ASD_CUDA(cudaEventRecord(turn.done, stream));
+    if (const int rc = grid_in_turn(stream, [&] { return cudaLaunchKernelEx(&cfg, fn, a); })) return rc;
     count_kernel(KERNEL_ONE_STEP);
     for (int i = 0; i < 4 * s.n_layers; ++i) note_kernel(KERNEL_GEMV);
     return 0;

@@ -42,7 +42,7 @@ inline bool one_step_sizes(const OneStep& s, int grid) {
 int one_step_sums();
 size_t one_step_bytes(int h, int nqkv, int qdim, int ffn);
 bool one_step_takes(const OneStep& s);     // on the current device
-// 0, -1 (error), or 1: sizes that it does not take after all, nothing launched
+// 0, -1 (error), or 1: sizes that it does not take after all or not its turn (grid_turn.h), nothing launched
 int one_step_launch(const OneStep& s, int max_kv_len, cudaStream_t stream);
 int preload_one_step();
 

@@ -60,6 +60,7 @@ constexpr int kPersistSyncWords = kPersistMaxPhases + 512;   // phase counters, 
 bool persist_supported(int M, int n_logit_rows, int max_qlen, int nh, int nkv, int hd, int page_size, int h, int n_layers);
 int persist_num_ctas();
 size_t persist_part_ws_bytes();
+// 0, -1 (error), or 1: not its turn (grid_turn.h), nothing launched
 int persist_launch(const PersistLaunch& L, cudaStream_t stream);
 
 }  // namespace asd

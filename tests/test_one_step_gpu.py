@@ -119,3 +119,44 @@ def test_one_launch_on_two_streams_and_under_capture():
     for eng in engines:
         eng.check_device()
         eng.close()
+
+
+def test_one_launch_beside_a_persistent_forward():
+    """steps of two engines on two streams, one in one launch and one in the persistent forward kernel (both wait for their own CTAs), end with the
+    right results; a captured step of either is a chain of kernels"""
+    from asd_b200.engine import QwenEngine
+    cfg = Qwen2Config(896, 2, 14, 2, 4864, 1000, head_dim=64, name="step-persist")
+    w = random_hf_weights(cfg, seed=39, logit_std=0.4)
+    engines = [QwenEngine(cfg, max_seqs=1, max_seq_len=64, max_tokens=16).load_hf_weights(w) for _ in range(2)]
+    engines[1].set_option("persist", 1)
+    slot = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tok, pos, cu = slot + 7, slot.clone(), torch.tensor([0, 1], dtype=torch.int32, device="cuda")
+    out = [torch.empty(1, cfg.vocab_size, device="cuda") for _ in range(2)]
+    want = [eng.forward(tok, pos, slot, cu, slot, 1, 1).clone() for eng in engines]
+    check(torch.cat(want).cpu(), qwen2_forward(w, cfg, torch.tensor([[7]]))[0].expand(2, -1))
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    torch.cuda.synchronize()
+
+    def steps():
+        for _ in range(50):
+            for eng, s, o in zip(engines, streams, out):
+                with torch.cuda.stream(s):
+                    eng.forward(tok, pos, slot, cu, slot, 1, 1, logits_out=o)
+        torch.cuda.synchronize()
+
+    assert _launched("one_step", steps) == 50
+    for eng, o, x in zip(engines, out, want):
+        assert (o - x).abs().max().item() <= MAX_ABS
+        eng.check_device()
+        graph = torch.cuda.CUDAGraph()
+
+        def captured():
+            with torch.cuda.graph(graph):
+                eng.forward(tok, pos, slot, cu, slot, 1, 1, logits_out=o)
+
+        assert _launched("gemv", captured) > 0
+        o.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert (o - x).abs().max().item() <= MAX_ABS
+        eng.close()
