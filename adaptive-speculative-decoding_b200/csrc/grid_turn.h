@@ -20,7 +20,8 @@ inline GridTurn* grid_turns() {
 
 // `launch` (which returns cudaError_t) behind the last such grid of the current device: two of them would share the SMs between them and
 // each wait for CTAs that find no place.  Returns 0, -1 (error), or 1: nothing was launched, a chain of kernels has to do.  That is so for a
-// captured step, which could not keep its turn when it is replayed.
+// captured step, which could not keep its turn when it is replayed, and where the device refuses the grid as a whole (a context with a part
+// of the SMs).
 template <typename F>
 int grid_in_turn(cudaStream_t stream, F&& launch) {
     cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
@@ -34,6 +35,10 @@ int grid_in_turn(cudaStream_t stream, F&& launch) {
         if (!turn.done) e = cudaEventCreateWithFlags(&turn.done, cudaEventDisableTiming);
         if (e == cudaSuccess) e = cudaStreamWaitEvent(stream, turn.done, 0);       // (nothing recorded yet: no wait)
         if (e == cudaSuccess) e = launch();
+        if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+            cudaGetLastError();          // nobody else's error
+            return 1;
+        }
         if (e == cudaSuccess) e = cudaEventRecord(turn.done, stream);
     }
     return e == cudaSuccess ? 0 : set_error("launch of a grid that waits for itself: %s", cudaGetErrorString(e));

@@ -41,6 +41,10 @@ int main() {
     printf("= %d\n", go(3, cudaSuccess));                                  // a device of its own
     device = 64;
     printf("= %d\n", go(3, cudaSuccess));
+    device = 0;
+    printf("= %d\n", go(1, cudaErrorCooperativeLaunchTooLarge));
+    printf("= %d\n", go(1, cudaErrorNotSupported));
+    printf("= %d\n", go(1, cudaSuccess));
 }
 """
 
@@ -63,6 +67,13 @@ def test_one_grid_behind_another(lines):
     assert lines[3] == "= 1"
     assert lines[4] == "wait3:2 launch record3:2 = 0"
     assert lines[5] == "= 1"
+
+
+def test_a_refused_grid_is_no_error(lines):
+    """a grid that finds no room as a whole (fewer SMs than the device has, say) leaves the step to a chain of kernels, and no error behind"""
+    assert lines[6] == "wait1:1 launch cleared = 1"
+    assert lines[7] == "wait1:1 launch cleared = 1"
+    assert lines[8] == "wait1:1 launch record1:1 = 0"
 
 
 def test_every_such_grid_takes_its_turn():
