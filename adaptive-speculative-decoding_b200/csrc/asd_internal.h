@@ -28,7 +28,14 @@ void note_kernel(CountedKernel k);                      // of a launch that is c
 // ---- Bounded device waits.  A kernel whose barrier does not complete gives up after some seconds (ptx.cuh, mbar_wait), writes
 // (kernel << 8 | place) into a word of mapped host memory and ends.  The host reads that word without touching the device: every
 // entry point of an engine does before it launches anything, and so does whoever hands results to the host.
-enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, WAIT_LINEAR, WAIT_LATENT, WAIT_PERSIST, WAIT_WINDOW, WAIT_LATENT_PROMPT, WAIT_LATENT_STEP, WAIT_ONE_STEP };
+enum WaitKernel { WAIT_GEMM = 1, WAIT_GEMM_PAIR, WAIT_ATTENTION, WAIT_SAMPLER, WAIT_LINEAR, WAIT_LATENT, WAIT_PERSIST, WAIT_WINDOW, WAIT_LATENT_PROMPT, WAIT_LATENT_STEP, WAIT_ONE_STEP, WAIT_KERNELS };
+inline const char* wait_kernel_name(int k) {
+    static const char* const names[] = {"diagnostic kernel", "weight-streaming GEMM", "CTA-pair GEMM", "paged attention", "sampler", "tcgen05 linear",
+                                        "latent attention", "persistent forward", "windowed attention", "latent attention of prompts",
+                                        "latent attention of few rows", "one-token step"};
+    static_assert(sizeof(names) / sizeof(names[0]) == WAIT_KERNELS, "a name for every kernel that waits");
+    return names[k >= 1 && k < WAIT_KERNELS ? k : 0];
+}
 int* wait_word_alloc();                                 // a zeroed word that every device and stream can write, or nullptr
 void wait_word_free(int* word);
 int wait_word_check(const int* word, const char* who);  // 0, or the error that names the kernel and the place

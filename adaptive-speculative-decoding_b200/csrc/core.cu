@@ -83,12 +83,8 @@ void wait_word_free(int* word) {        // after the engine's last kernel has en
 int wait_word_check(const int* word, const char* who) {
     const int v = word ? *static_cast<const volatile int*>(word) : 0;
     if (v == 0) return 0;
-    static const char* const kernels[] = {"diagnostic kernel", "weight-streaming GEMM", "CTA-pair GEMM", "paged attention",
-                                          "sampler", "tcgen05 linear", "latent attention", "persistent forward", "windowed attention", "latent attention of prompts",
-                                          "latent attention of few rows", "one-token step"};
-    const int k = v >> 8;
     return set_error("%s: a bounded wait of an earlier launch ran out (%s, place %d); its results are not valid", who,
-                     kernels[k >= 1 && k <= 8 ? k : 0], v & 255);
+                     wait_kernel_name(v >> 8), v & 255);
 }
 // one CTA that waits on a barrier nobody arrives at, with the shortest limit
 __global__ void wait_expiry_kernel(int* err) {
