@@ -16,7 +16,6 @@ void count_launch(int n);
 // launches of the kernels that a rule chooses between, by name (asd_kernel_launches): what the tests of those rules look at
 enum CountedKernel { KERNEL_GEMM, KERNEL_GEMM_PAIR, KERNEL_GEMM_GROUPED, KERNEL_GEMV, KERNEL_ONE_STEP, KERNEL_LINEAR_FEW, KERNEL_ATTENTION_TC, KERNEL_ATTENTION_FEW, KERNEL_LATENT_TC, KERNEL_LATENT_PROMPT, KERNEL_LATENT_STEP, KERNEL_WINDOW_TC, KERNEL_SAMPLER_DRAW, KERNEL_COUNTED };
 void count_kernel(CountedKernel k);                     // count_launch(1) too
-void note_kernel(CountedKernel k);                      // of a launch that is counted by another name as well
 
 #define ASD_CUDA(expr)                                                                        \
     do {                                                                                      \

@@ -134,6 +134,7 @@ struct AttnSplit {
     float* ml = nullptr;
     long long rows = 0, o_elems = 0;
     int tiled = 2;
+    int few_rows = 1;                    // 0: latent_step_tc.cu is not taken
 };
 // out_lat fp32 [M][heads][R].  cu_q / seq_slot as in asd_engine_forward; a sequence's tokens are consecutive positions;
 // max_kv_len bounds position + 1 over the batch.

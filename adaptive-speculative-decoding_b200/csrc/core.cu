@@ -29,9 +29,8 @@ int set_error(const char* fmt, ...) {
 }
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 static std::atomic<long long> g_kernels[KERNEL_COUNTED];
-void note_kernel(CountedKernel k) { g_kernels[k].fetch_add(1, std::memory_order_relaxed); }
 void count_kernel(CountedKernel k) {
-    note_kernel(k);
+    g_kernels[k].fetch_add(1, std::memory_order_relaxed);
     count_launch(1);
 }
 

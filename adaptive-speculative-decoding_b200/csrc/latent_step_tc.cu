@@ -500,7 +500,6 @@ int launch_latent_step(const SeqIndex& ix, const int* cu_q, const int* seq_slot,
     latent_step_kernel<<<dim3(p.q_tiles * p.hgs, nseq * a.nsplit), kLsThreads, smem, stream>>>(mk, a);
     ASD_CUDA(cudaGetLastError());
     count_kernel(KERNEL_LATENT_STEP);
-    if (p.HG * p.TQ >= 32) note_kernel(KERNEL_LATENT_TC);
     if (a.nsplit > 1) return launch_latent_combine(ws.o, ws.ml, a.nsplit, d.R, out_lat, rows, stream);
     return 0;
 }

@@ -125,7 +125,7 @@ static int forward(MzEngine* e, const int* tokens, const int* positions, const i
         lp.w = ly.wukv;
         const bool head_space = !f32 && e->dn.tc_linear && latent_prompt_takes(dm, cache, M, nseq, max_qlen, max_kv_len, e->qd, ly.nqd, lp,
                                                                                e->attn_ws.tiled);
-        const bool few_rows = latent_step_takes(dm, cache, max_qlen, max_kv_len, e->attn_ws.tiled);
+        const bool few_rows = e->attn_ws.few_rows && latent_step_takes(dm, cache, max_qlen, max_kv_len, e->attn_ws.tiled);
         if (!head_space && !f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
             (few_rows || latent_attention_tc_takes(dm, cache, max_qlen, e->attn_ws.tiled))) {
             q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
@@ -402,6 +402,10 @@ int asd_mezilix_set_option(asd_mezilix_engine_t* h, const char* name, int value)
     }
     if (!strcmp(name, "latent_prompt")) {
         e->prompt_ws.mode = value;
+        return 0;
+    }
+    if (!strcmp(name, "latent_step")) {
+        e->attn_ws.few_rows = value;
         return 0;
     }
     if (!strcmp(name, "attn_tiled")) {

@@ -633,7 +633,6 @@ int one_step_launch(const OneStep& s, int max_kv_len, cudaStream_t stream) {
     cfg.numAttrs = 1;
     if (const int rc = grid_in_turn(stream, [&] { return cudaLaunchKernelEx(&cfg, fn, a); })) return rc;
     count_kernel(KERNEL_ONE_STEP);
-    for (int i = 0; i < 4 * s.n_layers; ++i) note_kernel(KERNEL_GEMV);
     return 0;
 }
 

@@ -154,7 +154,7 @@ static int mix_latent(RvEngine* e, const RvLayer& ly, const RvRun& run, int li, 
         return launch_latent_prompt(b.ix, b.cu_q, b.seq_slot, b.nseq, b.max_qlen, b.max_kv_len, e->qbuf, nq, dm, cache, lp, e->mixed,
                                     e->dev_error, s);
     }
-    const bool few_rows = latent_step_takes(dm, cache, b.max_qlen, b.max_kv_len, e->attn_ws.tiled);
+    const bool few_rows = e->attn_ws.few_rows && latent_step_takes(dm, cache, b.max_qlen, b.max_kv_len, e->attn_ws.tiled);
     if (!f32 && e->dn.tc_linear && tc_linear_supports(ql) &&
         (few_rows || latent_attention_tc_takes(dm, cache, b.max_qlen, e->attn_ws.tiled))) {
         q_terms = reinterpret_cast<__nv_bfloat16*>(e->qlat);
@@ -533,6 +533,10 @@ int asd_rivetar_set_option(asd_rivetar_engine_t* h, const char* name, int value)
     if (e->dn.set_option(name, value)) return 0;
     if (!strcmp(name, "latent_prompt")) {
         e->prompt_ws.mode = value;
+        return 0;
+    }
+    if (!strcmp(name, "latent_step")) {
+        e->attn_ws.few_rows = value;
         return 0;
     }
     if (!strcmp(name, "attn_tiled")) {

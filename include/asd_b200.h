@@ -38,8 +38,8 @@ ASD_API const char* asd_last_error(void);
 ASD_API long long asd_launch_count(void);
 ASD_API void asd_reset_launch_count(void);
 /* launches since load of one of the kernels that a rule on sizes chooses: "gemm" (weight-streaming), "gemm_pair", "gemm_grouped",
- * "gemv" (projections of one token: launches, or phases of a one_step), "one_step", "linear_few", "attention_tc", "attention_few", "latent_tc" (calls of at
- * least 32 query rows a tile in latent space), "latent_step", "latent_prompt", "window_tc", "sampler_draw"; -1 for another name */
+ * "gemv", "one_step", "linear_few", "attention_tc", "attention_few", "latent_tc", "latent_step", "latent_prompt", "window_tc", "sampler_draw"; -1 for
+ * another name */
 ASD_API long long asd_kernel_launches(const char* name);
 /* Every wait inside a kernel is bounded (about nine seconds).  A wait that ran out makes the results of its launch invalid:
  * engines then refuse every later forward (asd_*_device_error names the kernel), a sampler call is refused once.
@@ -325,7 +325,8 @@ ASD_API int asd_mezilix_set_cache(asd_mezilix_engine_t* e, void* pool, int num_p
  * expert, on average, from which its products run on CTA pairs; 0, default: the measured rule), "attn_tiled" (2, default: attention of bf16 cache rows on the tensor cores with fp32 operands as two
  * bf16 terms, else as 1; 1: register-tiled fp32 kernel with key-range shares where the latent size allows; 0: one warp
  * per (token, head)), "latent_prompt" (attention of prompts in head space, which needs asd_mezilix_set_latent_up; 1, default:
- * where it measured better, 2: wherever the sizes allow, 0: never), "profile" (1: CUDA events around every launch, read with
+ * where it measured better, 2: wherever the sizes allow, 0: never), "latent_step" (1, default: few query rows on a kernel of their own;
+ * 0: as larger steps), "profile" (1: CUDA events around every launch, read with
  * asd_mezilix_profile_read) */
 ASD_API int asd_mezilix_set_option(asd_mezilix_engine_t* e, const char* name, int value);
 /* Same contract as asd_engine_forward (M <= max_tokens).  layer_out (optional, fp32 [n_layers][M][width]) receives
@@ -408,7 +409,7 @@ ASD_API size_t asd_rivetar_cache_bytes(const asd_rivetar_engine_t* e, int num_pa
 ASD_API size_t asd_rivetar_state_bytes(const asd_rivetar_engine_t* e, int max_seqs);
 ASD_API int asd_rivetar_set_cache(asd_rivetar_engine_t* e, void* pool, int num_pages, const int32_t* page_table,
                                   int max_seqs, int max_pages_per_seq, float* state);
-/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_tiled", "latent_prompt" as for the Mezilix engine (attn_tiled 2: windowed attention of
+/* options: "tc_linear", "tc_min_rows", "linear_few", "attn_tiled", "latent_prompt", "latent_step" as for the Mezilix engine (attn_tiled 2: windowed attention of
  * 17 query rows a tile and more on tcgen05 too); "fused_attn" (1, default: tiled windowed
  * attention kernel; 0: one warp per (token, head)); "profile" */
 ASD_API int asd_rivetar_set_option(asd_rivetar_engine_t* e, const char* name, int value);

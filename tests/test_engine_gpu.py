@@ -339,28 +339,30 @@ def test_engine_one_token(cfg):
         eng.prefill(idc[:nseq, :T - q].contiguous(), slots, want_logits=False)
         start = torch.full((nseq,), T - q, dtype=torch.int32, device="cuda")
         got = {}
-        for on in (1, 0):
+        for on in (2, 0):                   # (1, in one launch: test_one_step_gpu.py)
             eng.set_option("one_token", on)
 
             def step():
                 got[on] = eng.forward_uniform(idc[:nseq, T - q:].contiguous(), start, slots, T).view(nseq, q, -1).cpu()
 
             assert _launched("gemv", step) == (4 * cfg.num_hidden_layers + 1 if on and nseq * q == 1 else 0)
-        check(got[1], ref[:nseq, T - q:])
+        check(got[2], ref[:nseq, T - q:])
         if nseq * q == 1:
-            assert (got[1] - got[0]).abs().max().item() <= MAX_ABS
+            assert (got[2] - got[0]).abs().max().item() <= MAX_ABS
         else:
-            assert torch.equal(got[1], got[0])
-    eng.set_option("one_token", 1)
+            assert torch.equal(got[2], got[0])
     one, slot = torch.tensor([0], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
     pos, cu = slot + T - 1, torch.tensor([0, 1], dtype=torch.int32, device="cuda")
-    eng.prefill(idc[:1, :T - 1].contiguous(), slot, want_logits=False)
-    rows = eng.forward(idc[0, T - 1:].contiguous(), pos, slot, cu, slot, 1, T, logit_rows=one).cpu()
-    check(rows, ref[:1, T - 1])
+    for on in (2, 1):
+        eng.set_option("one_token", on)
+        eng.prefill(idc[:1, :T - 1].contiguous(), slot, want_logits=False)
+        rows = eng.forward(idc[0, T - 1:].contiguous(), pos, slot, cu, slot, 1, T, logit_rows=one).cpu()
+        check(rows, ref[:1, T - 1])
     eng.close()
 
 
-def test_engine_one_token_of_an_engine_for_one():
+@pytest.mark.parametrize("mode", [2, 1])
+def test_engine_one_token_of_an_engine_for_one(mode):
     """an engine that takes one token at a time has room for the statistics of as many blocks as any other"""
     from asd_b200.engine import QwenEngine
     cfg = Qwen2Config(896, 2, 14, 2, 4864, 1024, head_dim=64, name="one-only")
@@ -371,6 +373,7 @@ def test_engine_one_token_of_an_engine_for_one():
     outs = []
     for max_tokens in (1, 64):
         eng = QwenEngine(cfg, max_seqs=1, max_seq_len=16, max_tokens=max_tokens).load_hf_weights(w)
+        eng.set_option("one_token", mode)
         outs.append(torch.cat([eng.forward_uniform(idc[:, i:i + 1].contiguous(), slot + i, slot, i + 1) for i in range(6)]).cpu())
         eng.close()
     check(outs[0], ref[0])

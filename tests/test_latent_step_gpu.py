@@ -32,16 +32,20 @@ def test_latent_attention_of_few_rows(heads, kv_rank, window, page_size, scale, 
         eng.set_option("attn_tiled", mode)
         if mode == 2:
             eng.cache_pool.fill_(255)
-        before = lib().asd_kernel_launches(b"latent_step")
+        names = (b"latent_step", b"latent_tc")
+        before = [lib().asd_kernel_launches(n) for n in names]
         outs.append(mz.feed(eng, eng.open_sequence(), ids, portions).cpu())
-        ran, want, at = lib().asd_kernel_launches(b"latent_step") - before, 0, 0
+        ran, want, at = [lib().asd_kernel_launches(n) - b for n, b in zip(names, before)], [0, 0], 0
         for p in portions:
             at += p
             hg = min(heads, 32)
             tq = min(32 // hg, p)
             tiles = -(-p // tq) * -(-heads // hg)
-            want += tiles <= 2 and (hg * tq >= 32 or min(at, window) > 64)
-        assert ran == (want if mode == 2 else 0)
+            if tiles <= 2 and (hg * tq >= 32 or min(at, window) > 64):
+                want[0] += 1
+            elif min(128 // min(heads, 128), p) * min(heads, 128) >= 32:       # rows of a tile of latent_attention_tc.cu
+                want[1] += 1
+        assert ran == (want if mode == 2 else [0, 0])
         eng.check_device()
         mz.close(eng)
     assert torch.isfinite(outs[0]).all()

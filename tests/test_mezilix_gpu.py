@@ -570,6 +570,7 @@ def test_latent_attention_on_tcgen05(heads, kv_rank, rot_dim, window, page_size,
     for mode in (2, 1):
         eng = make_engine(cfg, w, dtype=torch.bfloat16, max_tokens=512, max_seq_len=1024, page_size=page_size)
         eng.set_option("attn_tiled", mode)
+        eng.set_option("latent_step", 0)         # its few rows are tested in test_latent_step_gpu.py
         if mode == 2:
             eng.cache_pool.fill_(255)
         before = lib().asd_kernel_launches(b"latent_tc")

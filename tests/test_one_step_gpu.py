@@ -16,6 +16,7 @@ from test_engine_gpu import MAX_ABS, Qwen2Config, _launched, check, qwen2_forwar
 def test_one_token_in_one_launch(cfg, page, contexts):
     """three steps in a row behind every context, so that each reads what the ones before appended: against the oracle and the chain of
     kernels, which rounds at the same points"""
+    from asd_b200._lib import lib
     from asd_b200.engine import QwenEngine
     w = random_hf_weights(cfg, seed=31, logit_std=0.4)
     top = max(contexts) + 3
@@ -33,7 +34,9 @@ def test_one_token_in_one_launch(cfg, page, contexts):
             def steps():
                 got[mode] = torch.cat([eng.forward_uniform(idc[:, i:i + 1].contiguous(), slot + i, slot, i + 1) for i in range(n, n + 3)]).cpu()
 
+            before = lib().asd_kernel_launches(b"gemv")
             assert _launched("one_step", steps) == (3 if mode == 1 else 0)
+            assert lib().asd_kernel_launches(b"gemv") - before == 3 * (1 if mode == 1 else 4 * cfg.num_hidden_layers + 1)      # 1: the logits
             eng.close()
         check(got[1], ref[0, n:n + 3])
         assert (got[1] - got[2]).abs().max().item() <= MAX_ABS
