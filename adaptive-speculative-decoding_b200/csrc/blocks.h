@@ -6,6 +6,8 @@
 #pragma once
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <stddef.h>
 #include <stdint.h>
 
@@ -169,6 +171,25 @@ struct LatentPromptWs {
     long long row_elems = 0, plane_elems = 0;
     int mode = 1;                        // 0 never, 1 where it measured better, 2 wherever the sizes allow
 };
+// What latent space costs above head space, us: two head products a (token, head), its tiles of 128 (query row, key) pairs a tile a CTA;
+// against every position's way through the up-projections, of all sequences as if they saw max_kv_len, and 128-token tiles of one head, of
+// which an SM has one at least.  Least squares over 297 calls (1, 4, 16 sequences of 9 to 256 tokens behind 0 to 2560 positions, 8, 16 and 32
+// heads), one layer, us in latent and in head space: 1 x 256 of 16 heads 224, 190; 4 x 256 372, 306, behind 2560 positions 687, 449; 16 x 24
+// of 32 heads 396, 396, behind 384 443, 509; 1 x 17 of 8 heads behind 2560 146, 168.  The constant is 24 in the fit; with 12 no call of the
+// 297 was more than 1 % slower than in latent space.
+// Sequences of unequal length count as one of max_qlen tokens and the others of what is left for each, behind the same context (the call's
+// numbers tell no more).  Counted as max_qlen each, one prompt among many short ones went through the up-projections of all: 172 tokens and 23
+// of one behind up to 1108 positions, 32 heads, 382 us a layer in latent and 768 in head space; 761 tokens and 31 of one 622 and 859.  Over 501 unequal calls (2
+// to 64 sequences, fresh, behind one context, behind contexts of their own) 63 were slower than in latent space, now 8 of them by 2 to 7 %.
+inline double latent_prompt_gain(int heads, int R, int sms, int M, int nseq, int max_qlen, int max_kv_len) {
+    auto up = [](int n, int d) { return (double)((n + d - 1) / d); };
+    const int tq = std::min(std::max(128 / heads, 1), max_qlen), others = nseq - 1, rest = others > 0 ? std::max(M - max_qlen, 0) / others : 0;
+    const int context = std::max(max_kv_len - max_qlen, 0);
+    const double kt = up(max_kv_len, 128), th = 1e-3 * heads;
+    const double tiles = up(max_qlen, tq) * kt + others * up(rest, tq) * up(context + rest, 128);
+    const double latent = tiles * up(heads, 128) * (R > 256 ? 2 : 1) / sms, here = heads * (up(max_qlen, 128) + others * up(rest, 128)) / sms;
+    return 12.0 + 1.85 * th * M + 9.06 * latent - (0.512 * th * nseq * kt * 128.0 + 2.58 * std::max(here, 1.0) * kt);
+}
 bool latent_prompt_takes(const LatentDims& d, const PagedRows& cache, int M, int nseq, int max_qlen, int max_kv_len, const float* q,
                          long long ldq, const LatentPromptWs& ws, int tiled);
 int launch_latent_prompt(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen, int max_kv_len,

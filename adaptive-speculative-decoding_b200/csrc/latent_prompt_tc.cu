@@ -496,17 +496,7 @@ bool latent_prompt_takes(const LatentDims& d, const PagedRows& cache, int M, int
     if (rows * (d.R + kLpDr) > ws.row_elems || 2 * rows * cols > ws.plane_elems) return false;
     if (ws.mode > 1) return true;
     if (max_qlen < kLpMinTokens) return false;
-    // What latent space costs above this form, us: two head products a (token, head), its tiles of 128 (query row, key) pairs a tile a
-    // CTA; against every position's way through the up-projections and 128-token tiles of one head, of which an SM has one at least.
-    // Least squares over 297 calls (1, 4, 16 sequences of 9 to 256 tokens behind 0 to 2560 positions, 8, 16 and 32 heads), one layer,
-    // us in latent and in head space: 1 x 256 of 16 heads 224, 190; 4 x 256 372, 306, behind 2560 positions 687, 449; 16 x 24 of 32 heads
-    // 396, 396, behind 384 443, 509; 1 x 17 of 8 heads behind 2560 146, 168.  The constant is 24 in the fit; with 12 no call of the 297
-    // was more than 1 % slower than in latent space.
-    const double kt = (double)(rows / nseq) / kLpKeys, sms = sm_count(), th = 1e-3 * d.heads;
-    const int tq = std::min(std::max(128 / d.heads, 1), max_qlen);
-    const double here = (double)nseq * d.heads * ((max_qlen + 127) / 128) / sms;
-    const double latent = (double)nseq * ((max_qlen + tq - 1) / tq) * ((d.heads + 127) / 128) * (d.R > 256 ? 2 : 1) / sms;
-    return 12.0 + 1.85 * th * M + 9.06 * latent * kt > 0.512 * th * rows + 2.58 * std::max(here, 1.0) * kt;
+    return latent_prompt_gain(d.heads, d.R, sm_count(), M, nseq, max_qlen, max_kv_len) > 0.0;
 }
 
 int launch_latent_prompt(const SeqIndex& ix, const int* cu_q, const int* seq_slot, int nseq, int max_qlen, int max_kv_len,
