@@ -196,6 +196,11 @@ def random_weights(cfg: MezilixConfig, seed: int, device="cpu", dtype=torch.bflo
     return w
 
 
+def head_space_sizes(l) -> bool:
+    """whether prompts' attention of a latent-attention layer of these sizes can run in head space (csrc/latent_prompt_tc.cu)"""
+    return (l.dim, l.rot_dim, l.vdim) == (128, 64, 128) and l.kv_rank % 8 == 0
+
+
 def pack_layer(w: Dict[str, torch.Tensor], cfg: MezilixConfig, i: int, device, dtype) -> Dict[str, Optional[torch.Tensor]]:
     """checkpoint names -> engine layout of layer i: the query and latent projections stacked into one matrix, the key
     up-projection transposed per head, the experts stacked into [experts, ff, width] / [experts, width, ff]"""
@@ -214,7 +219,8 @@ def pack_layer(w: Dict[str, torch.Tensor], cfg: MezilixConfig, i: int, device, d
            "wuk": dev(w[p + "mix.uk"].reshape(l.heads, l.dim, l.kv_rank).transpose(1, 2)),
            "wukv": None, "wuv": dev(w[p + "mix.uv"]), "wo": dev(w[p + "mix.o"]),
            "router": None, "w_up": None, "w_down": None}
-    if dtype == torch.bfloat16:      # prompts carry the positions through both up-projections; one buffer for both value forms
+    if dtype == torch.bfloat16 and head_space_sizes(l):
+        # prompts carry the positions through both up-projections; one buffer for both value forms
         out["wukv"] = dev(torch.cat([w[p + "mix.uk"], w[p + "mix.uv"]], 0))
         out["wuv"] = out["wukv"][l.heads * l.dim:]
     if l.experts:

@@ -21,6 +21,8 @@ from typing import Dict, List, Optional, Tuple
 
 import torch
 
+from .mezilix import head_space_sizes
+
 ARCHITECTURE = "Rivetar"
 MIXERS = ("latent_attention", "gla", "attention")
 MIXER_CODE = {m: i for i, m in enumerate(MIXERS)}
@@ -301,7 +303,8 @@ def pack(w: Dict[str, torch.Tensor], cfg: RivetarConfig, device, dtype) -> Dict[
             out[(i, "w_uq")] = mat(w[p + "mix.uq"])
             out[(i, "w_uk")] = mat(w[p + "mix.uk"].reshape(l.heads, l.dim, l.kv_rank).transpose(1, 2))
             out[(i, "w_uv")] = mat(w[p + "mix.uv"])
-            if dtype == torch.bfloat16:      # prompts carry the positions through both up-projections; one buffer for both value forms
+            if dtype == torch.bfloat16 and head_space_sizes(l):
+                # prompts carry the positions through both up-projections; one buffer for both value forms
                 ukv = mat(torch.cat([w[p + "mix.uk"], w[p + "mix.uv"]], 0))
                 out[(i, "w_uv")], out[(i, "w_ukv")] = ukv[l.heads * l.dim:], ukv
         elif l.type == "gla":

@@ -71,6 +71,33 @@ def test_pack_layer_checks_shapes_and_stacks_experts():
         mezilix.pack_layer(bad, cfg, 0, "cpu", torch.float32)
 
 
+@pytest.mark.parametrize("family", ["mezilix", "rivetar"])
+def test_second_key_up_projection_only_where_it_is_read(family):
+    """the rows that prompts' attention in head space reads: bf16 layers of heads of 128 + 64 alone, the value rows shared with wuv"""
+    import dataclasses
+    from asd_b200.models import rivetar
+    for dim, kv_rank, dtype in ((128, 512, torch.bfloat16), (128, 512, torch.float32), (64, 512, torch.bfloat16), (128, 36, torch.bfloat16)):
+        if family == "mezilix":
+            cfg = mezilix.sized_config(256, 1, 2, ff=64, dim=dim, kv_rank=kv_rank)
+            w = mezilix.random_weights(cfg, seed=1)
+            t = mezilix.pack_layer(w, cfg, 0, "cpu", dtype)
+            ukv, uv = t["wukv"], t["wuv"]
+        else:
+            cfg = rivetar.sized_config(256, 1, 2, ff=64, dim=dim)
+            cfg = dataclasses.replace(cfg, layers=[dataclasses.replace(cfg.layers[0], kv_rank=kv_rank)])
+            w = rivetar.random_weights(cfg, seed=1)
+            t = rivetar.pack(w, cfg, "cpu", dtype)
+            ukv, uv = t.get((0, "w_ukv")), t[(0, "w_uv")]
+        l = cfg.layers[0]
+        assert torch.equal(uv, w["l0.mix.uv"].to(dtype))
+        assert (ukv is not None) == (dtype == torch.bfloat16 and dim == 128 and kv_rank == 512)
+        if ukv is None:
+            assert uv.untyped_storage().nbytes() == uv.numel() * uv.element_size()
+        else:
+            assert torch.equal(ukv, torch.cat([w["l0.mix.uk"], w["l0.mix.uv"]], 0).to(dtype))
+            assert uv.data_ptr() == ukv[l.heads * l.dim:].data_ptr()
+
+
 def test_page_table_allocates_frees_and_reuses():
     from asd_b200._lib import AsdError
     from asd_b200.engine import PageTable
