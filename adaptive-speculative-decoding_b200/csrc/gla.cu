@@ -419,7 +419,8 @@ int launch_gla_recurrence(const SeqIndex& ix, const int* cu_q, const int* seq_sl
     int cols = groups > 32 && run <= 1 ? 16 : 32;
     // 48 columns where 32 leave some SMs with two CTAs, which are then the last, and these give every CTA an SM of its own: 436 clocks a
     // position there, 390 here (3 prompts of up to 777 positions, 16 heads of 128 x 128: 167 -> 158 us; four warps of 8 rows x 6 columns
-    // a CTA instead of six of 8 x 4: 225)
+    // a CTA instead of six of 8 x 4: 225).  Eleven head shapes, 38 to 148 pairs of sequence and head, a layer's step with and without: runs of
+    // 2 to 64 positions within 2 us of each other or faster, of 128 and 256 up to 14 % faster (12 x 256, 8 heads of 32 x 48: 208 -> 179 us)
     const long long heads_all = (long long)nseq * d.heads, sms = sm_count();
     if (run > 1 && groups <= 16 && heads_all * ((d.dv + 31) / 32) > sms && heads_all * ((d.dv + 47) / 48) <= sms) cols = 48;
     const int cg = cols / GLA_C, whole = cols == 48 ? 96 : 32;         // threads: whole warps, and whole rows of column groups
