@@ -319,8 +319,9 @@ __global__ void __launch_bounds__(kLsThreads, 1) latent_step_kernel(const __grid
                     const uint32_t* v = &x[i >> 3][(i & 7) * 4];
                     dst[i] = make_float4(__uint_as_float(v[0]), __uint_as_float(v[1]), __uint_as_float(v[2]), __uint_as_float(v[3]));
                 }
-            } else if (lane == 0) {
-                mbar_arrive(&B->s_read);                       // has no scores to read, and has seen that they are there
+            } else {                                           // has no scores to read; every lane has seen that they are there
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&B->s_read);
             }
             if (key0 + kLsKeys > p_last + 1 || key0 < j_lo) {
                 // keys that no row may see: whatever the pool holds there must not meet the zero weights (the scores have read them)

@@ -50,3 +50,14 @@ def test_the_walk_finds_a_lapped_barrier():
 def test_scores_wait_for_every_warp_that_looks_for_them(name):
     text = open(os.path.join(CSRC, name)).read()
     assert not stuck(int(re.search(r"mbar_init\(&B->s_read, (\d)\)", text).group(1)))
+
+
+@pytest.mark.parametrize("name", ["latent_step_tc.cu", "latent_prompt_tc.cu"])
+def test_a_warp_arrives_when_all_its_lanes_have_looked(name):
+    """lanes look one by one: the one that arrives for its warp does so behind a __syncwarp"""
+    lines = [l.split("//")[0].strip() for l in open(os.path.join(CSRC, name))]
+    lines = [l for l in lines if l]
+    at = [i for i, l in enumerate(lines) if "mbar_arrive(&B->s_read)" in l]
+    assert at
+    for i in at:
+        assert lines[i] == "if (lane == 0) mbar_arrive(&B->s_read);" and lines[i - 1] == "__syncwarp();", lines[i - 1:i + 1]
